@@ -60,9 +60,21 @@ bool is_phj(hj_algo_t a) { return hj::algo_is_phj(a); }
 
 // Segment mode for a radix join (see HJ_F_SEGMENTS): by size unless a flag decides.
 bool want_seg(hj_algo_t algo, const hj_params_t &p, const hj::RadixGeom &g, size_t nR, size_t nS) {
-    if (!is_phj(algo) || (p.flags & HJ_F_EXACT)) return false;
+    if (!is_phj(algo) || (p.flags & HJ_F_EXACT) || g.single) return false;
     if (p.flags & HJ_F_SEGMENTS) return hj::phj_seg_applies(g, hj::algo_lp(algo), 1ull << 40, 0);
     return hj::phj_seg_applies(g, hj::algo_lp(algo), nR, nS);
+}
+
+// Flags that name a pipeline or its element layout: the two-pass pipelines run as asked.
+constexpr uint32_t kPipelineFlags = HJ_F_SEGMENTS | HJ_F_EXACT | HJ_F_WIDE | HJ_F_WORDS | HJ_F_TEST_STALL;
+
+// The geometry of a radix join: the one-pass pipeline where the build relation needs few partitions,
+// unless the flags name another, else as asked.
+int join_geom(const hj_params_t &p, size_t nR, size_t nS, hj::RadixGeom *g) {
+    const int rc = hj::radix_geom(p.num_radix_bits, p.num_passes, g, p.radix_bits_pass1);
+    if (rc) return rc;
+    if (!(p.flags & kPipelineFlags)) hj::radix_geom_single(p.num_radix_bits, nR, nS, g);
+    return HJ_OK;
 }
 
 int scratch_need(hj_algo_t algo, const hj_params_t &p, size_t nR, size_t nS, bool host_inputs, int num_sms,
@@ -71,7 +83,7 @@ int scratch_need(hj_algo_t algo, const hj_params_t &p, size_t nR, size_t nS, boo
     if (host_inputs) need += align256(nR * 16) + align256(nS * 16);
     if (is_phj(algo)) {
         hj::RadixGeom g;
-        int rc = hj::radix_geom(p.num_radix_bits, p.num_passes, &g, p.radix_bits_pass1);
+        int rc = join_geom(p, nR, nS, &g);
         if (rc) return rc;
         need += hj::phj_scratch_bytes(g, nR, nS, num_sms, seg);
     } else {
@@ -251,7 +263,7 @@ int hj_ctx_reserve(hj_ctx_t *c, hj_algo_t algo, const hj_params_t *pin, size_t n
     bool seg = false;
     if (is_phj(algo)) {
         hj::RadixGeom geom;
-        const int rc = hj::radix_geom(p.num_radix_bits, p.num_passes, &geom, p.radix_bits_pass1);
+        const int rc = join_geom(p, nR, nS, &geom);
         if (rc) return rc;
         seg = want_seg(algo, p, geom, nR, nS);
     }
@@ -277,7 +289,7 @@ int hj_join_ctx(hj_ctx_t *c, hj_algo_t algo, const hj_params_t *pin, const hj_tu
     if (p.device != c->device) return out->status = HJ_E_INVAL;
     hj::RadixGeom geom = {};
     if (is_phj(algo)) {
-        int rc = hj::radix_geom(p.num_radix_bits, p.num_passes, &geom, p.radix_bits_pass1);
+        int rc = join_geom(p, nR, nS, &geom);
         if (rc) return out->status = rc;
         out->physical_passes = geom.passes;
     }
@@ -325,9 +337,12 @@ int hj_join_ctx(hj_ctx_t *c, hj_algo_t algo, const hj_params_t *pin, const hj_tu
     // tuple matched two build tuples (the first match then depends on the order inside a partition),
     // again with ordered ones. The second run needs the first one's flag on the host, so these joins
     // are not captured into a graph; a build relation that needed it runs ordered at once next time.
-    const bool lp_try = is_phj(algo) && hj::algo_lp(algo) && !(p.flags & (HJ_F_ORDERED | HJ_F_TEST_STALL)) &&
-                        p.watchdog_ms <= 0 && !(c->lp_ordered_R == (const void *)R && c->lp_ordered_nR == nR);
-    const bool lp_ordered = is_phj(algo) && hj::algo_lp(algo) && !lp_try;
+    // The one-pass pipeline needs neither: its build elements carry their input position. It reports
+    // HJ_RES_ORDERED_PASSES for the joins that the two-pass pipelines would have run ordered.
+    const bool lp_first = is_phj(algo) && hj::algo_lp(algo) && !(p.flags & (HJ_F_ORDERED | HJ_F_TEST_STALL)) &&
+                          p.watchdog_ms <= 0 && !(c->lp_ordered_R == (const void *)R && c->lp_ordered_nR == nR);
+    const bool lp_try = lp_first && !geom.single;
+    const bool lp_ordered = is_phj(algo) && hj::algo_lp(algo) && !lp_first;
     bool lp_rerun = false;
     // Everything from the result reset to the result copy; a repeated device-resident join replays it
     // from a CUDA graph (the key holds every input of the enqueued work).
@@ -455,6 +470,7 @@ int hj_join_ctx(hj_ctx_t *c, hj_algo_t algo, const hj_params_t *pin, const hj_tu
     out->checksum = c->acc_host->checksum;
     out->large_partitions = c->acc_host->large_parts;
     out->flags = (uint32_t)c->acc_host->flags;
+    if (lp_first && geom.single) lp_rerun = c->acc_host->dup_flag != 0;
     if (lp_ordered || lp_rerun) out->flags |= HJ_RES_ORDERED_PASSES;
     if (lp_rerun) {
         c->lp_ordered_R = R;
@@ -491,7 +507,7 @@ static int join_mat(hj_ctx *c, hj_algo_t algo, const hj_params_t &p, const hj_tu
                     unsigned long long cap_guess, hj_result_t *out) {
     hj::RadixGeom geom = {};
     if (is_phj(algo)) {
-        int rc = hj::radix_geom(p.num_radix_bits, p.num_passes, &geom, p.radix_bits_pass1);
+        int rc = join_geom(p, nR, nS, &geom);
         if (rc) return out->status = rc;
         out->physical_passes = geom.passes;
     }

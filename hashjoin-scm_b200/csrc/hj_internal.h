@@ -19,6 +19,8 @@ struct RadixGeom {
     int passes;     // physical passes (1 or 2)
     int b1, b2;     // bits of pass 1 / pass 2 (b2 = 0 for one pass)
     int F1, F2;     // fanouts (F2 = 1 for one pass)
+    bool single = false;  // the one-pass pipeline (hj_single.cu): bits <= kSingleMaxBits, passes 1
+    int req_bits = 0;     // the radix bits asked for (bits is smaller in the one-pass pipeline)
     int nparts() const { return 1 << bits; }
 };
 
@@ -34,6 +36,11 @@ inline cudaError_t record_event(cudaEvent_t ev, cudaStream_t st) {
 
 // b1_req > 0 asks for that many pass-1 bits (clamped so that both passes have 1..8 bits).
 int radix_geom(int bits, int passes, RadixGeom *g, int b1_req = 0);
+
+// The one-pass pipeline's geometry for a build relation of nR tuples and `bits` requested radix bits:
+// false when the two-pass pipelines should run.
+constexpr int kSingleMaxBits = 11;
+bool radix_geom_single(int bits, size_t nR, size_t nS, RadixGeom *g);
 
 // Result semantics of an algorithm: radix-partitioned or not; first match per probe tuple (lp) or
 // every match; build key 0 never matches (the phj_radix_lp empty-slot rule, src/algo/phj.c:614).
@@ -73,6 +80,7 @@ struct PhjScratch {
     size_t max_large;
     uint32_t *large_table;   // head/next chains for large partitions (>= 12 B per R tuple)
     size_t large_table_words;
+    unsigned long long *ors; // one-pass pipeline: [cR][3] ORs of build keys, build row ids, probe row ids
     ulonglong2 *tmp1;        // pass-1 output [nR + nS]; segment storage [max_segs * kTile] in segment mode
     ulonglong2 *tmp2;        // pass-2 output [nR + nS] (== tmp1 for one pass)
     // Segment mode (phj_seg_applies): pass 1 writes chains of kTile-tuple segments and counts the
@@ -119,6 +127,14 @@ int phj_enqueue(const RadixGeom &g, bool lp, bool skip0, const ulonglong2 *R, si
                 size_t nS, const PhjScratch &s, JoinAccum *acc, cudaStream_t st, cudaEvent_t ev_mid,
                 int num_sms, cudaEvent_t *ph, uint32_t *launches, const MatOut *mat = nullptr,
                 int test_flags = 0, bool ordered = true);
+
+// The partition phase of the one-pass pipeline (g.single): count, plan, scatter into s.tmp1. lp: build
+// elements carry their input position. Records ph[1..4].
+int single_prepare_device();
+uint32_t single_grid(size_t nR, size_t nS, int num_sms);
+int single_partition_enqueue(const RadixGeom &g, bool lp, bool skip0, bool ci_ok, const ulonglong2 *R, size_t nR,
+                             const ulonglong2 *S, size_t nS, const PhjScratch &s, cudaStream_t st, bool agg_ok,
+                             cudaEvent_t *ph, uint32_t *launches);
 
 // The events of phase slot i (HJ_PH_*) that phj_enqueue recorded: elapsed(ph[*from], ph[*to]);
 // false for a slot that the mode does not time (segment mode has no histogram pass).

@@ -46,184 +46,9 @@
 
 #include "hj_common.cuh"
 #include "hj_internal.h"
+#include "hj_partition.cuh"
 
 namespace hj {
-
-// ------------------------------------------------------------------------------------------------
-// Device-side plan structures
-// ------------------------------------------------------------------------------------------------
-struct JoinItem {
-    uint64_t r_begin;  // index into the final R buffer
-    uint64_t s_begin;  // index into the final S buffer
-    uint32_t r_len;
-    uint32_t s_len;
-    uint32_t part0;    // 1: the partition of the keys whose radix bits are 0 (key 0's partition)
-    uint32_t pad;
-};
-
-struct LargePart {
-    uint64_t r_begin, s_begin;
-    uint64_t r_len, s_len;
-    uint64_t table_off;  // u32 words into the large table: head[nb] then next[r_len]
-    uint64_t r_flat, s_flat;
-    uint32_t nb_log;
-    uint32_t part0;  // as JoinItem::part0
-};
-
-// counters[] slots
-enum : int {
-    kCtrItem1 = 0,       // scatter pass-1 work-item counter
-    kCtrItem2 = 1,       // scatter pass-2 work-item counter
-    kCtrNItemsA = 2,     // join items whose build side fits the compact shared-memory table (listed first)
-    kCtrItemA = 3,       // compact join work-item counter
-    kCtrSegAlloc = 4,    // segment mode: segment ids handed out
-    kCtrLargeAgg = 5,    // 1: large partitions use key-aggregated tables (see join_large_build)
-    kCtrNItems = 6,
-    kCtrNLarge = 7,
-    kCtrItem = 8,        // join work-item counter
-    kCtrLargeR = 9,      // total R tuples in large partitions (u32 pairs: lo, hi)
-    kCtrLargeS = 11,     // total S tuples in large partitions (lo, hi)
-    kCtrLargeWords = 13, // table words used (lo, hi)
-    kCtrErr = 15,
-    kCtrMaxKey = 16,     // u64: OR of all R keys (words 16-17)
-    kCtrMaxRid = 18,     // u64: OR of all R row ids (words 18-19)
-    kCtrOrRidS = 20,     // u64: OR of all S row ids (words 20-21)
-    kCtrItem1S = 22,     // first-match joins: pass-1 work-item counter of the probe relation's items
-    kCtrItem2S = 23,     // first-match joins: pass-2 work-item counter of the probe relation's items
-    kNumCounters = 24
-};
-
-// Compact final partitions. When every build key shifted right by the radix bits is below 2^31 and
-// every row id (build and probe) below 2^32, the last partition pass stores each tuple as one 8-byte
-// word, (key >> bits) << 32 | row id, and the joins read 8 bytes per tuple instead of 16. Inside a
-// final partition the low `bits` key bits are equal, so comparing key >> bits compares keys. A probe
-// key whose high part is 2^31 or more is stored as 0xffffffff: no build key has that high part. Joins
-// where a build key 0 never matches (lp_join's empty-slot rule): a last pass that reads tuples stores
-// that key's words with high part 0x80000000, which no build key and no probe word has (ci_word_z0);
-// from segment-mode pass-1 words it keeps high part 0, and since key 0 lies in the partition of the
-// keys whose radix bits are 0, where a high part of 0 means key 0, the joins skip such build words
-// there (JoinItem::part0). The widths are ORed together by the pass that reads the relations first (hist_chunk_kernel or
-// seg_pass1_kernel), so the choice is made on the device, before the last pass.
-__device__ __forceinline__ bool ci_applies(const uint32_t *counters, int bits) {
-    const unsigned long long *mx = reinterpret_cast<const unsigned long long *>(counters + kCtrMaxKey);
-    return (mx[0] >> bits) < (1ull << 31) && mx[1] < (1ull << 32) && mx[2] < (1ull << 32);
-}
-
-// Segment mode can go further: pass 1 stores (key >> b1) << 32 | row id (w8_word) in segments of 4096
-// words (the same 32 KB as 2048 tuples) when every build key >> b1 is below 2^31 and every row id below
-// 2^32; pass 2 then reads 8-byte words in tiles of 4096 and writes compact final partitions. A probe
-// key whose key >> b1 does not fit keeps its low 31 bits and gets bit 31 set: its pass-2 digit stays
-// right, and after pass 2's shift its high part is still above every build key's.
-__device__ __forceinline__ bool w8_fits(const uint32_t *counters, int b1) {
-    const unsigned long long *mx = reinterpret_cast<const unsigned long long *>(counters + kCtrMaxKey);
-    return (mx[0] >> b1) < (1ull << 31) && mx[1] < (1ull << 32) && mx[2] < (1ull << 32);
-}
-
-__device__ __forceinline__ unsigned long long w8_word(unsigned long long key, unsigned long long rid, int b1) {
-    const unsigned long long hi = key >> b1;
-    const unsigned long long h32 = hi < (1ull << 31) ? hi : (0x80000000ull | (hi & 0x7fffffffull));
-    return (h32 << 32) | (rid & 0xffffffffull);
-}
-
-// Build relations whose key 0 never matches (z0), in the exact-offset pipeline's word pass 1: key 0's
-// word takes the high part 0x80000000, which no other build word has; the last pass keeps it
-// (store_elem) and stores every probe word whose high part has bit 31 set as 0xffffffff, so nothing
-// matches it. (Segment mode's pass 1 stores key 0 as any key; the joins skip it in its partition.)
-__device__ __forceinline__ unsigned long long w8_word_z0(unsigned long long key, unsigned long long rid, int b1,
-                                                         bool z0) {
-    return z0 && key == 0 ? (0x80000000ull << 32) | (rid & 0xffffffffull) : w8_word(key, rid, b1);
-}
-
-__device__ __forceinline__ unsigned long long ci_word(unsigned long long key, unsigned long long rid, int bits) {
-    const unsigned long long hi = key >> bits;
-    return ((hi < 0x80000000ull ? hi : 0xffffffffull) << 32) | (rid & 0xffffffffull);
-}
-
-__device__ __forceinline__ unsigned long long ci_word_z0(unsigned long long key, unsigned long long rid, int bits,
-                                                         bool z0) {
-    return z0 && key == 0 ? (0x80000000ull << 32) | (rid & 0xffffffffull) : ci_word(key, rid, bits);
-}
-
-// Build partitions up to this size whose keys (above the radix bits) and row ids fit 32 bits are
-// joined with a 4-byte-per-field shared-memory table, two CTAs per SM.
-constexpr int kCompactCap = 8192;
-constexpr int kCompactThreads = 512;
-
-// Chunking of the two relations (identical for the histogram and both scatter passes).
-struct ChunkGeom {
-    uint64_t chunk;  // tuples per chunk (a multiple of the tile)
-    uint32_t cR, cS; // chunks of R, chunks of S (R's come first)
-    uint64_t sub;    // tuples per sub-chunk (a multiple of the tile): the pass-1 work item
-    uint32_t spc;    // sub-chunks per chunk
-    uint32_t pad;
-};
-
-__device__ __forceinline__ uint64_t ld_u64_pair(const uint32_t *p) {
-    return (uint64_t)p[0] | ((uint64_t)p[1] << 32);
-}
-__device__ __forceinline__ void st_u64_pair(uint32_t *p, uint64_t v) {
-    p[0] = (uint32_t)v;
-    p[1] = (uint32_t)(v >> 32);
-}
-
-__host__ __device__ __forceinline__ uint32_t ceil_div_u64(uint64_t a, uint64_t b) {
-    return (uint32_t)((a + b - 1) / b);
-}
-
-__device__ __forceinline__ uint32_t next_pow2_u32(uint32_t x) {
-    return x <= 1 ? 1u : 1u << (32 - __clz(x - 1));
-}
-
-__device__ __forceinline__ uint32_t smem_addr(const void *p) {
-    return (uint32_t)__cvta_generic_to_shared(p);
-}
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-
-// Bounded wait for the completion of phase `parity` of an mbarrier.
-__device__ __forceinline__ uint64_t globaltimer_ns() {
-    uint64_t t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-// Bounded wait for an mbarrier phase: gives up after kWaitNs of wall time (try_wait may suspend the
-// thread for a hardware-defined time per call, so an iteration count alone is no time bound).
-constexpr uint64_t kWaitNs = 2000000000ull;
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-    const uint64_t t0 = globaltimer_ns();
-    for (uint32_t it = 0; it < (1u << 30); it++) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(done)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (done) return true;
-        if ((it & 63u) == 63u && globaltimer_ns() - t0 > kWaitNs) return false;
-    }
-    return false;
-}
-
-// TMA bulk copy global -> shared of `bytes` (a multiple of 16, <= 1 MiB per phase), completing on
-// `bar`. Issued by one thread.
-__device__ __forceinline__ void tma_load_1d(void *dst_smem, const void *src, uint32_t bytes, uint32_t bar) {
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-    const char *s = reinterpret_cast<const char *>(src);
-    const uint32_t d = smem_addr(dst_smem);
-    for (uint32_t off = 0; off < bytes; off += 32768u) {
-        const uint32_t sz = bytes - off < 32768u ? bytes - off : 32768u;
-        asm volatile(
-            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(d + off),
-            "l"(s + off), "r"(sz), "r"(bar)
-            : "memory");
-    }
-}
 
 // Count the tuples [lo, hi) of `in`, read by one warp (four 512-byte loads in flight), into the joint
 // histogram and into the warp's histogram of the pass-1 digit, ORing together all row ids and (BUILD)
@@ -379,34 +204,6 @@ __global__ void colscan_kernel(const uint32_t *__restrict__ chunk_hist, uint32_t
 // 3. Plan: final partition starts (in (pass-1 digit, pass-2 digit) order), join work items, large
 //    partitions. One CTA of 1024 threads.
 // ------------------------------------------------------------------------------------------------
-struct PlanArgs {
-    int bits, passes, b1, F1, F2;
-    uint64_t nR, nS;
-    const uint32_t *total;  // [2][2^B]
-    uint64_t *start;        // [2][2^B + 1]
-    uint32_t *counters;
-    JoinItem *items;
-    uint64_t max_items;
-    LargePart *large;
-    uint64_t max_large;
-    uint64_t large_table_words;
-    int agg_ok;  // joins that need no per-match output may use key-aggregated large-partition tables
-};
-
-__device__ __forceinline__ uint32_t part_to_value(int f, int passes, int b1, int F2) {
-    if (passes == 1) return (uint32_t)f;
-    const uint32_t d1 = (uint32_t)f / (uint32_t)F2, d2 = (uint32_t)f % (uint32_t)F2;
-    return d1 | (d2 << b1);
-}
-
-// u32 words of one large partition's table. Chains: head[nb] then next[r_len]. Key-aggregated:
-// sum[r_len] (u64), head[nb], next[r_len], cnt[r_len], negpos[r_len], rounded to an even count so the
-// next table's sums stay 8-byte aligned.
-__device__ __forceinline__ uint64_t large_words_chain(const LargePart &L) { return (1ull << L.nb_log) + L.r_len; }
-__device__ __forceinline__ uint64_t large_words_agg(const LargePart &L) {
-    return ((1ull << L.nb_log) + 5 * L.r_len + 1) & ~1ull;
-}
-
 // Dynamic shared memory: the relation totals ([2][2^B] u32) when they fit (B <= 14), so that the
 // per-partition loops below read shared memory instead of waiting on one global load after another.
 constexpr int kPlanStageBits = 14;
@@ -414,7 +211,7 @@ constexpr int kPlanStageBits = 14;
 __global__ void __launch_bounds__(1024, 1) plan_kernel(PlanArgs a) {
     extern __shared__ uint32_t sm_tot[];
     __shared__ uint32_t tmp[32];
-    __shared__ uint64_t s_item_run, s_large_run;
+    __shared__ uint64_t s_run[2];
     const int tid = threadIdx.x;
     const int nparts = 1 << a.bits;
     const uint32_t *tot_all = a.total;
@@ -424,125 +221,7 @@ __global__ void __launch_bounds__(1024, 1) plan_kernel(PlanArgs a) {
         __syncthreads();
         tot_all = sm_tot;
     }
-    // Each thread owns a contiguous range of partitions.
-    const int per = (nparts + 1023) / 1024;
-    const int f0 = tid * per < nparts ? tid * per : nparts;
-    const int f1 = f0 + per < nparts ? f0 + per : nparts;
-    uint64_t base[2];  // start of this thread's first partition, per relation
-    for (int rel = 0; rel < 2; rel++) {
-        uint64_t *start = a.start + (size_t)rel * (nparts + 1);
-        const uint32_t *tot = tot_all + (size_t)rel * nparts;
-        uint32_t sum = 0;
-        for (int f = f0; f < f1; f++) sum += tot[part_to_value(f, a.passes, a.b1, a.F2)];
-        uint32_t all;
-        uint64_t run = block_excl_scan_u32(sum, tmp, &all);
-        base[rel] = run;
-        for (int f = f0; f < f1; f++) {
-            start[f] = run;
-            run += tot[part_to_value(f, a.passes, a.b1, a.F2)];
-        }
-        if (tid == 0) start[nparts] = all;
-    }
-
-    // Join work items (partitions with both sides non-empty, src/algo/phj.c:459-491) and large
-    // partitions. Partition sizes come from the totals, starts from the running sums above.
-    const uint32_t *totR = tot_all, *totS = tot_all + nparts;
-    const uint64_t small_cap = (uint64_t)kSmemCap;
-    uint32_t asum = 0, bsum = 0, lsum = 0;  // items with |R_p| <= compact cap, other small items, large
-    for (int f = f0; f < f1; f++) {
-        const uint32_t v = part_to_value(f, a.passes, a.b1, a.F2);
-        const uint64_t nr = totR[v], ns = totS[v];
-        if (nr > 0 && ns > 0) {
-            if (nr <= (uint64_t)kCompactCap) asum += ceil_div_u64(ns, kProbeChunk);
-            else if (nr <= small_cap) bsum += ceil_div_u64(ns, kProbeChunk);
-            else lsum++;
-        }
-    }
-    uint32_t atot, btot, ltot;
-    uint64_t a_idx = block_excl_scan_u32(asum, tmp, &atot);
-    uint64_t b_idx = block_excl_scan_u32(bsum, tmp, &btot) + atot;
-    uint64_t large_idx = block_excl_scan_u32(lsum, tmp, &ltot);
-    const uint32_t ktot = atot + btot;
-    uint64_t rR = base[0], rS = base[1];
-    for (int f = f0; f < f1; f++) {
-        const uint32_t v = part_to_value(f, a.passes, a.b1, a.F2);
-        const uint64_t nr = totR[v], ns = totS[v];
-        const uint64_t sR = rR, sS = rS;
-        rR += nr;
-        rS += ns;
-        if (!(nr > 0 && ns > 0)) continue;
-        if (nr <= small_cap) {
-            uint64_t &item_idx = nr <= (uint64_t)kCompactCap ? a_idx : b_idx;
-            const uint32_t k = ceil_div_u64(ns, kProbeChunk);
-            for (uint32_t q = 0; q < k; q++, item_idx++) {
-                if (item_idx < a.max_items) {
-                    JoinItem it;
-                    it.r_begin = sR;
-                    it.s_begin = sS + (uint64_t)q * kProbeChunk;
-                    it.r_len = (uint32_t)nr;
-                    const uint64_t rem = ns - (uint64_t)q * kProbeChunk;
-                    it.s_len = (uint32_t)(rem < (uint64_t)kProbeChunk ? rem : (uint64_t)kProbeChunk);
-                    it.part0 = v == 0 ? 1u : 0u;
-                    it.pad = 0;
-                    a.items[item_idx] = it;
-                } else {
-                    atomicOr(&a.counters[kCtrErr], kErrCapacity);
-                }
-            }
-        } else {
-            if (large_idx < a.max_large) {
-                LargePart lp;
-                lp.r_begin = sR;
-                lp.s_begin = sS;
-                lp.r_len = nr;
-                lp.s_len = ns;
-                uint32_t nb_log = 0;
-                while ((1ull << nb_log) < nr) nb_log++;
-                lp.nb_log = nb_log;
-                lp.part0 = v == 0 ? 1u : 0u;
-                lp.table_off = 0;
-                lp.r_flat = lp.s_flat = 0;
-                a.large[large_idx] = lp;
-            } else {
-                atomicOr(&a.counters[kCtrErr], kErrCapacity);
-            }
-            large_idx++;
-        }
-    }
-    if (tid == 0) a.counters[kCtrNItemsA] = atot < a.max_items ? atot : (uint32_t)a.max_items;
-    if (tid == 0) {
-        s_item_run = ktot;
-        s_large_run = ltot;
-    }
-    __syncthreads();
-    const uint64_t item_run = s_item_run, large_run = s_large_run;
-    __syncthreads();
-    if (tid == 0) {
-        const uint64_t nl = large_run < a.max_large ? large_run : a.max_large;
-        // Key-aggregated tables (large_words_agg) when the join allows them and they fit the table
-        // area, else plain chains (large_words_chain).
-        uint64_t need_agg = 0;
-        for (uint64_t l = 0; l < nl; l++) need_agg += large_words_agg(a.large[l]);
-        const bool agg = a.agg_ok && need_agg <= a.large_table_words;
-        a.counters[kCtrLargeAgg] = agg ? 1u : 0u;
-        uint64_t off = 0, rf = 0, sf = 0;
-        for (uint64_t l = 0; l < nl; l++) {
-            LargePart &lp = a.large[l];
-            lp.table_off = off;
-            lp.r_flat = rf;
-            lp.s_flat = sf;
-            off += agg ? large_words_agg(lp) : large_words_chain(lp);
-            rf += lp.r_len;
-            sf += lp.s_len;
-        }
-        const bool fits = off <= a.large_table_words;
-        if (!fits) atomicOr(&a.counters[kCtrErr], kErrCapacity);
-        a.counters[kCtrNItems] = (uint32_t)(item_run < a.max_items ? item_run : a.max_items);
-        a.counters[kCtrNLarge] = (uint32_t)nl;
-        st_u64_pair(&a.counters[kCtrLargeR], fits ? rf : 0);
-        st_u64_pair(&a.counters[kCtrLargeS], fits ? sf : 0);
-        st_u64_pair(&a.counters[kCtrLargeWords], fits ? off : 0);
-    }
+    plan_body(a, tot_all, tmp, s_run);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -1699,6 +1378,12 @@ struct JoinArgs {
     MatOut mat; // materialising joins (MAT kernels): where the (r.row_id, s.row_id) pairs go
     int ci;     // the final partitions may be compact words (when ci_applies holds) at finR8 / finS8
     const unsigned long long *finR8, *finS8;
+    // First-match joins of the one-pass pipeline: build elements are {ci_word or key, input position}, and
+    // a wide match reads its row id from the build relation itself.
+    int lp_pos;
+    const tuple_v *relR;
+    uint64_t nR;
+    int flag_bits;  // HJ_RES_COMPACT_PARTITIONS tells whether words of this many radix bits fit
     int w8_b1;  // a pass 1 that may store words (either pipeline): its shift (reported when w8_fits held); -1 otherwise
 };
 
@@ -1713,6 +1398,10 @@ __device__ __forceinline__ tuple_v ld_fin(const tuple_v *p16, const unsigned lon
 }
 
 __device__ __forceinline__ tuple_v fin_r(const JoinArgs &a, bool ci, uint64_t i) {
+    if (a.lp_pos) {  // y: the input position
+        const tuple_v t = a.finR[i];
+        return make_ulonglong2(ci ? t.x >> 32 : t.x, t.y);
+    }
     if (ci) {
         const unsigned long long w = a.finR8[i];
         return make_ulonglong2(w >> 32, w & 0xffffffffull);
@@ -1898,6 +1587,123 @@ __global__ void __launch_bounds__(kCompactThreads, 2) join_compact_kernel(JoinAr
     }
     block_sum2_to(cnt, sum, red, &a.acc->matched, &a.acc->checksum);
     if (LP && !MAT) flag_multi(multi, &a.acc->dup_flag);
+}
+
+// First-match join of the one-pass pipeline. Build elements come with their input position, and the match
+// with the lowest one wins, so the partition may hold them in any order. Key, position and row id in
+// separate arrays (20 bytes per build tuple, 16-bit bucket heads and chains: 214 KB, one CTA per SM);
+// a wide element's row id is gathered from the build relation once per build tuple.
+constexpr uint32_t kFirstHeads = 8192;
+constexpr size_t kFirstSmem = (size_t)kFirstCap * (8 + 8 + 4 + 2) + kFirstHeads * 2;
+
+template <bool MAT>
+__global__ void __launch_bounds__(kJoinThreads, 1) join_first_kernel(JoinArgs a) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    unsigned long long *kx = reinterpret_cast<unsigned long long *>(smem);  // [kFirstCap] key (or its high part)
+    unsigned long long *rid = kx + kFirstCap;                              // [kFirstCap]
+    uint32_t *pos = reinterpret_cast<uint32_t *>(rid + kFirstCap);         // [kFirstCap]
+    uint16_t *head = reinterpret_cast<uint16_t *>(pos + kFirstCap);        // [kFirstHeads]
+    uint16_t *nxt = head + kFirstHeads;                                    // [kFirstCap]
+    __shared__ unsigned long long red[64];
+    __shared__ uint32_t s_item;
+    __shared__ uint32_t scan_tmp[32];
+    __shared__ unsigned long long s_base;
+    const int tid = threadIdx.x;
+    unsigned int *err = &a.counters[kCtrErr];
+    const uint32_t nitems = a.counters[kCtrNItems];
+    const bool ci = !MAT && a.ci && ci_applies(a.counters, a.bits);
+    const int B = ci ? 0 : a.bits;
+    const bool skip0 = a.skip0 != 0;
+    unsigned long long cnt = 0, sum = 0;
+    bool multi = false;
+    constexpr int U = 4;
+    for (;;) {
+        if (tid == 0) s_item = atomicAdd(&a.counters[kCtrItemA], 1u);
+        __syncthreads();
+        const uint32_t it = s_item;
+        if (it >= nitems) break;
+        const JoinItem item = a.items[it];
+        const uint32_t nr = item.r_len;
+        const uint32_t nb = min(next_pow2_u32(nr), kFirstHeads);
+        const uint64_t hmask = nb - 1;
+        uint32_t *head32 = reinterpret_cast<uint32_t *>(head);
+        for (uint32_t q = tid; q < (nb + 1) / 2; q += kJoinThreads) head32[q] = 0;
+        __syncthreads();
+        const tuple_v *R = a.finR + item.r_begin;
+        for (uint32_t i0 = tid; i0 < nr; i0 += U * kJoinThreads) {
+            tuple_v t[U];
+            unsigned long long y[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const uint32_t i = i0 + u * kJoinThreads;
+                t[u] = i < nr ? ld_stream(R + i) : make_ulonglong2(0, 0);
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const bool live = i0 + u * kJoinThreads < nr && t[u].y < a.nR;
+                y[u] = ci ? t[u].x & 0xffffffffull : live ? a.relR[t[u].y].y : 0ull;
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const uint32_t i = i0 + u * kJoinThreads;
+                if (i >= nr) continue;
+                const unsigned long long k = ci ? t[u].x >> 32 : t[u].x;
+                kx[i] = k;
+                rid[i] = y[u];
+                pos[i] = (uint32_t)t[u].y;
+                // In compact words a key 0 that never matches has a high part that no probe word has.
+                if (skip0 && k == 0 && !ci) continue;
+                nxt[i] = (uint16_t)atomic_exch_u16(&head[(k >> B) & hmask], i + 1);
+            }
+        }
+        __syncthreads();
+        const tuple_v *S = a.finS + item.s_begin;
+        const unsigned long long *S8 = a.finS8 + item.s_begin;
+        const uint32_t ns = item.s_len;
+        for (uint32_t base = 0; base < ns; base += U * kJoinThreads) {
+            tuple_v sv[U];
+            uint32_t best[U], m = 0;
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const uint32_t j = base + u * kJoinThreads + tid;
+                sv[u] = j < ns ? ld_fin(S, S8, j, ci) : make_ulonglong2(0, 0);
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                best[u] = 0;
+                if (base + u * kJoinThreads + tid >= ns) continue;
+                uint32_t e = head[(sv[u].x >> B) & hmask], steps = 0, nm = 0, bp = 0;
+                while (e) {
+                    if (kx[e - 1] == sv[u].x) {
+                        const uint32_t p = pos[e - 1];
+                        if (nm++ == 0 || p < bp) {
+                            best[u] = e;
+                            bp = p;
+                        }
+                    }
+                    e = nxt[e - 1];
+                    if (++steps > nr) {
+                        set_error(err, kErrProbeLimit);
+                        break;
+                    }
+                }
+                if (!best[u]) continue;
+                m++;
+                if (!MAT) sum += rid[best[u] - 1] + sv[u].y;
+                multi |= nm > 1;
+            }
+            cnt += m;
+            if constexpr (MAT) {
+                unsigned long long o = mat_reserve(m, scan_tmp, &s_base, &a.acc->pairs);
+#pragma unroll
+                for (int u = 0; u < U; u++)
+                    if (best[u]) mat_put(a.mat, o++, rid[best[u] - 1], sv[u].y, err);
+            }
+        }
+        __syncthreads();
+    }
+    block_sum2_to(cnt, sum, red, &a.acc->matched, &a.acc->checksum);
+    if (!MAT) flag_multi(multi, &a.acc->dup_flag);
 }
 
 template <bool MAT, bool CI = false>
@@ -2183,7 +1989,7 @@ __global__ void join_large_build(JoinArgs a) {
             const unsigned s0 = __reduce_add_sync(peers, (unsigned)(r.y & 0xffffffu));
             const unsigned s1 = __reduce_add_sync(peers, (unsigned)((r.y >> 24) & 0xffffffu));
             const unsigned s2 = __reduce_add_sync(peers, (unsigned)(r.y >> 48));
-            const unsigned minpos = __reduce_min_sync(peers, (unsigned)i);
+            const unsigned minpos = __reduce_min_sync(peers, a.lp_pos ? (unsigned)r.y : (unsigned)i);
             if ((int)lane != __ffs(peers) - 1) continue;
             const LargePart &L = a.large[l];
             const LargeAgg t = large_agg(a.large_table, L);
@@ -2242,7 +2048,7 @@ __global__ void join_large_probe(JoinArgs a) {
                 for (uint32_t e = e0; e;) {
                     if (rr[e - 1].x == s.x) {
                         if (!a.lp) m++;
-                        else if (best == 0 || e < best) best = e;
+                        else if (best == 0 || (a.lp_pos ? rr[e - 1].y < rr[best - 1].y : e < best)) best = e;
                     }
                     e = nxt[e - 1];
                     if (++steps > Lp->r_len) {
@@ -2258,7 +2064,8 @@ __global__ void join_large_probe(JoinArgs a) {
                 const uint32_t *nxt = a.large_table + Lp->table_off + (1ull << Lp->nb_log);
                 const tuple_v *rr = a.finR + Lp->r_begin;
                 if (a.lp) {
-                    mat_put(a.mat, o, rr[best - 1].y, s.y, err);
+                    const unsigned long long y = rr[best - 1].y;
+                    mat_put(a.mat, o, !a.lp_pos ? y : y < a.nR ? a.relR[y].y : 0ull, s.y, err);
                 } else {
                     uint64_t steps = 0;
                     for (uint32_t e = e0; e && steps++ <= Lp->r_len; e = nxt[e - 1])
@@ -2286,9 +2093,9 @@ __global__ void join_large_probe(JoinArgs a) {
             if (a.lp) {
                 const uint32_t first = ~t.negpos[e - 1];
                 multi |= t.cnt[e - 1] > 1;
-                if (first < L.r_len) {
+                if (first < (a.lp_pos ? a.nR : L.r_len)) {
                     cnt++;
-                    sum += fin_r(a, ci, L.r_begin + first).y + s.y;
+                    sum += (a.lp_pos ? a.relR[first].y : fin_r(a, ci, L.r_begin + first).y) + s.y;
                 } else {
                     set_error(&a.counters[kCtrErr], kErrBounds);
                 }
@@ -2308,12 +2115,16 @@ __global__ void join_large_probe(JoinArgs a) {
         const uint32_t *nxt = head + (1ull << L.nb_log);
         uint32_t e = head[(s.x >> bshift) & ((1ull << L.nb_log) - 1)];
         uint32_t best = 0, nm = 0;
+        unsigned long long best_y = 0;  // the match's row id, or its input position (lp_pos)
         uint64_t steps = 0;
         while (e) {
             const tuple_v r = fin_r(a, ci, L.r_begin + e - 1);
             if (r.x == s.x) {
                 if (a.lp) {
-                    if (best == 0 || e < best) best = e;
+                    if (best == 0 || (a.lp_pos ? r.y < best_y : e < best)) {
+                        best = e;
+                        best_y = r.y;
+                    }
                     nm++;
                 } else {
                     cnt++;
@@ -2328,7 +2139,7 @@ __global__ void join_large_probe(JoinArgs a) {
         }
         if (a.lp && best) {
             cnt++;
-            sum += fin_r(a, ci, L.r_begin + best - 1).y + s.y;
+            sum += (!a.lp_pos ? best_y : best_y < a.nR ? a.relR[best_y].y : 0ull) + s.y;
             multi |= nm > 1;
         }
     }
@@ -2336,7 +2147,8 @@ __global__ void join_large_probe(JoinArgs a) {
     if (!MAT) flag_multi(multi, &a.acc->dup_flag);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         if (nl) atomicAdd(&a.acc->large_parts, (unsigned long long)nl);
-        if (ci) atomicOr(&a.acc->flags, (unsigned long long)HJ_RES_COMPACT_PARTITIONS);
+        if (!MAT && a.ci && ci_applies(a.counters, a.flag_bits))
+            atomicOr(&a.acc->flags, (unsigned long long)HJ_RES_COMPACT_PARTITIONS);
         if (a.w8_b1 >= 0 && w8_fits(a.counters, a.w8_b1))
             atomicOr(&a.acc->flags, (unsigned long long)HJ_RES_WORD_PASS1);
     }
@@ -2358,6 +2170,8 @@ int radix_geom(int bits, int passes, RadixGeom *g, int b1_req) {
     if (P == 1 && bits > 8) P = 2;
     if (P == 2 && bits < 2) P = 1;
     g->bits = bits;
+    g->req_bits = bits;
+    g->single = false;
     g->passes = P;
     int b1 = bits / 2;
     if (b1_req > 0) {
@@ -2373,6 +2187,28 @@ int radix_geom(int bits, int passes, RadixGeom *g, int b1_req) {
     g->F1 = 1 << g->b1;
     g->F2 = 1 << g->b2;
     return HJ_OK;
+}
+
+// The lowest bits that bring build partitions to kSingleTarget tuples on average, at least
+// kSingleMinBits (items for every SM), at most what the caller asked for. Above 2^kSingleMaxBits
+// partitions of kSingleMaxAvg tuples the two-pass pipelines run.
+constexpr uint64_t kSingleTarget = 6144, kSingleMaxAvg = 8192;
+constexpr int kSingleMinBits = 8;
+
+bool radix_geom_single(int bits, size_t nR, size_t nS, RadixGeom *g) {
+    if ((nR >> kSingleMaxBits) > kSingleMaxAvg || nR >= (1ull << 32) || nS >= (1ull << 32)) return false;
+    int b = kSingleMinBits;
+    while (b < kSingleMaxBits && (nR >> b) > kSingleTarget) b++;
+    if (b > bits) b = bits;
+    g->bits = b;
+    g->req_bits = bits;
+    g->passes = 1;
+    g->b1 = b;
+    g->b2 = 0;
+    g->F1 = 1 << b;
+    g->F2 = 1;
+    g->single = true;
+    return true;
 }
 
 static inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
@@ -2401,7 +2237,7 @@ static ChunkGeom chunk_geom(size_t nR, size_t nS, int num_sms) {
 
 struct PhjSizes {
     size_t chunk_hist, prefix, total, start, units_off, units_cnt, subhist, counters, items, large, large_table,
-        tmp1, tmp2, seg_head, seg_next;
+        tmp1, tmp2, seg_head, seg_next, ors;
     size_t max_items, max_large, large_table_words;
     uint32_t max_segs, seg_grid, it_tiles;
     ChunkGeom cg;
@@ -2437,6 +2273,12 @@ static PhjSizes phj_sizes(const RadixGeom &g, size_t nR, size_t nS, int num_sms,
         // fewer than kSegSlab ids of its last slab unused.
         const uint64_t segs = (uint64_t)(nR + nS) / kTile + 2ull * z.seg_grid * g.F1 + (uint64_t)z.seg_grid * kSegSlab;
         z.max_segs = (uint32_t)segs;
+    } else if (g.single) {
+        z.seg_grid = z.it_tiles = z.max_segs = 0;
+        z.cg.chunk = z.cg.sub = 0;
+        z.cg.cR = z.cg.cS = single_grid(nR, nS, sms);
+        z.cg.spc = 0;
+        z.cg.pad = 0;
     } else {
         z.cg = chunk_geom(nR, nS, num_sms);
         z.seg_grid = 0;
@@ -2445,16 +2287,18 @@ static PhjSizes phj_sizes(const RadixGeom &g, size_t nR, size_t nS, int num_sms,
     }
     const size_t nchunks = (size_t)z.cg.cR + z.cg.cS;
     z.chunk_hist = align_up(nchunks * np * 4, 256);
-    z.prefix = z.chunk_hist;
+    z.prefix = g.single ? 0 : z.chunk_hist;  // the one-pass pipeline's prefixes replace its histogram rows
+    z.ors = g.single ? align_up((size_t)z.cg.cR * 3 * 8, 256) : 0;
     z.total = align_up(2 * np * 4, 256);
     z.start = align_up(2 * (np + 1) * 8, 256);
-    z.units_off = align_up(nchunks * (size_t)g.F1 * 8, 256);
-    z.units_cnt = align_up(nchunks * (size_t)g.F1 * 4, 256);
+    z.units_off = g.single ? 0 : align_up(nchunks * (size_t)g.F1 * 8, 256);
+    z.units_cnt = g.single ? 0 : align_up(nchunks * (size_t)g.F1 * 4, 256);
     z.subhist = align_up(nchunks * (size_t)z.cg.spc * g.F1 * 4, 256);
     z.counters = 256;
     z.max_items = np + nS / kProbeChunk + 2;
     z.items = align_up(z.max_items * sizeof(JoinItem), 256);
-    z.max_large = np < nR / kSmemCap + 1 ? np : nR / kSmemCap + 1;
+    const size_t min_large = g.single ? kFirstCap : kSmemCap;
+    z.max_large = np < nR / min_large + 1 ? np : nR / min_large + 1;
     z.large = align_up(z.max_large * sizeof(LargePart), 256);
     z.tmp1 = seg ? align_up((size_t)z.max_segs * kTile * 16, 256) : align_up((nR + nS) * 16, 256);
     z.tmp2 = g.passes == 2 ? align_up((nR + nS) * 16, 256) : 0;
@@ -2471,7 +2315,7 @@ static PhjSizes phj_sizes(const RadixGeom &g, size_t nR, size_t nS, int num_sms,
 size_t phj_scratch_bytes(const RadixGeom &g, size_t nR, size_t nS, int num_sms, bool seg) {
     PhjSizes z = phj_sizes(g, nR, nS, num_sms, seg);
     return z.chunk_hist + z.prefix + z.total + z.start + z.units_off + z.units_cnt + z.subhist + z.counters + z.items +
-           z.large + z.large_table + z.tmp1 + z.tmp2 + z.seg_head + z.seg_next;
+           z.large + z.large_table + z.tmp1 + z.tmp2 + z.seg_head + z.seg_next + z.ors;
 }
 
 void phj_carve(const RadixGeom &g, size_t nR, size_t nS, int num_sms, char *base, PhjScratch *s, bool seg) {
@@ -2495,6 +2339,7 @@ void phj_carve(const RadixGeom &g, size_t nR, size_t nS, int num_sms, char *base
     s->subhist = reinterpret_cast<uint32_t *>(p); p += z.subhist;
     s->seg_head = reinterpret_cast<uint32_t *>(p); p += z.seg_head;
     s->seg_next = reinterpret_cast<uint32_t *>(p); p += z.seg_next;
+    s->ors = reinterpret_cast<unsigned long long *>(p); p += z.ors;
     s->counters = reinterpret_cast<uint32_t *>(p); p += z.counters;
     s->items = p; p += z.items;
     s->max_items = z.max_items;
@@ -2575,11 +2420,17 @@ int phj_prepare_device() {
                                (int)kCompactSmem));
     HJ_CU(cudaFuncSetAttribute(join_compact_kernel<true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)kCompactSmem));
+    HJ_CU(cudaFuncSetAttribute(join_first_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFirstSmem));
+    HJ_CU(cudaFuncSetAttribute(join_first_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFirstSmem));
     HJ_CU(cudaFuncSetAttribute(join_small_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kJoinSmem));
     HJ_CU(cudaFuncSetAttribute(join_compact_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)kCompactSmem));
     HJ_CU(cudaFuncSetAttribute(join_compact_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)kCompactSmem));
+    {
+        const int rc = single_prepare_device();
+        if (rc) return rc;
+    }
     g_attr_done[cur_dev] = true;
     return nphj_prepare_device();
 }
@@ -2590,7 +2441,7 @@ int phj_enqueue(const RadixGeom &g, bool lp, bool skip0, const ulonglong2 *R, si
                 bool ordered) {
     uint32_t nlaunch = 0;
     // Stable ranks of the build relation: first-match joins that keep the input order.
-    const bool stable = lp && ordered;
+    const bool stable = lp && ordered && !g.single;
 #define HJ_PH(i) \
     if (ph) HJ_CU(record_event(ph[i], st))
     if (nR >= (1ull << 32) || nS >= (1ull << 32)) return HJ_E_INVAL;
@@ -2630,7 +2481,10 @@ int phj_enqueue(const RadixGeom &g, bool lp, bool skip0, const ulonglong2 *R, si
     HJ_CU(cudaMemsetAsync(s.counters, 0, kNumCounters * 4, st));
 
     HJ_PH(0);
-    if (segm) {
+    if (g.single) {
+        const int rc = single_partition_enqueue(g, lp, skip0, ci_ok != 0, R, nR, S, nS, s, st, !mat, ph, &nlaunch);
+        if (rc) return rc;
+    } else if (segm) {
         // 1'. pass 1 into segment chains, with the per-CTA histograms
         SegArgs ga;
         ga.R = R;
@@ -2697,6 +2551,7 @@ int phj_enqueue(const RadixGeom &g, bool lp, bool skip0, const ulonglong2 *R, si
                                                            s.counters + kCtrMaxKey);
         HJ_CU(cudaGetLastError());
     }
+    if (!g.single) {
     HJ_PH(1);
     // 2. prefix over chunks, 3. plan, 4. units
     colscan_kernel<<<(8 * np + 255) / 256, 256, 0, st>>>(s.chunk_hist, s.prefix, s.total, np, cg);
@@ -2717,6 +2572,7 @@ int phj_enqueue(const RadixGeom &g, bool lp, bool skip0, const ulonglong2 *R, si
     pa.max_large = s.max_large;
     pa.large_table_words = s.large_table_words;
     pa.agg_ok = mat ? 0 : 1;
+    pa.small_cap = kSmemCap;
     plan_kernel<<<1, 1024, g.bits <= kPlanStageBits ? (size_t)2 * np * 4 : 0, st>>>(pa);
     {
         const int ut = F1 < 32 ? 32 : F1;
@@ -2726,10 +2582,11 @@ int phj_enqueue(const RadixGeom &g, bool lp, bool skip0, const ulonglong2 *R, si
     HJ_CU(cudaGetLastError());
     nlaunch += segm ? 3 : 4;
     HJ_PH(2);
+    }
 
     // 5. scatter passes (segment mode: pass 2 only, its units are the pass-1 chains)
     const int scatter_grid = num_sms * kScatterCtasPerSm;
-    for (int pass = segm ? 1 : 0; pass < g.passes; pass++) {
+    for (int pass = segm ? 1 : 0; pass < g.passes && !g.single; pass++) {
         ScatterArgs sa;
         sa.pass = pass;
         sa.F = pass == 0 ? F1 : F2;
@@ -2813,7 +2670,7 @@ int phj_enqueue(const RadixGeom &g, bool lp, bool skip0, const ulonglong2 *R, si
         nlaunch++;
         HJ_PH(segm ? 3 : 3 + pass);
     }
-    if (ph && g.passes == 1) HJ_CU(record_event(ph[4], st));
+    if (ph && g.passes == 1 && !g.single) HJ_CU(record_event(ph[4], st));
     if (ev_mid) HJ_CU(record_event(ev_mid, st));
 
     // 6. joins
@@ -2831,9 +2688,18 @@ int phj_enqueue(const RadixGeom &g, bool lp, bool skip0, const ulonglong2 *R, si
     ja.mat = mat ? *mat : MatOut{nullptr, 0};
     ja.ci = ci_ok;
     ja.finR8 = reinterpret_cast<const unsigned long long *>(s.tmp2);
-    ja.finS8 = ja.finR8 + nR;
+    ja.finS8 = g.single ? single_probe_words(s, nR, lp) : ja.finR8 + nR;
+    ja.lp_pos = g.single && lp ? 1 : 0;
+    ja.relR = R;
+    ja.nR = nR;
+    ja.flag_bits = g.req_bits;
     ja.w8_b1 = (seg_words || exact_words) ? g.b1 : -1;
-    if (mat) {
+    if (ja.lp_pos) {
+        if (mat)
+            join_first_kernel<true><<<num_sms, kJoinThreads, kFirstSmem, st>>>(ja);
+        else
+            join_first_kernel<false><<<num_sms, kJoinThreads, kFirstSmem, st>>>(ja);
+    } else if (mat) {
         if (lp)
             join_compact_kernel<true, false, true><<<num_sms * 2, kCompactThreads, kCompactSmem, st>>>(ja);
         else

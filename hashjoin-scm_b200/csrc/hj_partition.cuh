@@ -1,0 +1,354 @@
+// hj_partition.cuh - plan structures, compact words and counters shared by the kernels of the radix
+// joins: the two-pass pipelines (hj_partition.cu) and the one-pass pipeline (hj_single.cu).
+#pragma once
+
+#include "hj_common.cuh"
+#include "hj_internal.h"
+
+namespace hj {
+
+// ------------------------------------------------------------------------------------------------
+// Device-side plan structures
+// ------------------------------------------------------------------------------------------------
+struct JoinItem {
+    uint64_t r_begin;  // index into the final R buffer
+    uint64_t s_begin;  // index into the final S buffer
+    uint32_t r_len;
+    uint32_t s_len;
+    uint32_t part0;    // 1: the partition of the keys whose radix bits are 0 (key 0's partition)
+    uint32_t pad;
+};
+
+struct LargePart {
+    uint64_t r_begin, s_begin;
+    uint64_t r_len, s_len;
+    uint64_t table_off;  // u32 words into the large table: head[nb] then next[r_len]
+    uint64_t r_flat, s_flat;
+    uint32_t nb_log;
+    uint32_t part0;  // as JoinItem::part0
+};
+
+// counters[] slots
+enum : int {
+    kCtrItem1 = 0,       // scatter pass-1 work-item counter
+    kCtrItem2 = 1,       // scatter pass-2 work-item counter
+    kCtrNItemsA = 2,     // join items whose build side fits the compact shared-memory table (listed first)
+    kCtrItemA = 3,       // compact join work-item counter
+    kCtrSegAlloc = 4,    // segment mode: segment ids handed out
+    kCtrLargeAgg = 5,    // 1: large partitions use key-aggregated tables (see join_large_build)
+    kCtrNItems = 6,
+    kCtrNLarge = 7,
+    kCtrItem = 8,        // join work-item counter
+    kCtrLargeR = 9,      // total R tuples in large partitions (u32 pairs: lo, hi)
+    kCtrLargeS = 11,     // total S tuples in large partitions (lo, hi)
+    kCtrLargeWords = 13, // table words used (lo, hi)
+    kCtrErr = 15,
+    kCtrMaxKey = 16,     // u64: OR of all R keys (words 16-17)
+    kCtrMaxRid = 18,     // u64: OR of all R row ids (words 18-19)
+    kCtrOrRidS = 20,     // u64: OR of all S row ids (words 20-21)
+    kCtrItem1S = 22,     // first-match joins: pass-1 work-item counter of the probe relation's items
+    kCtrItem2S = 23,     // first-match joins: pass-2 work-item counter of the probe relation's items
+    kCtrTicket = 24,     // one-pass pipeline: CTAs of single_plan that have written their totals
+    kNumCounters = 26
+};
+
+// Compact final partitions. When every build key shifted right by the radix bits is below 2^31 and
+// every row id (build and probe) below 2^32, the last partition pass stores each tuple as one 8-byte
+// word, (key >> bits) << 32 | row id, and the joins read 8 bytes per tuple instead of 16. Inside a
+// final partition the low `bits` key bits are equal, so comparing key >> bits compares keys. A probe
+// key whose high part is 2^31 or more is stored as 0xffffffff: no build key has that high part. Joins
+// where a build key 0 never matches (lp_join's empty-slot rule): a last pass that reads tuples stores
+// that key's words with high part 0x80000000, which no build key and no probe word has (ci_word_z0);
+// from segment-mode pass-1 words it keeps high part 0, and since key 0 lies in the partition of the
+// keys whose radix bits are 0, where a high part of 0 means key 0, the joins skip such build words
+// there (JoinItem::part0). The widths are ORed together by the pass that reads the relations first (hist_chunk_kernel or
+// seg_pass1_kernel), so the choice is made on the device, before the last pass.
+__device__ __forceinline__ bool ci_applies(const uint32_t *counters, int bits) {
+    const unsigned long long *mx = reinterpret_cast<const unsigned long long *>(counters + kCtrMaxKey);
+    return (mx[0] >> bits) < (1ull << 31) && mx[1] < (1ull << 32) && mx[2] < (1ull << 32);
+}
+
+// Segment mode can go further: pass 1 stores (key >> b1) << 32 | row id (w8_word) in segments of 4096
+// words (the same 32 KB as 2048 tuples) when every build key >> b1 is below 2^31 and every row id below
+// 2^32; pass 2 then reads 8-byte words in tiles of 4096 and writes compact final partitions. A probe
+// key whose key >> b1 does not fit keeps its low 31 bits and gets bit 31 set: its pass-2 digit stays
+// right, and after pass 2's shift its high part is still above every build key's.
+__device__ __forceinline__ bool w8_fits(const uint32_t *counters, int b1) {
+    const unsigned long long *mx = reinterpret_cast<const unsigned long long *>(counters + kCtrMaxKey);
+    return (mx[0] >> b1) < (1ull << 31) && mx[1] < (1ull << 32) && mx[2] < (1ull << 32);
+}
+
+__device__ __forceinline__ unsigned long long w8_word(unsigned long long key, unsigned long long rid, int b1) {
+    const unsigned long long hi = key >> b1;
+    const unsigned long long h32 = hi < (1ull << 31) ? hi : (0x80000000ull | (hi & 0x7fffffffull));
+    return (h32 << 32) | (rid & 0xffffffffull);
+}
+
+// Build relations whose key 0 never matches (z0), in the exact-offset pipeline's word pass 1: key 0's
+// word takes the high part 0x80000000, which no other build word has; the last pass keeps it
+// (store_elem) and stores every probe word whose high part has bit 31 set as 0xffffffff, so nothing
+// matches it. (Segment mode's pass 1 stores key 0 as any key; the joins skip it in its partition.)
+__device__ __forceinline__ unsigned long long w8_word_z0(unsigned long long key, unsigned long long rid, int b1,
+                                                         bool z0) {
+    return z0 && key == 0 ? (0x80000000ull << 32) | (rid & 0xffffffffull) : w8_word(key, rid, b1);
+}
+
+__device__ __forceinline__ unsigned long long ci_word(unsigned long long key, unsigned long long rid, int bits) {
+    const unsigned long long hi = key >> bits;
+    return ((hi < 0x80000000ull ? hi : 0xffffffffull) << 32) | (rid & 0xffffffffull);
+}
+
+__device__ __forceinline__ unsigned long long ci_word_z0(unsigned long long key, unsigned long long rid, int bits,
+                                                         bool z0) {
+    return z0 && key == 0 ? (0x80000000ull << 32) | (rid & 0xffffffffull) : ci_word(key, rid, bits);
+}
+
+// Build partitions up to this size whose keys (above the radix bits) and row ids fit 32 bits are
+// joined with a 4-byte-per-field shared-memory table, two CTAs per SM.
+constexpr int kCompactCap = 8192;
+constexpr int kCompactThreads = 512;
+// Largest build partition of the one-pass pipeline's first-match join.
+constexpr int kFirstCap = 9216;
+
+__device__ __forceinline__ uint32_t smem_addr(const void *p) {
+    return (uint32_t)__cvta_generic_to_shared(p);
+}
+
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+
+// Bounded wait for the completion of phase `parity` of an mbarrier.
+__device__ __forceinline__ uint64_t globaltimer_ns() {
+    uint64_t t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+// Bounded wait for an mbarrier phase: gives up after kWaitNs of wall time (try_wait may suspend the
+// thread for a hardware-defined time per call, so an iteration count alone is no time bound).
+constexpr uint64_t kWaitNs = 2000000000ull;
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return done != 0;
+}
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
+    if (mbar_try(bar, parity)) return true;
+    const uint64_t t0 = globaltimer_ns();
+    for (uint32_t it = 0; it < (1u << 30); it++) {
+        if (mbar_try(bar, parity)) return true;
+        if ((it & 63u) == 63u && globaltimer_ns() - t0 > kWaitNs) return false;
+    }
+    return false;
+}
+
+// TMA bulk copy global -> shared of `bytes` (a multiple of 16, <= 1 MiB per phase), completing on
+// `bar`. Issued by one thread.
+__device__ __forceinline__ void tma_load_1d(void *dst_smem, const void *src, uint32_t bytes, uint32_t bar) {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+    const char *s = reinterpret_cast<const char *>(src);
+    const uint32_t d = smem_addr(dst_smem);
+    for (uint32_t off = 0; off < bytes; off += 32768u) {
+        const uint32_t sz = bytes - off < 32768u ? bytes - off : 32768u;
+        asm volatile(
+            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(d + off),
+            "l"(s + off), "r"(sz), "r"(bar)
+            : "memory");
+    }
+}
+
+// Chunking of the two relations (identical for the histogram and both scatter passes).
+struct ChunkGeom {
+    uint64_t chunk;  // tuples per chunk (a multiple of the tile)
+    uint32_t cR, cS; // chunks of R, chunks of S (R's come first)
+    uint64_t sub;    // tuples per sub-chunk (a multiple of the tile): the pass-1 work item
+    uint32_t spc;    // sub-chunks per chunk
+    uint32_t pad;
+};
+
+__device__ __forceinline__ uint64_t ld_u64_pair(const uint32_t *p) {
+    return (uint64_t)p[0] | ((uint64_t)p[1] << 32);
+}
+__device__ __forceinline__ void st_u64_pair(uint32_t *p, uint64_t v) {
+    p[0] = (uint32_t)v;
+    p[1] = (uint32_t)(v >> 32);
+}
+
+__host__ __device__ __forceinline__ uint32_t ceil_div_u64(uint64_t a, uint64_t b) {
+    return (uint32_t)((a + b - 1) / b);
+}
+
+__device__ __forceinline__ uint32_t next_pow2_u32(uint32_t x) {
+    return x <= 1 ? 1u : 1u << (32 - __clz(x - 1));
+}
+
+struct PlanArgs {
+    int bits, passes, b1, F1, F2;
+    uint64_t nR, nS;
+    const uint32_t *total;  // [2][2^B]
+    uint64_t *start;        // [2][2^B + 1]
+    uint32_t *counters;
+    JoinItem *items;
+    uint64_t max_items;
+    LargePart *large;
+    uint64_t max_large;
+    uint64_t large_table_words;
+    uint64_t small_cap;  // build partitions above this many tuples are large
+    int agg_ok;  // joins that need no per-match output may use key-aggregated large-partition tables
+};
+
+__device__ __forceinline__ uint32_t part_to_value(int f, int passes, int b1, int F2) {
+    if (passes == 1) return (uint32_t)f;
+    const uint32_t d1 = (uint32_t)f / (uint32_t)F2, d2 = (uint32_t)f % (uint32_t)F2;
+    return d1 | (d2 << b1);
+}
+
+// u32 words of one large partition's table. Chains: head[nb] then next[r_len]. Key-aggregated:
+// sum[r_len] (u64), head[nb], next[r_len], cnt[r_len], negpos[r_len], rounded to an even count so the
+// next table's sums stay 8-byte aligned.
+__device__ __forceinline__ uint64_t large_words_chain(const LargePart &L) { return (1ull << L.nb_log) + L.r_len; }
+__device__ __forceinline__ uint64_t large_words_agg(const LargePart &L) {
+    return ((1ull << L.nb_log) + 5 * L.r_len + 1) & ~1ull;
+}
+
+// Final partition starts, join work items and large partitions from the relation totals tot_all
+// ([2][2^B], readable by the calling CTA of 1024 threads). tmp: 32 u32, s_run: 2 u64 of shared memory.
+__device__ __forceinline__ void plan_body(const PlanArgs &a, const uint32_t *tot_all, uint32_t *tmp, uint64_t *s_run) {
+    const int tid = threadIdx.x;
+    const int nparts = 1 << a.bits;
+    // Each thread owns a contiguous range of partitions.
+    const int per = (nparts + 1023) / 1024;
+    const int f0 = tid * per < nparts ? tid * per : nparts;
+    const int f1 = f0 + per < nparts ? f0 + per : nparts;
+    uint64_t base[2];  // start of this thread's first partition, per relation
+    for (int rel = 0; rel < 2; rel++) {
+        uint64_t *start = a.start + (size_t)rel * (nparts + 1);
+        const uint32_t *tot = tot_all + (size_t)rel * nparts;
+        uint32_t sum = 0;
+        for (int f = f0; f < f1; f++) sum += tot[part_to_value(f, a.passes, a.b1, a.F2)];
+        uint32_t all;
+        uint64_t run = block_excl_scan_u32(sum, tmp, &all);
+        base[rel] = run;
+        for (int f = f0; f < f1; f++) {
+            start[f] = run;
+            run += tot[part_to_value(f, a.passes, a.b1, a.F2)];
+        }
+        if (tid == 0) start[nparts] = all;
+    }
+
+    // Join work items (partitions with both sides non-empty, src/algo/phj.c:459-491) and large
+    // partitions. Partition sizes come from the totals, starts from the running sums above.
+    const uint32_t *totR = tot_all, *totS = tot_all + nparts;
+    const uint64_t small_cap = a.small_cap;
+    uint32_t asum = 0, bsum = 0, lsum = 0;  // items with |R_p| <= compact cap, other small items, large
+    for (int f = f0; f < f1; f++) {
+        const uint32_t v = part_to_value(f, a.passes, a.b1, a.F2);
+        const uint64_t nr = totR[v], ns = totS[v];
+        if (nr > 0 && ns > 0) {
+            if (nr <= (uint64_t)kCompactCap) asum += ceil_div_u64(ns, kProbeChunk);
+            else if (nr <= small_cap) bsum += ceil_div_u64(ns, kProbeChunk);
+            else lsum++;
+        }
+    }
+    uint32_t atot, btot, ltot;
+    uint64_t a_idx = block_excl_scan_u32(asum, tmp, &atot);
+    uint64_t b_idx = block_excl_scan_u32(bsum, tmp, &btot) + atot;
+    uint64_t large_idx = block_excl_scan_u32(lsum, tmp, &ltot);
+    const uint32_t ktot = atot + btot;
+    uint64_t rR = base[0], rS = base[1];
+    for (int f = f0; f < f1; f++) {
+        const uint32_t v = part_to_value(f, a.passes, a.b1, a.F2);
+        const uint64_t nr = totR[v], ns = totS[v];
+        const uint64_t sR = rR, sS = rS;
+        rR += nr;
+        rS += ns;
+        if (!(nr > 0 && ns > 0)) continue;
+        if (nr <= small_cap) {
+            uint64_t &item_idx = nr <= (uint64_t)kCompactCap ? a_idx : b_idx;
+            const uint32_t k = ceil_div_u64(ns, kProbeChunk);
+            for (uint32_t q = 0; q < k; q++, item_idx++) {
+                if (item_idx < a.max_items) {
+                    JoinItem it;
+                    it.r_begin = sR;
+                    it.s_begin = sS + (uint64_t)q * kProbeChunk;
+                    it.r_len = (uint32_t)nr;
+                    const uint64_t rem = ns - (uint64_t)q * kProbeChunk;
+                    it.s_len = (uint32_t)(rem < (uint64_t)kProbeChunk ? rem : (uint64_t)kProbeChunk);
+                    it.part0 = v == 0 ? 1u : 0u;
+                    it.pad = 0;
+                    a.items[item_idx] = it;
+                } else {
+                    atomicOr(&a.counters[kCtrErr], kErrCapacity);
+                }
+            }
+        } else {
+            if (large_idx < a.max_large) {
+                LargePart lp;
+                lp.r_begin = sR;
+                lp.s_begin = sS;
+                lp.r_len = nr;
+                lp.s_len = ns;
+                uint32_t nb_log = 0;
+                while ((1ull << nb_log) < nr) nb_log++;
+                lp.nb_log = nb_log;
+                lp.part0 = v == 0 ? 1u : 0u;
+                lp.table_off = 0;
+                lp.r_flat = lp.s_flat = 0;
+                a.large[large_idx] = lp;
+            } else {
+                atomicOr(&a.counters[kCtrErr], kErrCapacity);
+            }
+            large_idx++;
+        }
+    }
+    if (tid == 0) a.counters[kCtrNItemsA] = atot < a.max_items ? atot : (uint32_t)a.max_items;
+    if (tid == 0) {
+        s_run[0] = ktot;
+        s_run[1] = ltot;
+    }
+    __syncthreads();
+    const uint64_t item_run = s_run[0], large_run = s_run[1];
+    __syncthreads();
+    if (tid == 0) {
+        const uint64_t nl = large_run < a.max_large ? large_run : a.max_large;
+        // Key-aggregated tables (large_words_agg) when the join allows them and they fit the table
+        // area, else plain chains (large_words_chain).
+        uint64_t need_agg = 0;
+        for (uint64_t l = 0; l < nl; l++) need_agg += large_words_agg(a.large[l]);
+        const bool agg = a.agg_ok && need_agg <= a.large_table_words;
+        a.counters[kCtrLargeAgg] = agg ? 1u : 0u;
+        uint64_t off = 0, rf = 0, sf = 0;
+        for (uint64_t l = 0; l < nl; l++) {
+            LargePart &lp = a.large[l];
+            lp.table_off = off;
+            lp.r_flat = rf;
+            lp.s_flat = sf;
+            off += agg ? large_words_agg(lp) : large_words_chain(lp);
+            rf += lp.r_len;
+            sf += lp.s_len;
+        }
+        const bool fits = off <= a.large_table_words;
+        if (!fits) atomicOr(&a.counters[kCtrErr], kErrCapacity);
+        a.counters[kCtrNItems] = (uint32_t)(item_run < a.max_items ? item_run : a.max_items);
+        a.counters[kCtrNLarge] = (uint32_t)nl;
+        st_u64_pair(&a.counters[kCtrLargeR], fits ? rf : 0);
+        st_u64_pair(&a.counters[kCtrLargeS], fits ? sf : 0);
+        st_u64_pair(&a.counters[kCtrLargeWords], fits ? off : 0);
+    }
+}
+
+// Compact words of the probe relation in the one-pass pipeline: behind the build relation's words, or
+// behind its 16-byte elements for first-match joins.
+inline unsigned long long *single_probe_words(const PhjScratch &s, size_t nR, bool lp) {
+    return lp ? reinterpret_cast<unsigned long long *>(s.tmp1 + nR) : reinterpret_cast<unsigned long long *>(s.tmp1) + nR;
+}
+
+}  // namespace hj
