@@ -45,6 +45,7 @@ std::mutex g_default_mu;
 hj_ctx *g_default[64] = {};
 
 constexpr size_t kAccBytes = 256;
+constexpr size_t kSmallBufBytes = 256 + hj::kSmallMaxGrid * sizeof(hj::SmallPart);
 
 size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
@@ -223,6 +224,8 @@ int hj_ctx_create(int device, hj_ctx_t **out) {
     CU_OR(cudaEventCreateWithFlags(&c->ev_done, cudaEventDisableTiming), HJ_E_DEVICE);
     for (int i = 0; i <= HJ_PH_COUNT; i++) CU_OR(cudaEventCreate(&c->ev_ph[i]), HJ_E_DEVICE);
     CU_OR(cudaMallocHost(&c->acc_host, sizeof(JoinAccum)), HJ_E_OOM);
+    CU_OR(cudaMalloc(&c->small_buf, kSmallBufBytes), HJ_E_OOM);
+    CU_OR(cudaMemset(c->small_buf, 0, kSmallBufBytes), HJ_E_DEVICE);
     c->tuner.nphj_max_table_bytes = 64e6;
     c->tuner.wave_table_bytes = 64e6;
     c->tuner.partition_target = 6144;
@@ -240,6 +243,7 @@ int hj_ctx_destroy(hj_ctx_t *c) {
         drop_graphs(c);
         if (c->arena) cudaFree(c->arena);
         if (c->acc_host) cudaFreeHost(c->acc_host);
+        if (c->small_buf) cudaFree(c->small_buf);
         cudaEventDestroy(c->ev_h2d);
         cudaEventDestroy(c->ev_start);
         cudaEventDestroy(c->ev_mid);
@@ -299,8 +303,16 @@ int hj_join_ctx(hj_ctx_t *c, hj_algo_t algo, const hj_params_t *pin, const hj_tu
     std::lock_guard<std::mutex> lk(c->mu);
     const bool host_in = !p.inputs_on_device;
     size_t need = 0;
-    bool seg = want_seg(algo, p, geom, nR, nS);
-    int rc = scratch_need(algo, p, nR, nS, host_in, c->num_sms, &need, seg);
+    // Few build tuples: one kernel, without scratch.
+    const bool small = nR <= hj::kSmallMaxBuild && !(p.flags & kPipelineFlags);
+    bool seg = !small && want_seg(algo, p, geom, nR, nS);
+    int rc = HJ_OK;
+    if (small) {
+        out->physical_passes = 0;
+        if (host_in) need = kAccBytes + align256(nR * 16) + align256(nS * 16);
+    } else {
+        rc = scratch_need(algo, p, nR, nS, host_in, c->num_sms, &need, seg);
+    }
     if (rc) return out->status = rc;
     rc = ensure_arena(c, need);
     if (rc == HJ_E_OOM && seg) {  // the exact-offset pipeline needs less memory
@@ -311,7 +323,10 @@ int hj_join_ctx(hj_ctx_t *c, hj_algo_t algo, const hj_params_t *pin, const hj_tu
     if (rc) return out->status = rc;
     cudaStream_t st = p.stream ? (cudaStream_t)p.stream : c->stream;
     // A join that a watchdog gave up on may still run; its arena use must end before this one starts.
-    CU_OR(cudaStreamWaitEvent(st, c->ev_done, 0), out->status = HJ_E_DEVICE);
+    if (c->gave_up) {
+        CU_OR(cudaStreamWaitEvent(st, c->ev_done, 0), out->status = HJ_E_DEVICE);
+        c->gave_up = false;
+    }
     const bool timing = !(p.flags & HJ_F_NO_TIMING);
     const bool phases = (p.flags & HJ_F_PHASE_TIMES) != 0;
     cudaEvent_t *ph = phases ? c->ev_ph : nullptr;
@@ -341,12 +356,29 @@ int hj_join_ctx(hj_ctx_t *c, hj_algo_t algo, const hj_params_t *pin, const hj_tu
     // HJ_RES_ORDERED_PASSES for the joins that the two-pass pipelines would have run ordered.
     const bool lp_first = is_phj(algo) && hj::algo_lp(algo) && !(p.flags & (HJ_F_ORDERED | HJ_F_TEST_STALL)) &&
                           p.watchdog_ms <= 0 && !(c->lp_ordered_R == (const void *)R && c->lp_ordered_nR == nR);
-    const bool lp_try = lp_first && !geom.single;
+    const bool lp_try = lp_first && !geom.single && !small;
     const bool lp_ordered = is_phj(algo) && hj::algo_lp(algo) && !lp_first;
     bool lp_rerun = false;
     // Everything from the result reset to the result copy; a repeated device-resident join replays it
     // from a CUDA graph (the key holds every input of the enqueued work).
     auto enqueue = [&]() -> int {
+        if (small) {
+            // The build and the probe are one kernel, timed as the probe.
+            if (timing && hj::record_event(c->ev_start, st) != cudaSuccess) return HJ_E_DEVICE;
+            for (int i = 0; ph && i < HJ_PH_LARGE; i++)
+                if (hj::record_event(ph[i], st) != cudaSuccess) return HJ_E_DEVICE;
+            int erc = hj::phj_prepare_device();
+            if (!erc)
+                erc = hj::small_enqueue(hj::algo_lp(algo), hj::algo_skip0(algo), is_phj(algo) ? geom.req_bits : -1, dR,
+                                        nR, dS, nS, reinterpret_cast<hj::SmallPart *>(c->small_buf + 256),
+                                        reinterpret_cast<uint32_t *>(c->small_buf), c->acc_host, st, c->num_sms);
+            if (erc) return erc;
+            launches = 1;
+            for (int i = HJ_PH_LARGE; ph && i <= HJ_PH_COUNT; i++)
+                if (hj::record_event(ph[i], st) != cudaSuccess) return HJ_E_DEVICE;
+            if (timing && hj::record_event(c->ev_end, st) != cudaSuccess) return HJ_E_DEVICE;
+            return HJ_OK;
+        }
         if (cudaMemsetAsync(acc, 0, sizeof(JoinAccum), st) != cudaSuccess) return HJ_E_DEVICE;
         if (timing && hj::record_event(c->ev_start, st) != cudaSuccess) return HJ_E_DEVICE;
         int erc;
@@ -382,7 +414,7 @@ int hj_join_ctx(hj_ctx_t *c, hj_algo_t algo, const hj_params_t *pin, const hj_tu
         return HJ_OK;
     };
     hj_graph_key key;
-    const bool graphable = !host_in && st == c->stream && !(p.flags & HJ_F_TEST_STALL) && !lp_try;
+    const bool graphable = !host_in && st == c->stream && !(p.flags & HJ_F_TEST_STALL) && !lp_try && !small;
     if (graphable) {
         key.algo = (int)algo;
         key.R = R;
@@ -460,7 +492,10 @@ int hj_join_ctx(hj_ctx_t *c, hj_algo_t algo, const hj_params_t *pin, const hj_tu
             const cudaError_t q = cudaEventQuery(c->ev_done);
             if (q == cudaSuccess) break;
             if (q != cudaErrorNotReady) return out->status = HJ_E_DEVICE;
-            if (std::chrono::steady_clock::now() > deadline) return out->status = HJ_E_TIMEOUT;
+            if (std::chrono::steady_clock::now() > deadline) {
+                c->gave_up = true;
+                return out->status = HJ_E_TIMEOUT;
+            }
             std::this_thread::sleep_for(std::chrono::microseconds(50));
         }
     } else {
@@ -470,7 +505,7 @@ int hj_join_ctx(hj_ctx_t *c, hj_algo_t algo, const hj_params_t *pin, const hj_tu
     out->checksum = c->acc_host->checksum;
     out->large_partitions = c->acc_host->large_parts;
     out->flags = (uint32_t)c->acc_host->flags;
-    if (lp_first && geom.single) lp_rerun = c->acc_host->dup_flag != 0;
+    if (lp_first && !lp_try) lp_rerun = c->acc_host->dup_flag != 0;
     if (lp_ordered || lp_rerun) out->flags |= HJ_RES_ORDERED_PASSES;
     if (lp_rerun) {
         c->lp_ordered_R = R;
@@ -478,8 +513,8 @@ int hj_join_ctx(hj_ctx_t *c, hj_algo_t algo, const hj_params_t *pin, const hj_tu
     }
     if (timing) {
         float a = 0, b = 0, h = 0;
-        cudaEventElapsedTime(&a, c->ev_start, c->ev_mid);
-        cudaEventElapsedTime(&b, c->ev_mid, c->ev_end);
+        if (!small) cudaEventElapsedTime(&a, c->ev_start, c->ev_mid);
+        cudaEventElapsedTime(&b, small ? c->ev_start : c->ev_mid, c->ev_end);
         if (host_in) cudaEventElapsedTime(&h, c->ev_h2d, c->ev_start);
         out->buildpart = a * 1e-3;
         out->probejoin = b * 1e-3;

@@ -49,6 +49,8 @@ struct hj_ctx {
     char *arena = nullptr;
     size_t arena_bytes = 0;
     hj::JoinAccum *acc_host = nullptr;  // pinned
+    char *small_buf = nullptr;          // device: the ticket and partial results of one-kernel joins
+    bool gave_up = false;               // a watchdog gave up on a join: the next one waits for ev_done
     hj_tuner_t tuner = {};              // autotuner state used by batches
     // Joins repeated on the same device buffers: the second consecutive identical call is captured into
     // a CUDA graph, later ones replay it (one launch instead of one per kernel, copy and event).

@@ -42,6 +42,20 @@ int radix_geom(int bits, int passes, RadixGeom *g, int b1_req = 0);
 constexpr int kSingleMaxBits = 11;
 bool radix_geom_single(int bits, size_t nR, size_t nS, RadixGeom *g);
 
+// Joins of at most kSmallMaxBuild build tuples run as one kernel (hj_small.cu).
+constexpr uint32_t kSmallMaxBuild = 8192;
+constexpr int kSmallMaxGrid = 512;
+struct SmallPart {  // one CTA's partial result
+    unsigned long long cnt, sum, sor;
+    uint32_t multi, over;
+};
+int small_prepare_device();
+// flag_bits: radix bits of a radix join's HJ_RES_COMPACT_PARTITIONS test, -1 otherwise. part: kSmallMaxGrid
+// records, ticket: one zero word (zero again after the join), both device; out_host: pinned host memory,
+// filled when the kernel ends.
+int small_enqueue(bool lp, bool skip0, int flag_bits, const ulonglong2 *R, size_t nR, const ulonglong2 *S, size_t nS,
+                  SmallPart *part, uint32_t *ticket, JoinAccum *out_host, cudaStream_t st, int num_sms);
+
 // Result semantics of an algorithm: radix-partitioned or not; first match per probe tuple (lp) or
 // every match; build key 0 never matches (the phj_radix_lp empty-slot rule, src/algo/phj.c:614).
 inline bool algo_is_phj(hj_algo_t a) { return a >= HJ_ALGO_PHJ_RADIX_BC && a < HJ_ALGO_COUNT; }

@@ -2428,7 +2428,8 @@ int phj_prepare_device() {
     HJ_CU(cudaFuncSetAttribute(join_compact_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)kCompactSmem));
     {
-        const int rc = single_prepare_device();
+        int rc = single_prepare_device();
+        if (!rc) rc = small_prepare_device();
         if (rc) return rc;
     }
     g_attr_done[cur_dev] = true;

@@ -1,0 +1,232 @@
+// hj_small.cu - joins whose build relation fits one CTA's shared memory, as one kernel.
+//
+// A build relation of at most kSmallMaxBuild tuples needs neither partitions nor a global table: every
+// CTA builds the whole table in its own shared memory (from L2 after the first) and probes its share of
+// the probe relation, which is read once. The pipelines' dozen launches, memsets and copies cost such a
+// join 90-160 us, of which its data took a few. The CTA that finishes last adds up the CTAs' partial
+// results and writes them to the caller's pinned host record, so there is nothing to clear before and
+// nothing to copy after the kernel (whole calls: phj_radix_bc 1000 x 4000 158 -> 29 us).
+//
+// The table: 32-bit bucket heads, tuples and 16-bit chain links by build position (22 bytes per tuple plus
+// the heads, at most 208 KB, one CTA of 1024 threads per SM). Keys may share low bits, so buckets are
+// taken from the top of a multiplicative hash. First-match joins take the lowest position on the chain,
+// which is the first in input order. Bound by the read of the probe relation (four 16-byte loads per
+// thread in flight) when that is large, else by the latency of its four dependent steps.
+#include <cstdio>
+
+#include "hj_common.cuh"
+#include "hj_internal.h"
+#include "hj_partition.cuh"
+
+namespace hj {
+
+constexpr int kSmallThreads = 1024;
+
+struct SmallArgs {
+    const tuple_v *R, *S;
+    uint32_t nR;
+    uint64_t nS;
+    int nb_log;       // buckets
+    int lp, skip0;
+    int flag_bits;    // radix bits of the HJ_RES_COMPACT_PARTITIONS test; -1: not a radix join
+    SmallPart *part;  // [gridDim.x]
+    uint32_t *ticket; // 0 before and after every join
+    JoinAccum *out;   // pinned host memory
+};
+
+__global__ void __launch_bounds__(kSmallThreads, 1) small_join(SmallArgs a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    tuple_v *rt = reinterpret_cast<tuple_v *>(smem);                 // [nR]
+    uint32_t *head = reinterpret_cast<uint32_t *>(rt + a.nR);        // [2^nb_log]
+    uint16_t *nxt = reinterpret_cast<uint16_t *>(head + (1u << a.nb_log));  // [nR]
+    __shared__ unsigned long long s_red[5][kSmallThreads / 32];
+    __shared__ bool s_last;
+    const int tid = threadIdx.x;
+    constexpr int UR = kSmallMaxBuild / kSmallThreads, U = 4;
+    const int shift = 64 - a.nb_log;
+    constexpr unsigned long long kMul = 0x9e3779b97f4a7c15ull;
+    // The first probe tuples are requested before the build.
+    const uint64_t stride = (uint64_t)gridDim.x * kSmallThreads;
+    uint64_t j0 = (uint64_t)blockIdx.x * kSmallThreads + tid;
+    tuple_v s[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const uint64_t j = j0 + u * stride;
+        s[u] = j < a.nS ? ld_stream(a.S + j) : make_ulonglong2(0, 0);
+    }
+    tuple_v t[UR];
+#pragma unroll
+    for (int u = 0; u < UR; u++) {
+        const uint32_t i = tid + u * kSmallThreads;
+        if (i < a.nR) t[u] = __ldg(a.R + i);
+    }
+    for (uint32_t q = tid; q < (1u << a.nb_log); q += kSmallThreads) head[q] = 0;
+    __syncthreads();
+    unsigned long long kor = 0, ror = 0, sor = 0;
+#pragma unroll
+    for (int u = 0; u < UR; u++) {
+        const uint32_t i = tid + u * kSmallThreads;
+        if (i >= a.nR) break;
+        rt[i] = t[u];
+        kor |= t[u].x;
+        ror |= t[u].y;
+        if (a.skip0 && t[u].x == 0) continue;
+        nxt[i] = (uint16_t)atomicExch(&head[(t[u].x * kMul) >> shift], i + 1);
+    }
+    __syncthreads();
+    unsigned long long cnt = 0, sum = 0;
+    bool multi = false, over = false;
+    for (; j0 < a.nS; j0 += U * stride) {
+        tuple_v nx[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const uint64_t j = j0 + (U + u) * stride;
+            nx[u] = j < a.nS ? ld_stream(a.S + j) : make_ulonglong2(0, 0);
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            if (j0 + u * stride >= a.nS) continue;
+            sor |= s[u].y;
+            uint32_t e = head[(s[u].x * kMul) >> shift];
+            uint32_t best = 0, nm = 0, steps = 0;
+            while (e) {
+                const tuple_v r = rt[e - 1];
+                if (r.x == s[u].x) {
+                    if (a.lp) {
+                        if (nm++ == 0 || e < best) best = e;
+                    } else {
+                        cnt++;
+                        sum += r.y + s[u].y;
+                    }
+                }
+                e = nxt[e - 1];
+                if (++steps > a.nR) {
+                    over = true;
+                    break;
+                }
+            }
+            if (nm) {  // first match
+                cnt++;
+                sum += rt[best - 1].y + s[u].y;
+                multi |= nm > 1;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) s[u] = nx[u];
+    }
+    // This CTA's partial result: sums, ORs and flags.
+    const unsigned lane = lane_id(), w = tid >> 5;
+    cnt = warp_sum_u64(cnt);
+    sum = warp_sum_u64(sum);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        kor |= __shfl_xor_sync(0xffffffffu, kor, o);
+        ror |= __shfl_xor_sync(0xffffffffu, ror, o);
+        sor |= __shfl_xor_sync(0xffffffffu, sor, o);
+    }
+    if (lane == 0) {
+        s_red[0][w] = cnt;
+        s_red[1][w] = sum;
+        s_red[2][w] = kor;
+        s_red[3][w] = ror;
+        s_red[4][w] = sor;
+    }
+    const bool any_multi = __syncthreads_or(multi), any_over = __syncthreads_or(over);
+    if (w == 0) {
+        cnt = warp_sum_u64(s_red[0][lane]);
+        sum = warp_sum_u64(s_red[1][lane]);
+        kor = s_red[2][lane];
+        ror = s_red[3][lane];
+        sor = s_red[4][lane];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            kor |= __shfl_xor_sync(0xffffffffu, kor, o);
+            ror |= __shfl_xor_sync(0xffffffffu, ror, o);
+            sor |= __shfl_xor_sync(0xffffffffu, sor, o);
+        }
+        if (lane == 0) {
+            SmallPart p;
+            p.cnt = cnt;
+            p.sum = sum;
+            p.sor = sor;
+            p.multi = any_multi;
+            p.over = any_over;
+            a.part[blockIdx.x] = p;
+            __threadfence();
+            s_last = atomicAdd(a.ticket, 1u) == gridDim.x - 1;
+        }
+    }
+    __syncthreads();
+    if (!s_last || w != 0) return;
+    __threadfence();
+    unsigned long long tc = 0, ts = 0, to = 0;
+    bool tm = false, tv = false;
+    for (uint32_t q = lane; q < gridDim.x; q += 32) {
+        const volatile SmallPart *p = a.part + q;
+        tc += p->cnt;
+        ts += p->sum;
+        to |= p->sor;
+        tm |= p->multi != 0;
+        tv |= p->over != 0;
+    }
+    tc = warp_sum_u64(tc);
+    ts = warp_sum_u64(ts);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) to |= __shfl_xor_sync(0xffffffffu, to, o);
+    tm = __any_sync(0xffffffffu, tm);
+    tv = __any_sync(0xffffffffu, tv);
+    if (lane == 0) {
+        JoinAccum r = {};
+        r.matched = tc;
+        r.checksum = ts;
+        r.error = tv ? kErrProbeLimit : 0u;
+        r.dup_flag = tm ? 1u : 0u;
+        // Every CTA has seen the whole build relation, so kor and ror are its ORs.
+        if (a.flag_bits >= 0 && (kor >> a.flag_bits) < (1ull << 31) && ror < (1ull << 32) && to < (1ull << 32))
+            r.flags = HJ_RES_COMPACT_PARTITIONS;
+        *a.out = r;
+        *a.ticket = 0;
+    }
+}
+
+#define HJ_CU(call)                                                                   \
+    do {                                                                              \
+        cudaError_t e_ = (call);                                                      \
+        if (e_ != cudaSuccess) {                                                      \
+            fprintf(stderr, "hjscm: %s failed: %s\n", #call, cudaGetErrorString(e_)); \
+            return HJ_E_DEVICE;                                                       \
+        }                                                                             \
+    } while (0)
+
+int small_prepare_device() {
+    HJ_CU(cudaFuncSetAttribute(small_join, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               kSmallMaxBuild * (16 + 4 + 2)));
+    return HJ_OK;
+}
+
+int small_enqueue(bool lp, bool skip0, int flag_bits, const ulonglong2 *R, size_t nR, const ulonglong2 *S, size_t nS,
+                  SmallPart *part, uint32_t *ticket, JoinAccum *out_host, cudaStream_t st, int num_sms) {
+    if (nR > kSmallMaxBuild) return HJ_E_INVAL;
+    SmallArgs a;
+    a.R = R;
+    a.S = S;
+    a.nR = (uint32_t)nR;
+    a.nS = nS;
+    a.nb_log = 1;
+    while ((1u << a.nb_log) < nR) a.nb_log++;
+    a.lp = lp ? 1 : 0;
+    a.skip0 = skip0 ? 1 : 0;
+    a.flag_bits = flag_bits;
+    a.part = part;
+    a.ticket = ticket;
+    a.out = out_host;
+    const uint64_t want = ((uint64_t)nS + kSmallThreads - 1) / kSmallThreads;
+    const uint64_t sms = (uint64_t)(num_sms < kSmallMaxGrid ? num_sms : kSmallMaxGrid);
+    const unsigned grid = (unsigned)(want < 1 ? 1 : want < sms ? want : sms);
+    const size_t smem = nR * 16 + ((size_t)4 << a.nb_log) + nR * 2;
+    small_join<<<grid, kSmallThreads, smem, st>>>(a);
+    HJ_CU(cudaGetLastError());
+    return HJ_OK;
+}
+
+}  // namespace hj
