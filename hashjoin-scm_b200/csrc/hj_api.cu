@@ -61,7 +61,7 @@ bool is_phj(hj_algo_t a) { return hj::algo_is_phj(a); }
 
 // Segment mode for a radix join (see HJ_F_SEGMENTS): by size unless a flag decides.
 bool want_seg(hj_algo_t algo, const hj_params_t &p, const hj::RadixGeom &g, size_t nR, size_t nS) {
-    if (!is_phj(algo) || (p.flags & HJ_F_EXACT) || g.single) return false;
+    if ((p.flags & HJ_F_EXACT) || g.single) return false;
     if (p.flags & HJ_F_SEGMENTS) return hj::phj_seg_applies(g, hj::algo_lp(algo), 1ull << 40, 0);
     return hj::phj_seg_applies(g, hj::algo_lp(algo), nR, nS);
 }
@@ -71,27 +71,59 @@ constexpr uint32_t kPipelineFlags = HJ_F_SEGMENTS | HJ_F_EXACT | HJ_F_WIDE | HJ_
 
 // The geometry of a radix join: the one-pass pipeline where the build relation needs few partitions,
 // unless the flags name another, else as asked.
-int join_geom(const hj_params_t &p, size_t nR, size_t nS, hj::RadixGeom *g) {
+int join_geom(hj_algo_t algo, const hj_params_t &p, size_t nR, size_t nS, hj::RadixGeom *g) {
     const int rc = hj::radix_geom(p.num_radix_bits, p.num_passes, g, p.radix_bits_pass1);
     if (rc) return rc;
-    if (!(p.flags & kPipelineFlags)) hj::radix_geom_single(p.num_radix_bits, nR, nS, g);
+    if (!(p.flags & kPipelineFlags)) hj::radix_geom_single(p.num_radix_bits, hj::algo_lp(algo), nR, nS, g);
     return HJ_OK;
 }
 
-int scratch_need(hj_algo_t algo, const hj_params_t &p, size_t nR, size_t nS, bool host_inputs, int num_sms,
-                 size_t *bytes, bool seg) {
+// Non-partitioned joins of these sizes run a radix pipeline (14 bits, or the one-pass geometry): what a
+// join reports does not depend on how it was computed, and beyond L2 partitioning both sides beats one
+// random table access per tuple (unique keys, device time: nphj_sc 2^22 x 2^23 191 us against 230 by the
+// table, 2^24 x 2^24 575 against 968, 2^26 x 2^28 4.6 ms against 10.7; nphj_lp 2^24 x 2^26 with four
+// duplicates a key 1.5 against 1.8 ms). Below kNphjRadixMinBuild the 16-byte table sits in L2 and is as fast
+// (2^18 x 2^20: both 53 us; 20000 x 20000: 43 against 35), and up to kNphjTableBuild the compact one does,
+// which wins from about five probe tuples a build tuple (2^22 x 2^26: 892 against 745 us). A load factor
+// asks for the table itself; build partitions above 6144 tuples on average, and scratch that cannot be had,
+// take it too.
+constexpr size_t kNphjRadixMinBuild = 1u << 21, kNphjTableBuild = 5000000, kNphjRadixMaxBuild = (size_t)6144 << 14;
+bool nphj_by_radix(const hj_params_t &p, size_t nR, size_t nS) {
+    if (p.table_load > 0.0 || nR < kNphjRadixMinBuild || nR > kNphjRadixMaxBuild || nS >= (1ull << 32)) return false;
+    return nR > kNphjTableBuild || nS <= 5 * nR;
+}
+
+// How a join runs: by a radix pipeline (radix, geom, seg) or on the non-partitioned table.
+struct JoinPlan {
+    bool radix = false, seg = false;
+    hj::RadixGeom geom = {};
+};
+
+int plan_join(hj_algo_t algo, hj_params_t *p, size_t nR, size_t nS, JoinPlan *jp) {
+    *jp = JoinPlan();
+    if (is_phj(algo)) {
+        const int rc = join_geom(algo, *p, nR, nS, &jp->geom);
+        if (rc) return rc;
+    } else if (nphj_by_radix(*p, nR, nS)) {
+        p->flags &= ~(kPipelineFlags | HJ_F_ORDERED);  // radix joins' flags
+        hj::radix_geom(14, 2, &jp->geom);
+        hj::radix_geom_single(14, hj::algo_lp(algo), nR, nS, &jp->geom);
+    } else {
+        return HJ_OK;
+    }
+    jp->radix = true;
+    jp->seg = want_seg(algo, *p, jp->geom, nR, nS);
+    return HJ_OK;
+}
+
+size_t scratch_need(const JoinPlan &jp, const hj_params_t &p, size_t nR, size_t nS, bool host_inputs, int num_sms) {
     size_t need = kAccBytes;
     if (host_inputs) need += align256(nR * 16) + align256(nS * 16);
-    if (is_phj(algo)) {
-        hj::RadixGeom g;
-        int rc = join_geom(p, nR, nS, &g);
-        if (rc) return rc;
-        need += hj::phj_scratch_bytes(g, nR, nS, num_sms, seg);
-    } else {
+    if (jp.radix)
+        need += hj::phj_scratch_bytes(jp.geom, nR, nS, num_sms, jp.seg);
+    else
         need += align256(hj::nphj_scratch_bytes(nR, p.table_load));
-    }
-    *bytes = need;
-    return HJ_OK;
+    return need;
 }
 
 // Drop the context's join graphs (they address the arena).
@@ -127,6 +159,21 @@ int ensure_arena(hj_ctx *c, size_t bytes) {
     }
     c->arena_bytes = bytes;
     return HJ_OK;
+}
+
+// Scratch for the plan; one that cannot be had falls back to a plan that needs less (segment mode to the
+// exact-offset pipeline, a non-partitioned join's radix pipeline to the table).
+int ensure_plan(hj_ctx *c, hj_algo_t algo, const hj_params_t &p, size_t nR, size_t nS, bool host_inputs, JoinPlan *jp) {
+    int rc = ensure_arena(c, scratch_need(*jp, p, nR, nS, host_inputs, c->num_sms));
+    if (rc == HJ_E_OOM && jp->seg) {
+        jp->seg = false;
+        rc = ensure_arena(c, scratch_need(*jp, p, nR, nS, host_inputs, c->num_sms));
+    }
+    if (rc == HJ_E_OOM && jp->radix && !is_phj(algo)) {
+        *jp = JoinPlan();
+        rc = ensure_arena(c, scratch_need(*jp, p, nR, nS, host_inputs, c->num_sms));
+    }
+    return rc;
 }
 
 int map_error_bits(unsigned bits) {
@@ -263,24 +310,12 @@ int hj_ctx_reserve(hj_ctx_t *c, hj_algo_t algo, const hj_params_t *pin, size_t n
     if (!c || (int)algo < 0 || algo >= HJ_ALGO_COUNT) return HJ_E_INVAL;
     hj_params_t p;
     resolve_params(pin, &p);
-    size_t need = 0;
-    bool seg = false;
-    if (is_phj(algo)) {
-        hj::RadixGeom geom;
-        const int rc = join_geom(p, nR, nS, &geom);
-        if (rc) return rc;
-        seg = want_seg(algo, p, geom, nR, nS);
-    }
-    int rc = scratch_need(algo, p, nR, nS, !p.inputs_on_device, c->num_sms, &need, seg);
+    JoinPlan jp;
+    const int rc = plan_join(algo, &p, nR, nS, &jp);
     if (rc) return rc;
     DeviceGuard g(c->device);
     std::lock_guard<std::mutex> lk(c->mu);
-    rc = ensure_arena(c, need);
-    if (rc == HJ_E_OOM && seg) {
-        rc = scratch_need(algo, p, nR, nS, !p.inputs_on_device, c->num_sms, &need, false);
-        if (!rc) rc = ensure_arena(c, need);
-    }
-    return rc;
+    return ensure_plan(c, algo, p, nR, nS, !p.inputs_on_device, &jp);
 }
 
 int hj_join_ctx(hj_ctx_t *c, hj_algo_t algo, const hj_params_t *pin, const hj_tuple_t *R, size_t nR,
@@ -291,36 +326,26 @@ int hj_join_ctx(hj_ctx_t *c, hj_algo_t algo, const hj_params_t *pin, const hj_tu
     hj_params_t p;
     resolve_params(pin, &p);
     if (p.device != c->device) return out->status = HJ_E_INVAL;
-    hj::RadixGeom geom = {};
-    if (is_phj(algo)) {
-        int rc = join_geom(p, nR, nS, &geom);
-        if (rc) return out->status = rc;
-        out->physical_passes = geom.passes;
-    }
+    JoinPlan jp;
+    int rc = plan_join(algo, &p, nR, nS, &jp);
+    if (rc) return out->status = rc;
+    if (is_phj(algo)) out->physical_passes = jp.geom.passes;
     if (nR == 0 || nS == 0) return out->status = HJ_OK;  // no join task (src/algo/phj.c:1290)
 
     DeviceGuard g(c->device);
     std::lock_guard<std::mutex> lk(c->mu);
     const bool host_in = !p.inputs_on_device;
-    size_t need = 0;
     // Few build tuples: one kernel, without scratch.
     const bool small = nR <= hj::kSmallMaxBuild && !(p.flags & kPipelineFlags);
-    bool seg = !small && want_seg(algo, p, geom, nR, nS);
-    int rc = HJ_OK;
     if (small) {
         out->physical_passes = 0;
-        if (host_in) need = kAccBytes + align256(nR * 16) + align256(nS * 16);
+        if (host_in) rc = ensure_arena(c, kAccBytes + align256(nR * 16) + align256(nS * 16));
     } else {
-        rc = scratch_need(algo, p, nR, nS, host_in, c->num_sms, &need, seg);
+        rc = ensure_plan(c, algo, p, nR, nS, host_in, &jp);
     }
     if (rc) return out->status = rc;
-    rc = ensure_arena(c, need);
-    if (rc == HJ_E_OOM && seg) {  // the exact-offset pipeline needs less memory
-        seg = false;
-        rc = scratch_need(algo, p, nR, nS, host_in, c->num_sms, &need, false);
-        if (!rc) rc = ensure_arena(c, need);
-    }
-    if (rc) return out->status = rc;
+    const bool radix = jp.radix, seg = jp.seg && !small;
+    const hj::RadixGeom &geom = jp.geom;
     cudaStream_t st = p.stream ? (cudaStream_t)p.stream : c->stream;
     // A join that a watchdog gave up on may still run; its arena use must end before this one starts.
     if (c->gave_up) {
@@ -354,11 +379,16 @@ int hj_join_ctx(hj_ctx_t *c, hj_algo_t algo, const hj_params_t *pin, const hj_tu
     // are not captured into a graph; a build relation that needed it runs ordered at once next time.
     // The one-pass pipeline needs neither: its build elements carry their input position. It reports
     // HJ_RES_ORDERED_PASSES for the joins that the two-pass pipelines would have run ordered.
-    const bool lp_first = is_phj(algo) && hj::algo_lp(algo) && !(p.flags & (HJ_F_ORDERED | HJ_F_TEST_STALL)) &&
+    // A non-partitioned join in two passes runs ordered at once: it must not pay for two runs where the table
+    // would have been one.
+    const bool lp_first = radix && hj::algo_lp(algo) && (is_phj(algo) || geom.single) && !(p.flags & (HJ_F_ORDERED | HJ_F_TEST_STALL)) &&
                           p.watchdog_ms <= 0 && !(c->lp_ordered_R == (const void *)R && c->lp_ordered_nR == nR);
     const bool lp_try = lp_first && !geom.single && !small;
-    const bool lp_ordered = is_phj(algo) && hj::algo_lp(algo) && !lp_first;
+    const bool lp_ordered = radix && hj::algo_lp(algo) && !lp_first;
     bool lp_rerun = false;
+    // The one-pass pipeline writes its result to acc_host itself and leaves large partitions, if any, to a
+    // second step below (a watchdog's deadline covers one step only, so such a join has none).
+    const bool one_pass = radix && geom.single && !small && p.watchdog_ms <= 0;
     // Everything from the result reset to the result copy; a repeated device-resident join replays it
     // from a CUDA graph (the key holds every input of the enqueued work).
     auto enqueue = [&]() -> int {
@@ -379,10 +409,10 @@ int hj_join_ctx(hj_ctx_t *c, hj_algo_t algo, const hj_params_t *pin, const hj_tu
             if (timing && hj::record_event(c->ev_end, st) != cudaSuccess) return HJ_E_DEVICE;
             return HJ_OK;
         }
-        if (cudaMemsetAsync(acc, 0, sizeof(JoinAccum), st) != cudaSuccess) return HJ_E_DEVICE;
+        if (!one_pass && cudaMemsetAsync(acc, 0, sizeof(JoinAccum), st) != cudaSuccess) return HJ_E_DEVICE;
         if (timing && hj::record_event(c->ev_start, st) != cudaSuccess) return HJ_E_DEVICE;
         int erc;
-        if (is_phj(algo)) {
+        if (radix) {
             hj::PhjScratch s;
             hj::phj_carve(geom, nR, nS, c->num_sms, cur, &s, seg);
             const int tf = ((p.flags & HJ_F_TEST_STALL) ? 1 : 0) | ((p.flags & HJ_F_WIDE) ? 2 : 0) |
@@ -400,7 +430,8 @@ int hj_join_ctx(hj_ctx_t *c, hj_algo_t algo, const hj_params_t *pin, const hj_tu
             }
             if (!lp_try || lp_rerun)
                 erc = hj::phj_enqueue(geom, hj::algo_lp(algo), hj::algo_skip0(algo), dR, nR, dS, nS, s, acc, st,
-                                      timing ? c->ev_mid : nullptr, c->num_sms, ph, &launches, nullptr, tf);
+                                      timing ? c->ev_mid : nullptr, c->num_sms, ph, &launches, nullptr, tf, true,
+                                      one_pass ? c->acc_host : nullptr);
             launches += first;
         } else {
             const size_t tb = c->arena_bytes - (size_t)(cur - c->arena);
@@ -409,6 +440,7 @@ int hj_join_ctx(hj_ctx_t *c, hj_algo_t algo, const hj_params_t *pin, const hj_tu
         }
         if (erc) return erc;
         if (timing && hj::record_event(c->ev_end, st) != cudaSuccess) return HJ_E_DEVICE;
+        if (one_pass) return HJ_OK;  // its last kernel writes the result to acc_host
         if (cudaMemcpyAsync(c->acc_host, acc, sizeof(JoinAccum), cudaMemcpyDeviceToHost, st) != cudaSuccess)
             return HJ_E_DEVICE;
         return HJ_OK;
@@ -501,12 +533,31 @@ int hj_join_ctx(hj_ctx_t *c, hj_algo_t algo, const hj_params_t *pin, const hj_tu
     } else {
         CU_OR(cudaStreamSynchronize(st), out->status = HJ_E_DEVICE);
     }
-    out->matched_cnt = c->acc_host->matched;
-    out->checksum = c->acc_host->checksum;
-    out->large_partitions = c->acc_host->large_parts;
-    out->flags = (uint32_t)c->acc_host->flags;
-    if (lp_first && !lp_try) lp_rerun = c->acc_host->dup_flag != 0;
-    if (lp_ordered || lp_rerun) out->flags |= HJ_RES_ORDERED_PASSES;
+    JoinAccum res = *c->acc_host;
+    if (one_pass && res.large_parts) {
+        // Partitions beyond shared memory (rare: a hot build key, or keys that share their low bits) are
+        // joined by a second batch of kernels, launched only now that there are some.
+        hj::PhjScratch s;
+        hj::phj_carve(geom, nR, nS, c->num_sms, cur, &s, false);
+        rc = hj::phj_large_enqueue(geom, hj::algo_lp(algo), hj::algo_skip0(algo), dR, nR, nS, s, acc, st, c->num_sms,
+                                   &launches);
+        if (rc) return out->status = rc;
+        if (phases) CU_OR(cudaEventRecord(c->ev_ph[HJ_PH_COUNT], st), out->status = HJ_E_DEVICE);
+        if (timing) CU_OR(cudaEventRecord(c->ev_end, st), out->status = HJ_E_DEVICE);
+        CU_OR(cudaMemcpyAsync(c->acc_host, acc, sizeof(JoinAccum), cudaMemcpyDeviceToHost, st),
+              out->status = HJ_E_DEVICE);
+        CU_OR(cudaStreamSynchronize(st), out->status = HJ_E_DEVICE);
+        res.matched += c->acc_host->matched;
+        res.checksum += c->acc_host->checksum;
+        res.error |= c->acc_host->error;
+        res.dup_flag |= c->acc_host->dup_flag;
+    }
+    out->matched_cnt = res.matched;
+    out->checksum = res.checksum;
+    out->large_partitions = is_phj(algo) ? res.large_parts : 0;
+    out->flags = is_phj(algo) ? (uint32_t)res.flags : 0u;
+    if (lp_first && !lp_try) lp_rerun = res.dup_flag != 0;
+    if (is_phj(algo) && (lp_ordered || lp_rerun)) out->flags |= HJ_RES_ORDERED_PASSES;
     if (lp_rerun) {
         c->lp_ordered_R = R;
         c->lp_ordered_nR = nR;
@@ -525,12 +576,19 @@ int hj_join_ctx(hj_ctx_t *c, hj_algo_t algo, const hj_params_t *pin, const hj_tu
         for (int i = 0; i < HJ_PH_COUNT; i++) {
             float ms = 0;
             int from = 0, to = 0;
-            if (hj::phj_phase_span(seg, i, &from, &to)) cudaEventElapsedTime(&ms, c->ev_ph[from], c->ev_ph[to]);
+            if (!is_phj(algo) && radix) {
+                // Non-partitioned joins report a build and a probe phase: partitioning and the joins.
+                from = i == HJ_PH_JOIN ? (seg ? 3 : 4) : 0;
+                to = i == HJ_PH_JOIN ? (seg ? 5 : 6) : (seg ? 3 : 4);
+                if (i == HJ_PH_HIST || i == HJ_PH_JOIN) cudaEventElapsedTime(&ms, c->ev_ph[from], c->ev_ph[to]);
+            } else if (hj::phj_phase_span(seg, i, &from, &to)) {
+                cudaEventElapsedTime(&ms, c->ev_ph[from], c->ev_ph[to]);
+            }
             out->phase[i] = ms * 1e-3;
         }
     }
     out->kernel_launches = launches;
-    out->status = map_error_bits(c->acc_host->error);
+    out->status = map_error_bits(res.error);
     return out->status;
 }
 
@@ -542,7 +600,7 @@ static int join_mat(hj_ctx *c, hj_algo_t algo, const hj_params_t &p, const hj_tu
                     unsigned long long cap_guess, hj_result_t *out) {
     hj::RadixGeom geom = {};
     if (is_phj(algo)) {
-        int rc = join_geom(p, nR, nS, &geom);
+        int rc = join_geom(algo, p, nR, nS, &geom);
         if (rc) return out->status = rc;
         out->physical_passes = geom.passes;
     }

@@ -40,7 +40,7 @@ int radix_geom(int bits, int passes, RadixGeom *g, int b1_req = 0);
 // The one-pass pipeline's geometry for a build relation of nR tuples and `bits` requested radix bits:
 // false when the two-pass pipelines should run.
 constexpr int kSingleMaxBits = 11;
-bool radix_geom_single(int bits, size_t nR, size_t nS, RadixGeom *g);
+bool radix_geom_single(int bits, bool lp, size_t nR, size_t nS, RadixGeom *g);
 
 // Joins of at most kSmallMaxBuild build tuples run as one kernel (hj_small.cu).
 constexpr uint32_t kSmallMaxBuild = 8192;
@@ -140,15 +140,22 @@ void phj_carve(const RadixGeom &g, size_t nR, size_t nS, int num_sms, char *base
 int phj_enqueue(const RadixGeom &g, bool lp, bool skip0, const ulonglong2 *R, size_t nR, const ulonglong2 *S,
                 size_t nS, const PhjScratch &s, JoinAccum *acc, cudaStream_t st, cudaEvent_t ev_mid,
                 int num_sms, cudaEvent_t *ph, uint32_t *launches, const MatOut *mat = nullptr,
-                int test_flags = 0, bool ordered = true);
+                int test_flags = 0, bool ordered = true, JoinAccum *host_out = nullptr);
+
+// A one-pass join (g.single, not materialising) given host_out, pinned host memory: the call clears *acc, and
+// the last kernel writes the result there, except that partitions too large for shared memory are left
+// out (host_out->large_parts tells how many). The caller then runs them with phj_large_enqueue, which adds
+// to *acc (their part of the result only).
+int phj_large_enqueue(const RadixGeom &g, bool lp, bool skip0, const ulonglong2 *R, size_t nR, size_t nS,
+                      const PhjScratch &s, JoinAccum *acc, cudaStream_t st, int num_sms, uint32_t *launches);
 
 // The partition phase of the one-pass pipeline (g.single): count, plan, scatter into s.tmp1. lp: build
-// elements carry their input position. Records ph[1..4].
+// elements carry their input position. Clears s.counters, and *acc if clear_acc. Records ph[1..4].
 int single_prepare_device();
 uint32_t single_grid(size_t nR, size_t nS, int num_sms);
 int single_partition_enqueue(const RadixGeom &g, bool lp, bool skip0, bool ci_ok, const ulonglong2 *R, size_t nR,
-                             const ulonglong2 *S, size_t nS, const PhjScratch &s, cudaStream_t st, bool agg_ok,
-                             cudaEvent_t *ph, uint32_t *launches);
+                             const ulonglong2 *S, size_t nS, const PhjScratch &s, JoinAccum *acc, bool clear_acc,
+                             cudaStream_t st, bool agg_ok, cudaEvent_t *ph, uint32_t *launches);
 
 // The events of phase slot i (HJ_PH_*) that phj_enqueue recorded: elapsed(ph[*from], ph[*to]);
 // false for a slot that the mode does not time (segment mode has no histogram pass).

@@ -1384,6 +1384,9 @@ struct JoinArgs {
     const tuple_v *relR;
     uint64_t nR;
     int flag_bits;  // HJ_RES_COMPACT_PARTITIONS tells whether words of this many radix bits fit
+    // One-pass pipeline: one launch takes the items of every size; host_out: see join_finish.
+    int all_items;
+    JoinAccum *host_out;
     int w8_b1;  // a pass 1 that may store words (either pipeline): its shift (reported when w8_fits held); -1 otherwise
 };
 
@@ -1589,17 +1592,305 @@ __global__ void __launch_bounds__(kCompactThreads, 2) join_compact_kernel(JoinAr
     if (LP && !MAT) flag_multi(multi, &a.acc->dup_flag);
 }
 
-// First-match join of the one-pass pipeline. Build elements come with their input position, and the match
-// with the lowest one wins, so the partition may hold them in any order. Key, position and row id in
+// End of the one-pass pipeline's partition join, called by every thread of every CTA after it has added its
+// sums to *a.acc. With host_out, the CTA that finishes last writes the join's result there (pinned host
+// memory), so that nothing has to be copied or launched after the join unless there are large partitions.
+__device__ __forceinline__ void join_finish(const JoinArgs &a, bool ci) {
+    if (!a.host_out || threadIdx.x != 0) return;
+    __threadfence();
+    if (atomicAdd(&a.counters[kCtrTicketJoin], 1u) != gridDim.x - 1) return;
+    __threadfence();
+    const volatile JoinAccum *acc = a.acc;
+    JoinAccum r = {};
+    r.matched = acc->matched;
+    r.checksum = acc->checksum;
+    r.error = acc->error | *reinterpret_cast<const volatile uint32_t *>(&a.counters[kCtrErr]);
+    r.dup_flag = acc->dup_flag;
+    r.large_parts = a.counters[kCtrNLarge];
+    if (a.ci && ci_applies(a.counters, a.flag_bits)) r.flags = HJ_RES_COMPACT_PARTITIONS;
+    *a.host_out = r;
+    // Large partitions add to the result after this: start them from zero.
+    a.acc->matched = a.acc->checksum = 0;
+    a.acc->dup_flag = a.acc->error = 0;
+}
+
+// Partition join over compact words in an open-addressing table of the words themselves (every match
+// counted): two CTAs of 512 threads per SM with 13312 slots each. A probe is one 8-byte shared load when its
+// key sits in its first slot and the build saw no key twice, where a chain costs a head, a word and a link.
+// Slots come from the high product of a multiplicative hash, so the table takes any size: twice the build
+// partition (less for the largest, 10240 tuples). Equal keys sit in a row; a build that walks more than
+// kOaMaxSteps slots (a key repeated often) is done again with chains in the same memory.
+constexpr uint32_t kOaSlots = 13312, kOaMaxSteps = 64, kOaHeads = 2048;
+constexpr size_t kOaSmem = (size_t)kOaSlots * 8;
+static_assert(kOaSmem >= (size_t)kSmemCap * 10 + kOaHeads * 2, "the chains fit the same memory");
+
+__device__ __forceinline__ uint32_t oa_hash(uint32_t hi) { return hi * 0x9e3779b1u; }
+
+__global__ void __launch_bounds__(kCompactThreads, 2) join_words_kernel(JoinArgs a) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    unsigned long long *slots = reinterpret_cast<unsigned long long *>(smem);
+    __shared__ unsigned long long red[64];
+    __shared__ uint32_t s_item, s_flags;  // s_flags: 1 a key occurs twice, 2 a walk was too long
+    if (!(a.ci && ci_applies(a.counters, a.bits))) return;
+    const int tid = threadIdx.x;
+    constexpr int NT = kCompactThreads, UR = 4, U = 8;
+    constexpr unsigned long long kNone = ~0ull;  // no build word has this high part
+    unsigned int *err = &a.counters[kCtrErr];
+    const uint32_t nitems = a.counters[kCtrNItems];
+    unsigned long long cnt = 0, sum = 0;
+    for (;;) {
+        if (tid == 0) {
+            s_item = atomicAdd(&a.counters[kCtrItemA], 1u);
+            s_flags = 0;
+        }
+        __syncthreads();
+        const uint32_t it = s_item;
+        if (it >= nitems) break;
+        const JoinItem item = a.items[it];
+        const uint32_t nr = item.r_len, ns = item.s_len;
+        const unsigned long long *R8 = a.finR8 + item.r_begin, *S8 = a.finS8 + item.s_begin;
+        const uint32_t nslots = min(kOaSlots, (2 * nr + 511u) & ~511u);
+        unsigned long long r[UR], s[U];
+#pragma unroll
+        for (int u = 0; u < UR; u++) r[u] = tid + u * NT < nr ? ld_stream8(R8 + tid + u * NT) : kNone;
+        for (uint32_t q = tid; q < nslots / 2; q += NT) reinterpret_cast<ulonglong2 *>(slots)[q] = make_ulonglong2(kNone, kNone);
+        __syncthreads();
+        uint32_t fl = 0;
+        for (uint32_t i0 = tid; i0 < nr; i0 += UR * NT) {
+            unsigned long long nx[UR];
+#pragma unroll
+            for (int u = 0; u < UR; u++) {
+                const uint32_t i = i0 + (UR + u) * NT;
+                nx[u] = i < nr ? ld_stream8(R8 + i) : kNone;
+            }
+#pragma unroll
+            for (int u = 0; u < UR; u++) {
+                if (r[u] == kNone) continue;
+                const uint32_t hi = (uint32_t)(r[u] >> 32);
+                uint32_t h = __umulhi(oa_hash(hi), nslots);
+                for (uint32_t steps = 0;;) {
+                    const unsigned long long cur = atomicCAS(&slots[h], kNone, r[u]);
+                    if (cur == kNone) break;
+                    if ((uint32_t)(cur >> 32) == hi) fl |= 1u;
+                    if (++h == nslots) h = 0;
+                    if (++steps >= kOaMaxSteps) {
+                        fl |= 2u;
+                        break;
+                    }
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < UR; u++) r[u] = nx[u];
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) s[u] = tid + u * NT < ns ? ld_stream8(S8 + tid + u * NT) : kNone;
+        if (fl) atomicOr(&s_flags, fl);
+        __syncthreads();
+        const bool dups = s_flags != 0;
+        if (s_flags & 2u) {
+            // Chains: words, links by position, bucket heads.
+            uint16_t *nxt = reinterpret_cast<uint16_t *>(slots + kSmemCap), *head = nxt + kSmemCap;
+            uint32_t *head32 = reinterpret_cast<uint32_t *>(head);
+            for (uint32_t q = tid; q < kOaHeads / 2; q += NT) head32[q] = 0;
+            __syncthreads();
+            for (uint32_t i = tid; i < nr; i += NT) {
+                const unsigned long long w = R8[i];
+                slots[i] = w;
+                nxt[i] = (uint16_t)atomic_exch_u16(&head[oa_hash((uint32_t)(w >> 32)) >> 21], i + 1);
+            }
+            __syncthreads();
+            for (uint32_t j = tid; j < ns; j += NT) {
+                const unsigned long long w = ld_stream8(S8 + j);
+                const uint32_t hi = (uint32_t)(w >> 32);
+                uint32_t steps = 0;
+                for (uint32_t e = head[oa_hash(hi) >> 21]; e; e = nxt[e - 1]) {
+                    const unsigned long long b = slots[e - 1];
+                    if ((uint32_t)(b >> 32) == hi) {
+                        cnt++;
+                        sum += (b & 0xffffffffull) + (w & 0xffffffffull);
+                    }
+                    if (++steps > nr) {
+                        set_error(err, kErrProbeLimit);
+                        break;
+                    }
+                }
+            }
+            __syncthreads();
+            continue;
+        }
+        for (uint32_t j0 = tid; j0 < ns; j0 += U * NT) {
+            unsigned long long nx[U], e[U];
+            uint32_t h[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const uint32_t j = j0 + (U + u) * NT;
+                nx[u] = j < ns ? ld_stream8(S8 + j) : kNone;
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                h[u] = __umulhi(oa_hash((uint32_t)(s[u] >> 32)), nslots);
+                e[u] = slots[h[u]];
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const uint32_t hi = (uint32_t)(s[u] >> 32);
+                // A word past the end (kNone), as a probe key beyond every build key, matches nothing.
+                for (uint32_t steps = 0; e[u] != kNone;) {
+                    if ((uint32_t)(e[u] >> 32) == hi) {
+                        cnt++;
+                        sum += (e[u] & 0xffffffffull) + (s[u] & 0xffffffffull);
+                        if (!dups) break;
+                    }
+                    if (++h[u] == nslots) h[u] = 0;
+                    if (++steps >= nslots) {
+                        set_error(err, kErrProbeLimit);
+                        break;
+                    }
+                    e[u] = slots[h[u]];
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) s[u] = nx[u];
+        }
+        __syncthreads();
+    }
+    block_sum2_to(cnt, sum, red, &a.acc->matched, &a.acc->checksum);
+    join_finish(a, true);
+}
+
+// First-match join over {compact word, position} elements in an open-addressing table: a slot holds (key
+// high part << 32 | position), equal keys share a slot and lower its position, and the row ids of the winners
+// stand beside the slots. Equal keys never lengthen a walk. A bitmap marks the slots that two build tuples
+// share: a probe that matches one sets acc->dup_flag (see flag_multi). One CTA of 1024 threads per SM, 194 KB;
+// a thread keeps its build tuples in registers from the insert to the row-id store.
+constexpr uint32_t kFwSlots = 16384;
+constexpr size_t kFwSmem = (size_t)kFwSlots * 12 + kFwSlots / 8;
+
+__global__ void __launch_bounds__(kJoinThreads, 1) join_first_words_kernel(JoinArgs a) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    unsigned long long *slots = reinterpret_cast<unsigned long long *>(smem);  // [kFwSlots]
+    uint32_t *rid = reinterpret_cast<uint32_t *>(slots + kFwSlots);             // [kFwSlots]
+    uint32_t *dup = rid + kFwSlots;                                             // [kFwSlots / 32]
+    __shared__ unsigned long long red[64];
+    __shared__ uint32_t s_item, s_dups;
+    if (!(a.ci && ci_applies(a.counters, a.bits))) return;
+    const uint32_t tid = threadIdx.x;
+    constexpr int NT = kJoinThreads, UR = kFirstCap / NT, U = 8;
+    static_assert(UR * NT == kFirstCap, "a thread's build tuples");
+    constexpr unsigned long long kNone = ~0ull;  // no build element has this high part
+    unsigned int *err = &a.counters[kCtrErr];
+    const uint32_t nitems = a.counters[kCtrNItems];
+    unsigned long long cnt = 0, sum = 0;
+    bool multi = false;
+    for (;;) {
+        if (tid == 0) {
+            s_item = atomicAdd(&a.counters[kCtrItemA], 1u);
+            s_dups = 0;
+        }
+        __syncthreads();
+        const uint32_t it = s_item;
+        if (it >= nitems) break;
+        const JoinItem item = a.items[it];
+        const uint32_t nr = item.r_len, ns = item.s_len;
+        const tuple_v *R = a.finR + item.r_begin;
+        const unsigned long long *S8 = a.finS8 + item.s_begin;
+        const uint32_t nslots = min(kFwSlots, (2 * nr + 511u) & ~511u);
+        tuple_v r[UR];
+#pragma unroll
+        for (int u = 0; u < UR; u++)
+            r[u] = tid + u * NT < nr ? ld_stream(R + tid + u * NT) : make_ulonglong2(kNone, 0);
+        for (uint32_t q = tid; q < nslots / 2; q += NT) reinterpret_cast<ulonglong2 *>(slots)[q] = make_ulonglong2(kNone, kNone);
+        for (uint32_t q = tid; q < nslots / 32; q += NT) dup[q] = 0;
+        __syncthreads();
+        uint32_t at[UR];
+        bool any_dup = false;
+#pragma unroll
+        for (int u = 0; u < UR; u++) {
+            at[u] = ~0u;
+            if (r[u].x == kNone) continue;
+            const uint32_t hi = (uint32_t)(r[u].x >> 32);
+            const unsigned long long v = ((unsigned long long)hi << 32) | (uint32_t)r[u].y;
+            uint32_t h = __umulhi(oa_hash(hi), nslots);
+            for (uint32_t steps = 0;;) {
+                const unsigned long long cur = atomicCAS(&slots[h], kNone, v);
+                if (cur == kNone) break;
+                if ((uint32_t)(cur >> 32) == hi) {
+                    atomicMin(&slots[h], v);
+                    atomicOr(&dup[h >> 5], 1u << (h & 31));
+                    any_dup = true;
+                    break;
+                }
+                if (++h == nslots) h = 0;
+                if (++steps >= nslots) {
+                    set_error(err, kErrProbeLimit);
+                    break;
+                }
+            }
+            at[u] = h;
+        }
+        unsigned long long s[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) s[u] = tid + u * NT < ns ? ld_stream8(S8 + tid + u * NT) : kNone;
+        if (any_dup) s_dups = 1u;
+        __syncthreads();
+        // The tuple whose position won its slot stores its row id there.
+#pragma unroll
+        for (int u = 0; u < UR; u++)
+            if (at[u] != ~0u && (uint32_t)slots[at[u]] == (uint32_t)r[u].y) rid[at[u]] = (uint32_t)r[u].x;
+        const bool dups = s_dups != 0;
+        __syncthreads();
+        for (uint32_t j0 = tid; j0 < ns; j0 += U * NT) {
+            unsigned long long nx[U], e[U];
+            uint32_t h[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const uint32_t j = j0 + (U + u) * NT;
+                nx[u] = j < ns ? ld_stream8(S8 + j) : kNone;
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                h[u] = __umulhi(oa_hash((uint32_t)(s[u] >> 32)), nslots);
+                e[u] = slots[h[u]];
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const uint32_t hi = (uint32_t)(s[u] >> 32);
+                for (uint32_t steps = 0; e[u] != kNone;) {
+                    if ((uint32_t)(e[u] >> 32) == hi) {
+                        cnt++;
+                        sum += (unsigned long long)rid[h[u]] + (s[u] & 0xffffffffull);
+                        if (dups) multi |= (dup[h[u] >> 5] >> (h[u] & 31)) & 1u;
+                        break;
+                    }
+                    if (++h[u] == nslots) h[u] = 0;
+                    if (++steps >= nslots) {
+                        set_error(err, kErrProbeLimit);
+                        break;
+                    }
+                    e[u] = slots[h[u]];
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) s[u] = nx[u];
+        }
+        __syncthreads();
+    }
+    block_sum2_to(cnt, sum, red, &a.acc->matched, &a.acc->checksum);
+    flag_multi(multi, &a.acc->dup_flag);
+    join_finish(a, true);
+}
+
+// First-match join of the one-pass pipeline over {key, position} elements (wide). The match with the lowest
+// position wins, so the partition may hold them in any order. Key, position and row id in
 // separate arrays (20 bytes per build tuple, 16-bit bucket heads and chains: 214 KB, one CTA per SM);
-// a wide element's row id is gathered from the build relation once per build tuple.
+// a build tuple's row id is gathered from the build relation once.
 constexpr uint32_t kFirstHeads = 8192;
 constexpr size_t kFirstSmem = (size_t)kFirstCap * (8 + 8 + 4 + 2) + kFirstHeads * 2;
 
 template <bool MAT>
 __global__ void __launch_bounds__(kJoinThreads, 1) join_first_kernel(JoinArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
-    unsigned long long *kx = reinterpret_cast<unsigned long long *>(smem);  // [kFirstCap] key (or its high part)
+    unsigned long long *kx = reinterpret_cast<unsigned long long *>(smem);  // [kFirstCap] keys
     unsigned long long *rid = kx + kFirstCap;                              // [kFirstCap]
     uint32_t *pos = reinterpret_cast<uint32_t *>(rid + kFirstCap);         // [kFirstCap]
     uint16_t *head = reinterpret_cast<uint16_t *>(pos + kFirstCap);        // [kFirstHeads]
@@ -1611,8 +1902,8 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_kernel(JoinArgs a)
     const int tid = threadIdx.x;
     unsigned int *err = &a.counters[kCtrErr];
     const uint32_t nitems = a.counters[kCtrNItems];
-    const bool ci = !MAT && a.ci && ci_applies(a.counters, a.bits);
-    const int B = ci ? 0 : a.bits;
+    if (!MAT && a.ci && ci_applies(a.counters, a.bits)) return;  // join_first_words_kernel
+    const int B = a.bits;
     const bool skip0 = a.skip0 != 0;
     unsigned long long cnt = 0, sum = 0;
     bool multi = false;
@@ -1641,24 +1932,22 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_kernel(JoinArgs a)
 #pragma unroll
             for (int u = 0; u < U; u++) {
                 const bool live = i0 + u * kJoinThreads < nr && t[u].y < a.nR;
-                y[u] = ci ? t[u].x & 0xffffffffull : live ? a.relR[t[u].y].y : 0ull;
+                y[u] = live ? a.relR[t[u].y].y : 0ull;
             }
 #pragma unroll
             for (int u = 0; u < U; u++) {
                 const uint32_t i = i0 + u * kJoinThreads;
                 if (i >= nr) continue;
-                const unsigned long long k = ci ? t[u].x >> 32 : t[u].x;
+                const unsigned long long k = t[u].x;
                 kx[i] = k;
                 rid[i] = y[u];
                 pos[i] = (uint32_t)t[u].y;
-                // In compact words a key 0 that never matches has a high part that no probe word has.
-                if (skip0 && k == 0 && !ci) continue;
+                if (skip0 && k == 0) continue;
                 nxt[i] = (uint16_t)atomic_exch_u16(&head[(k >> B) & hmask], i + 1);
             }
         }
         __syncthreads();
         const tuple_v *S = a.finS + item.s_begin;
-        const unsigned long long *S8 = a.finS8 + item.s_begin;
         const uint32_t ns = item.s_len;
         for (uint32_t base = 0; base < ns; base += U * kJoinThreads) {
             tuple_v sv[U];
@@ -1666,7 +1955,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_kernel(JoinArgs a)
 #pragma unroll
             for (int u = 0; u < U; u++) {
                 const uint32_t j = base + u * kJoinThreads + tid;
-                sv[u] = j < ns ? ld_fin(S, S8, j, ci) : make_ulonglong2(0, 0);
+                sv[u] = j < ns ? ld_stream(S + j) : make_ulonglong2(0, 0);
             }
 #pragma unroll
             for (int u = 0; u < U; u++) {
@@ -1704,6 +1993,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_kernel(JoinArgs a)
     }
     block_sum2_to(cnt, sum, red, &a.acc->matched, &a.acc->checksum);
     if (!MAT) flag_multi(multi, &a.acc->dup_flag);
+    join_finish(a, false);
 }
 
 template <bool MAT, bool CI = false>
@@ -1733,7 +2023,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_small_kernel(JoinArgs a)
     const bool lp = a.lp != 0;
     const bool skip0 = a.skip0 != 0;
     // Items [0, nA) went to the compact kernel if the build side's keys and row ids fit it.
-    const uint32_t first_item = compact_applies(a) ? a.counters[kCtrNItemsA] : 0u;
+    const uint32_t first_item = !a.all_items && compact_applies(a) ? a.counters[kCtrNItemsA] : 0u;
     unsigned long long cnt = 0, sum = 0;
     uint32_t phase = 0;
     bool ok = true, multi = false;
@@ -1881,6 +2171,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_small_kernel(JoinArgs a)
     }
     block_sum2_to(cnt, sum, red, &a.acc->matched, &a.acc->checksum);
     if (!MAT) flag_multi(multi, &a.acc->dup_flag);
+    join_finish(a, ci);
 }
 
 // Large partitions: chained tables in global memory, one flattened index space for all of them.
@@ -2191,14 +2482,19 @@ int radix_geom(int bits, int passes, RadixGeom *g, int b1_req) {
 
 // The lowest bits that bring build partitions to kSingleTarget tuples on average, at least
 // kSingleMinBits (items for every SM), at most what the caller asked for. Above 2^kSingleMaxBits
-// partitions of kSingleMaxAvg tuples the two-pass pipelines run.
-constexpr uint64_t kSingleTarget = 6144, kSingleMaxAvg = 8192;
+// partitions of kSingleMaxAvg tuples the two-pass pipelines run, and with 2^11 partitions also from
+// kSingleManyTuples tuples: the scatter visits every page of its output once per tile, and those visits
+// grow with the output (2^24 x 2^24, 12 bits: 0.57 ms in one pass, 0.74 in two; 2^24 x 2^26: 1.34 and 1.32;
+// 2^24 x 2^28: 4.50 and 3.38). First-match joins stay up to twice that size: two passes may have to run
+// again in order where build keys repeat (2^24 x 2^26, four a key: 1.55 ms against 2 x 1.4 and more).
+constexpr uint64_t kSingleTarget = 6144, kSingleMaxAvg = 8192, kSingleManyTuples = 80000000;
 constexpr int kSingleMinBits = 8;
 
-bool radix_geom_single(int bits, size_t nR, size_t nS, RadixGeom *g) {
+bool radix_geom_single(int bits, bool lp, size_t nR, size_t nS, RadixGeom *g) {
     if ((nR >> kSingleMaxBits) > kSingleMaxAvg || nR >= (1ull << 32) || nS >= (1ull << 32)) return false;
     int b = kSingleMinBits;
     while (b < kSingleMaxBits && (nR >> b) > kSingleTarget) b++;
+    if (b == kSingleMaxBits && (uint64_t)nR + nS > (lp ? 2 : 1) * kSingleManyTuples) return false;
     if (b > bits) b = bits;
     g->bits = b;
     g->req_bits = bits;
@@ -2420,6 +2716,8 @@ int phj_prepare_device() {
                                (int)kCompactSmem));
     HJ_CU(cudaFuncSetAttribute(join_compact_kernel<true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)kCompactSmem));
+    HJ_CU(cudaFuncSetAttribute(join_words_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOaSmem));
+    HJ_CU(cudaFuncSetAttribute(join_first_words_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwSmem));
     HJ_CU(cudaFuncSetAttribute(join_first_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFirstSmem));
     HJ_CU(cudaFuncSetAttribute(join_first_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFirstSmem));
     HJ_CU(cudaFuncSetAttribute(join_small_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kJoinSmem));
@@ -2436,10 +2734,57 @@ int phj_prepare_device() {
     return nphj_prepare_device();
 }
 
+static JoinArgs join_args(const RadixGeom &g, bool lp, bool skip0, const ulonglong2 *R, size_t nR, const PhjScratch &s,
+                          JoinAccum *acc, const MatOut *mat, int ci_ok, int w8_b1, JoinAccum *host_out) {
+    JoinArgs ja;
+    ja.items = reinterpret_cast<const JoinItem *>(s.items);
+    ja.large = reinterpret_cast<const LargePart *>(s.large);
+    ja.counters = s.counters;
+    ja.finR = s.tmp2;
+    ja.finS = s.tmp2 + nR;
+    ja.large_table = s.large_table;
+    ja.bits = g.bits;
+    ja.lp = lp ? 1 : 0;
+    ja.skip0 = skip0 ? 1 : 0;
+    ja.acc = acc;
+    ja.mat = mat ? *mat : MatOut{nullptr, 0};
+    ja.ci = ci_ok;
+    ja.finR8 = reinterpret_cast<const unsigned long long *>(s.tmp2);
+    ja.finS8 = g.single ? single_probe_words(s, nR, lp) : ja.finR8 + nR;
+    ja.lp_pos = g.single && lp ? 1 : 0;
+    ja.relR = R;
+    ja.nR = nR;
+    ja.flag_bits = g.req_bits;
+    ja.w8_b1 = w8_b1;
+    ja.all_items = g.single && !mat ? 1 : 0;
+    ja.host_out = host_out;
+    return ja;
+}
+
+// Partitions beyond shared memory, then the error word of all kernels.
+static int large_launch(const JoinArgs &ja, bool mat, const PhjScratch &s, JoinAccum *acc, cudaStream_t st, int num_sms) {
+    join_large_clear<<<num_sms * 2, 256, 0, st>>>(ja);
+    join_large_build<<<num_sms * 2, 256, 0, st>>>(ja);
+    if (mat)
+        join_large_probe<true><<<num_sms * 2, 256, 0, st>>>(ja);
+    else
+        join_large_probe<false><<<num_sms * 2, 256, 0, st>>>(ja);
+    copy_error<<<1, 32, 0, st>>>(s.counters, acc);
+    HJ_CU(cudaGetLastError());
+    return HJ_OK;
+}
+
+int phj_large_enqueue(const RadixGeom &g, bool lp, bool skip0, const ulonglong2 *R, size_t nR, size_t nS,
+                      const PhjScratch &s, JoinAccum *acc, cudaStream_t st, int num_sms, uint32_t *launches) {
+    (void)nS;
+    *launches += 4;
+    return large_launch(join_args(g, lp, skip0, R, nR, s, acc, nullptr, 1, -1, nullptr), false, s, acc, st, num_sms);
+}
+
 int phj_enqueue(const RadixGeom &g, bool lp, bool skip0, const ulonglong2 *R, size_t nR, const ulonglong2 *S,
                 size_t nS, const PhjScratch &s, JoinAccum *acc, cudaStream_t st, cudaEvent_t ev_mid,
                 int num_sms, cudaEvent_t *ph, uint32_t *launches, const MatOut *mat, int test_flags,
-                bool ordered) {
+                bool ordered, JoinAccum *host_out) {
     uint32_t nlaunch = 0;
     // Stable ranks of the build relation: first-match joins that keep the input order.
     const bool stable = lp && ordered && !g.single;
@@ -2479,11 +2824,12 @@ int phj_enqueue(const RadixGeom &g, bool lp, bool skip0, const ulonglong2 *R, si
         const int rc = phj_prepare_device();
         if (rc) return rc;
     }
-    HJ_CU(cudaMemsetAsync(s.counters, 0, kNumCounters * 4, st));
+    if (!g.single) HJ_CU(cudaMemsetAsync(s.counters, 0, kNumCounters * 4, st));  // the one-pass count clears them
 
     HJ_PH(0);
     if (g.single) {
-        const int rc = single_partition_enqueue(g, lp, skip0, ci_ok != 0, R, nR, S, nS, s, st, !mat, ph, &nlaunch);
+        const int rc = single_partition_enqueue(g, lp, skip0, ci_ok != 0, R, nR, S, nS, s, acc, host_out && !mat, st, !mat,
+                                                ph, &nlaunch);
         if (rc) return rc;
     } else if (segm) {
         // 1'. pass 1 into segment chains, with the per-CTA histograms
@@ -2675,37 +3021,30 @@ int phj_enqueue(const RadixGeom &g, bool lp, bool skip0, const ulonglong2 *R, si
     if (ev_mid) HJ_CU(record_event(ev_mid, st));
 
     // 6. joins
-    JoinArgs ja;
-    ja.items = reinterpret_cast<const JoinItem *>(s.items);
-    ja.large = reinterpret_cast<const LargePart *>(s.large);
-    ja.counters = s.counters;
-    ja.finR = s.tmp2;
-    ja.finS = s.tmp2 + nR;
-    ja.large_table = s.large_table;
-    ja.bits = g.bits;
-    ja.lp = lp ? 1 : 0;
-    ja.skip0 = skip0 ? 1 : 0;
-    ja.acc = acc;
-    ja.mat = mat ? *mat : MatOut{nullptr, 0};
-    ja.ci = ci_ok;
-    ja.finR8 = reinterpret_cast<const unsigned long long *>(s.tmp2);
-    ja.finS8 = g.single ? single_probe_words(s, nR, lp) : ja.finR8 + nR;
-    ja.lp_pos = g.single && lp ? 1 : 0;
-    ja.relR = R;
-    ja.nR = nR;
-    ja.flag_bits = g.req_bits;
-    ja.w8_b1 = (seg_words || exact_words) ? g.b1 : -1;
+    const JoinArgs ja = join_args(g, lp, skip0, R, nR, s, acc, mat, ci_ok, (seg_words || exact_words) ? g.b1 : -1,
+                                  g.single && !mat ? host_out : nullptr);
     if (ja.lp_pos) {
         if (mat)
             join_first_kernel<true><<<num_sms, kJoinThreads, kFirstSmem, st>>>(ja);
-        else
+        else {
+            // One launch per element layout; the one that does not match the device's choice returns at once.
+            join_first_words_kernel<<<num_sms, kJoinThreads, kFwSmem, st>>>(ja);
             join_first_kernel<false><<<num_sms, kJoinThreads, kFirstSmem, st>>>(ja);
+            nlaunch++;
+        }
+        nlaunch++;
     } else if (mat) {
         if (lp)
             join_compact_kernel<true, false, true><<<num_sms * 2, kCompactThreads, kCompactSmem, st>>>(ja);
         else
             join_compact_kernel<true><<<num_sms * 2, kCompactThreads, kCompactSmem, st>>>(ja);
         join_small_kernel<true><<<num_sms, kJoinThreads, kJoinSmem, st>>>(ja);
+        nlaunch += 2;
+    } else if (g.single) {
+        // One launch per element layout; the one that does not match the device's choice returns at once.
+        join_words_kernel<<<num_sms * 2, kCompactThreads, kOaSmem, st>>>(ja);
+        join_small_kernel<false, false><<<num_sms, kJoinThreads, kJoinSmem, st>>>(ja);
+        nlaunch += 2;
     } else {
         // One launch per partition layout (tuples, compact words); the one that does not match the
         // device's choice returns at once.
@@ -2714,6 +3053,7 @@ int phj_enqueue(const RadixGeom &g, bool lp, bool skip0, const ulonglong2 *R, si
         else
             join_compact_kernel<false, false><<<num_sms * 2, kCompactThreads, kCompactSmem, st>>>(ja);
         join_small_kernel<false, false><<<num_sms, kJoinThreads, kJoinSmem, st>>>(ja);
+        nlaunch += 2;
         if (ci_ok) {
             if (lp)
                 join_compact_kernel<false, true, true><<<num_sms * 2, kCompactThreads, kCompactSmem, st>>>(ja);
@@ -2725,16 +3065,12 @@ int phj_enqueue(const RadixGeom &g, bool lp, bool skip0, const ulonglong2 *R, si
     }
     HJ_CU(cudaGetLastError());
     HJ_PH(segm ? 4 : 5);
-    join_large_clear<<<num_sms * 2, 256, 0, st>>>(ja);
-    join_large_build<<<num_sms * 2, 256, 0, st>>>(ja);
-    if (mat)
-        join_large_probe<true><<<num_sms * 2, 256, 0, st>>>(ja);
-    else
-        join_large_probe<false><<<num_sms * 2, 256, 0, st>>>(ja);
-    copy_error<<<1, 32, 0, st>>>(s.counters, acc);
-    HJ_CU(cudaGetLastError());
+    if (!ja.host_out) {
+        const int rc = large_launch(ja, mat != nullptr, s, acc, st, num_sms);
+        if (rc) return rc;
+        nlaunch += 4;
+    }
     HJ_PH(segm ? 5 : 6);
-    nlaunch += 6;
     if (launches) *launches = nlaunch;
 #undef HJ_PH
     return HJ_OK;

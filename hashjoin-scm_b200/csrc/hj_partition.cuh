@@ -49,6 +49,7 @@ enum : int {
     kCtrItem1S = 22,     // first-match joins: pass-1 work-item counter of the probe relation's items
     kCtrItem2S = 23,     // first-match joins: pass-2 work-item counter of the probe relation's items
     kCtrTicket = 24,     // one-pass pipeline: CTAs of single_plan that have written their totals
+    kCtrTicketJoin = 25, // one-pass pipeline: CTAs of the partition join that have finished
     kNumCounters = 26
 };
 
@@ -139,14 +140,16 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
         : "memory");
     return done != 0;
 }
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-    if (mbar_try(bar, parity)) return true;
+__device__ __forceinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity) {
     const uint64_t t0 = globaltimer_ns();
     for (uint32_t it = 0; it < (1u << 30); it++) {
         if (mbar_try(bar, parity)) return true;
         if ((it & 63u) == 63u && globaltimer_ns() - t0 > kWaitNs) return false;
     }
     return false;
+}
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
+    return mbar_try(bar, parity) || mbar_wait_slow(bar, parity);
 }
 
 // TMA bulk copy global -> shared of `bytes` (a multiple of 16, <= 1 MiB per phase), completing on

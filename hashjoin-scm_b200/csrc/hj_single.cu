@@ -26,13 +26,10 @@
 
 namespace hj {
 
-constexpr int kCountThreads = 1024, kSingleThreads = 512;
-// Scatter: one CTA per SM, 512 threads that place tuples and one warp that loads them.
-constexpr int kScatThreads = kSingleThreads + 32;
-constexpr int kRingChunk = 1024, kRingChunks = 4;  // input ring: chunks of 1024 tuples (16 KB)
-constexpr int kTileChunks = 12;                    // a tile of words: 12 chunks; of 16-byte elements: 6
-constexpr int kSingleWordItems = kTileChunks * kRingChunk / kSingleThreads, kSingleTupleItems = kSingleWordItems / 2;
-constexpr int kSingleDigitsPerThread = ((1 << kSingleMaxBits) + kSingleThreads - 1) / kSingleThreads;
+constexpr int kCountThreads = 1024;
+constexpr int kPlaceThreads = 512;  // scatter: one CTA per SM
+constexpr int kWordItems = 16, kTupleItems = kWordItems / 2;  // staged 8-byte / 16-byte elements per thread and tile
+constexpr int kSingleDigitsPerThread = ((1 << kSingleMaxBits) + kPlaceThreads - 1) / kPlaceThreads;
 
 // CTA c's contiguous range of n tuples (a multiple of 8 tuples, one 128-byte line).
 __device__ __forceinline__ void single_range(uint64_t n, uint64_t *lo, uint64_t *hi) {
@@ -41,13 +38,9 @@ __device__ __forceinline__ void single_range(uint64_t n, uint64_t *lo, uint64_t 
     *hi = *lo + per < n ? *lo + per : n;
 }
 
-// Shared memory of the scatter: a staged tile with its digits, and four words per digit.
-constexpr size_t kSingleStage = (size_t)kSingleThreads * kSingleWordItems * 8;
-static_assert(kSingleStage == (size_t)kSingleThreads * kSingleTupleItems * 16, "one staging area for both layouts");
-inline size_t single_scatter_smem(int bits) {
-    return (size_t)kRingChunks * kRingChunk * 16 + kSingleStage + (size_t)kSingleThreads * kSingleWordItems * 2 +
-           ((size_t)4 << bits) * 4;
-}
+// Shared memory of the scatter: a staged tile, and four words per digit.
+constexpr size_t kSingleStage = (size_t)kPlaceThreads * kWordItems * 8;
+inline size_t single_scatter_smem(int bits) { return kSingleStage + 128 + ((size_t)4 << bits) * 4; }
 
 // Input tuple of the count: read again by the scatter, so its line keeps the normal L2 priority.
 __device__ __forceinline__ tuple_v ld_twice(const tuple_v *p) {
@@ -65,6 +58,8 @@ struct SingleArgs {
     unsigned long long *ors; // [G][3]: ORs of build keys, build row ids, probe row ids
     const uint64_t *start;   // [2][P + 1]
     uint32_t *counters;
+    JoinAccum *acc;          // cleared by the count if clear_acc
+    int clear_acc;
     int ci_ok;               // compact words allowed
     int lp;                  // first match: build elements carry their input position
     int z0;                  // build key 0 never matches
@@ -84,6 +79,9 @@ __global__ void __launch_bounds__(kCountThreads, 1) single_count(SingleArgs a) {
     uint32_t *mine = sh + (size_t)((uint32_t)(tid >> 5) % (uint32_t)a.copies) * P;
     __shared__ unsigned long long s_or[3];
     if (tid < 3) s_or[tid] = 0;
+    // The kernels after this one find their counters (and the result) at zero.
+    if (blockIdx.x == 0 && tid < kNumCounters) a.counters[tid] = 0;
+    if (blockIdx.x == 0 && a.clear_acc && tid == 0) *a.acc = JoinAccum{};
     for (int rel = 0; rel < 2; rel++) {
         for (uint32_t j = tid; j < P * a.copies; j += kCountThreads) sh[j] = 0;
         __syncthreads();
@@ -201,40 +199,66 @@ __global__ void __launch_bounds__(1024, 1) single_plan(SingleArgs a, uint32_t G,
 }
 
 // ------------------------------------------------------------------------------------------------
-// 3. Scatter. One CTA per SM with the largest tile that fits (12288 words or 6144 16-byte elements): what a
-//    run of a digit costs in L2 does not depend on its length (about 35 G runs per second here, whatever
-//    the tile), so the runs N * P / tile have to be few. A producer warp keeps a ring of bulk copies in
-//    flight through all phases of a tile; per tile the 512 placing threads take the elements' ranks within
-//    their digit from shared-memory atomics, a block scan over the digits gives each digit's start in the
-//    tile, and the tile is staged in digit order and written out, consecutive threads to consecutive places
-//    of a digit's run. A CTA's elements of a digit go to its own consecutive places, so the next place of
-//    every digit is a counter in shared memory.
+// 3. Scatter. Tiles of 8192 8-byte or 4096 16-byte elements: a thread takes 16 (8) elements, all their loads
+//    in flight together and issued under the previous tile's write-out; their ranks within their digit come
+//    from shared-memory atomics; a block scan over the digits gives each digit's start in the tile; the tile
+//    is staged in digit order and written out, consecutive threads to consecutive places of a digit's run. A
+//    CTA's elements of a digit go to its own consecutive places, so the next place of every digit is a
+//    counter in shared memory. A staged element still tells its digit, so none is kept beside it.
+//    One CTA per SM: every tile visits every page of the output, and those visits, not the length of the
+//    runs, are what scattered stores cost (12.6 M words to 1024 partitions of 100 MB: 77 us stored in
+//    place, 76 us scattered over 8 MB, 98 us over the 100 MB; 2 CTAs with half the tile: 125 us; 4 CTAs:
+//    153 us; direct stores without staging: 36-65 G elements per second).
 // ------------------------------------------------------------------------------------------------
-// KIND 0: tuples, 1: compact words, 2: {word or key, position} of first-match builds.
-template <int KIND>
+enum SingleMode {
+    kModeWord,      // staged {low 32 key bits, row id} (build keys below 2^31), written as a compact word
+    kModeTuple,     // staged and written as a tuple
+    kModeTupleWord, // staged as a tuple, written as a compact word
+    kModePosWord,   // first-match builds: {compact word, position | digit << 32}, written as {word, position}
+    kModePos,       // first-match builds, wide: {key, position}
+};
+
+// Staged and written element of a mode. bits: radix bits; mask = 2^bits - 1.
+template <int MODE>
 struct SingleElem {
-    using type = tuple_v;
+    using Staged = tuple_v;
+    using Out = tuple_v;
+    static __device__ __forceinline__ tuple_v stage(const tuple_v &t, uint64_t i, int bits, uint32_t mask, bool z0) {
+        if (MODE == kModePosWord)
+            return make_ulonglong2(ci_word_z0(t.x, t.y, bits, z0), i | ((unsigned long long)((uint32_t)t.x & mask) << 32));
+        return MODE == kModePos ? make_ulonglong2(t.x, i) : t;
+    }
+    static __device__ __forceinline__ uint32_t digit(const tuple_v &v, uint32_t mask) {
+        return MODE == kModePosWord ? (uint32_t)(v.y >> 32) : (uint32_t)v.x & mask;
+    }
+    static __device__ __forceinline__ tuple_v out(const tuple_v &v, int) {
+        return MODE == kModePosWord ? make_ulonglong2(v.x, v.y & 0xffffffffull) : v;
+    }
 };
 template <>
-struct SingleElem<1> {
-    using type = unsigned long long;
+struct SingleElem<kModeTupleWord> {
+    using Staged = tuple_v;
+    using Out = unsigned long long;
+    static __device__ __forceinline__ tuple_v stage(const tuple_v &t, uint64_t, int, uint32_t, bool) { return t; }
+    static __device__ __forceinline__ uint32_t digit(const tuple_v &v, uint32_t mask) { return (uint32_t)v.x & mask; }
+    static __device__ __forceinline__ unsigned long long out(const tuple_v &v, int bits) { return ci_word(v.x, v.y, bits); }
+};
+template <>
+struct SingleElem<kModeWord> {
+    using Staged = uint2;  // x: row id, y: key (a probe key of 2^31 or more: its digit with bit 31 set)
+    using Out = unsigned long long;
+    static __device__ __forceinline__ uint2 stage(const tuple_v &t, uint64_t, int, uint32_t mask, bool) {
+        const uint32_t lo = (uint32_t)t.x, hi = (uint32_t)(t.x >> 32);
+        return make_uint2((uint32_t)t.y, (hi | (lo & 0x80000000u)) ? 0x80000000u | (lo & mask) : lo);
+    }
+    static __device__ __forceinline__ uint32_t digit(const uint2 &v, uint32_t mask) { return v.y & mask; }
+    static __device__ __forceinline__ unsigned long long out(const uint2 &v, int bits) {
+        const uint32_t h = (int)v.y < 0 ? 0xffffffffu : v.y >> bits;
+        return ((unsigned long long)h << 32) | v.x;
+    }
 };
 
-template <int KIND>
-__device__ __forceinline__ typename SingleElem<KIND>::type single_elem(const tuple_v &t, uint64_t i, bool ci, int bits,
-                                                                       bool z0) {
-    if constexpr (KIND == 0)
-        return t;
-    else if constexpr (KIND == 1)
-        return ci_word_z0(t.x, t.y, bits, z0);
-    else
-        return make_ulonglong2(ci ? ci_word_z0(t.x, t.y, bits, z0) : t.x, i);
-}
-
-// Barrier of the placing threads (the producer warp takes no part).
-__device__ __forceinline__ void place_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kSingleThreads) : "memory"); }
-
-// Exclusive scan of one u32 per placing thread.
+// Exclusive scan of one u32 per thread; tmp is reused only after two more barriers.
 __device__ __forceinline__ uint32_t place_scan(uint32_t v, uint32_t *tmp) {
     const unsigned lane = lane_id(), w = threadIdx.x >> 5;
     uint32_t x = v;
@@ -244,194 +268,132 @@ __device__ __forceinline__ uint32_t place_scan(uint32_t v, uint32_t *tmp) {
         if (lane >= (unsigned)o) x += y;
     }
     if (lane == 31) tmp[w] = x;
-    place_sync();
-    uint32_t before = 0;  // every warp sums the totals of the warps before it
-    uint32_t tot = lane < (unsigned)(kSingleThreads / 32) ? tmp[lane] : 0u;
-    before = __reduce_add_sync(0xffffffffu, lane < w ? tot : 0u);
-    return before + x - v;
+    __syncthreads();
+    // Every warp adds up the totals of the warps before it.
+    return __reduce_add_sync(0xffffffffu, lane < w ? tmp[lane] : 0u) + x - v;
 }
 
-struct SingleShared {
-    unsigned long long full[kRingChunks], empty[kRingChunks];
-    uint32_t scan_tmp[32];
-    uint32_t stop;  // a placing thread's bounded wait expired (written before a barrier of theirs only)
-};
-
-// The order in which a CTA reads its ranges: S before R, each from its last tile to its first, a tile's
-// chunks in order. Producer and placing threads walk it alike.
-template <class F>
-__device__ __forceinline__ bool single_walk(uint32_t len, uint32_t tile, F &&f) {
-    for (uint32_t k = (len + tile - 1) / tile; k > 0; k--)
-        if (!f((k - 1) * tile, len - (k - 1) * tile < tile ? len - (k - 1) * tile : tile)) return false;
-    return true;
-}
-
-__device__ __forceinline__ void single_produce(const SingleArgs &a, uint32_t tile_r, uint32_t tile_s, tuple_v *ring,
-                                               SingleShared &sh) {
-    uint32_t c = 0;  // chunks issued
-    bool ok = true;
-    for (int rel = 1; rel >= 0 && ok; rel--) {
-        uint64_t lo, hi;
-        single_range(rel ? a.nS : a.nR, &lo, &hi);
-        const tuple_v *in = (rel ? a.S : a.R) + lo;
-        ok = single_walk((uint32_t)(hi - lo), rel ? tile_s : tile_r, [&](uint32_t base, uint32_t m) {
-            for (uint32_t o = 0; o < m; o += kRingChunk, c++) {
-                const uint32_t slot = c % kRingChunks;
-                if (c >= kRingChunks && !mbar_wait(smem_addr(&sh.empty[slot]), (c / kRingChunks - 1) & 1u)) return false;
-                if (*reinterpret_cast<volatile uint32_t *>(&sh.stop)) return false;
-                const uint32_t cnt = m - o < (uint32_t)kRingChunk ? m - o : (uint32_t)kRingChunk;
-                tma_load_1d(ring + (size_t)slot * kRingChunk, in + base + o, cnt * 16u, smem_addr(&sh.full[slot]));
-            }
-            return true;
-        });
-    }
-    if (!ok) set_error(&a.counters[kCtrErr], kErrSpinLimit);
-    // Let what is in flight land (bounded) before the CTA may give up its shared memory.
-    for (uint32_t q = c > (uint32_t)kRingChunks ? c - kRingChunks : 0u; q < c; q++)
-        mbar_wait(smem_addr(&sh.full[q % kRingChunks]), (q / kRingChunks) & 1u);
-}
-
-// Place one relation's range; c counts the ring chunks taken so far. False: a wait expired.
-template <int KIND>
-__device__ __forceinline__ bool single_scatter_rel(const SingleArgs &a, bool ci, int rel, unsigned char *smem,
-                                                   SingleShared &sh, uint32_t &c) {
-    using E = typename SingleElem<KIND>::type;
-    constexpr int NT = kSingleThreads, ITEMS = KIND == 1 ? kSingleWordItems : kSingleTupleItems;
-    constexpr int PC = kRingChunk / NT;  // tuples of a chunk per thread
-    constexpr uint32_t T = NT * ITEMS;
+// Place one relation's range. A function of its own per mode: inlined side by side the modes spilled.
+template <int MODE>
+__device__ __noinline__ void single_scatter_rel(const SingleArgs &a, int rel) {
+    using Elem = SingleElem<MODE>;
+    using E = typename Elem::Staged;
+    using O = typename Elem::Out;
+    constexpr int NT = kPlaceThreads, ITEMS = MODE == kModeWord ? kWordItems : kTupleItems;
     constexpr int D = kSingleDigitsPerThread;
-    const int tid = threadIdx.x;
-    const uint32_t P = 1u << a.bits, mask = P - 1;
-    unsigned int *err = &a.counters[kCtrErr];
-    const tuple_v *ring = reinterpret_cast<const tuple_v *>(smem);                     // [kRingChunks][kRingChunk]
-    E *stage = reinterpret_cast<E *>(smem + (size_t)kRingChunks * kRingChunk * 16);    // [T]
-    uint16_t *dig = reinterpret_cast<uint16_t *>(smem + (size_t)kRingChunks * kRingChunk * 16 + kSingleStage);  // [T]
-    uint32_t *cnt = reinterpret_cast<uint32_t *>(dig + NT * kSingleWordItems);         // [P] elements of the tile
-    uint32_t *tst = cnt + P;                                                           // [P] start in the tile
-    uint32_t *gofs = tst + P;                                                          // [P] place - staged index
-    uint32_t *place = gofs + P;                                                        // [P] next place in the output
-    const uint64_t n = rel ? a.nS : a.nR;
-    const uint32_t *pre = a.hist + ((size_t)rel * gridDim.x + blockIdx.x) * P;
-    const uint64_t *start = a.start + (size_t)rel * (P + 1);
-    const uint32_t per = (P + NT - 1) / NT;  // this thread's digits in the scan: [tid * per, tid * per + per)
-    for (uint32_t j = tid; j < P; j += NT) {
-        place[j] = (uint32_t)start[j] + pre[j];
-        cnt[j] = 0;
-    }
-    E *out;
-    if constexpr (KIND == 1)
+    constexpr uint32_t T = NT * ITEMS;
+    extern __shared__ __align__(128) unsigned char smem[];
+    const uint32_t tid = threadIdx.x;
+    const int bits = a.bits;
+    const uint32_t P = 1u << bits, mask = P - 1;
+    E *stage = reinterpret_cast<E *>(smem);                                   // [T]
+    uint32_t *scan_tmp = reinterpret_cast<uint32_t *>(smem + kSingleStage);   // [32]
+    uint32_t *cnt = scan_tmp + 32;                                            // [P] elements of the tile
+    uint32_t *tst = cnt + P;                                                  // [P] start in the tile
+    uint32_t *gofs = tst + P;                                                 // [P] place - staged index
+    uint32_t *place = gofs + P;                                               // [P] next place in the output
+    const uint32_t n = (uint32_t)(rel ? a.nS : a.nR);
+    O *out;
+    if constexpr (sizeof(O) == 8)
         out = rel ? a.outS8 : a.outR8;
     else
         out = rel ? a.outS : a.outR;
     const bool z0 = a.z0 && rel == 0;
     uint64_t lo, hi;
-    single_range(n, &lo, &hi);
-    place_sync();
-    return single_walk((uint32_t)(hi - lo), T, [&](uint32_t base, uint32_t m) {
-        E v[ITEMS];
-        uint32_t dr[ITEMS];  // digit << 16 | rank
+    single_range(rel ? a.nS : a.nR, &lo, &hi);
+    const tuple_v *in = (rel ? a.S : a.R) + lo;
+    const uint32_t len = (uint32_t)(hi - lo);
+    if (len == 0) return;
+    tuple_v t[ITEMS];
+    uint32_t base = (len - 1) / T * T;
 #pragma unroll
-        for (int ch = 0; ch < ITEMS / PC; ch++) {
-            if ((uint32_t)(ch * kRingChunk) < m) {
-                const uint32_t slot = c % kRingChunks;
-                if (!mbar_wait(smem_addr(&sh.full[slot]), (c / kRingChunks) & 1u)) {
-                    set_error(err, kErrSpinLimit);
-                    *reinterpret_cast<volatile uint32_t *>(&sh.stop) = 1u;
-                }
-                tuple_v t[PC];
-#pragma unroll
-                for (int u = 0; u < PC; u++) t[u] = ring[(size_t)slot * kRingChunk + u * NT + tid];
-                __syncwarp();
-                if ((tid & 31) == 0)
-                    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(&sh.empty[slot])) : "memory");
-                c++;
-#pragma unroll
-                for (int u = 0; u < PC; u++) {
-                    const uint32_t i = ch * kRingChunk + u * NT + tid;
-                    const uint32_t d = (uint32_t)t[u].x & mask;
-                    v[ch * PC + u] = single_elem<KIND>(t[u], lo + base + i, ci, a.bits, z0);
-                    dr[ch * PC + u] = i < m ? (d << 16) | atomicAdd(&cnt[d], 1u) : 0xffffffffu;
-                }
-            } else {
-#pragma unroll
-                for (int u = 0; u < PC; u++) dr[ch * PC + u] = 0xffffffffu;
-            }
+    for (int q = 0; q < ITEMS; q++) t[q] = base + q * NT + tid < len ? ld_stream(in + base + q * NT + tid) : make_ulonglong2(0, 0);
+    {
+        const uint32_t *pre = a.hist + ((size_t)rel * gridDim.x + blockIdx.x) * P;
+        const uint64_t *start = a.start + (size_t)rel * (P + 1);
+        for (uint32_t j = tid; j < P; j += NT) {
+            place[j] = (uint32_t)start[j] + pre[j];
+            cnt[j] = 0;
         }
-        place_sync();
-        if (*reinterpret_cast<volatile uint32_t *>(&sh.stop)) return false;  // the same for every thread
-        uint32_t cq[D], sum = 0;
-#pragma unroll
-        for (int q = 0; q < D; q++) {
-            cq[q] = q < per && tid * per + q < P ? cnt[tid * per + q] : 0u;
-            sum += cq[q];
-        }
-        uint32_t ex = place_scan(sum, sh.scan_tmp);
-#pragma unroll
-        for (int q = 0; q < D; q++) {
-            if (q < per && tid * per + q < P) {
-                const uint32_t pl = place[tid * per + q];
-                cnt[tid * per + q] = 0;
-                tst[tid * per + q] = ex;
-                gofs[tid * per + q] = pl - ex;
-                place[tid * per + q] = pl + cq[q];
-                ex += cq[q];
-            }
-        }
-        place_sync();
-#pragma unroll
-        for (int q = 0; q < ITEMS; q++) {
-            if (dr[q] == 0xffffffffu) continue;
-            const uint32_t d = dr[q] >> 16, p = tst[d] + (dr[q] & 0xffffu);
-            stage[p] = v[q];
-            dig[p] = (uint16_t)d;
-        }
-        place_sync();
-#pragma unroll 4
-        for (uint32_t j = tid; j < m; j += NT) {
-            const uint32_t dst = gofs[dig[j]] + j;
-            if (dst < n)
-                out[dst] = stage[j];
-            else
-                set_error(err, kErrBounds);
-        }
-        return true;
-    });
-}
-
-__global__ void __launch_bounds__(kScatThreads, 1) single_scatter(SingleArgs a) {
-    extern __shared__ __align__(128) unsigned char smem[];
-    __shared__ SingleShared sh;
-    const bool ci = a.ci_ok && ci_applies(a.counters, a.bits);
-    if (threadIdx.x == 0) {
-        for (int q = 0; q < kRingChunks; q++) {
-            mbar_init(smem_addr(&sh.full[q]), 1);
-            mbar_init(smem_addr(&sh.empty[q]), kSingleThreads / 32);
-        }
-        sh.stop = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    constexpr uint32_t kWordTile = kSingleThreads * kSingleWordItems, kTupleTile = kSingleThreads * kSingleTupleItems;
-    if (threadIdx.x >= kSingleThreads) {
-        if (threadIdx.x == kSingleThreads)
-            single_produce(a, ci && !a.lp ? kWordTile : kTupleTile, ci ? kWordTile : kTupleTile,
-                           reinterpret_cast<tuple_v *>(smem), sh);
-        return;
+    for (;;) {
+        const uint32_t m = len - base < T ? len - base : T;
+        E v[ITEMS];
+        uint32_t rk[ITEMS / 2];  // ranks, two 16-bit ones per word
+#pragma unroll
+        for (int q = 0; q < ITEMS; q++) {
+            v[q] = Elem::stage(t[q], lo + base + q * NT + tid, bits, mask, z0);
+            uint32_t r = 0;
+            if (q * NT + tid < m) r = atomicAdd(&cnt[Elem::digit(v[q], mask)], 1u);
+            rk[q / 2] = (q & 1) ? rk[q / 2] | (r << 16) : r;
+        }
+        __syncthreads();
+        {
+            const uint32_t per = (P + NT - 1) / NT;  // this thread's digits: [tid * per, tid * per + per)
+            uint32_t cq[D], sum = 0;
+#pragma unroll
+            for (int q = 0; q < D; q++) {
+                cq[q] = q < per && tid * per + q < P ? cnt[tid * per + q] : 0u;
+                sum += cq[q];
+            }
+            uint32_t ex = place_scan(sum, scan_tmp);
+#pragma unroll
+            for (int q = 0; q < D; q++) {
+                if (q < per && tid * per + q < P) {
+                    const uint32_t pl = place[tid * per + q];
+                    cnt[tid * per + q] = 0;
+                    tst[tid * per + q] = ex;
+                    gofs[tid * per + q] = pl - ex;
+                    place[tid * per + q] = pl + cq[q];
+                    ex += cq[q];
+                }
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < ITEMS; q++)
+            if (q * NT + tid < m)
+                stage[tst[Elem::digit(v[q], mask)] + ((q & 1) ? rk[q / 2] >> 16 : rk[q / 2] & 0xffffu)] = v[q];
+        const bool more = base != 0;
+        if (more) {  // the next tile's loads pass under the write-out
+            base -= T;
+#pragma unroll
+            for (int q = 0; q < ITEMS; q++) t[q] = ld_stream(in + base + q * NT + tid);
+        }
+        __syncthreads();
+#pragma unroll 4
+        for (uint32_t j = tid; j < m; j += NT) {
+            const E e = stage[j];
+            const uint32_t dst = gofs[Elem::digit(e, mask)] + j;
+            if (dst < n)
+                out[dst] = Elem::out(e, bits);
+            else
+                set_error(&a.counters[kCtrErr], kErrBounds);
+        }
+        if (!more) break;
     }
-    uint32_t c = 0;
-    bool ok;
-    if (ci)
-        ok = single_scatter_rel<1>(a, true, 1, smem, sh, c);
-    else
-        ok = single_scatter_rel<0>(a, false, 1, smem, sh, c);
-    if (!ok) return;
-    place_sync();
-    if (a.lp)
-        single_scatter_rel<2>(a, ci, 0, smem, sh, c);
-    else if (ci)
-        single_scatter_rel<1>(a, true, 0, smem, sh, c);
-    else
-        single_scatter_rel<0>(a, false, 0, smem, sh, c);
+    __syncthreads();
+}
+
+__global__ void __launch_bounds__(kPlaceThreads, 1) single_scatter(SingleArgs a) {
+    const bool ci = a.ci_ok && ci_applies(a.counters, a.bits);
+    const bool narrow = ci && *reinterpret_cast<const unsigned long long *>(a.counters + kCtrMaxKey) < (1ull << 31);
+    // S, then R; one instantiation per mode serves both.
+    for (int rel = 1; rel >= 0; rel--) {
+        if (rel == 0 && a.lp) {
+            if (ci)
+                single_scatter_rel<kModePosWord>(a, rel);
+            else
+                single_scatter_rel<kModePos>(a, rel);
+        } else if (narrow) {
+            single_scatter_rel<kModeWord>(a, rel);
+        } else if (ci) {
+            single_scatter_rel<kModeTupleWord>(a, rel);
+        } else {
+            single_scatter_rel<kModeTuple>(a, rel);
+        }
+    }
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -459,8 +421,8 @@ int single_prepare_device() {
 }
 
 int single_partition_enqueue(const RadixGeom &g, bool lp, bool skip0, bool ci_ok, const ulonglong2 *R, size_t nR,
-                             const ulonglong2 *S, size_t nS, const PhjScratch &s, cudaStream_t st, bool agg_ok,
-                             cudaEvent_t *ph, uint32_t *launches) {
+                             const ulonglong2 *S, size_t nS, const PhjScratch &s, JoinAccum *acc, bool clear_acc,
+                             cudaStream_t st, bool agg_ok, cudaEvent_t *ph, uint32_t *launches) {
     const uint32_t P = 1u << g.bits;
     SingleArgs a;
     a.R = R;
@@ -473,6 +435,8 @@ int single_partition_enqueue(const RadixGeom &g, bool lp, bool skip0, bool ci_ok
     a.ors = s.ors;
     a.start = s.start;
     a.counters = s.counters;
+    a.acc = acc;
+    a.clear_acc = clear_acc ? 1 : 0;
     a.ci_ok = ci_ok ? 1 : 0;
     a.lp = lp ? 1 : 0;
     a.z0 = skip0 ? 1 : 0;
@@ -503,7 +467,7 @@ int single_partition_enqueue(const RadixGeom &g, bool lp, bool skip0, bool ci_ok
     if (ph) HJ_CU(record_event(ph[1], st));
     single_plan<<<(2 * P + 31) / 32, 1024, (size_t)2 * P * 4, st>>>(a, G, s.total, pa);
     if (ph) HJ_CU(record_event(ph[2], st));
-    single_scatter<<<G, kScatThreads, single_scatter_smem(g.bits), st>>>(a);
+    single_scatter<<<G, kPlaceThreads, single_scatter_smem(g.bits), st>>>(a);
     HJ_CU(cudaGetLastError());
     if (ph) {
         HJ_CU(record_event(ph[3], st));
