@@ -74,7 +74,8 @@ constexpr uint32_t kPipelineFlags = HJ_F_SEGMENTS | HJ_F_EXACT | HJ_F_WIDE | HJ_
 int join_geom(hj_algo_t algo, const hj_params_t &p, size_t nR, size_t nS, hj::RadixGeom *g) {
     const int rc = hj::radix_geom(p.num_radix_bits, p.num_passes, g, p.radix_bits_pass1);
     if (rc) return rc;
-    if (!(p.flags & kPipelineFlags)) hj::radix_geom_single(p.num_radix_bits, hj::algo_lp(algo), nR, nS, g);
+    if (!(p.flags & kPipelineFlags) && !hj::radix_geom_single(p.num_radix_bits, hj::algo_lp(algo), nR, nS, g))
+        hj::radix_geom_by_size(nR, g);
     return HJ_OK;
 }
 
@@ -107,7 +108,7 @@ int plan_join(hj_algo_t algo, hj_params_t *p, size_t nR, size_t nS, JoinPlan *jp
     } else if (nphj_by_radix(*p, nR, nS)) {
         p->flags &= ~(kPipelineFlags | HJ_F_ORDERED);  // radix joins' flags
         hj::radix_geom(14, 2, &jp->geom);
-        hj::radix_geom_single(14, hj::algo_lp(algo), nR, nS, &jp->geom);
+        if (!hj::radix_geom_single(14, hj::algo_lp(algo), nR, nS, &jp->geom)) hj::radix_geom_by_size(nR, &jp->geom);
     } else {
         return HJ_OK;
     }

@@ -42,6 +42,9 @@ int radix_geom(int bits, int passes, RadixGeom *g, int b1_req = 0);
 constexpr int kSingleMaxBits = 11;
 bool radix_geom_single(int bits, bool lp, size_t nR, size_t nS, RadixGeom *g);
 
+// Lower the bits of a two-pass geometry to what a build relation of nR tuples needs.
+void radix_geom_by_size(size_t nR, RadixGeom *g);
+
 // Joins of at most kSmallMaxBuild build tuples run as one kernel (hj_small.cu).
 constexpr uint32_t kSmallMaxBuild = 8192;
 constexpr int kSmallMaxGrid = 512;

@@ -38,7 +38,7 @@
 // The join kernels have a materialising variant (MAT) for the ptr_* joins: one (r.row_id, s.row_id)
 // pair per match instead of the sums.
 //
-// Segment mode (joins that count every match, two passes, <= 14 bits, from 2^27 tuples): no histogram
+// Segment mode (joins that count every match, two passes, <= 14 bits, from 2^26 tuples): no histogram
 // pass. seg_pass1_kernel writes pass 1 into per-(CTA, relation, digit) chains of tile-sized segments
 // and counts each CTA's joint histogram itself; colscan/plan/units then treat the pass-1 CTAs as the
 // chunks, and pass 2 (scatter_kernel) walks the chains as its units.
@@ -858,6 +858,7 @@ constexpr uint32_t kSegSlab = 32;          // segment ids a CTA takes from the g
 constexpr int kSegCtasPerSm = 2;           // shared memory: two tile buffers + 32 KB of counters
 constexpr int kSegMaxBits = 14;
 constexpr uint32_t kSegSpillAt = 8192;
+constexpr uint32_t kSegEndItems = 0x40000000;  // more than the work items of any relation (2^32 / kTile each)
 
 struct SegArgs {
     const tuple_v *R, *S;
@@ -898,7 +899,7 @@ __device__ __forceinline__ SegSlot seg_next_tile(const SegArgs &a, uint32_t &ite
                                                  uint32_t &t_end, uint32_t &r_next, uint32_t r_end) {
     SegSlot s;
     while (item == ~0u || t_next >= t_end) {
-        if (STATIC_R && r_next < r_end)
+        if (STATIC_R && r_next < r_end && !*reinterpret_cast<volatile uint32_t *>(&a.counters[kCtrSegWide]))
             item = r_next++;
         else
             item = atomicAdd(&a.counters[kCtrItem1], 1u) + (STATIC_R ? a.itemsR : 0u);
@@ -1120,6 +1121,13 @@ __global__ void __launch_bounds__(THREADS, kSegCtasPerSm) seg_pass1_kernel(SegAr
         } else {
             rors |= yo;
         }
+        // A value too wide for words: the tuple pass will have to run, so end this one. The claims of every
+        // CTA run past the last item from now on (a relation of 63-bit keys costs a tile per CTA here, not
+        // a whole pass).
+        if (W8 && (yo || (sl.rel == 0 && (xo >> (a.b1 - 1)))) &&
+            !*reinterpret_cast<volatile uint32_t *>(&a.counters[kCtrSegWide]) &&
+            atomicExch(&a.counters[kCtrSegWide], 1u) == 0)
+            atomicAdd(&a.counters[kCtrItem1], kSegEndItems);
         if (STABLE_R && st) {
             // Stable rank within the warp: items in order, lanes in order; the lanes holding one digit
             // are found with one ballot per digit bit (plus the bit that marks padding lanes).
@@ -1344,6 +1352,7 @@ __global__ void seg_reset_if_wide(uint32_t *counters, int b1) {
     if (threadIdx.x == 0 && !w8_fits(counters, b1)) {
         counters[kCtrItem1] = 0;
         counters[kCtrSegAlloc] = 0;
+        counters[kCtrSegWide] = 0;
     }
 }
 
@@ -2539,12 +2548,24 @@ struct PhjSizes {
     ChunkGeom cg;
 };
 
-// Segment mode from 2^27 tuples. Its pass 2 has one unit per (pass-1 CTA, relation, digit) and a
-// partial tile per unit whatever the size, and its pass 1 runs at two CTAs per SM. At 2^24 x 2^26
-// (2^26.3 tuples) the joins of both pipelines took the same time; the saved histogram read grows with
-// the size (1.3 ms of 11.8 at 2^27 x 2^29). The partly filled segments also reserve storage
-// (2 * CTAs * F1 * kTile tuples).
-constexpr uint64_t kSegMinTuples = 1ull << 27;
+// The two-pass pipelines' geometry: the lowest bits that bring build partitions to kSingleTarget tuples, at
+// most what the caller asked for. Fewer digits make longer runs and fewer, fuller units (2^24 x 2^26 in
+// segment mode: 1.32 ms with 12 bits, 1.40 with 13, 2.00 with 14; 2^24 x 2^28 3.38 / 3.47 / 4.09).
+void radix_geom_by_size(size_t nR, RadixGeom *g) {
+    if (g->passes != 2) return;
+    int b = 2;
+    while (b < g->bits && (nR >> b) > kSingleTarget) b++;
+    const int req = g->req_bits;
+    if (b < g->bits) radix_geom(b, 2, g);
+    g->req_bits = req;
+}
+
+// Segment mode from 2^26 tuples. Its pass 2 has one unit per (pass-1 CTA, relation, digit) and a
+// partial tile per unit whatever the size, its pass 1 runs at two CTAs per SM, and the partly filled
+// segments reserve storage (2 * CTAs * F1 * kTile tuples); the histogram read it saves grows with the
+// size. Fewest bits, unique keys: 2^24 x 2^24 0.86 ms against 0.74 in the exact-offset pipeline, 2^25 x
+// 2^25 1.25 against 1.34 (63-bit keys 1.52 against 1.67), 2^26 x 2^28 4.61 against 5.01 (6.41 / 7.09).
+constexpr uint64_t kSegMinTuples = 1ull << 26;
 
 bool phj_seg_applies(const RadixGeom &g, bool, size_t nR, size_t nS) {
     return g.passes == 2 && g.bits <= kSegMaxBits && (uint64_t)nR + nS >= kSegMinTuples;

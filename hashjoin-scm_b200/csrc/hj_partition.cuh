@@ -50,7 +50,8 @@ enum : int {
     kCtrItem2S = 23,     // first-match joins: pass-2 work-item counter of the probe relation's items
     kCtrTicket = 24,     // one-pass pipeline: CTAs of single_plan that have written their totals
     kCtrTicketJoin = 25, // one-pass pipeline: CTAs of the partition join that have finished
-    kNumCounters = 26
+    kCtrSegWide = 26,    // segment mode: the word pass 1 met a value too wide for words and stopped
+    kNumCounters = 28
 };
 
 // Compact final partitions. When every build key shifted right by the radix bits is below 2^31 and
