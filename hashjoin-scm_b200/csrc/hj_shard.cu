@@ -11,12 +11,17 @@
 // tuples keep their input order, so after an all-to-all that concatenates the ranks' pieces in rank
 // order, each rank's build relation is in global input order (first-match joins stay exact).
 //
-// Kernels (all block ranges are contiguous slices of the input, in block order):
-//   route_count    per block and owner: tuples (shared-memory counters)
+// Kernels (all block ranges are contiguous slices of the input, in block order, four blocks per SM):
+//   route_count    per block and owner: tuples. Every lane counts in a shared-memory column of its own, so
+//                  that 32 lanes on a few owners do not serialise; four loads per thread in flight
 //   route_offsets  one CTA: each block's start per owner (exclusive scan down the columns, then owner
 //                  bases), and the owner totals
-//   route_scatter  per block, tiles of 8 tuples per thread: per-owner exclusive scans across the
-//                  block's threads give each tuple its stable position.
+//   route_scatter  per block, tiles of 8 rows of 32 tuples per warp: a tuple's stable rank is the number of
+//                  lanes before it with its owner (one ballot per bit of the owner) plus what its warp has
+//                  seen; a prefix over the warps and the owners gives its place in the tile, which is
+//                  staged by owner and written out coalesced
+// Bound by the two reads and the write (48 bytes a tuple): 2^24 tuples to 8 owners 174 us, where one block scan
+// per owner and tile, strided loads and a single load in flight took 462 us.
 #include <cstdio>
 
 #include "../host/hj_feistel.h"
@@ -28,6 +33,14 @@ namespace hj {
 constexpr int kRouteThreads = 256;
 constexpr int kRouteItems = 8;
 constexpr int kRouteMaxShards = 32;
+constexpr int kRouteCtas = 4;  // blocks per SM
+
+// The count's loads: the scatter reads the tuples again, so their lines keep the normal L2 priority.
+__device__ __forceinline__ tuple_v ld_once_more(const tuple_v *p) {
+    tuple_v v;
+    asm volatile("ld.global.nc.L1::no_allocate.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p));
+    return v;
+}
 
 __device__ __forceinline__ unsigned shard_of(unsigned long long key, unsigned nshards) {
     return (unsigned)__umul64hi(hj_mix64(key ^ 0x5ca1ab1e5eed0001ull), (unsigned long long)nshards);
@@ -43,17 +56,31 @@ __device__ __forceinline__ void route_block_range(unsigned long long n, unsigned
     *hi = *lo + per < n ? *lo + per : n;
 }
 
-__global__ void __launch_bounds__(kRouteThreads) route_count(const tuple_v *__restrict__ in, unsigned long long n,
-                                                             unsigned nshards, uint32_t *__restrict__ blk_cnt) {
-    __shared__ uint32_t cnt[kRouteMaxShards];
-    if (threadIdx.x < kRouteMaxShards) cnt[threadIdx.x] = 0;
-    __syncthreads();
+__global__ void __launch_bounds__(kRouteThreads, kRouteCtas) route_count(const tuple_v *__restrict__ in,
+                                                                         unsigned long long n, unsigned nshards,
+                                                                         uint32_t *__restrict__ blk_cnt) {
+    __shared__ uint32_t cnt[kRouteThreads / 32][kRouteMaxShards][32];  // [warp][owner][lane]
+    const unsigned lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (unsigned s = 0; s < nshards; s++) cnt[w][s][lane] = 0;
     unsigned long long lo, hi;
     route_block_range(n, &lo, &hi);
-    for (unsigned long long i = lo + threadIdx.x; i < hi; i += blockDim.x)
-        atomicAdd(&cnt[shard_of(ld_stream(in + i).x, nshards)], 1u);
+    constexpr int U = 4;
+    for (unsigned long long i0 = lo + threadIdx.x; i0 < hi; i0 += U * kRouteThreads) {
+        tuple_v v[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) v[u] = i0 + u * kRouteThreads < hi ? ld_once_more(in + i0 + u * kRouteThreads) : make_ulonglong2(0, 0);
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (i0 + u * kRouteThreads < hi) cnt[w][shard_of(v[u].x, nshards)][lane]++;
+    }
     __syncthreads();
-    if (threadIdx.x < nshards) blk_cnt[(size_t)blockIdx.x * nshards + threadIdx.x] = cnt[threadIdx.x];
+    for (unsigned s = w; s < nshards; s += kRouteThreads / 32) {
+        uint32_t c = 0;
+#pragma unroll
+        for (int q = 0; q < kRouteThreads / 32; q++) c += cnt[q][s][lane];
+        c = __reduce_add_sync(0xffffffffu, c);
+        if (lane == 0) blk_cnt[(size_t)blockIdx.x * nshards + s] = c;
+    }
 }
 
 // One CTA of 1024 threads; lane = owner, warp w sums a contiguous run of block rows.
@@ -96,69 +123,93 @@ __global__ void __launch_bounds__(1024) route_offsets(const uint32_t *__restrict
     }
 }
 
-__global__ void __launch_bounds__(kRouteThreads) route_scatter(const tuple_v *__restrict__ in, unsigned long long n,
-                                                               unsigned nshards,
-                                                               const unsigned long long *__restrict__ blk_off,
-                                                               tuple_v *__restrict__ out, unsigned int *err) {
-    __shared__ unsigned long long base[kRouteMaxShards];  // next output index of each owner for this block
-    __shared__ uint32_t warp_tot[kRouteMaxShards][kRouteThreads / 32];
+__global__ void __launch_bounds__(kRouteThreads, kRouteCtas) route_scatter(const tuple_v *__restrict__ in,
+                                                                           unsigned long long n, unsigned nshards,
+                                                                           int owner_bits,
+                                                                           const unsigned long long *__restrict__ blk_off,
+                                                                           tuple_v *__restrict__ out, unsigned int *err) {
+    constexpr int NW = kRouteThreads / 32;
+    constexpr unsigned T = kRouteThreads * kRouteItems;
+    __shared__ __align__(16) tuple_v stage[T];
+    __shared__ uint8_t own_of[T];                         // owner of each staged tuple
+    __shared__ uint32_t wcnt[NW][kRouteMaxShards];        // a warp's tuples per owner, then its start in the tile
+    __shared__ unsigned long long gofs[kRouteMaxShards];  // output index of a staged tuple - its staged index
     const unsigned lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (threadIdx.x < nshards) base[threadIdx.x] = blk_off[(size_t)blockIdx.x * nshards + threadIdx.x];
-    __syncthreads();
+    const unsigned ltmask = lanemask_lt();
+    // Warp 0, lane = owner: the block's next output index.
+    unsigned long long base = 0;
+    if (w == 0 && lane < nshards) base = blk_off[(size_t)blockIdx.x * nshards + lane];
     unsigned long long lo, hi;
     route_block_range(n, &lo, &hi);
-    constexpr unsigned T = kRouteThreads * kRouteItems;
     for (unsigned long long t0 = lo; t0 < hi; t0 += T) {
-        // Thread t takes tuples [t * ITEMS, (t + 1) * ITEMS) of the tile, in order.
+        const unsigned m = hi - t0 < T ? (unsigned)(hi - t0) : T;
         tuple_v v[kRouteItems];
-        unsigned own[kRouteItems];
+        unsigned pr[kRouteItems];  // owner << 16 | rank within the warp; owner kRouteMaxShards: no tuple
 #pragma unroll
         for (int u = 0; u < kRouteItems; u++) {
-            const unsigned long long i = t0 + (unsigned long long)threadIdx.x * kRouteItems + u;
-            if (i < hi) {
-                v[u] = ld_stream(in + i);
-                own[u] = shard_of(v[u].x, nshards);
-            } else {
-                v[u] = make_ulonglong2(0, 0);
-                own[u] = kRouteMaxShards;
-            }
+            const unsigned j = (w * kRouteItems + u) * 32 + lane;
+            v[u] = j < m ? ld_stream(in + t0 + j) : make_ulonglong2(0, 0);
         }
-        unsigned long long my_pos[kRouteItems];
-        for (unsigned s = 0; s < nshards; s++) {
-            uint32_t c = 0;
+        wcnt[w][lane] = 0;
+        __syncwarp();
 #pragma unroll
-            for (int u = 0; u < kRouteItems; u++) c += own[u] == s;
-            // Exclusive scan of c across the block's threads (thread order = input order).
-            uint32_t incl = c;
+        for (int u = 0; u < kRouteItems; u++) {
+            const bool live = (w * kRouteItems + u) * 32 + lane < m;
+            const unsigned d = live ? shard_of(v[u].x, nshards) : 0u;
+            unsigned peers = __ballot_sync(0xffffffffu, live);
+            for (int b = 0; b < owner_bits; b++) {
+                const unsigned bit = (d >> b) & 1u;
+                peers &= __ballot_sync(0xffffffffu, bit) ^ (bit - 1u);  // bit ? ballot : ~ballot
+            }
+            const unsigned before = wcnt[w][d];
+            __syncwarp();
+            if (live && (peers & ltmask) == 0) wcnt[w][d] = before + __popc(peers);
+            __syncwarp();
+            pr[u] = ((live ? d : (unsigned)kRouteMaxShards) << 16) | (before + __popc(peers & ltmask));
+        }
+        __syncthreads();
+        if (w == 0) {
+            // Lane = owner: each warp's start within the owner's run, then the runs' starts in the tile.
+            uint32_t run = 0;
+#pragma unroll
+            for (int q = 0; q < NW; q++) {
+                const uint32_t c = wcnt[q][lane];
+                wcnt[q][lane] = run;
+                run += c;
+            }
+            uint32_t incl = run;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= (unsigned)o) incl += x;
+                const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= (unsigned)o) incl += y;
             }
-            if (lane == 31) warp_tot[s][w] = incl;
-            __syncthreads();
-            uint32_t before = 0, total = 0;
-            for (unsigned q = 0; q < kRouteThreads / 32; q++) {
-                const uint32_t x = warp_tot[s][q];
-                if (q < w) before += x;
-                total += x;
-            }
-            unsigned long long p = base[s] + before + incl - c;
+            const uint32_t start = incl - run;
 #pragma unroll
-            for (int u = 0; u < kRouteItems; u++)
-                if (own[u] == s) my_pos[u] = p++;
-            __syncthreads();
-            if (threadIdx.x == 0) base[s] += total;
+            for (int q = 0; q < NW; q++) wcnt[q][lane] += start;
+            gofs[lane] = base - start;
+            base += run;
         }
         __syncthreads();
 #pragma unroll
         for (int u = 0; u < kRouteItems; u++) {
-            if (own[u] >= nshards) continue;
-            if (my_pos[u] < n)
-                out[my_pos[u]] = v[u];
+            const unsigned d = pr[u] >> 16;
+            if (d == (unsigned)kRouteMaxShards) continue;
+            const unsigned p = wcnt[w][d] + (pr[u] & 0xffffu);
+            stage[p] = v[u];
+            own_of[p] = (uint8_t)d;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < kRouteItems; u++) {
+            const unsigned j = u * kRouteThreads + threadIdx.x;
+            if (j >= m) continue;
+            const unsigned long long dst = gofs[own_of[j]] + j;
+            if (dst < n)
+                out[dst] = stage[j];
             else
                 set_error(err, kErrBounds);
         }
+        __syncthreads();
     }
 }
 
@@ -168,7 +219,7 @@ namespace {
 size_t route_blocks(size_t n, int num_sms) {
     const size_t T = (size_t)hj::kRouteThreads * hj::kRouteItems;
     const size_t tiles = (n + T - 1) / T;
-    size_t b = (size_t)num_sms * 2;
+    size_t b = (size_t)num_sms * hj::kRouteCtas;
     if (tiles < b) b = tiles ? tiles : 1;
     return b;
 }
@@ -179,8 +230,8 @@ extern "C" {
 
 size_t hj_shard_route_scratch_bytes(size_t n, int nshards) {
     if (nshards < 1) nshards = 1;
-    // Enough for any device's SM count (the block count is at most 2 * 1024 SMs).
-    const size_t blocks = route_blocks(n, 1024);
+    // Enough for any device's SM count (up to 512 SMs at kRouteCtas blocks each).
+    const size_t blocks = route_blocks(n, 512);
     return a256(blocks * nshards * 4) + a256(blocks * nshards * 8) + 256;
 }
 
@@ -205,7 +256,9 @@ int hj_shard_route(const hj_tuple_t *in_dev, size_t n, int nshards, hj_tuple_t *
     hj::route_count<<<blocks, hj::kRouteThreads, 0, st>>>(in, n, (unsigned)nshards, blk_cnt);
     hj::route_offsets<<<1, 1024, 0, st>>>(blk_cnt, blocks, (unsigned)nshards, blk_off,
                                           reinterpret_cast<unsigned long long *>(counts_dev));
-    hj::route_scatter<<<blocks, hj::kRouteThreads, 0, st>>>(in, n, (unsigned)nshards, blk_off,
+    int owner_bits = 0;
+    while ((1 << owner_bits) < nshards) owner_bits++;
+    hj::route_scatter<<<blocks, hj::kRouteThreads, 0, st>>>(in, n, (unsigned)nshards, owner_bits, blk_off,
                                                             reinterpret_cast<hj::tuple_v *>(out_dev), err);
     return cudaGetLastError() == cudaSuccess ? HJ_OK : HJ_E_DEVICE;
 }
