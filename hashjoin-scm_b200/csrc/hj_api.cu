@@ -292,6 +292,7 @@ int hj_ctx_destroy(hj_ctx_t *c) {
         if (c->arena) cudaFree(c->arena);
         if (c->acc_host) cudaFreeHost(c->acc_host);
         if (c->small_buf) cudaFree(c->small_buf);
+        hj::free_copy_buffers(c);
         cudaEventDestroy(c->ev_h2d);
         cudaEventDestroy(c->ev_start);
         cudaEventDestroy(c->ev_mid);
@@ -369,8 +370,12 @@ int hj_join_ctx(hj_ctx_t *c, hj_algo_t algo, const hj_params_t *pin, const hj_tu
         ulonglong2 *s = reinterpret_cast<ulonglong2 *>(cur);
         cur += align256(nS * 16);
         if (timing) CU_OR(cudaEventRecord(c->ev_h2d, st), out->status = HJ_E_DEVICE);
-        CU_OR(cudaMemcpyAsync(r, R, nR * 16, cudaMemcpyHostToDevice, st), out->status = HJ_E_DEVICE);
-        CU_OR(cudaMemcpyAsync(s, S, nS * 16, cudaMemcpyHostToDevice, st), out->status = HJ_E_DEVICE);
+        const hj::HostCopy copies[2] = {{r, R, nR * 16}, {s, S, nS * 16}};
+        rc = hj::copy_in(c, copies, 2, (p.flags & HJ_F_PINNED_HOST) != 0, st);
+        if (rc) {
+            cudaStreamSynchronize(st);
+            return out->status = rc;
+        }
         dR = r;
         dS = s;
     }
@@ -644,8 +649,12 @@ static int join_mat(hj_ctx *c, hj_algo_t algo, const hj_params_t &p, const hj_tu
         ulonglong2 *s = reinterpret_cast<ulonglong2 *>(cur);
         cur += align256(nS * 16);
         if (timing) CU_OR(cudaEventRecord(c->ev_h2d, st), out->status = HJ_E_DEVICE);
-        CU_OR(cudaMemcpyAsync(r, R, nR * 16, cudaMemcpyHostToDevice, st), out->status = HJ_E_DEVICE);
-        CU_OR(cudaMemcpyAsync(s, S, nS * 16, cudaMemcpyHostToDevice, st), out->status = HJ_E_DEVICE);
+        const hj::HostCopy copies[2] = {{r, R, nR * 16}, {s, S, nS * 16}};
+        rc = hj::copy_in(c, copies, 2, (p.flags & HJ_F_PINNED_HOST) != 0, st);
+        if (rc) {
+            cudaStreamSynchronize(st);
+            return out->status = rc;
+        }
         dR = r;
         dS = s;
     }

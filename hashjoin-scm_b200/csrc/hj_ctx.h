@@ -49,6 +49,8 @@ struct hj_ctx {
     char *arena = nullptr;
     size_t arena_bytes = 0;
     hj::JoinAccum *acc_host = nullptr;  // pinned
+    char *copy_buf = nullptr;           // page-locked pieces of copies from pageable memory (hj_hostcopy.cu)
+    std::vector<cudaEvent_t> copy_ev;   // one per piece: its last copy has been read
     char *small_buf = nullptr;          // device: the ticket and partial results of one-kernel joins
     bool gave_up = false;               // a watchdog gave up on a join: the next one waits for ev_done
     hj_tuner_t tuner = {};              // autotuner state used by batches
@@ -63,3 +65,16 @@ struct hj_ctx {
     size_t lp_ordered_nR = 0;
     std::mutex mu;
 };
+
+namespace hj {
+// Copies of host memory to the device on `st`: through the context's page-locked pieces when they are pageable
+// and large enough. The caller holds c->mu; a source has been read when the call returns, or (plain copies
+// of page-locked memory) when the stream gets there.
+struct HostCopy {
+    void *dst;
+    const void *src;
+    size_t bytes;
+};
+int copy_in(hj_ctx *c, const HostCopy *copies, int ncopies, bool pinned, cudaStream_t st);
+void free_copy_buffers(hj_ctx *c);
+}  // namespace hj
