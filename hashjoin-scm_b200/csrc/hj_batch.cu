@@ -10,13 +10,15 @@
 //      (phj_radix_lp) - are kept whichever implementation runs, so results equal the named algorithm's.
 //      With HJ_F_TUNE the budget is chosen by timing the batch's own graph under several budgets; a
 //      calibrated cost model (hj_tuner_calibrate) serves single joins;
-//   2. packs the non-partitioned joins into waves whose tables together stay within the wave budget,
-//      and runs each wave as one set of multi-join kernels over a flattened index space (build over all
-//      build tuples of the wave, then probe over all probe tuples), so the tables are still in L2 when
-//      probed;
-//   3. enqueues the partitioned joins on up to kPhjLanes streams forked from the first (each with its own
-//      scratch area; largest joins first, each on the least loaded stream), so they overlap the waves
-//      and each other;
+//   2. packs the joins into waves by the tuner's table budget, whatever implementation it decided (results do
+//      not depend on it), and runs each wave as one launch per step over all its joins: one shared-memory
+//      table per probe range for joins of at most 8192 build tuples, the one-pass radix pipeline for the
+//      others (hj_wave.cuh). Waves alternate between three streams. When that scratch (16 bytes a tuple)
+//      cannot be had, waves of global tables run instead: one multi-join build and one probe kernel, bound
+//      by the L2's atomic rate (96 joins of 2^10..2^22 build tuples: 10.7 ms, 6.3 in one pass);
+//   3. enqueues the joins that are too large for a wave on up to kPhjLanes streams forked from the first (each
+//      with its own scratch area; largest joins first, each on the least loaded stream), so they overlap
+//      the waves and each other;
 //   4. captures the whole sequence in a CUDA graph once (parallel branches), so a run is one graph
 //      launch.
 #include <algorithm>
@@ -307,13 +309,26 @@ unsigned long long nphj_slots(size_t nR) { return hj::mj_slots(nR); }
 // branches when their scratch would take more than a quarter of the free device memory. (512 joins:
 // 40.4 ms on one branch, 33.7 on four, 33.0 on eight.)
 constexpr int kPhjLanes = 8;
+// Waves of one-pass joins alternate between this many branches, each with the scratch of its largest wave, so
+// that one wave's kernels fill the SMs that the end of another's leaves idle (96 joins: one branch 7.7 ms, two
+// 6.6, three 6.3, four 6.3).
+constexpr int kWaveLanes = 3;
 
 struct hj_batch {
     hj_ctx *ctx = nullptr;
     int njobs = 0;
     std::vector<hj_batch_job_t> jobs;
     std::vector<int> impl, bits, passes;
-    std::vector<Wave> waves;
+    std::vector<Wave> waves;          // table waves (when scratch is short)
+    struct OnePassWave {
+        hj::WavePlan wp;
+        const char *image;            // device
+        int lane;
+    };
+    std::vector<OnePassWave> onewaves;  // waves of one-pass and small joins
+    int wave_lanes = 1;
+    cudaStream_t stream_wave[kWaveLanes] = {};  // [0] is `stream`
+    cudaEvent_t ev_wave[kWaveLanes] = {};
     std::vector<int> phj_jobs;
     char *mem = nullptr;
     size_t mem_bytes = 0;
@@ -383,6 +398,15 @@ void decide(const hj_ctx *c, size_t nR, size_t nS, int *impl, int *bits, int *pa
         }                                                                              \
     } while (0)
 
+// Geometry of a join that runs a pipeline of its own: the tuner's, or for a join decided as non-partitioned
+// (too large for a wave) the two-pass one that its size needs.
+int lane_geom(const hj_batch *b, int j, hj::RadixGeom *g) {
+    if (b->impl[j] == kImplPhj) return hj::radix_geom(b->bits[j], b->passes[j], g);
+    const int rc = hj::radix_geom(14, 2, g);
+    hj::radix_geom_by_size(b->jobs[j].nR, g);
+    return rc;
+}
+
 int enqueue_batch(hj_batch *b) {
     const int sms = b->ctx->num_sms;
     cudaStream_t st = b->stream;
@@ -392,11 +416,17 @@ int enqueue_batch(hj_batch *b) {
     // the waves of non-partitioned joins or with each other, and their kernels fill the SMs that a
     // wave's small kernels, or a small pipeline's, leave idle (in the captured graph these become
     // parallel branches).
-    const bool fork = !b->phj_jobs.empty();
-    const int lanes = fork ? b->phj_lanes : 0;
+    const int wlanes = b->onewaves.size() > 1 ? b->wave_lanes : 1;
+    const bool fork = !b->phj_jobs.empty() || wlanes > 1;
+    const int lanes = b->phj_jobs.empty() ? 0 : b->phj_lanes;
     if (fork) {
         BCU(cudaEventRecord(b->ev_fork, st));
         for (int l = 0; l < lanes; l++) BCU(cudaStreamWaitEvent(b->stream_phj[l], b->ev_fork, 0));
+        for (int l = 1; l < wlanes; l++) BCU(cudaStreamWaitEvent(b->stream_wave[l], b->ev_fork, 0));
+    }
+    for (const hj_batch::OnePassWave &w : b->onewaves) {
+        const int rc = hj::wave_enqueue(w.wp, w.image, w.lane ? b->stream_wave[w.lane] : st, &launches);
+        if (rc) return rc;
     }
     for (const Wave &w : b->waves) {
         if (w.total_r == 0 && w.total_s == 0) continue;
@@ -430,7 +460,7 @@ int enqueue_batch(hj_batch *b) {
             if (load[q] < load[l]) l = q;
         load[l] += J.nR + J.nS;
         hj::RadixGeom g;
-        if (hj::radix_geom(b->bits[j], b->passes[j], &g)) return HJ_E_INVAL;
+        if (lane_geom(b, j, &g)) return HJ_E_INVAL;
         hj::PhjScratch s;
         hj::phj_carve(g, J.nR, J.nS, sms, b->phj_scratch + (size_t)l * b->phj_lane_bytes, &s);
         uint32_t nl = 0;
@@ -443,6 +473,10 @@ int enqueue_batch(hj_batch *b) {
     for (int l = 0; l < lanes; l++) {
         BCU(cudaEventRecord(b->ev_join[l], b->stream_phj[l]));
         BCU(cudaStreamWaitEvent(st, b->ev_join[l], 0));
+    }
+    for (int l = 1; l < wlanes; l++) {
+        BCU(cudaEventRecord(b->ev_wave[l], b->stream_wave[l]));
+        BCU(cudaStreamWaitEvent(st, b->ev_wave[l], 0));
     }
     b->launches = launches;
     return HJ_OK;
@@ -470,7 +504,14 @@ int hj_tuner_decide(hj_ctx_t *c, size_t nR, size_t nS, int *impl, int *bits, int
     return HJ_OK;
 }
 
-static int plan_one(hj_ctx_t *c, const hj_batch_job_t *jobs, int njobs, const hj_params_t *p, hj_batch_t **out);
+static int plan_tables(hj_ctx_t *c, const hj_batch_job_t *jobs, int njobs, const hj_params_t *p, bool tables,
+                       hj_batch_t **out);
+
+// Waves of one-pass joins; when their scratch cannot be had, waves over global tables, which need less.
+static int plan_one(hj_ctx_t *c, const hj_batch_job_t *jobs, int njobs, const hj_params_t *p, hj_batch_t **out) {
+    const int rc = plan_tables(c, jobs, njobs, p, false, out);
+    return rc == HJ_E_OOM ? plan_tables(c, jobs, njobs, p, true, out) : rc;
+}
 
 // Empirical tuning of a batch (HJ_F_TUNE): plan it under a few table budgets around the current one,
 // time each plan's graph, keep the fastest and leave its budget in the context's tuner. Timings of
@@ -531,7 +572,8 @@ int hj_batch_plan(hj_ctx_t *c, const hj_batch_job_t *jobs, int njobs, const hj_p
     return HJ_OK;
 }
 
-static int plan_one(hj_ctx_t *c, const hj_batch_job_t *jobs, int njobs, const hj_params_t *p, hj_batch_t **out) {
+static int plan_tables(hj_ctx_t *c, const hj_batch_job_t *jobs, int njobs, const hj_params_t *p, bool tables,
+                       hj_batch_t **out) {
     if (!c || !out || njobs < 0 || (njobs && !jobs)) return HJ_E_INVAL;
     *out = nullptr;
     for (int j = 0; j < njobs; j++) {
@@ -556,7 +598,9 @@ static int plan_one(hj_ctx_t *c, const hj_batch_job_t *jobs, int njobs, const hj
     double acc = 0;
     int wfirst = 0;
     for (int j = 0; j < njobs; j++) {
-        if (b->impl[j] != kImplNphj) {
+        // What a join reports does not depend on how it ran: one-pass waves take every join that their
+        // geometry fits, whatever the tuner decided.
+        if (tables ? b->impl[j] != kImplNphj : !hj::wave_takes(jobs[j].nR, jobs[j].nS)) {
             b->phj_jobs.push_back(j);
             continue;
         }
@@ -574,6 +618,41 @@ static int plan_one(hj_ctx_t *c, const hj_batch_job_t *jobs, int njobs, const hj
     // Device memory of the batch: results, wave tables (the largest wave), wave descriptors, and the
     // scratch of the largest partitioned join.
     size_t max_wave_tables = 0, desc_bytes = 0;
+    // The joins of wave wr; their result records are set once there is memory.
+    auto wave_joins = [&](const std::pair<int, int> &wr) {
+        std::vector<hj::WaveJoin> v;
+        for (int q = 0; q < wr.second; q++) {
+            const hj_batch_job_t &J = jobs[order[wr.first + q]];
+            hj::WaveJoin w;
+            w.lp = sem_lp(J.algo);
+            w.skip0 = sem_skip0(J.algo);
+            w.R = reinterpret_cast<const ulonglong2 *>(J.R);
+            w.nR = J.nR;
+            w.S = reinterpret_cast<const ulonglong2 *>(J.S);
+            w.nS = J.nS;
+            w.acc = b->accs + order[wr.first + q];
+            v.push_back(w);
+        }
+        return v;
+    };
+    size_t lane_bytes[kWaveLanes] = {};
+    auto lane_total = [&] {
+        size_t t = 0;
+        for (size_t x : lane_bytes) t += x;
+        return t;
+    };
+    if (!tables) {
+        for (size_t i = 0; i < wave_ranges.size(); i++) {
+            const std::vector<hj::WaveJoin> v = wave_joins(wave_ranges[i]);
+            hj_batch::OnePassWave w;
+            hj::wave_plan(v.data(), v.size(), c->num_sms, &w.wp);
+            w.image = nullptr;
+            w.lane = (int)(i % kWaveLanes);
+            lane_bytes[w.lane] = std::max(lane_bytes[w.lane], a256(w.wp.scratch_bytes));
+            desc_bytes += a256(w.wp.image_bytes);
+            b->onewaves.push_back(w);
+        }
+    } else
     for (auto &wr : wave_ranges) {
         size_t t = 0;
         for (int q = 0; q < wr.second; q++) t += nphj_slots(jobs[order[wr.first + q]].nR) * 16;
@@ -590,7 +669,7 @@ static int plan_one(hj_ctx_t *c, const hj_batch_job_t *jobs, int njobs, const hj
     size_t phj_bytes = 0;
     for (int j : b->phj_jobs) {
         hj::RadixGeom g;
-        if (hj::radix_geom(b->bits[j], b->passes[j], &g)) {
+        if (lane_geom(b, j, &g)) {
             delete b;
             return HJ_E_INVAL;
         }
@@ -612,6 +691,16 @@ static int plan_one(hj_ctx_t *c, const hj_batch_job_t *jobs, int njobs, const hj
         size_t lanes = std::min<size_t>(kPhjLanes, b->phj_jobs.size() ? b->phj_jobs.size() : 1);
         while (lanes > 1 && lanes * b->phj_lane_bytes > free_b / 4) lanes--;
         b->phj_lanes = (int)lanes;
+        b->wave_lanes = kWaveLanes;
+        if (lane_total() > free_b / 4) {  // one branch
+            b->wave_lanes = 1;
+            for (size_t &x : lane_bytes) {
+                lane_bytes[0] = std::max(lane_bytes[0], x);
+                if (&x != lane_bytes) x = 0;
+            }
+            for (hj_batch::OnePassWave &w : b->onewaves) w.lane = 0;
+        }
+        max_wave_tables += lane_total();
     }
     b->mem_bytes = acc_bytes + max_wave_tables + desc_bytes + (size_t)b->phj_lanes * b->phj_lane_bytes;
     int dev_prev = -1;
@@ -635,12 +724,32 @@ static int plan_one(hj_ctx_t *c, const hj_batch_job_t *jobs, int njobs, const hj
         if (cudaStreamCreateWithFlags(&b->stream_phj[l], cudaStreamNonBlocking) != cudaSuccess ||
             cudaEventCreateWithFlags(&b->ev_join[l], cudaEventDisableTiming) != cudaSuccess)
             return fail(HJ_E_DEVICE);
+    for (int l = 0; l < kWaveLanes; l++)
+        if (cudaStreamCreateWithFlags(&b->stream_wave[l], cudaStreamNonBlocking) != cudaSuccess ||
+            cudaEventCreateWithFlags(&b->ev_wave[l], cudaEventDisableTiming) != cudaSuccess)
+            return fail(HJ_E_DEVICE);
     if (cudaEventCreate(&b->e0) != cudaSuccess || cudaEventCreate(&b->e1) != cudaSuccess) return fail(HJ_E_DEVICE);
     char *cur = b->mem;
     b->accs = reinterpret_cast<JoinAccum *>(cur);
     cur += acc_bytes;
-    char *tables = cur;
+    char *table_area = cur;
     cur += max_wave_tables;
+    auto lane_area = [&](int lane) {
+        char *p = table_area;
+        for (int l = 0; l < lane; l++) p += lane_bytes[l];
+        return p;
+    };
+    for (size_t i = 0; i < b->onewaves.size(); i++) {
+        hj_batch::OnePassWave &w = b->onewaves[i];
+        const std::vector<hj::WaveJoin> v = wave_joins(wave_ranges[i]);
+        std::vector<char> image(w.wp.image_bytes ? w.wp.image_bytes : 1);
+        if (hj::wave_image(v.data(), v.size(), c->num_sms, w.wp, lane_area(w.lane), image.data()))
+            return fail(HJ_E_INVAL);
+        if (cudaMemcpy(cur, image.data(), w.wp.image_bytes, cudaMemcpyHostToDevice) != cudaSuccess) return fail(HJ_E_DEVICE);
+        w.image = cur;
+        cur += a256(w.wp.image_bytes);
+    }
+    if (tables)
     for (auto &wr : wave_ranges) {
         Wave w;
         w.first = wr.first;
@@ -648,10 +757,10 @@ static int plan_one(hj_ctx_t *c, const hj_batch_job_t *jobs, int njobs, const hj
         std::vector<hj::MJob> mj(w.count);
         std::vector<unsigned long long> rf(w.count + 1, 0), sf(w.count + 1, 0), tf(w.count + 1, 0);
         std::vector<hj::MChunk> rch, sch;
-        char *tp = tables;
+        char *tp = table_area;
         size_t slots_total = 0;
         for (int q = 0; q < w.count; q++) slots_total += nphj_slots(jobs[order[w.first + q]].nR);
-        hj::MSide *sides = reinterpret_cast<hj::MSide *>(tables + slots_total * 16);
+        hj::MSide *sides = reinterpret_cast<hj::MSide *>(table_area + slots_total * 16);
         w.any_lp = false;
         for (int q = 0; q < w.count; q++) {
             const int j = order[w.first + q];
@@ -676,7 +785,7 @@ static int plan_one(hj_ctx_t *c, const hj_batch_job_t *jobs, int njobs, const hj
             sf[q + 1] = sf[q] + J.nS;
             tf[q + 1] = tf[q] + m.cap;
         }
-        w.tables = reinterpret_cast<ulonglong2 *>(tables);
+        w.tables = reinterpret_cast<ulonglong2 *>(table_area);
         w.sides = sides;
         w.total_r = rf[w.count];
         w.total_s = sf[w.count];
@@ -749,7 +858,7 @@ int hj_batch_run(hj_batch_t *b, hj_batch_result_t *results, hj_batch_stats_t *st
         memset(stats, 0, sizeof(*stats));
         stats->seconds = ms * 1e-3;
         stats->kernel_launches = b->launches;
-        stats->waves = (int)b->waves.size();
+        stats->waves = (int)(b->waves.size() + b->onewaves.size());
         for (int j = 0; j < b->njobs; j++) stats->nphj_jobs += b->impl[j] == kImplNphj;
         stats->phj_jobs = b->njobs - stats->nphj_jobs;
     }
@@ -780,6 +889,10 @@ int hj_batch_destroy(hj_batch_t *b) {
     for (int l = 0; l < kPhjLanes; l++) {
         if (b->stream_phj[l]) cudaStreamDestroy(b->stream_phj[l]);
         if (b->ev_join[l]) cudaEventDestroy(b->ev_join[l]);
+    }
+    for (int l = 0; l < kWaveLanes; l++) {
+        if (b->stream_wave[l]) cudaStreamDestroy(b->stream_wave[l]);
+        if (b->ev_wave[l]) cudaEventDestroy(b->ev_wave[l]);
     }
     if (b->ev_fork) cudaEventDestroy(b->ev_fork);
     delete b;

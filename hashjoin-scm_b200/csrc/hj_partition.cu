@@ -1374,31 +1374,6 @@ __device__ __forceinline__ uint32_t atomic_exch_u16(uint16_t *addr, uint32_t val
     return (assumed >> shift) & 0xffffu;
 }
 
-struct JoinArgs {
-    const JoinItem *items;
-    const LargePart *large;
-    uint32_t *counters;
-    const tuple_v *finR, *finS;
-    uint32_t *large_table;
-    int bits;
-    int lp;     // first match per probe tuple (lowest build position) instead of all matches
-    int skip0;  // build tuples with key 0 never match (key 0 marks an empty slot in lp_join)
-    JoinAccum *acc;
-    MatOut mat; // materialising joins (MAT kernels): where the (r.row_id, s.row_id) pairs go
-    int ci;     // the final partitions may be compact words (when ci_applies holds) at finR8 / finS8
-    const unsigned long long *finR8, *finS8;
-    // First-match joins of the one-pass pipeline: build elements are {ci_word or key, input position}, and
-    // a wide match reads its row id from the build relation itself.
-    int lp_pos;
-    const tuple_v *relR;
-    uint64_t nR;
-    int flag_bits;  // HJ_RES_COMPACT_PARTITIONS tells whether words of this many radix bits fit
-    // One-pass pipeline: one launch takes the items of every size; host_out: see join_finish.
-    int all_items;
-    JoinAccum *host_out;
-    int w8_b1;  // a pass 1 that may store words (either pipeline): its shift (reported when w8_fits held); -1 otherwise
-};
-
 // A tuple of a final partition: the stored tuple, or for compact partitions {key >> bits, row id}.
 // Joins compare x for equality and hash x >> shift with shift = bits (tuples) or 0 (compact words).
 __device__ __forceinline__ tuple_v ld_fin(const tuple_v *p16, const unsigned long long *p8, uint64_t i, bool ci) {
@@ -1635,7 +1610,15 @@ static_assert(kOaSmem >= (size_t)kSmemCap * 10 + kOaHeads * 2, "the chains fit t
 
 __device__ __forceinline__ uint32_t oa_hash(uint32_t hi) { return hi * 0x9e3779b1u; }
 
-__global__ void __launch_bounds__(kCompactThreads, 2) join_words_kernel(JoinArgs a) {
+template <bool MULTI>
+__global__ void __launch_bounds__(kCompactThreads, 2) join_words_kernel(JoinArgs a0, MultiRef mr) {
+    __shared__ JoinArgs s_a;
+    if (MULTI) {
+        const uint2 e = mr.map[blockIdx.x];
+        multi_copy(&s_a, &mr.jobs[e.x].ja);
+        __syncthreads();
+    }
+    const JoinArgs &a = MULTI ? s_a : a0;
     extern __shared__ __align__(128) unsigned char smem[];
     unsigned long long *slots = reinterpret_cast<unsigned long long *>(smem);
     __shared__ unsigned long long red[64];
@@ -1775,7 +1758,15 @@ __global__ void __launch_bounds__(kCompactThreads, 2) join_words_kernel(JoinArgs
 constexpr uint32_t kFwSlots = 16384;
 constexpr size_t kFwSmem = (size_t)kFwSlots * 12 + kFwSlots / 8;
 
-__global__ void __launch_bounds__(kJoinThreads, 1) join_first_words_kernel(JoinArgs a) {
+template <bool MULTI>
+__global__ void __launch_bounds__(kJoinThreads, 1) join_first_words_kernel(JoinArgs a0, MultiRef mr) {
+    __shared__ JoinArgs s_a;
+    if (MULTI) {
+        const uint2 e = mr.map[blockIdx.x];
+        multi_copy(&s_a, &mr.jobs[e.x].ja);
+        __syncthreads();
+    }
+    const JoinArgs &a = MULTI ? s_a : a0;
     extern __shared__ __align__(128) unsigned char smem[];
     unsigned long long *slots = reinterpret_cast<unsigned long long *>(smem);  // [kFwSlots]
     uint32_t *rid = reinterpret_cast<uint32_t *>(slots + kFwSlots);             // [kFwSlots]
@@ -1896,8 +1887,15 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_words_kernel(JoinA
 constexpr uint32_t kFirstHeads = 8192;
 constexpr size_t kFirstSmem = (size_t)kFirstCap * (8 + 8 + 4 + 2) + kFirstHeads * 2;
 
-template <bool MAT>
-__global__ void __launch_bounds__(kJoinThreads, 1) join_first_kernel(JoinArgs a) {
+template <bool MAT, bool MULTI = false>
+__global__ void __launch_bounds__(kJoinThreads, 1) join_first_kernel(JoinArgs a0, MultiRef mr) {
+    __shared__ JoinArgs s_a;
+    if (MULTI) {
+        const uint2 e = mr.map[blockIdx.x];
+        multi_copy(&s_a, &mr.jobs[e.x].ja);
+        __syncthreads();
+    }
+    const JoinArgs &a = MULTI ? s_a : a0;
     extern __shared__ __align__(128) unsigned char smem[];
     unsigned long long *kx = reinterpret_cast<unsigned long long *>(smem);  // [kFirstCap] keys
     unsigned long long *rid = kx + kFirstCap;                              // [kFirstCap]
@@ -2005,8 +2003,15 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_kernel(JoinArgs a)
     join_finish(a, false);
 }
 
-template <bool MAT, bool CI = false>
-__global__ void __launch_bounds__(kJoinThreads, 1) join_small_kernel(JoinArgs a) {
+template <bool MAT, bool CI = false, bool MULTI = false>
+__global__ void __launch_bounds__(kJoinThreads, 1) join_small_kernel(JoinArgs a0, MultiRef mr) {
+    __shared__ JoinArgs s_a;
+    if (MULTI) {
+        const uint2 e = mr.map[blockIdx.x];
+        multi_copy(&s_a, &mr.jobs[e.x].ja);
+        __syncthreads();
+    }
+    const JoinArgs &a = MULTI ? s_a : a0;
     extern __shared__ __align__(128) unsigned char smem[];
     tuple_v *rt = reinterpret_cast<tuple_v *>(smem);                      // [kSmemCap]
     uint16_t *head = reinterpret_cast<uint16_t *>(rt + kSmemCap);         // [kHeadMax]
@@ -2194,10 +2199,10 @@ __device__ __forceinline__ int find_large(const LargePart *L, int nl, uint64_t g
     return lo;
 }
 
-__global__ void join_large_clear(JoinArgs a) {
+__device__ __forceinline__ void large_clear(const JoinArgs &a, uint32_t blk, uint32_t nblk) {
     const uint64_t words = ld_u64_pair(&a.counters[kCtrLargeWords]);
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < words;
-         i += (uint64_t)gridDim.x * blockDim.x)
+    for (uint64_t i = blk * (uint64_t)blockDim.x + threadIdx.x; i < words;
+         i += (uint64_t)nblk * blockDim.x)
         a.large_table[i] = 0;
 }
 
@@ -2257,7 +2262,7 @@ __device__ __forceinline__ uint32_t large_agg_find_or_insert(const LargeAgg &t, 
     }
 }
 
-__global__ void join_large_build(JoinArgs a) {
+__device__ __forceinline__ void large_build(const JoinArgs &a, uint32_t blk, uint32_t nblk) {
     const int nl = (int)a.counters[kCtrNLarge];
     const uint64_t total = ld_u64_pair(&a.counters[kCtrLargeR]);
     const bool ci = a.ci && ci_applies(a.counters, a.bits);
@@ -2266,8 +2271,8 @@ __global__ void join_large_build(JoinArgs a) {
         // Warp-uniform rounds: lanes holding equal keys of one partition combine their count, row-id sum
         // and smallest position first, so a hot key costs one update per warp.
         const unsigned lane = threadIdx.x & 31;
-        for (uint64_t g0 = blockIdx.x * (uint64_t)blockDim.x + (threadIdx.x & ~31u); g0 < total;
-             g0 += (uint64_t)gridDim.x * blockDim.x) {
+        for (uint64_t g0 = blk * (uint64_t)blockDim.x + (threadIdx.x & ~31u); g0 < total;
+             g0 += (uint64_t)nblk * blockDim.x) {
             const uint64_t g = g0 + lane;
             bool act = g < total;
             int l = 0;
@@ -2304,8 +2309,8 @@ __global__ void join_large_build(JoinArgs a) {
         }
         return;
     }
-    for (uint64_t g = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; g < total;
-         g += (uint64_t)gridDim.x * blockDim.x) {
+    for (uint64_t g = blk * (uint64_t)blockDim.x + threadIdx.x; g < total;
+         g += (uint64_t)nblk * blockDim.x) {
         const int l = find_large(a.large, nl, g, true);
         const LargePart &L = a.large[l];
         const uint64_t i = g - L.r_flat;
@@ -2319,7 +2324,7 @@ __global__ void join_large_build(JoinArgs a) {
 }
 
 template <bool MAT>
-__global__ void join_large_probe(JoinArgs a) {
+__device__ __forceinline__ void large_probe(const JoinArgs &a, uint32_t blk, uint32_t nblk) {
     __shared__ unsigned long long red[64];
     __shared__ uint32_t scan_tmp[32];
     __shared__ unsigned long long s_base;
@@ -2332,7 +2337,7 @@ __global__ void join_large_probe(JoinArgs a) {
     if constexpr (MAT) {
         unsigned int *err = &a.counters[kCtrErr];
         // Block-uniform rounds over the flattened probe tuples of all large partitions.
-        for (uint64_t g0 = blockIdx.x * (uint64_t)blockDim.x; g0 < total; g0 += (uint64_t)gridDim.x * blockDim.x) {
+        for (uint64_t g0 = blk * (uint64_t)blockDim.x; g0 < total; g0 += (uint64_t)nblk * blockDim.x) {
             const uint64_t g = g0 + threadIdx.x;
             uint32_t m = 0, best = 0, e0 = 0;
             tuple_v s = make_ulonglong2(0, 0);
@@ -2374,8 +2379,8 @@ __global__ void join_large_probe(JoinArgs a) {
             }
         }
     } else if (a.counters[kCtrLargeAgg]) {
-        for (uint64_t g = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; g < total;
-             g += (uint64_t)gridDim.x * blockDim.x) {
+        for (uint64_t g = blk * (uint64_t)blockDim.x + threadIdx.x; g < total;
+             g += (uint64_t)nblk * blockDim.x) {
             const int l = find_large(a.large, nl, g, false);
             const LargePart &L = a.large[l];
             const tuple_v s = ld_fin(a.finS, a.finS8, L.s_begin + (g - L.s_flat), ci);
@@ -2406,8 +2411,8 @@ __global__ void join_large_probe(JoinArgs a) {
             }
         }
     } else
-    for (uint64_t g = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; g < total;
-         g += (uint64_t)gridDim.x * blockDim.x) {
+    for (uint64_t g = blk * (uint64_t)blockDim.x + threadIdx.x; g < total;
+         g += (uint64_t)nblk * blockDim.x) {
         const int l = find_large(a.large, nl, g, false);
         const LargePart &L = a.large[l];
         const tuple_v s = ld_fin(a.finS, a.finS8, L.s_begin + (g - L.s_flat), ci);
@@ -2445,12 +2450,41 @@ __global__ void join_large_probe(JoinArgs a) {
     }
     block_sum2_to(cnt, sum, red, &a.acc->matched, &a.acc->checksum);
     if (!MAT) flag_multi(multi, &a.acc->dup_flag);
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (blk == 0 && threadIdx.x == 0) {
         if (nl) atomicAdd(&a.acc->large_parts, (unsigned long long)nl);
         if (!MAT && a.ci && ci_applies(a.counters, a.flag_bits))
             atomicOr(&a.acc->flags, (unsigned long long)HJ_RES_COMPACT_PARTITIONS);
         if (a.w8_b1 >= 0 && w8_fits(a.counters, a.w8_b1))
             atomicOr(&a.acc->flags, (unsigned long long)HJ_RES_WORD_PASS1);
+    }
+}
+
+__global__ void join_large_clear(JoinArgs a) { large_clear(a, blockIdx.x, gridDim.x); }
+__global__ void join_large_build(JoinArgs a) { large_build(a, blockIdx.x, gridDim.x); }
+template <bool MAT>
+__global__ void join_large_probe(JoinArgs a) {
+    large_probe<MAT>(a, blockIdx.x, gridDim.x);
+}
+
+// End of a wave, one block per join: its partitions beyond shared memory (rare: the block takes all three
+// steps by itself) and its error word.
+__global__ void __launch_bounds__(kJoinThreads, 1) multi_finish(const MultiJob *jobs) {
+    __shared__ JoinArgs a;
+    multi_copy(&a, &jobs[blockIdx.x].ja);
+    __syncthreads();
+    if (a.counters[kCtrNLarge]) {
+        large_clear(a, 0, 1);
+        __threadfence();
+        __syncthreads();
+        large_build(a, 0, 1);
+        __threadfence();
+        __syncthreads();
+        large_probe<false>(a, 0, 1);
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        const uint32_t e = *reinterpret_cast<const volatile uint32_t *>(&a.counters[kCtrErr]);
+        if (e) atomicOr(&a.acc->error, e);
     }
 }
 
@@ -2737,8 +2771,13 @@ int phj_prepare_device() {
                                (int)kCompactSmem));
     HJ_CU(cudaFuncSetAttribute(join_compact_kernel<true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)kCompactSmem));
-    HJ_CU(cudaFuncSetAttribute(join_words_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOaSmem));
-    HJ_CU(cudaFuncSetAttribute(join_first_words_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwSmem));
+    HJ_CU(cudaFuncSetAttribute(join_words_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOaSmem));
+    HJ_CU(cudaFuncSetAttribute(join_words_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOaSmem));
+    HJ_CU(cudaFuncSetAttribute(join_first_words_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwSmem));
+    HJ_CU(cudaFuncSetAttribute(join_first_words_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwSmem));
+    HJ_CU(cudaFuncSetAttribute(join_first_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFirstSmem));
+    HJ_CU(cudaFuncSetAttribute(join_small_kernel<false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)kJoinSmem));
     HJ_CU(cudaFuncSetAttribute(join_first_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFirstSmem));
     HJ_CU(cudaFuncSetAttribute(join_first_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFirstSmem));
     HJ_CU(cudaFuncSetAttribute(join_small_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kJoinSmem));
@@ -2755,9 +2794,9 @@ int phj_prepare_device() {
     return nphj_prepare_device();
 }
 
-static JoinArgs join_args(const RadixGeom &g, bool lp, bool skip0, const ulonglong2 *R, size_t nR, const PhjScratch &s,
+JoinArgs join_args(const RadixGeom &g, bool lp, bool skip0, const ulonglong2 *R, size_t nR, const PhjScratch &s,
                           JoinAccum *acc, const MatOut *mat, int ci_ok, int w8_b1, JoinAccum *host_out) {
-    JoinArgs ja;
+    JoinArgs ja = {};
     ja.items = reinterpret_cast<const JoinItem *>(s.items);
     ja.large = reinterpret_cast<const LargePart *>(s.large);
     ja.counters = s.counters;
@@ -2791,6 +2830,26 @@ static int large_launch(const JoinArgs &ja, bool mat, const PhjScratch &s, JoinA
     else
         join_large_probe<false><<<num_sms * 2, 256, 0, st>>>(ja);
     copy_error<<<1, 32, 0, st>>>(s.counters, acc);
+    HJ_CU(cudaGetLastError());
+    return HJ_OK;
+}
+
+int multi_join_launch(const MultiJob *jobs, int njobs, const uint2 *every_map, unsigned every_blocks,
+                      const uint2 *first_map, unsigned first_blocks, cudaStream_t st, uint32_t *launches) {
+    const JoinArgs none = {};
+    const MultiRef every = {jobs, every_map}, first = {jobs, first_map};
+    if (every_blocks) {
+        join_words_kernel<true><<<every_blocks, kCompactThreads, kOaSmem, st>>>(none, every);
+        join_small_kernel<false, false, true><<<every_blocks, kJoinThreads, kJoinSmem, st>>>(none, every);
+        *launches += 2;
+    }
+    if (first_blocks) {
+        join_first_words_kernel<true><<<first_blocks, kJoinThreads, kFwSmem, st>>>(none, first);
+        join_first_kernel<false, true><<<first_blocks, kJoinThreads, kFirstSmem, st>>>(none, first);
+        *launches += 2;
+    }
+    multi_finish<<<njobs, kJoinThreads, 0, st>>>(jobs);
+    *launches += 1;
     HJ_CU(cudaGetLastError());
     return HJ_OK;
 }
@@ -3044,13 +3103,14 @@ int phj_enqueue(const RadixGeom &g, bool lp, bool skip0, const ulonglong2 *R, si
     // 6. joins
     const JoinArgs ja = join_args(g, lp, skip0, R, nR, s, acc, mat, ci_ok, (seg_words || exact_words) ? g.b1 : -1,
                                   g.single && !mat ? host_out : nullptr);
+    const MultiRef none = {};
     if (ja.lp_pos) {
         if (mat)
-            join_first_kernel<true><<<num_sms, kJoinThreads, kFirstSmem, st>>>(ja);
+            join_first_kernel<true><<<num_sms, kJoinThreads, kFirstSmem, st>>>(ja, none);
         else {
             // One launch per element layout; the one that does not match the device's choice returns at once.
-            join_first_words_kernel<<<num_sms, kJoinThreads, kFwSmem, st>>>(ja);
-            join_first_kernel<false><<<num_sms, kJoinThreads, kFirstSmem, st>>>(ja);
+            join_first_words_kernel<false><<<num_sms, kJoinThreads, kFwSmem, st>>>(ja, none);
+            join_first_kernel<false><<<num_sms, kJoinThreads, kFirstSmem, st>>>(ja, none);
             nlaunch++;
         }
         nlaunch++;
@@ -3059,12 +3119,12 @@ int phj_enqueue(const RadixGeom &g, bool lp, bool skip0, const ulonglong2 *R, si
             join_compact_kernel<true, false, true><<<num_sms * 2, kCompactThreads, kCompactSmem, st>>>(ja);
         else
             join_compact_kernel<true><<<num_sms * 2, kCompactThreads, kCompactSmem, st>>>(ja);
-        join_small_kernel<true><<<num_sms, kJoinThreads, kJoinSmem, st>>>(ja);
+        join_small_kernel<true><<<num_sms, kJoinThreads, kJoinSmem, st>>>(ja, none);
         nlaunch += 2;
     } else if (g.single) {
         // One launch per element layout; the one that does not match the device's choice returns at once.
-        join_words_kernel<<<num_sms * 2, kCompactThreads, kOaSmem, st>>>(ja);
-        join_small_kernel<false, false><<<num_sms, kJoinThreads, kJoinSmem, st>>>(ja);
+        join_words_kernel<false><<<num_sms * 2, kCompactThreads, kOaSmem, st>>>(ja, none);
+        join_small_kernel<false, false><<<num_sms, kJoinThreads, kJoinSmem, st>>>(ja, none);
         nlaunch += 2;
     } else {
         // One launch per partition layout (tuples, compact words); the one that does not match the
@@ -3073,14 +3133,14 @@ int phj_enqueue(const RadixGeom &g, bool lp, bool skip0, const ulonglong2 *R, si
             join_compact_kernel<false, false, true><<<num_sms * 2, kCompactThreads, kCompactSmem, st>>>(ja);
         else
             join_compact_kernel<false, false><<<num_sms * 2, kCompactThreads, kCompactSmem, st>>>(ja);
-        join_small_kernel<false, false><<<num_sms, kJoinThreads, kJoinSmem, st>>>(ja);
+        join_small_kernel<false, false><<<num_sms, kJoinThreads, kJoinSmem, st>>>(ja, none);
         nlaunch += 2;
         if (ci_ok) {
             if (lp)
                 join_compact_kernel<false, true, true><<<num_sms * 2, kCompactThreads, kCompactSmem, st>>>(ja);
             else
                 join_compact_kernel<false, true><<<num_sms * 2, kCompactThreads, kCompactSmem, st>>>(ja);
-            join_small_kernel<false, true><<<num_sms, kJoinThreads, kJoinSmem, st>>>(ja);
+            join_small_kernel<false, true><<<num_sms, kJoinThreads, kJoinSmem, st>>>(ja, none);
             nlaunch += 2;
         }
     }

@@ -349,10 +349,92 @@ __device__ __forceinline__ void plan_body(const PlanArgs &a, const uint32_t *tot
     }
 }
 
+struct SingleArgs {
+    const tuple_v *R, *S;
+    uint64_t nR, nS;
+    int bits;                // P = 2^bits partitions
+    int copies;              // count: histograms per CTA (its warps spread over them)
+    uint32_t *hist;          // [2][G][P]: rows of R, rows of S; exclusive prefixes after single_plan
+    unsigned long long *ors; // [G][3]: ORs of build keys, build row ids, probe row ids
+    const uint64_t *start;   // [2][P + 1]
+    uint32_t *counters;
+    JoinAccum *acc;          // cleared by the count if clear_acc
+    int clear_acc;
+    int ci_ok;               // compact words allowed
+    int lp;                  // first match: build elements carry their input position
+    int z0;                  // build key 0 never matches
+    tuple_v *outR, *outS;    // tuples
+    unsigned long long *outR8, *outS8;  // compact words
+};
+
+struct JoinArgs {
+    const JoinItem *items;
+    const LargePart *large;
+    uint32_t *counters;
+    const tuple_v *finR, *finS;
+    uint32_t *large_table;
+    int bits;
+    int lp;     // first match per probe tuple (lowest build position) instead of all matches
+    int skip0;  // build tuples with key 0 never match (key 0 marks an empty slot in lp_join)
+    JoinAccum *acc;
+    MatOut mat; // materialising joins (MAT kernels): where the (r.row_id, s.row_id) pairs go
+    int ci;     // the final partitions may be compact words (when ci_applies holds) at finR8 / finS8
+    const unsigned long long *finR8, *finS8;
+    // First-match joins of the one-pass pipeline: build elements are {ci_word or key, input position}, and
+    // a wide match reads its row id from the build relation itself.
+    int lp_pos;
+    const tuple_v *relR;
+    uint64_t nR;
+    int flag_bits;  // HJ_RES_COMPACT_PARTITIONS tells whether words of this many radix bits fit
+    // One-pass pipeline: one launch takes the items of every size; host_out: see join_finish.
+    int all_items;
+    JoinAccum *host_out;
+    int w8_b1;  // a pass 1 that may store words (either pipeline): its shift (reported when w8_fits held); -1 otherwise
+};
+
+// Kernels of the one-pass pipeline run on one join (its arguments are the launch's) or on many (MULTI: a
+// block's job and its index among the job's blocks come from a map; the job's arguments are copied to shared
+// memory). One launch per step then serves a whole wave of joins.
+struct MultiJob {
+    SingleArgs sa;
+    PlanArgs pa;
+    JoinArgs ja;
+    uint32_t grid;         // blocks of the count and the scatter
+    uint32_t plan_blocks;  // blocks of the plan
+};
+static_assert(sizeof(MultiJob) % 8 == 0 && sizeof(SingleArgs) % 8 == 0 && sizeof(PlanArgs) % 8 == 0 &&
+              sizeof(JoinArgs) % 8 == 0, "copied by 8-byte words");
+
+struct MultiRef {
+    const MultiJob *jobs;
+    const uint2 *map;  // [gridDim.x] {job, block of the job}
+};
+
+template <class T>
+__device__ __forceinline__ void multi_copy(T *dst, const T *src) {
+    static_assert(sizeof(T) % 8 == 0, "8-byte words");
+    for (uint32_t i = threadIdx.x; i < sizeof(T) / 8; i += blockDim.x)
+        reinterpret_cast<unsigned long long *>(dst)[i] = reinterpret_cast<const unsigned long long *>(src)[i];
+}
+
 // Compact words of the probe relation in the one-pass pipeline: behind the build relation's words, or
 // behind its 16-byte elements for first-match joins.
 inline unsigned long long *single_probe_words(const PhjScratch &s, size_t nR, bool lp) {
     return lp ? reinterpret_cast<unsigned long long *>(s.tmp1 + nR) : reinterpret_cast<unsigned long long *>(s.tmp1) + nR;
 }
+
+// Arguments of a radix join's partition joins (hj_partition.cu).
+JoinArgs join_args(const RadixGeom &g, bool lp, bool skip0, const ulonglong2 *R, size_t nR, const PhjScratch &s,
+                   JoinAccum *acc, const MatOut *mat, int ci_ok, int w8_b1, JoinAccum *host_out);
+// Arguments of a one-pass join's partition phase (hj_single.cu).
+void single_args(const RadixGeom &g, bool lp, bool skip0, bool ci_ok, const ulonglong2 *R, size_t nR,
+                 const ulonglong2 *S, size_t nS, const PhjScratch &s, JoinAccum *acc, bool clear_acc, bool agg_ok,
+                 SingleArgs *a, PlanArgs *pa);
+// The steps of a wave of one-pass joins (hj_wave.cu): partition phase, partition joins (maps of the joins
+// that count every match and of the first-match ones), large partitions and error words.
+int multi_partition_launch(const MultiJob *jobs, const uint2 *part_map, unsigned part_blocks, const uint2 *plan_map,
+                           unsigned plan_blocks, int max_bits, cudaStream_t st, uint32_t *launches);
+int multi_join_launch(const MultiJob *jobs, int njobs, const uint2 *every_map, unsigned every_blocks,
+                      const uint2 *first_map, unsigned first_blocks, cudaStream_t st, uint32_t *launches);
 
 }  // namespace hj

@@ -140,6 +140,10 @@ struct WaveLayout {
     size_t sides_off, tables_off, copies_off, total;
     unsigned n_r_chunks, n_s_chunks;
     unsigned r_piece, s_piece;  // chunk lengths of the build and probe relations (mj_piece)
+    // One-pass form (wave_layout_one_pass): [results][image][scratch][device copies of host relations].
+    bool one_pass = false;
+    hj::WavePlan wp;
+    size_t scratch_off = 0;
 };
 
 struct WaveLane {
@@ -199,6 +203,48 @@ void wave_layout(const std::vector<Request> &reqs, int num_sms, WaveLayout *L) {
     L->tables_off = L->sides_off + a256(sizeof(hj::MSide) * n);
     L->copies_off = L->tables_off + a256(table_bytes);
     L->total = L->copies_off + copy_bytes;
+}
+
+// Waves of fewer mid-size requests than this keep the table form: a lone one is done sooner by two launches over
+// an L2-sized table than by the one-pass pipeline's nine (20000 x 20000: 35 against 43 us); a burst is done
+// sooner in one pass (64 joins of 2^10..2^18 build tuples queued together: 729 us by tables, 363 in one pass).
+constexpr size_t kOnePassWaveMin = 4;
+
+std::vector<hj::WaveJoin> wave_joins(const std::vector<Request> &reqs) {
+    std::vector<hj::WaveJoin> v;
+    v.reserve(reqs.size());
+    for (const Request &r : reqs) {
+        hj::WaveJoin w;
+        w.lp = hj::algo_lp(r.algo);
+        w.skip0 = hj::algo_skip0(r.algo);
+        w.R = reinterpret_cast<const ulonglong2 *>(r.R);
+        w.nR = r.nR;
+        w.S = reinterpret_cast<const ulonglong2 *>(r.S);
+        w.nS = r.nS;
+        w.acc = nullptr;
+        v.push_back(w);
+    }
+    return v;
+}
+
+// Layout of the wave without global tables; false where the table form is better or the only one.
+bool wave_layout_one_pass(const std::vector<Request> &reqs, int num_sms, WaveLayout *L) {
+    size_t mid = 0, copy_bytes = 0;
+    for (const Request &r : reqs) {
+        if (!hj::wave_takes(r.nR, r.nS)) return false;
+        mid += r.nR > hj::kSmallMaxBuild;
+        if (!r.on_device) copy_bytes += a256(r.nR * 16) + a256(r.nS * 16);
+    }
+    if (mid && mid < kOnePassWaveMin) return false;
+    const std::vector<hj::WaveJoin> v = wave_joins(reqs);
+    L->one_pass = true;
+    hj::wave_plan(v.data(), v.size(), num_sms, &L->wp);
+    L->desc_off = a256(sizeof(hj::JoinAccum) * reqs.size());
+    L->desc_bytes = L->wp.image_bytes;
+    L->scratch_off = L->desc_off + a256(L->desc_bytes);
+    L->copies_off = L->scratch_off + a256(L->wp.scratch_bytes);
+    L->total = L->copies_off + copy_bytes;
+    return true;
 }
 
 }  // namespace
@@ -362,7 +408,40 @@ void complete_wave(hj_server *s, WaveLane &L, int status) {
 // Enqueue one admitted wave on its lane's stream: host relations are copied into the block, the
 // descriptor image (built here in the lane's pinned buffer) goes over in one copy, then the wave's
 // kernels run and the results come back into pinned memory; nothing here waits for the device.
+int launch_wave_one_pass(hj_server *s, WaveLane &L) {
+    const size_t n = L.reqs.size();
+    const WaveLayout &lay = L.lay;
+    cudaStream_t st = L.stream;
+    char *base = s->pool_mem + L.off;
+    hj::JoinAccum *accs = reinterpret_cast<hj::JoinAccum *>(base);
+    char *cp = base + lay.copies_off;
+    std::vector<hj::WaveJoin> v = wave_joins(L.reqs);
+    for (size_t q = 0; q < n; q++) {
+        const Request &r = L.reqs[q];
+        v[q].acc = accs + q;
+        if (r.on_device) continue;
+        if (cudaMemcpyAsync(cp, r.R, r.nR * 16, cudaMemcpyHostToDevice, st) != cudaSuccess) return HJ_E_DEVICE;
+        v[q].R = reinterpret_cast<const ulonglong2 *>(cp);
+        cp += a256(r.nR * 16);
+        if (cudaMemcpyAsync(cp, r.S, r.nS * 16, cudaMemcpyHostToDevice, st) != cudaSuccess) return HJ_E_DEVICE;
+        v[q].S = reinterpret_cast<const ulonglong2 *>(cp);
+        cp += a256(r.nS * 16);
+    }
+    int rc = hj::wave_image(v.data(), n, s->ctx->num_sms, lay.wp, base + lay.scratch_off, L.stage);
+    if (rc) return rc;
+    if (cudaMemcpyAsync(base + lay.desc_off, L.stage, lay.desc_bytes, cudaMemcpyHostToDevice, st) != cudaSuccess ||
+        cudaMemsetAsync(accs, 0, sizeof(hj::JoinAccum) * n, st) != cudaSuccess)
+        return HJ_E_DEVICE;
+    rc = hj::wave_enqueue(lay.wp, base + lay.desc_off, st, nullptr);
+    if (rc) return rc;
+    if (cudaMemcpyAsync(L.acc_host, accs, sizeof(hj::JoinAccum) * n, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        cudaEventRecord(L.done, st) != cudaSuccess)
+        return HJ_E_DEVICE;
+    return HJ_OK;
+}
+
 int launch_wave(hj_server *s, WaveLane &L) {
+    if (L.lay.one_pass) return launch_wave_one_pass(s, L);
     const int n = (int)L.reqs.size();
     const WaveLayout &lay = L.lay;
     cudaStream_t st = L.stream;
@@ -545,14 +624,16 @@ void worker_main(hj_server *s) {
                 // The wave's block must fit the pool now; under memory pressure the wave shrinks (the
                 // requests left out stay queued, in order).
                 WaveLayout lay;
-                wave_layout(wave, s->ctx->num_sms, &lay);
                 size_t off = 0;
-                bool got = false;
-                for (;;) {
+                bool got = wave_layout_one_pass(wave, s->ctx->num_sms, &lay) && lay.desc_bytes <= s->stage_bytes &&
+                           s->pool.alloc(lay.total, &off);
+                // The table form, which needs less memory; then fewer requests.
+                while (!got) {
+                    lay = WaveLayout();
+                    wave_layout(wave, s->ctx->num_sms, &lay);
                     got = lay.desc_bytes <= s->stage_bytes && s->pool.alloc(lay.total, &off);
                     if (got || wave.size() == 1) break;
                     wave.resize(wave.size() / 2);
-                    wave_layout(wave, s->ctx->num_sms, &lay);
                 }
                 if (got) {
                     // Take the wave's requests out of the queue (they are in queue order).

@@ -31,10 +31,10 @@ constexpr int kPlaceThreads = 512;  // scatter: one CTA per SM
 constexpr int kWordItems = 16, kTupleItems = kWordItems / 2;  // staged 8-byte / 16-byte elements per thread and tile
 constexpr int kSingleDigitsPerThread = ((1 << kSingleMaxBits) + kPlaceThreads - 1) / kPlaceThreads;
 
-// CTA c's contiguous range of n tuples (a multiple of 8 tuples, one 128-byte line).
-__device__ __forceinline__ void single_range(uint64_t n, uint64_t *lo, uint64_t *hi) {
-    const uint64_t per = ((n + gridDim.x - 1) / gridDim.x + 7) & ~7ull;
-    *lo = blockIdx.x * per < n ? blockIdx.x * per : n;
+// The contiguous range of n tuples that block c of G takes (a multiple of 8 tuples, one 128-byte line).
+__device__ __forceinline__ void single_range(uint64_t n, uint32_t c, uint32_t G, uint64_t *lo, uint64_t *hi) {
+    const uint64_t per = ((n + G - 1) / G + 7) & ~7ull;
+    *lo = c * per < n ? c * per : n;
     *hi = *lo + per < n ? *lo + per : n;
 }
 
@@ -49,45 +49,38 @@ __device__ __forceinline__ tuple_v ld_twice(const tuple_v *p) {
     return v;
 }
 
-struct SingleArgs {
-    const tuple_v *R, *S;
-    uint64_t nR, nS;
-    int bits;                // P = 2^bits partitions
-    int copies;              // count: histograms per CTA (its warps spread over them)
-    uint32_t *hist;          // [2][G][P]: rows of R, rows of S; exclusive prefixes after single_plan
-    unsigned long long *ors; // [G][3]: ORs of build keys, build row ids, probe row ids
-    const uint64_t *start;   // [2][P + 1]
-    uint32_t *counters;
-    JoinAccum *acc;          // cleared by the count if clear_acc
-    int clear_acc;
-    int ci_ok;               // compact words allowed
-    int lp;                  // first match: build elements carry their input position
-    int z0;                  // build key 0 never matches
-    tuple_v *outR, *outS;    // tuples
-    unsigned long long *outR8, *outS8;  // compact words
-};
-
 // ------------------------------------------------------------------------------------------------
 // 1. Count. Bound by reading the relations (four 16-byte loads per thread in flight, 1024 threads per SM);
 //    the shared-memory increments return nothing. With few partitions the warps spread over `copies`
 //    histograms, since 32 lanes on a handful of counters serialise.
 // ------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(kCountThreads, 1) single_count(SingleArgs a) {
+template <bool MULTI>
+__global__ void __launch_bounds__(kCountThreads, 1) single_count(SingleArgs a0, MultiRef mr) {
     extern __shared__ uint32_t sh[];  // [copies][P]
+    __shared__ SingleArgs s_a;
+    uint32_t blk = blockIdx.x, G = gridDim.x;
+    if (MULTI) {
+        const uint2 e = mr.map[blockIdx.x];
+        multi_copy(&s_a, &mr.jobs[e.x].sa);
+        blk = e.y;
+        G = mr.jobs[e.x].grid;
+        __syncthreads();
+    }
+    const SingleArgs &a = MULTI ? s_a : a0;
     const int tid = threadIdx.x;
     const uint32_t P = 1u << a.bits, mask = P - 1;
     uint32_t *mine = sh + (size_t)((uint32_t)(tid >> 5) % (uint32_t)a.copies) * P;
     __shared__ unsigned long long s_or[3];
     if (tid < 3) s_or[tid] = 0;
     // The kernels after this one find their counters (and the result) at zero.
-    if (blockIdx.x == 0 && tid < kNumCounters) a.counters[tid] = 0;
-    if (blockIdx.x == 0 && a.clear_acc && tid == 0) *a.acc = JoinAccum{};
+    if (blk == 0 && tid < kNumCounters) a.counters[tid] = 0;
+    if (blk == 0 && a.clear_acc && tid == 0) *a.acc = JoinAccum{};
     for (int rel = 0; rel < 2; rel++) {
         for (uint32_t j = tid; j < P * a.copies; j += kCountThreads) sh[j] = 0;
         __syncthreads();
         const tuple_v *in = rel ? a.S : a.R;
         uint64_t lo, hi;
-        single_range(rel ? a.nS : a.nR, &lo, &hi);
+        single_range(rel ? a.nS : a.nR, blk, G, &lo, &hi);
         unsigned long long kor = 0, ror = 0;
         constexpr int U = 4;
         uint64_t i = lo + tid;
@@ -122,7 +115,7 @@ __global__ void __launch_bounds__(kCountThreads, 1) single_count(SingleArgs a) {
             }
         }
         __syncthreads();
-        uint32_t *row = a.hist + ((size_t)rel * gridDim.x + blockIdx.x) * P;
+        uint32_t *row = a.hist + ((size_t)rel * G + blk) * P;
         for (uint32_t j = tid; j < P; j += kCountThreads) {
             uint32_t n = 0;
             for (int c = 0; c < a.copies; c++) n += sh[(size_t)c * P + j];
@@ -130,22 +123,38 @@ __global__ void __launch_bounds__(kCountThreads, 1) single_count(SingleArgs a) {
         }
         __syncthreads();
     }
-    if (tid < 3) a.ors[(size_t)blockIdx.x * 3 + tid] = s_or[tid];
+    if (tid < 3) a.ors[(size_t)blk * 3 + tid] = s_or[tid];
 }
 
 // ------------------------------------------------------------------------------------------------
 // 2. Prefixes and plan. A CTA takes 32 columns (digits of one relation; consecutive lanes read
 //    consecutive digits of a row), its 32 warps share the rows. The CTA that finishes last plans.
 // ------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(1024, 1) single_plan(SingleArgs a, uint32_t G, uint32_t *total, PlanArgs pa) {
+template <bool MULTI>
+__global__ void __launch_bounds__(1024, 1) single_plan(SingleArgs a0, PlanArgs pa0, uint32_t G0, MultiRef mr) {
     __shared__ uint32_t part[32][33];
     __shared__ uint32_t tmp[32];
     __shared__ uint64_t s_run[2];
     __shared__ bool s_last;
     extern __shared__ uint32_t sm_tot[];  // [2][P]
+    __shared__ SingleArgs s_a;
+    __shared__ PlanArgs s_pa;
+    uint32_t blk = blockIdx.x, nblk = gridDim.x, G = G0;
+    if (MULTI) {
+        const uint2 e = mr.map[blockIdx.x];
+        multi_copy(&s_a, &mr.jobs[e.x].sa);
+        multi_copy(&s_pa, &mr.jobs[e.x].pa);
+        blk = e.y;
+        nblk = mr.jobs[e.x].plan_blocks;
+        G = mr.jobs[e.x].grid;
+        __syncthreads();
+    }
+    const SingleArgs &a = MULTI ? s_a : a0;
+    const PlanArgs &pa = MULTI ? s_pa : pa0;
+    uint32_t *total = const_cast<uint32_t *>(pa.total);
     const uint32_t P = 1u << a.bits;
     const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const uint32_t col = blockIdx.x * 32 + lane;
+    const uint32_t col = blk * 32 + lane;
     const uint32_t rel = col >= P;
     if (col < 2 * P) {
         uint32_t *h = a.hist + (size_t)rel * G * P + (col - rel * P);
@@ -169,7 +178,7 @@ __global__ void __launch_bounds__(1024, 1) single_plan(SingleArgs a, uint32_t G,
         __threadfence();
     }
     __syncthreads();
-    if (threadIdx.x == 0) s_last = atomicAdd(&a.counters[kCtrTicket], 1u) == gridDim.x - 1;
+    if (threadIdx.x == 0) s_last = atomicAdd(&a.counters[kCtrTicket], 1u) == nblk - 1;
     if (col < 2 * P) {
         uint32_t *h = a.hist + (size_t)rel * G * P + (col - rel * P);
         const uint32_t per = (G + 31) / 32;
@@ -275,7 +284,7 @@ __device__ __forceinline__ uint32_t place_scan(uint32_t v, uint32_t *tmp) {
 
 // Place one relation's range. A function of its own per mode: inlined side by side the modes spilled.
 template <int MODE>
-__device__ __noinline__ void single_scatter_rel(const SingleArgs &a, int rel) {
+__device__ __noinline__ void single_scatter_rel(const SingleArgs &a, int rel, uint32_t blk, uint32_t G) {
     using Elem = SingleElem<MODE>;
     using E = typename Elem::Staged;
     using O = typename Elem::Out;
@@ -300,7 +309,7 @@ __device__ __noinline__ void single_scatter_rel(const SingleArgs &a, int rel) {
         out = rel ? a.outS : a.outR;
     const bool z0 = a.z0 && rel == 0;
     uint64_t lo, hi;
-    single_range(rel ? a.nS : a.nR, &lo, &hi);
+    single_range(rel ? a.nS : a.nR, blk, G, &lo, &hi);
     const tuple_v *in = (rel ? a.S : a.R) + lo;
     const uint32_t len = (uint32_t)(hi - lo);
     if (len == 0) return;
@@ -309,7 +318,7 @@ __device__ __noinline__ void single_scatter_rel(const SingleArgs &a, int rel) {
 #pragma unroll
     for (int q = 0; q < ITEMS; q++) t[q] = base + q * NT + tid < len ? ld_stream(in + base + q * NT + tid) : make_ulonglong2(0, 0);
     {
-        const uint32_t *pre = a.hist + ((size_t)rel * gridDim.x + blockIdx.x) * P;
+        const uint32_t *pre = a.hist + ((size_t)rel * G + blk) * P;
         const uint64_t *start = a.start + (size_t)rel * (P + 1);
         for (uint32_t j = tid; j < P; j += NT) {
             place[j] = (uint32_t)start[j] + pre[j];
@@ -376,22 +385,33 @@ __device__ __noinline__ void single_scatter_rel(const SingleArgs &a, int rel) {
     __syncthreads();
 }
 
-__global__ void __launch_bounds__(kPlaceThreads, 1) single_scatter(SingleArgs a) {
+template <bool MULTI>
+__global__ void __launch_bounds__(kPlaceThreads, 1) single_scatter(SingleArgs a0, MultiRef mr) {
+    __shared__ SingleArgs s_a;
+    uint32_t blk = blockIdx.x, G = gridDim.x;
+    if (MULTI) {
+        const uint2 e = mr.map[blockIdx.x];
+        multi_copy(&s_a, &mr.jobs[e.x].sa);
+        blk = e.y;
+        G = mr.jobs[e.x].grid;
+        __syncthreads();
+    }
+    const SingleArgs &a = MULTI ? s_a : a0;
     const bool ci = a.ci_ok && ci_applies(a.counters, a.bits);
     const bool narrow = ci && *reinterpret_cast<const unsigned long long *>(a.counters + kCtrMaxKey) < (1ull << 31);
     // S, then R; one instantiation per mode serves both.
     for (int rel = 1; rel >= 0; rel--) {
         if (rel == 0 && a.lp) {
             if (ci)
-                single_scatter_rel<kModePosWord>(a, rel);
+                single_scatter_rel<kModePosWord>(a, rel, blk, G);
             else
-                single_scatter_rel<kModePos>(a, rel);
+                single_scatter_rel<kModePos>(a, rel, blk, G);
         } else if (narrow) {
-            single_scatter_rel<kModeWord>(a, rel);
+            single_scatter_rel<kModeWord>(a, rel, blk, G);
         } else if (ci) {
-            single_scatter_rel<kModeTupleWord>(a, rel);
+            single_scatter_rel<kModeTupleWord>(a, rel, blk, G);
         } else {
-            single_scatter_rel<kModeTuple>(a, rel);
+            single_scatter_rel<kModeTuple>(a, rel, blk, G);
         }
     }
 }
@@ -399,6 +419,13 @@ __global__ void __launch_bounds__(kPlaceThreads, 1) single_scatter(SingleArgs a)
 // ------------------------------------------------------------------------------------------------
 // Host side
 // ------------------------------------------------------------------------------------------------
+// Histograms per CTA of the count (32 KB of them) for 2^bits digits.
+constexpr size_t kCountSmem = 32768;
+static int single_copies(int bits) {
+    const uint32_t n = (uint32_t)(kCountSmem / 4) >> bits;
+    return n < 1 ? 1 : n < 32 ? (int)n : 32;
+}
+
 uint32_t single_grid(size_t nR, size_t nS, int num_sms) {
     const uint64_t sms = (uint64_t)(num_sms > 0 ? num_sms : 148);
     const uint64_t want = ((uint64_t)nR + nS + 4095) / 4096;
@@ -415,22 +442,25 @@ uint32_t single_grid(size_t nR, size_t nS, int num_sms) {
     } while (0)
 
 int single_prepare_device() {
-    HJ_CU(cudaFuncSetAttribute(single_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    HJ_CU(cudaFuncSetAttribute(single_scatter<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)single_scatter_smem(kSingleMaxBits)));
+    HJ_CU(cudaFuncSetAttribute(single_scatter<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)single_scatter_smem(kSingleMaxBits)));
     return HJ_OK;
 }
 
-int single_partition_enqueue(const RadixGeom &g, bool lp, bool skip0, bool ci_ok, const ulonglong2 *R, size_t nR,
-                             const ulonglong2 *S, size_t nS, const PhjScratch &s, JoinAccum *acc, bool clear_acc,
-                             cudaStream_t st, bool agg_ok, cudaEvent_t *ph, uint32_t *launches) {
+void single_args(const RadixGeom &g, bool lp, bool skip0, bool ci_ok, const ulonglong2 *R, size_t nR,
+                 const ulonglong2 *S, size_t nS, const PhjScratch &s, JoinAccum *acc, bool clear_acc, bool agg_ok,
+                 SingleArgs *out, PlanArgs *pout) {
     const uint32_t P = 1u << g.bits;
-    SingleArgs a;
+    SingleArgs &a = *out;
+    a = SingleArgs{};
     a.R = R;
     a.S = S;
     a.nR = nR;
     a.nS = nS;
     a.bits = g.bits;
-    a.copies = P >= 8192 ? 1 : (int)(8192u / P < 32u ? 8192u / P : 32u);
+    a.copies = single_copies(g.bits);
     a.hist = s.chunk_hist;
     a.ors = s.ors;
     a.start = s.start;
@@ -444,8 +474,8 @@ int single_partition_enqueue(const RadixGeom &g, bool lp, bool skip0, bool ci_ok
     a.outS = s.tmp1 + nR;
     a.outR8 = reinterpret_cast<unsigned long long *>(s.tmp1);
     a.outS8 = single_probe_words(s, nR, lp);
-    const uint32_t G = s.cR;
-    PlanArgs pa;
+    PlanArgs &pa = *pout;
+    pa = PlanArgs{};
     pa.bits = g.bits;
     pa.passes = 1;
     pa.b1 = g.bits;
@@ -463,16 +493,39 @@ int single_partition_enqueue(const RadixGeom &g, bool lp, bool skip0, bool ci_ok
     pa.large_table_words = s.large_table_words;
     pa.small_cap = lp ? kFirstCap : kSmemCap;
     pa.agg_ok = agg_ok ? 1 : 0;
-    single_count<<<G, kCountThreads, (size_t)a.copies * P * 4, st>>>(a);
+}
+
+int single_partition_enqueue(const RadixGeom &g, bool lp, bool skip0, bool ci_ok, const ulonglong2 *R, size_t nR,
+                             const ulonglong2 *S, size_t nS, const PhjScratch &s, JoinAccum *acc, bool clear_acc,
+                             cudaStream_t st, bool agg_ok, cudaEvent_t *ph, uint32_t *launches) {
+    const uint32_t P = 1u << g.bits, G = s.cR;
+    SingleArgs a;
+    PlanArgs pa;
+    single_args(g, lp, skip0, ci_ok, R, nR, S, nS, s, acc, clear_acc, agg_ok, &a, &pa);
+    const MultiRef none = {};
+    single_count<false><<<G, kCountThreads, (size_t)a.copies * P * 4, st>>>(a, none);
     if (ph) HJ_CU(record_event(ph[1], st));
-    single_plan<<<(2 * P + 31) / 32, 1024, (size_t)2 * P * 4, st>>>(a, G, s.total, pa);
+    single_plan<false><<<(2 * P + 31) / 32, 1024, (size_t)2 * P * 4, st>>>(a, pa, G, none);
     if (ph) HJ_CU(record_event(ph[2], st));
-    single_scatter<<<G, kPlaceThreads, single_scatter_smem(g.bits), st>>>(a);
+    single_scatter<false><<<G, kPlaceThreads, single_scatter_smem(g.bits), st>>>(a, none);
     HJ_CU(cudaGetLastError());
     if (ph) {
         HJ_CU(record_event(ph[3], st));
         HJ_CU(record_event(ph[4], st));
     }
+    *launches += 3;
+    return HJ_OK;
+}
+
+int multi_partition_launch(const MultiJob *jobs, const uint2 *part_map, unsigned part_blocks, const uint2 *plan_map,
+                           unsigned plan_blocks, int max_bits, cudaStream_t st, uint32_t *launches) {
+    const SingleArgs none_a = {};
+    const PlanArgs none_p = {};
+    const MultiRef part = {jobs, part_map}, plan = {jobs, plan_map};
+    single_count<true><<<part_blocks, kCountThreads, kCountSmem, st>>>(none_a, part);
+    single_plan<true><<<plan_blocks, 1024, (size_t)8 << max_bits, st>>>(none_a, none_p, 0, plan);
+    single_scatter<true><<<part_blocks, kPlaceThreads, single_scatter_smem(max_bits), st>>>(none_a, part);
+    HJ_CU(cudaGetLastError());
     *launches += 3;
     return HJ_OK;
 }

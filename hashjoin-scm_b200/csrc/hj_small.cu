@@ -17,6 +17,7 @@
 #include "hj_common.cuh"
 #include "hj_internal.h"
 #include "hj_partition.cuh"
+#include "hj_wave.cuh"
 
 namespace hj {
 
@@ -34,86 +35,122 @@ struct SmallArgs {
     JoinAccum *out;   // pinned host memory
 };
 
-__global__ void __launch_bounds__(kSmallThreads, 1) small_join(SmallArgs a) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    tuple_v *rt = reinterpret_cast<tuple_v *>(smem);                 // [nR]
-    uint32_t *head = reinterpret_cast<uint32_t *>(rt + a.nR);        // [2^nb_log]
-    uint16_t *nxt = reinterpret_cast<uint16_t *>(head + (1u << a.nb_log));  // [nR]
-    __shared__ unsigned long long s_red[5][kSmallThreads / 32];
-    __shared__ bool s_last;
+struct SmallTable {  // in dynamic shared memory
+    tuple_v *rt;        // [nR]
+    uint32_t *head;     // [2^nb_log]
+    uint16_t *nxt;      // [nR]
+    int shift;
+    __device__ __forceinline__ SmallTable(unsigned char *smem, uint32_t nR, int nb_log)
+        : rt(reinterpret_cast<tuple_v *>(smem)), head(reinterpret_cast<uint32_t *>(rt + nR)),
+          nxt(reinterpret_cast<uint16_t *>(head + (1u << nb_log))), shift(64 - nb_log) {}
+    __device__ __forceinline__ uint32_t bucket(unsigned long long key) const {
+        return (uint32_t)((key * 0x9e3779b97f4a7c15ull) >> shift);
+    }
+};
+
+struct SmallSums {
+    unsigned long long cnt = 0, sum = 0, kor = 0, ror = 0, sor = 0;
+    bool multi = false, over = false;
+};
+
+// Build the whole table and probe it with S[j0], S[j0 + stride], ... below end. All threads of the block.
+__device__ __forceinline__ void small_block(const SmallTable &tb, const tuple_v *R, uint32_t nR, int nb_log, bool lp,
+                                            bool skip0, const tuple_v *S, uint64_t j0, uint64_t stride, uint64_t end,
+                                            SmallSums &o) {
     const int tid = threadIdx.x;
     constexpr int UR = kSmallMaxBuild / kSmallThreads, U = 4;
-    const int shift = 64 - a.nb_log;
-    constexpr unsigned long long kMul = 0x9e3779b97f4a7c15ull;
     // The first probe tuples are requested before the build.
-    const uint64_t stride = (uint64_t)gridDim.x * kSmallThreads;
-    uint64_t j0 = (uint64_t)blockIdx.x * kSmallThreads + tid;
     tuple_v s[U];
 #pragma unroll
     for (int u = 0; u < U; u++) {
         const uint64_t j = j0 + u * stride;
-        s[u] = j < a.nS ? ld_stream(a.S + j) : make_ulonglong2(0, 0);
+        s[u] = j < end ? ld_stream(S + j) : make_ulonglong2(0, 0);
     }
     tuple_v t[UR];
 #pragma unroll
     for (int u = 0; u < UR; u++) {
         const uint32_t i = tid + u * kSmallThreads;
-        if (i < a.nR) t[u] = __ldg(a.R + i);
+        if (i < nR) t[u] = __ldg(R + i);
     }
-    for (uint32_t q = tid; q < (1u << a.nb_log); q += kSmallThreads) head[q] = 0;
+    for (uint32_t q = tid; q < (1u << nb_log); q += kSmallThreads) tb.head[q] = 0;
     __syncthreads();
-    unsigned long long kor = 0, ror = 0, sor = 0;
 #pragma unroll
     for (int u = 0; u < UR; u++) {
         const uint32_t i = tid + u * kSmallThreads;
-        if (i >= a.nR) break;
-        rt[i] = t[u];
-        kor |= t[u].x;
-        ror |= t[u].y;
-        if (a.skip0 && t[u].x == 0) continue;
-        nxt[i] = (uint16_t)atomicExch(&head[(t[u].x * kMul) >> shift], i + 1);
+        if (i >= nR) break;
+        tb.rt[i] = t[u];
+        o.kor |= t[u].x;
+        o.ror |= t[u].y;
+        if (skip0 && t[u].x == 0) continue;
+        tb.nxt[i] = (uint16_t)atomicExch(&tb.head[tb.bucket(t[u].x)], i + 1);
     }
     __syncthreads();
-    unsigned long long cnt = 0, sum = 0;
-    bool multi = false, over = false;
-    for (; j0 < a.nS; j0 += U * stride) {
+    for (; j0 < end; j0 += U * stride) {
         tuple_v nx[U];
 #pragma unroll
         for (int u = 0; u < U; u++) {
             const uint64_t j = j0 + (U + u) * stride;
-            nx[u] = j < a.nS ? ld_stream(a.S + j) : make_ulonglong2(0, 0);
+            nx[u] = j < end ? ld_stream(S + j) : make_ulonglong2(0, 0);
         }
 #pragma unroll
         for (int u = 0; u < U; u++) {
-            if (j0 + u * stride >= a.nS) continue;
-            sor |= s[u].y;
-            uint32_t e = head[(s[u].x * kMul) >> shift];
+            if (j0 + u * stride >= end) continue;
+            o.sor |= s[u].y;
+            uint32_t e = tb.head[tb.bucket(s[u].x)];
             uint32_t best = 0, nm = 0, steps = 0;
             while (e) {
-                const tuple_v r = rt[e - 1];
+                const tuple_v r = tb.rt[e - 1];
                 if (r.x == s[u].x) {
-                    if (a.lp) {
+                    if (lp) {
                         if (nm++ == 0 || e < best) best = e;
                     } else {
-                        cnt++;
-                        sum += r.y + s[u].y;
+                        o.cnt++;
+                        o.sum += r.y + s[u].y;
                     }
                 }
-                e = nxt[e - 1];
-                if (++steps > a.nR) {
-                    over = true;
+                e = tb.nxt[e - 1];
+                if (++steps > nR) {
+                    o.over = true;
                     break;
                 }
             }
             if (nm) {  // first match
-                cnt++;
-                sum += rt[best - 1].y + s[u].y;
-                multi |= nm > 1;
+                o.cnt++;
+                o.sum += tb.rt[best - 1].y + s[u].y;
+                o.multi |= nm > 1;
             }
         }
 #pragma unroll
         for (int u = 0; u < U; u++) s[u] = nx[u];
     }
+}
+
+// Many small joins: block b takes the probe range chunks[b] of its job.
+__global__ void __launch_bounds__(kSmallThreads, 1) small_multi(const SmallJob *__restrict__ jobs,
+                                                               const MChunk *__restrict__ chunks) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ unsigned long long red[64];
+    const MChunk ch = chunks[blockIdx.x];
+    const SmallJob J = jobs[ch.job];
+    const SmallTable tb(smem, J.nR, J.nb_log);
+    SmallSums o;
+    small_block(tb, J.R, J.nR, J.nb_log, J.lp != 0, J.skip0 != 0, J.S, ch.begin + threadIdx.x, kSmallThreads,
+                ch.begin + ch.len, o);
+    block_sum2_to(o.cnt, o.sum, red, &J.acc->matched, &J.acc->checksum);
+    if (__syncthreads_or(o.over) && threadIdx.x == 0) set_error(&J.acc->error, kErrProbeLimit);
+}
+
+__global__ void __launch_bounds__(kSmallThreads, 1) small_join(SmallArgs a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ unsigned long long s_red[5][kSmallThreads / 32];
+    __shared__ bool s_last;
+    const int tid = threadIdx.x;
+    const SmallTable tb(smem, a.nR, a.nb_log);
+    SmallSums o;
+    small_block(tb, a.R, a.nR, a.nb_log, a.lp != 0, a.skip0 != 0, a.S, (uint64_t)blockIdx.x * kSmallThreads + tid,
+                (uint64_t)gridDim.x * kSmallThreads, a.nS, o);
+    unsigned long long cnt = o.cnt, sum = o.sum, kor = o.kor, ror = o.ror, sor = o.sor;
+    const bool multi = o.multi, over = o.over;
     // This CTA's partial result: sums, ORs and flags.
     const unsigned lane = lane_id(), w = tid >> 5;
     cnt = warp_sum_u64(cnt);
@@ -199,8 +236,34 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_join(SmallArgs a) {
     } while (0)
 
 int small_prepare_device() {
+    HJ_CU(cudaFuncSetAttribute(small_multi, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               kSmallMaxBuild * (16 + 4 + 2)));
     HJ_CU(cudaFuncSetAttribute(small_join, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                kSmallMaxBuild * (16 + 4 + 2)));
+    return HJ_OK;
+}
+
+static int small_buckets_log(size_t nR) {
+    int b = 1;
+    while ((1u << b) < nR) b++;
+    return b;
+}
+
+static size_t small_smem(size_t nR) { return nR * 16 + ((size_t)4 << small_buckets_log(nR)) + nR * 2; }
+
+void small_job(bool lp, bool skip0, const ulonglong2 *R, size_t nR, const ulonglong2 *S, JoinAccum *acc, SmallJob *j) {
+    j->R = R;
+    j->S = S;
+    j->acc = acc;
+    j->nR = (uint32_t)nR;
+    j->nb_log = small_buckets_log(nR);
+    j->lp = lp ? 1u : 0u;
+    j->skip0 = skip0 ? 1u : 0u;
+}
+
+int small_multi_launch(const SmallJob *jobs, const MChunk *chunks, unsigned nchunks, size_t max_build, cudaStream_t st) {
+    small_multi<<<nchunks, kSmallThreads, small_smem(max_build), st>>>(jobs, chunks);
+    HJ_CU(cudaGetLastError());
     return HJ_OK;
 }
 
@@ -212,8 +275,7 @@ int small_enqueue(bool lp, bool skip0, int flag_bits, const ulonglong2 *R, size_
     a.S = S;
     a.nR = (uint32_t)nR;
     a.nS = nS;
-    a.nb_log = 1;
-    while ((1u << a.nb_log) < nR) a.nb_log++;
+    a.nb_log = small_buckets_log(nR);
     a.lp = lp ? 1 : 0;
     a.skip0 = skip0 ? 1 : 0;
     a.flag_bits = flag_bits;
@@ -223,8 +285,7 @@ int small_enqueue(bool lp, bool skip0, int flag_bits, const ulonglong2 *R, size_
     const uint64_t want = ((uint64_t)nS + kSmallThreads - 1) / kSmallThreads;
     const uint64_t sms = (uint64_t)(num_sms < kSmallMaxGrid ? num_sms : kSmallMaxGrid);
     const unsigned grid = (unsigned)(want < 1 ? 1 : want < sms ? want : sms);
-    const size_t smem = nR * 16 + ((size_t)4 << a.nb_log) + nR * 2;
-    small_join<<<grid, kSmallThreads, smem, st>>>(a);
+    small_join<<<grid, kSmallThreads, small_smem(nR), st>>>(a);
     HJ_CU(cudaGetLastError());
     return HJ_OK;
 }

@@ -10,8 +10,10 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <vector>
 
 #include "hj_common.cuh"
+#include "hj_internal.h"
 
 namespace hj {
 
@@ -72,5 +74,48 @@ struct WaveDev {
 // Enqueue a wave on `st`: clear its tables and side records, build, resolve first-match joins with
 // duplicate build keys, probe. Results accumulate into each job's JoinAccum (which the caller zeroes).
 int mj_launch_wave(const WaveDev &w, int num_sms, cudaStream_t st, uint32_t *launches);
+
+// ------------------------------------------------------------------------------------------------
+// Waves without global tables. Joins of at most kSmallMaxBuild build tuples take one shared-memory table
+// per probe range (hj_small.cu); the others run the one-pass pipeline (hj_single.cu), each step as one
+// launch over all joins of the wave. A wave needs 16 bytes of scratch per tuple (and 28 per build tuple),
+// where table waves need 32 bytes per build tuple; the server falls back to those when its pool is short.
+// ------------------------------------------------------------------------------------------------
+struct SmallJob {
+    const tuple_v *R, *S;
+    JoinAccum *acc;
+    uint32_t nR;
+    int nb_log;
+    unsigned int lp, skip0;
+};
+void small_job(bool lp, bool skip0, const ulonglong2 *R, size_t nR, const ulonglong2 *S, JoinAccum *acc, SmallJob *j);
+int small_multi_launch(const SmallJob *jobs, const MChunk *chunks, unsigned nchunks, size_t max_build, cudaStream_t st);
+
+struct WaveJoin {
+    bool lp, skip0;
+    const ulonglong2 *R;
+    size_t nR;
+    const ulonglong2 *S;
+    size_t nS;
+    JoinAccum *acc;  // device, zeroed by the caller before the wave
+};
+
+// Whether a join may be part of such a wave.
+bool wave_takes(size_t nR, size_t nS);
+
+// Sizes and launches of one wave, from the joins' sizes alone; the descriptor image and the scratch are the
+// caller's (image: host copy of what goes to the device).
+struct WavePlan {
+    size_t scratch_bytes = 0, image_bytes = 0;
+    size_t jobs_off, small_off, chunk_off, part_off, plan_off, every_off, first_off;
+    unsigned n_jobs = 0, n_small = 0, n_chunks = 0, n_part = 0, n_plan = 0, n_every = 0, n_first = 0;
+    int max_bits = 0;
+    size_t max_build = 0;
+};
+void wave_plan(const WaveJoin *joins, size_t n, int num_sms, WavePlan *wp);
+// Fill the image for scratch at `scratch` (device, 256-byte aligned).
+int wave_image(const WaveJoin *joins, size_t n, int num_sms, const WavePlan &wp, char *scratch, char *image);
+// Enqueue the wave; image_dev: the image on the device.
+int wave_enqueue(const WavePlan &wp, const char *image_dev, cudaStream_t st, uint32_t *launches);
 
 }  // namespace hj
