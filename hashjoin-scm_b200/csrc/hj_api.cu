@@ -71,10 +71,10 @@ constexpr uint32_t kPipelineFlags = HJ_F_SEGMENTS | HJ_F_EXACT | HJ_F_WIDE | HJ_
 
 // The geometry of a radix join: the one-pass pipeline where the build relation needs few partitions,
 // unless the flags name another, else as asked.
-int join_geom(hj_algo_t algo, const hj_params_t &p, size_t nR, size_t nS, hj::RadixGeom *g) {
+int join_geom(hj_algo_t algo, const hj_params_t &p, size_t nR, size_t nS, bool mat, hj::RadixGeom *g) {
     const int rc = hj::radix_geom(p.num_radix_bits, p.num_passes, g, p.radix_bits_pass1);
     if (rc) return rc;
-    if (!(p.flags & kPipelineFlags) && !hj::radix_geom_single(p.num_radix_bits, hj::algo_lp(algo), nR, nS, g))
+    if (!(p.flags & kPipelineFlags) && !hj::radix_geom_single(p.num_radix_bits, hj::algo_lp(algo) || mat, nR, nS, g))
         hj::radix_geom_by_size(nR, g);
     return HJ_OK;
 }
@@ -100,15 +100,15 @@ struct JoinPlan {
     hj::RadixGeom geom = {};
 };
 
-int plan_join(hj_algo_t algo, hj_params_t *p, size_t nR, size_t nS, JoinPlan *jp) {
+int plan_join(hj_algo_t algo, hj_params_t *p, size_t nR, size_t nS, JoinPlan *jp, bool mat = false) {
     *jp = JoinPlan();
     if (is_phj(algo)) {
-        const int rc = join_geom(algo, *p, nR, nS, &jp->geom);
+        const int rc = join_geom(algo, *p, nR, nS, mat, &jp->geom);
         if (rc) return rc;
     } else if (nphj_by_radix(*p, nR, nS)) {
         p->flags &= ~(kPipelineFlags | HJ_F_ORDERED);  // radix joins' flags
         hj::radix_geom(14, 2, &jp->geom);
-        if (!hj::radix_geom_single(14, hj::algo_lp(algo), nR, nS, &jp->geom)) hj::radix_geom_by_size(nR, &jp->geom);
+        if (!hj::radix_geom_single(14, hj::algo_lp(algo) || mat, nR, nS, &jp->geom)) hj::radix_geom_by_size(nR, &jp->geom);
     } else {
         return HJ_OK;
     }
@@ -601,38 +601,41 @@ int hj_join_ctx(hj_ctx_t *c, hj_algo_t algo, const hj_params_t *pin, const hj_tu
 // Materialising joins (the reference's ptr_* joins, src/algo/ptr_phj.c, ptr_nphj.c): the join writes
 // one (r.row_id, s.row_id) pair per match, and a retrieve phase recomputes the checksum by gathering
 // R[r_row_id - 1].row_id + S[s_row_id - 1].row_id (src/inc/utils.c:712-724).
-static int join_mat(hj_ctx *c, hj_algo_t algo, const hj_params_t &p, const hj_tuple_t *R, size_t nR,
+static int join_mat(hj_ctx *c, hj_algo_t algo, hj_params_t p, const hj_tuple_t *R, size_t nR,
                     const hj_tuple_t *S, size_t nS, hj_pair_t *user_pairs, size_t user_cap,
                     unsigned long long cap_guess, hj_result_t *out) {
-    hj::RadixGeom geom = {};
-    if (is_phj(algo)) {
-        int rc = join_geom(algo, p, nR, nS, &geom);
-        if (rc) return out->status = rc;
-        out->physical_passes = geom.passes;
-    }
+    JoinPlan jp;
+    int rc = plan_join(algo, &p, nR, nS, &jp, true);
+    if (rc) return out->status = rc;
+    if (is_phj(algo)) out->physical_passes = jp.geom.passes;
     if (nR == 0 || nS == 0) return out->status = HJ_OK;
     const bool host_in = !p.inputs_on_device;
     // Pairs land in the caller's device buffer, or in the arena (library-owned, or staged for a host
     // buffer).
     const bool pairs_in_arena = !user_pairs || host_in;
     const unsigned long long cap = user_pairs ? (unsigned long long)user_cap : cap_guess;
-    bool seg = want_seg(algo, p, geom, nR, nS);
-    auto need_of = [&](bool sg) {
+    auto need_of = [&]() {
         size_t need = kAccBytes;
         if (host_in) need += align256(nR * 16) + align256(nS * 16);
-        if (is_phj(algo))
-            need += hj::phj_scratch_bytes(geom, nR, nS, c->num_sms, sg);
+        if (jp.radix)
+            need += hj::phj_scratch_bytes(jp.geom, nR, nS, c->num_sms, jp.seg);
         else
             need += align256(hj::nphj_scratch_bytes(nR, p.table_load, true));
         if (pairs_in_arena) need += align256(cap * 16);
         return need;
     };
-    int rc = ensure_arena(c, need_of(seg));
-    if (rc == HJ_E_OOM && seg) {
-        seg = false;
-        rc = ensure_arena(c, need_of(false));
+    rc = ensure_arena(c, need_of());
+    if (rc == HJ_E_OOM && jp.seg) {
+        jp.seg = false;
+        rc = ensure_arena(c, need_of());
+    }
+    if (rc == HJ_E_OOM && jp.radix && !is_phj(algo)) {
+        jp = JoinPlan();
+        rc = ensure_arena(c, need_of());
     }
     if (rc) return out->status = rc;
+    const bool seg = jp.seg;
+    const hj::RadixGeom &geom = jp.geom;
     cudaStream_t st = p.stream ? (cudaStream_t)p.stream : c->stream;
     CU_OR(cudaStreamWaitEvent(st, c->ev_done, 0), out->status = HJ_E_DEVICE);
     const bool timing = !(p.flags & HJ_F_NO_TIMING);
@@ -668,9 +671,13 @@ static int join_mat(hj_ctx *c, hj_algo_t algo, const hj_params_t &p, const hj_tu
     }
     CU_OR(cudaMemsetAsync(acc, 0, sizeof(JoinAccum), st), out->status = HJ_E_DEVICE);
     if (timing) CU_OR(cudaEventRecord(c->ev_start, st), out->status = HJ_E_DEVICE);
-    if (is_phj(algo)) {
+    void *dead = cur;  // scratch that the retrieve phase may use: the join's partitions, or its table
+    size_t dead_bytes = c->arena_bytes - (size_t)(cur - c->arena);
+    if (jp.radix) {
         hj::PhjScratch s;
         hj::phj_carve(geom, nR, nS, c->num_sms, cur, &s, seg);
+        dead = s.tmp1;
+        dead_bytes = (nR + nS) * 16;
         rc = hj::phj_enqueue(geom, hj::algo_lp(algo), hj::algo_skip0(algo), dR, nR, dS, nS, s, acc, st,
                              timing ? c->ev_mid : nullptr, c->num_sms, nullptr, &launches, &mat);
     } else {
@@ -680,8 +687,8 @@ static int join_mat(hj_ctx *c, hj_algo_t algo, const hj_params_t &p, const hj_tu
     }
     if (!rc) {
         if (timing) CU_OR(cudaEventRecord(c->ev_end, st), out->status = HJ_E_DEVICE);
-        rc = hj::mat_retrieve_enqueue(mat.pairs, &acc->pairs, cap, dR, nR, dS, nS, acc, st, c->num_sms);
-        launches++;
+        rc = hj::mat_retrieve_enqueue(mat.pairs, &acc->pairs, cap, dR, nR, dS, nS, dead, dead_bytes, acc, st,
+                                      c->num_sms, &launches);
     }
     if (rc) {
         cudaStreamSynchronize(st);
@@ -697,8 +704,10 @@ static int join_mat(hj_ctx *c, hj_algo_t algo, const hj_params_t &p, const hj_tu
               out->status = HJ_E_DEVICE);
     out->matched_cnt = n;
     out->checksum = c->acc_host->checksum;
-    out->large_partitions = c->acc_host->large_parts;
-    out->flags = (uint32_t)c->acc_host->flags;
+    if (is_phj(algo)) {
+        out->large_partitions = c->acc_host->large_parts;
+        out->flags = (uint32_t)c->acc_host->flags;
+    }
     if (timing) {
         float a = 0, b = 0, r = 0, h = 0;
         cudaEventElapsedTime(&a, c->ev_start, c->ev_mid);

@@ -32,7 +32,8 @@ struct JoinAccum {
     unsigned long long large_parts;
     unsigned long long pairs;   // materialising joins: output slots reserved so far
     unsigned long long flags;   // HJ_RES_* bits of hj_result_t.flags
-    unsigned long long pad[2];
+    unsigned long long wide_rids;  // materialising joins: OR of the row ids' high halves (mat_columns)
+    unsigned long long pad;
 };
 
 __device__ __forceinline__ void set_error(unsigned int *err, uint32_t bit) { atomicOr(err, bit); }

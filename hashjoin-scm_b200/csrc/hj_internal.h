@@ -193,9 +193,10 @@ int nphj_enqueue(bool lp, bool skip0, const ulonglong2 *R, size_t nR, const ulon
                  int phases = kNphjBuild | kNphjProbe);
 
 // Checksum of materialised pairs as the reference's retrieve phase computes it: the wrapping sum of
-// R[r_row_id - 1].row_id + S[s_row_id - 1].row_id over the first n pairs (into acc->checksum).
+// R[r_row_id - 1].row_id + S[s_row_id - 1].row_id over the first n pairs (into acc->checksum). scratch: device
+// memory that the join no longer uses.
 int mat_retrieve_enqueue(const ulonglong2 *pairs, const unsigned long long *n_dev, unsigned long long cap,
-                         const ulonglong2 *R, size_t nR, const ulonglong2 *S, size_t nS, JoinAccum *acc,
-                         cudaStream_t st, int num_sms);
+                         const ulonglong2 *R, size_t nR, const ulonglong2 *S, size_t nS, void *scratch,
+                         size_t scratch_bytes, JoinAccum *acc, cudaStream_t st, int num_sms, uint32_t *launches);
 
 }  // namespace hj

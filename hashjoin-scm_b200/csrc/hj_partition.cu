@@ -1438,7 +1438,7 @@ __global__ void __launch_bounds__(kCompactThreads, 2) join_compact_kernel(JoinAr
     unsigned int *err = &a.counters[kCtrErr];
     const uint32_t nA = a.counters[kCtrNItemsA];
     // Compiled once per partition layout; only the launch matching the device's choice runs.
-    if (CI != (!MAT && a.ci && ci_applies(a.counters, a.bits))) return;
+    if (CI != (a.ci && ci_applies(a.counters, a.bits))) return;
     constexpr bool ci = CI;
     const int B = ci ? 0 : a.bits;  // shift from a stored x to the key's bits above the radix bits
     constexpr bool lp = LP;
@@ -1610,7 +1610,76 @@ static_assert(kOaSmem >= (size_t)kSmemCap * 10 + kOaHeads * 2, "the chains fit t
 
 __device__ __forceinline__ uint32_t oa_hash(uint32_t hi) { return hi * 0x9e3779b1u; }
 
-template <bool MULTI>
+// Matches of probe word s in an open-addressing table of build words.
+__device__ __forceinline__ uint32_t oa_matches(const unsigned long long *slots, uint32_t nslots, unsigned long long s) {
+    const uint32_t hi = (uint32_t)(s >> 32);
+    uint32_t h = __umulhi(oa_hash(hi), nslots), m = 0;
+    for (uint32_t steps = 0; steps < nslots; steps++) {
+        const unsigned long long e = slots[h];
+        if (e == ~0ull) break;
+        m += (uint32_t)(e >> 32) == hi;
+        if (++h == nslots) h = 0;
+    }
+    return m;
+}
+
+// The first build word that matches, or ~0.
+__device__ __forceinline__ unsigned long long oa_find(const unsigned long long *slots, uint32_t nslots,
+                                                      unsigned long long s) {
+    const uint32_t hi = (uint32_t)(s >> 32);
+    uint32_t h = __umulhi(oa_hash(hi), nslots);
+    for (uint32_t steps = 0; steps < nslots; steps++) {
+        const unsigned long long e = slots[h];
+        if (e == ~0ull || (uint32_t)(e >> 32) == hi) return e;
+        if (++h == nslots) h = 0;
+    }
+    return ~0ull;
+}
+
+// One round of a materialising probe with at most one match per probe tuple: the matches' pairs (row ids of
+// build word e[u] and probe word s[u]; e[u] = ~0: none) go to consecutive output slots per warp and u.
+struct MatRound {
+    uint32_t count[32], at[32];  // a warp's pairs of the round, its start among them
+    unsigned long long base;     // the round's first output slot
+};
+
+template <int U, int NT>
+__device__ __forceinline__ void mat_write_round(MatRound &r, const unsigned long long (&e)[U],
+                                                const unsigned long long (&s)[U], const MatOut &out,
+                                                unsigned long long *cursor, unsigned int *err) {
+    const unsigned lane = lane_id(), w = threadIdx.x >> 5;
+    unsigned masks[U], total = 0;
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        masks[u] = __ballot_sync(0xffffffffu, e[u] != ~0ull);
+        total += __popc(masks[u]);
+    }
+    if (lane == 0) r.count[w] = total;
+    __syncthreads();
+    if (w == 0) {
+        const uint32_t x = lane < (unsigned)(NT / 32) ? r.count[lane] : 0u;
+        uint32_t incl = x;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= (unsigned)o) incl += y;
+        }
+        r.at[lane] = incl - x;
+        if (lane == 31) r.base = incl ? atomicAdd(cursor, (unsigned long long)incl) : 0ull;
+    }
+    __syncthreads();
+    unsigned long long o = r.base + r.at[w];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        if (e[u] != ~0ull)
+            mat_put(out, o + __popc(masks[u] & lanemask_lt()), e[u] & 0xffffffffull, s[u] & 0xffffffffull, err);
+        o += __popc(masks[u]);
+    }
+}
+
+// MAT: one pair per match. Without repeated build keys a probe has at most one match, and the block reserves
+// output for a round of eight probes per thread by ballots, so a warp writes consecutive pairs.
+template <bool MULTI, bool MAT = false>
 __global__ void __launch_bounds__(kCompactThreads, 2) join_words_kernel(JoinArgs a0, MultiRef mr) {
     __shared__ JoinArgs s_a;
     if (MULTI) {
@@ -1623,6 +1692,9 @@ __global__ void __launch_bounds__(kCompactThreads, 2) join_words_kernel(JoinArgs
     unsigned long long *slots = reinterpret_cast<unsigned long long *>(smem);
     __shared__ unsigned long long red[64];
     __shared__ uint32_t s_item, s_flags;  // s_flags: 1 a key occurs twice, 2 a walk was too long
+    __shared__ MatRound mat_round;
+    __shared__ uint32_t scan_tmp[32];
+    __shared__ unsigned long long s_base;
     if (!(a.ci && ci_applies(a.counters, a.bits))) return;
     const int tid = threadIdx.x;
     constexpr int NT = kCompactThreads, UR = 4, U = 8;
@@ -1691,6 +1763,24 @@ __global__ void __launch_bounds__(kCompactThreads, 2) join_words_kernel(JoinArgs
                 nxt[i] = (uint16_t)atomic_exch_u16(&head[oa_hash((uint32_t)(w >> 32)) >> 21], i + 1);
             }
             __syncthreads();
+            if constexpr (MAT) {
+                // Count, reserve, walk again and write.
+                for (uint32_t base = 0; base < ns; base += NT) {
+                    const uint32_t j = base + tid;
+                    const unsigned long long w = j < ns ? ld_stream8(S8 + j) : kNone;
+                    const uint32_t hi = (uint32_t)(w >> 32), e0 = j < ns ? head[oa_hash(hi) >> 21] : 0u;
+                    uint32_t m = 0, steps = 0;
+                    for (uint32_t e = e0; e && steps++ < nr; e = nxt[e - 1]) m += (uint32_t)(slots[e - 1] >> 32) == hi;
+                    unsigned long long o = mat_reserve(m, scan_tmp, &s_base, &a.acc->pairs);
+                    cnt += m;
+                    steps = 0;
+                    for (uint32_t e = e0; e && steps++ < nr; e = nxt[e - 1])
+                        if ((uint32_t)(slots[e - 1] >> 32) == hi)
+                            mat_put(a.mat, o++, slots[e - 1] & 0xffffffffull, w & 0xffffffffull, err);
+                }
+                __syncthreads();
+                continue;
+            }
             for (uint32_t j = tid; j < ns; j += NT) {
                 const unsigned long long w = ld_stream8(S8 + j);
                 const uint32_t hi = (uint32_t)(w >> 32);
@@ -1710,6 +1800,41 @@ __global__ void __launch_bounds__(kCompactThreads, 2) join_words_kernel(JoinArgs
             __syncthreads();
             continue;
         }
+        if constexpr (MAT) {
+            for (uint32_t base = 0; base < ns; base += U * NT) {  // the same rounds for every thread
+                unsigned long long nx[U], e[U];
+                uint32_t m = 0;
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const uint32_t j = base + tid + (U + u) * NT;
+                    nx[u] = j < ns ? ld_stream8(S8 + j) : kNone;
+                }
+                if (dups) {
+#pragma unroll
+                    for (int u = 0; u < U; u++) m += oa_matches(slots, nslots, s[u]);
+                    unsigned long long o = mat_reserve(m, scan_tmp, &s_base, &a.acc->pairs);
+                    cnt += m;
+#pragma unroll
+                    for (int u = 0; u < U; u++) {
+                        const uint32_t hi = (uint32_t)(s[u] >> 32);
+                        uint32_t h = __umulhi(oa_hash(hi), nslots);
+                        for (uint32_t steps = 0; steps < nslots && slots[h] != kNone; steps++) {
+                            if ((uint32_t)(slots[h] >> 32) == hi)
+                                mat_put(a.mat, o++, slots[h] & 0xffffffffull, s[u] & 0xffffffffull, err);
+                            if (++h == nslots) h = 0;
+                        }
+                    }
+                } else {
+#pragma unroll
+                    for (int u = 0; u < U; u++) e[u] = oa_find(slots, nslots, s[u]);
+                    mat_write_round<U, NT>(mat_round, e, s, a.mat, &a.acc->pairs, err);
+#pragma unroll
+                    for (int u = 0; u < U; u++) cnt += e[u] != kNone;
+                }
+#pragma unroll
+                for (int u = 0; u < U; u++) s[u] = nx[u];
+            }
+        } else
         for (uint32_t j0 = tid; j0 < ns; j0 += U * NT) {
             unsigned long long nx[U], e[U];
             uint32_t h[U];
@@ -1758,7 +1883,7 @@ __global__ void __launch_bounds__(kCompactThreads, 2) join_words_kernel(JoinArgs
 constexpr uint32_t kFwSlots = 16384;
 constexpr size_t kFwSmem = (size_t)kFwSlots * 12 + kFwSlots / 8;
 
-template <bool MULTI>
+template <bool MULTI, bool MAT = false>
 __global__ void __launch_bounds__(kJoinThreads, 1) join_first_words_kernel(JoinArgs a0, MultiRef mr) {
     __shared__ JoinArgs s_a;
     if (MULTI) {
@@ -1773,6 +1898,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_words_kernel(JoinA
     uint32_t *dup = rid + kFwSlots;                                             // [kFwSlots / 32]
     __shared__ unsigned long long red[64];
     __shared__ uint32_t s_item, s_dups;
+    __shared__ MatRound mat_round;
     if (!(a.ci && ci_applies(a.counters, a.bits))) return;
     const uint32_t tid = threadIdx.x;
     constexpr int NT = kJoinThreads, UR = kFirstCap / NT, U = 8;
@@ -1839,6 +1965,35 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_words_kernel(JoinA
             if (at[u] != ~0u && (uint32_t)slots[at[u]] == (uint32_t)r[u].y) rid[at[u]] = (uint32_t)r[u].x;
         const bool dups = s_dups != 0;
         __syncthreads();
+        if constexpr (MAT) {
+            for (uint32_t base = 0; base < ns; base += U * NT) {  // the same rounds for every thread
+                unsigned long long nx[U], e[U];
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const uint32_t j = base + tid + (U + u) * NT;
+                    nx[u] = j < ns ? ld_stream8(S8 + j) : kNone;
+                }
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const uint32_t hi = (uint32_t)(s[u] >> 32);
+                    uint32_t h = __umulhi(oa_hash(hi), nslots);
+                    e[u] = kNone;
+                    for (uint32_t steps = 0; steps < nslots && slots[h] != kNone; steps++) {
+                        if ((uint32_t)(slots[h] >> 32) == hi) {
+                            e[u] = rid[h];
+                            break;
+                        }
+                        if (++h == nslots) h = 0;
+                    }
+                }
+                mat_write_round<U, NT>(mat_round, e, s, a.mat, &a.acc->pairs, err);
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    cnt += e[u] != kNone;
+                    s[u] = nx[u];
+                }
+            }
+        } else
         for (uint32_t j0 = tid; j0 < ns; j0 += U * NT) {
             unsigned long long nx[U], e[U];
             uint32_t h[U];
@@ -1876,7 +2031,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_words_kernel(JoinA
         __syncthreads();
     }
     block_sum2_to(cnt, sum, red, &a.acc->matched, &a.acc->checksum);
-    flag_multi(multi, &a.acc->dup_flag);
+    if (!MAT) flag_multi(multi, &a.acc->dup_flag);
     join_finish(a, true);
 }
 
@@ -1909,7 +2064,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_kernel(JoinArgs a0
     const int tid = threadIdx.x;
     unsigned int *err = &a.counters[kCtrErr];
     const uint32_t nitems = a.counters[kCtrNItems];
-    if (!MAT && a.ci && ci_applies(a.counters, a.bits)) return;  // join_first_words_kernel
+    if (a.ci && ci_applies(a.counters, a.bits)) return;  // join_first_words_kernel
     const int B = a.bits;
     const bool skip0 = a.skip0 != 0;
     unsigned long long cnt = 0, sum = 0;
@@ -2031,7 +2186,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_small_kernel(JoinArgs a0
     __syncthreads();
     const uint32_t nitems = a.counters[kCtrNItems];
     // Compiled once per partition layout; only the launch matching the device's choice runs.
-    if (CI != (!MAT && a.ci && ci_applies(a.counters, a.bits))) return;
+    if (CI != (a.ci && ci_applies(a.counters, a.bits))) return;
     constexpr bool ci = CI;
     const int B = ci ? 0 : a.bits;  // shift from a stored x to the key's bits above the radix bits
     const bool lp = a.lp != 0;
@@ -2332,7 +2487,7 @@ __device__ __forceinline__ void large_probe(const JoinArgs &a, uint32_t blk, uin
     const uint64_t total = ld_u64_pair(&a.counters[kCtrLargeS]);
     unsigned long long cnt = 0, sum = 0;
     bool multi = false;  // first-match joins: a probe tuple matched two build tuples
-    const bool ci = !MAT && a.ci && ci_applies(a.counters, a.bits);
+    const bool ci = a.ci && ci_applies(a.counters, a.bits);
     const int bshift = ci ? 0 : a.bits;
     if constexpr (MAT) {
         unsigned int *err = &a.counters[kCtrErr];
@@ -2344,16 +2499,21 @@ __device__ __forceinline__ void large_probe(const JoinArgs &a, uint32_t blk, uin
             const LargePart *Lp = nullptr;
             if (g < total) {
                 Lp = &a.large[find_large(a.large, nl, g, false)];
-                s = ld_stream(a.finS + Lp->s_begin + (g - Lp->s_flat));
+                s = ld_fin(a.finS, a.finS8, Lp->s_begin + (g - Lp->s_flat), ci);
                 const uint32_t *head = a.large_table + Lp->table_off;
                 const uint32_t *nxt = head + (1ull << Lp->nb_log);
-                const tuple_v *rr = a.finR + Lp->r_begin;
-                e0 = head[(s.x >> a.bits) & ((1ull << Lp->nb_log) - 1)];
+                unsigned long long best_y = 0;
+                e0 = head[(s.x >> bshift) & ((1ull << Lp->nb_log) - 1)];
                 uint64_t steps = 0;
                 for (uint32_t e = e0; e;) {
-                    if (rr[e - 1].x == s.x) {
-                        if (!a.lp) m++;
-                        else if (best == 0 || (a.lp_pos ? rr[e - 1].y < rr[best - 1].y : e < best)) best = e;
+                    const tuple_v r = fin_r(a, ci, Lp->r_begin + e - 1);
+                    if (r.x == s.x) {
+                        if (!a.lp) {
+                            m++;
+                        } else if (best == 0 || (a.lp_pos ? r.y < best_y : e < best)) {
+                            best = e;
+                            best_y = r.y;
+                        }
                     }
                     e = nxt[e - 1];
                     if (++steps > Lp->r_len) {
@@ -2367,14 +2527,15 @@ __device__ __forceinline__ void large_probe(const JoinArgs &a, uint32_t blk, uin
             cnt += m;
             if (m) {
                 const uint32_t *nxt = a.large_table + Lp->table_off + (1ull << Lp->nb_log);
-                const tuple_v *rr = a.finR + Lp->r_begin;
                 if (a.lp) {
-                    const unsigned long long y = rr[best - 1].y;
+                    const unsigned long long y = fin_r(a, ci, Lp->r_begin + best - 1).y;
                     mat_put(a.mat, o, !a.lp_pos ? y : y < a.nR ? a.relR[y].y : 0ull, s.y, err);
                 } else {
                     uint64_t steps = 0;
-                    for (uint32_t e = e0; e && steps++ <= Lp->r_len; e = nxt[e - 1])
-                        if (rr[e - 1].x == s.x) mat_put(a.mat, o++, rr[e - 1].y, s.y, err);
+                    for (uint32_t e = e0; e && steps++ <= Lp->r_len; e = nxt[e - 1]) {
+                        const tuple_v r = fin_r(a, ci, Lp->r_begin + e - 1);
+                        if (r.x == s.x) mat_put(a.mat, o++, r.y, s.y, err);
+                    }
                 }
             }
         }
@@ -2529,7 +2690,8 @@ int radix_geom(int bits, int passes, RadixGeom *g, int b1_req) {
 // kSingleManyTuples tuples: the scatter visits every page of its output once per tile, and those visits
 // grow with the output (2^24 x 2^24, 12 bits: 0.57 ms in one pass, 0.74 in two; 2^24 x 2^26: 1.34 and 1.32;
 // 2^24 x 2^28: 4.50 and 3.38). First-match joins stay up to twice that size: two passes may have to run
-// again in order where build keys repeat (2^24 x 2^26, four a key: 1.55 ms against 2 x 1.4 and more).
+// again in order where build keys repeat (2^24 x 2^26, four a key: 1.55 ms against 2 x 1.4 and more). So do
+// materialising joins, which have words in one pass only (`lp` covers both).
 constexpr uint64_t kSingleTarget = 6144, kSingleMaxAvg = 8192, kSingleManyTuples = 80000000;
 constexpr int kSingleMinBits = 8;
 
@@ -2771,6 +2933,9 @@ int phj_prepare_device() {
                                (int)kCompactSmem));
     HJ_CU(cudaFuncSetAttribute(join_compact_kernel<true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)kCompactSmem));
+    HJ_CU(cudaFuncSetAttribute(join_words_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOaSmem));
+    HJ_CU(cudaFuncSetAttribute(join_first_words_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)kFwSmem));
     HJ_CU(cudaFuncSetAttribute(join_words_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOaSmem));
     HJ_CU(cudaFuncSetAttribute(join_words_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOaSmem));
     HJ_CU(cudaFuncSetAttribute(join_first_words_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwSmem));
@@ -2816,7 +2981,7 @@ JoinArgs join_args(const RadixGeom &g, bool lp, bool skip0, const ulonglong2 *R,
     ja.nR = nR;
     ja.flag_bits = g.req_bits;
     ja.w8_b1 = w8_b1;
-    ja.all_items = g.single && !mat ? 1 : 0;
+    ja.all_items = g.single ? 1 : 0;
     ja.host_out = host_out;
     return ja;
 }
@@ -2890,7 +3055,7 @@ int phj_enqueue(const RadixGeom &g, bool lp, bool skip0, const ulonglong2 *R, si
     // 8-byte words in the partitions (compact final partitions, and in segment mode an 8-byte pass 1):
     // joins without per-match output (all but the materialising ones), unless the caller asked for
     // tuples (test_flags bit 2), when the widths allow them (decided on the device).
-    const int ci_ok = (!mat && !(test_flags & 2)) ? 1 : 0;
+    const int ci_ok = ((!mat || g.single) && !(test_flags & 2)) ? 1 : 0;
     const bool seg_words = segm && ci_ok;
     // The exact-offset pipeline with two passes stores pass 1 as words too (when w8_fits holds, which
     // the histogram pass's ORs decide before pass 1) when its pass-2 units (chunk, pass-1 digit) average
@@ -3105,15 +3270,21 @@ int phj_enqueue(const RadixGeom &g, bool lp, bool skip0, const ulonglong2 *R, si
                                   g.single && !mat ? host_out : nullptr);
     const MultiRef none = {};
     if (ja.lp_pos) {
-        if (mat)
+        if (mat) {
+            join_first_words_kernel<false, true><<<num_sms, kJoinThreads, kFwSmem, st>>>(ja, none);
             join_first_kernel<true><<<num_sms, kJoinThreads, kFirstSmem, st>>>(ja, none);
-        else {
+            nlaunch++;
+        } else {
             // One launch per element layout; the one that does not match the device's choice returns at once.
             join_first_words_kernel<false><<<num_sms, kJoinThreads, kFwSmem, st>>>(ja, none);
             join_first_kernel<false><<<num_sms, kJoinThreads, kFirstSmem, st>>>(ja, none);
             nlaunch++;
         }
         nlaunch++;
+    } else if (mat && g.single) {
+        join_words_kernel<false, true><<<num_sms * 2, kCompactThreads, kOaSmem, st>>>(ja, none);
+        join_small_kernel<true><<<num_sms, kJoinThreads, kJoinSmem, st>>>(ja, none);
+        nlaunch += 2;
     } else if (mat) {
         if (lp)
             join_compact_kernel<true, false, true><<<num_sms * 2, kCompactThreads, kCompactSmem, st>>>(ja);

@@ -84,3 +84,58 @@ def test_materialised_pairs(hj, oracle, cuda, algo):
     got = out.cpu().numpy().view(np.uint64)
     assert r.matched_cnt == want.shape[0]
     assert np.array_equal(got[np.lexsort((got[:, 1], got[:, 0]))], want)
+
+
+@pytest.mark.parametrize("algo", ["phj_radix_bc", "phj_radix_lp", "nphj_sc", "nphj_lp"])
+@pytest.mark.parametrize("kind", ["unique", "dups", "hot", "wide_key", "wide_rid"])
+def test_materialised_words(hj, oracle, cuda, algo, kind):
+    """Pairs written from compact words and from tuples, with at most one match per probe and with many, a hot
+    build key in a large partition, and a row id that is not a position (refused with HJ_E_ROWID)."""
+    rng = np.random.default_rng(8)
+    nR, nS = 50_001, 120_007
+    R, S = relations(rng, nR, nS, "key" if kind == "wide_key" else "word", 3 if kind == "dups" else 1)
+    S[: nS // 8, 0] = R[rng.integers(0, nR, nS // 8), 0]
+    if kind == "hot":
+        R[: 12_000, 0] = R[0, 0]
+        S[(S[:, 0] == R[0, 0]), 0] += np.uint64(1)
+        S[:3, 0] = R[0, 0]
+    R[:, 1] = np.arange(1, nR + 1, dtype=np.uint64)
+    S[:, 1] = np.arange(1, nS + 1, dtype=np.uint64)
+    if kind == "wide_rid":
+        R[0, 1] = np.uint64(1 << 40)
+        S[0, 0] = R[0, 0]
+        r = hj.join_mat(algo, dev(cuda, R), dev(cuda, S), on_device=True, check=False)
+        assert r.status == hj.HJ_E_ROWID or (r.status == 0 and (R[0, 0] == 0 or R[0, 0] == 2**64 - 1))
+        return
+    want = oracle.join_pairs(algo, R, S)
+    out = cuda.zeros((want.shape[0], 2), dtype=cuda.int64, device="cuda")
+    r = hj.join_mat(algo, dev(cuda, R), dev(cuda, S), pairs=out, on_device=True)
+    got = out.cpu().numpy().view(np.uint64)
+    assert r.matched_cnt == want.shape[0]
+    assert np.array_equal(got[np.lexsort((got[:, 1], got[:, 0]))], want)
+    assert (r.matched_cnt, r.checksum) == oracle.join(algo, R, S)
+
+
+@pytest.mark.parametrize("algo", ["phj_radix_bc", "phj_radix_lp", "nphj_sc", "nphj_lp"])
+def test_retrieve_columns(hj, cuda, algo):
+    """Relations beyond 64 MB gather from row-id columns: permuted row ids (in range, so retrieved), and one
+    out of range."""
+    nR, nS = (1 << 21) + 5, (1 << 22) + 3
+    g = cuda.Generator(device="cuda")
+    g.manual_seed(2)
+    R = cuda.empty((nR, 2), dtype=cuda.int64, device="cuda")
+    S = cuda.empty((nS, 2), dtype=cuda.int64, device="cuda")
+    R[:, 0] = cuda.randperm(nR, generator=g, device="cuda") + 1
+    S[:, 0] = cuda.randint(1, nR + nR // 4, (nS,), generator=g, device="cuda")
+    R[:, 1] = cuda.randperm(nR, generator=g, device="cuda") + 1
+    S[:, 1] = cuda.randperm(nS, generator=g, device="cuda") + 1
+    rid = cuda.zeros(nR + nR // 4 + 1, dtype=cuda.int64, device="cuda")
+    rid[R[:, 0]] = R[:, 1]
+    hit = rid[S[:, 0]] > 0
+    r_id, s_id = rid[S[:, 0]][hit], S[:, 1][hit]
+    want = (int(hit.sum()), int((R[:, 1][r_id - 1] + S[:, 1][s_id - 1]).sum()))
+    r = hj.join_mat(algo, R, S, on_device=True)
+    assert (r.matched_cnt, r.checksum) == want
+    S[5, 0], S[5, 1] = R[0, 0], 1 << 33
+    r = hj.join_mat(algo, R, S, on_device=True, check=False)
+    assert r.status == hj.HJ_E_ROWID
