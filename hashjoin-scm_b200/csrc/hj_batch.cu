@@ -401,9 +401,9 @@ void decide(const hj_ctx *c, size_t nR, size_t nS, int *impl, int *bits, int *pa
 // Geometry of a join that runs a pipeline of its own: the tuner's, or for a join decided as non-partitioned
 // (too large for a wave) the two-pass one that its size needs.
 int lane_geom(const hj_batch *b, int j, hj::RadixGeom *g) {
-    if (b->impl[j] == kImplPhj) return hj::radix_geom(b->bits[j], b->passes[j], g);
-    const int rc = hj::radix_geom(14, 2, g);
-    hj::radix_geom_by_size(b->jobs[j].nR, g);
+    const bool phj = b->impl[j] == kImplPhj;
+    const int rc = hj::radix_geom(phj ? b->bits[j] : 14, phj ? b->passes[j] : 2, g);
+    hj::radix_geom_by_size(b->jobs[j].nR, false, g);
     return rc;
 }
 

@@ -42,8 +42,9 @@ int radix_geom(int bits, int passes, RadixGeom *g, int b1_req = 0);
 constexpr int kSingleMaxBits = 11;
 bool radix_geom_single(int bits, bool lp, size_t nR, size_t nS, RadixGeom *g);
 
-// Lower the bits of a two-pass geometry to what a build relation of nR tuples needs.
-void radix_geom_by_size(size_t nR, RadixGeom *g);
+// Lower the bits of a two-pass geometry to what a build relation of nR tuples needs, and split them for the
+// passes unless the caller gave the split (a split given for more bits than are needed does not apply).
+void radix_geom_by_size(size_t nR, bool split_given, RadixGeom *g);
 
 // Joins of at most kSmallMaxBuild build tuples run as one kernel (hj_small.cu).
 constexpr uint32_t kSmallMaxBuild = 8192;

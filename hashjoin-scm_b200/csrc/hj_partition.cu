@@ -884,12 +884,28 @@ struct SegSlot {
     int rel;
 };
 
-// Where a digit's run of the staged tile goes: staged index j < split to base + j (the rest of the
-// current segment), j >= split to base2 + j (the new segment).
-struct SegRun {
-    long long base, base2;
-    uint32_t split, pad;
+// Where a digit's run of the staged tile goes: staged index j < split to base + j - kTile (the rest of the
+// current segment), j >= split to base2 + j - kTile (the new segment). 40-bit bases, biased so that they are
+// not negative, in one 16-byte load; kSegNowhere fails the bounds check of the store.
+constexpr unsigned long long kSegNowhere = (1ull << 40) - 1;
+struct __align__(16) SegRun {
+    uint32_t base_lo, base2_lo, split_hi, pad;  // split_hi: split | base >> 32 << 16 | base2 >> 32 << 24
 };
+__device__ __forceinline__ SegRun seg_run(unsigned long long base, unsigned long long base2, uint32_t split) {
+    SegRun r;
+    r.base_lo = (uint32_t)base;
+    r.base2_lo = (uint32_t)base2;
+    r.split_hi = split | (uint32_t)(base >> 32) << 16 | (uint32_t)(base2 >> 32) << 24;
+    r.pad = 0;
+    return r;
+}
+__device__ __forceinline__ unsigned long long seg_dst(const SegRun *run, uint32_t j) {
+    const uint4 r = *reinterpret_cast<const uint4 *>(run);
+    const bool first = j < (r.z & 0xffffu);
+    const unsigned long long base =
+        ((unsigned long long)(first ? (r.z >> 16) & 0xffu : r.z >> 24) << 32) | (first ? r.x : r.y);
+    return base + j - kTile;
+}
 
 // Thread 0: the next tile of this CTA's current work item, claiming items as needed. STATIC_R: the build
 // relation's items [r_next, r_end) belong to this CTA and come first, in order; the probe relation's
@@ -1088,7 +1104,7 @@ __global__ void __launch_bounds__(THREADS, kSegCtasPerSm) seg_pass1_kernel(SegAr
         tuple_v v[ITEMS];
         uint32_t rk[ITEMS];
         const bool st = STABLE_R && sl.rel == 0;  // uniform: this tile takes the stable rank
-        uint32_t xo = 0, yo = 0;
+        uint32_t xo = 0, yo = 0, lo = 0;
         if (cnt == (uint32_t)T) {
 #pragma unroll
             for (int i = 0; i < ITEMS; i++) {
@@ -1099,6 +1115,7 @@ __global__ void __launch_bounds__(THREADS, kSegCtasPerSm) seg_pass1_kernel(SegAr
                 atomicAdd(&jh[bin >> 1], 1u << ((bin & 1u) << 4));
                 xo |= (uint32_t)(v[i].x >> 32);
                 yo |= (uint32_t)(v[i].y >> 32);
+                lo |= (uint32_t)v[i].x;
             }
         } else {
 #pragma unroll
@@ -1112,6 +1129,7 @@ __global__ void __launch_bounds__(THREADS, kSegCtasPerSm) seg_pass1_kernel(SegAr
                     atomicAdd(&jh[bin >> 1], 1u << ((bin & 1u) << 4));
                     xo |= (uint32_t)(v[i].x >> 32);
                     yo |= (uint32_t)(v[i].y >> 32);
+                    lo |= (uint32_t)v[i].x;
                 }
             }
         }
@@ -1165,7 +1183,13 @@ __global__ void __launch_bounds__(THREADS, kSegCtasPerSm) seg_pass1_kernel(SegAr
                 thist[tid] = h;
             }
         }
-        __syncthreads();
+        // Words: a tile whose keys are below 2^31 and row ids below 2^32 is staged as 8-byte {row id, key}, half
+        // the shared-memory traffic of a tuple; the word is made from it when it is written.
+        bool narrow = false;
+        if (W8)
+            narrow = !__syncthreads_or((xo | yo | (lo >> 31)) != 0);
+        else
+            __syncthreads();
         // Warp 0, step 1: digit starts in the staged tile, and which digits' runs need a new segment
         // (a run that does not fit the rest of its current segment). Lane l owns digits [l*K, l*K + K).
         uint32_t hv[K];      // warp 0: tile count of each owned digit
@@ -1206,7 +1230,11 @@ __global__ void __launch_bounds__(THREADS, kSegCtasPerSm) seg_pass1_kernel(SegAr
             const uint32_t idx = (uint32_t)(w * 32 * ITEMS + i * 32 + lane);
             if (idx < cnt) {
                 const uint32_t d = (uint32_t)v[i].x & dmask;
-                buf[tdstart[d] + (STABLE_R && st ? (uint32_t)whist[w * F + d] : 0u) + rk[i]] = v[i];
+                const uint32_t p = tdstart[d] + (STABLE_R && st ? (uint32_t)whist[w * F + d] : 0u) + rk[i];
+                if (W8 && narrow)
+                    reinterpret_cast<uint2 *>(buf)[p] = make_uint2((uint32_t)v[i].y, (uint32_t)v[i].x);
+                else
+                    buf[p] = v[i];
             }
         }
         // Warp 0, step 2 (while the other warps stage): where each digit's run goes, the rest of its
@@ -1242,10 +1270,10 @@ __global__ void __launch_bounds__(THREADS, kSegCtasPerSm) seg_pass1_kernel(SegAr
                     const uint32_t h = hv[j];
                     if (h) {
                         const uint32_t sc = scur[j], fill = sfill[j];
-                        SegRun r;
+                        unsigned long long b1 = kSegNowhere, b2 = kSegNowhere;
+                        uint32_t split = ex + h;
                         if (sc != kSegNone && fill + h <= SEGW) {
-                            r.base = r.base2 = (long long)sc * SEGW + fill - ex;
-                            r.split = ex + h;
+                            b1 = b2 = (unsigned long long)sc * SEGW + fill + kTile - ex;
                             sfill[j] = fill + h;
                         } else {
                             const uint32_t id = e < old_rem ? old_lo + e : nb + (e - old_rem);
@@ -1254,16 +1282,15 @@ __global__ void __launch_bounds__(THREADS, kSegCtasPerSm) seg_pass1_kernel(SegAr
                                 if (sc == kSegNone) {
                                     // The whole run starts the chain.
                                     a.seg_head[((size_t)phase_rel * G + c) * F + d] = id;
-                                    r.base = r.base2 = (long long)id * SEGW - ex;
-                                    r.split = ex + h;
+                                    b1 = b2 = (unsigned long long)id * SEGW + kTile - ex;
                                     sfill[j] = h;
                                 } else {
                                     // The run fills the current segment, then goes on in segment
                                     // id: staged index ex + (SEGW - fill) lands at id * SEGW.
                                     a.seg_next[sc] = id;
-                                    r.base = (long long)sc * SEGW + fill - ex;
-                                    r.base2 = r.base + ((long long)id - (long long)sc - 1) * SEGW;
-                                    r.split = ex + (SEGW - fill);
+                                    b1 = (unsigned long long)sc * SEGW + fill + kTile - ex;
+                                    b2 = (unsigned long long)id * SEGW + kTile - ex - (SEGW - fill);
+                                    split = ex + (SEGW - fill);
                                     sfill[j] = h - (SEGW - fill);
                                 }
                                 scur[j] = id;
@@ -1271,13 +1298,11 @@ __global__ void __launch_bounds__(THREADS, kSegCtasPerSm) seg_pass1_kernel(SegAr
                                 // Cannot happen with the storage phj_carve reserves; the run's
                                 // stores fail their bounds check and report it.
                                 set_error(err, kErrCapacity);
-                                r.base = r.base2 = -(long long)cap - (long long)SEGW;
-                                r.split = ex + h;
                                 scur[j] = kSegNone;
                                 sfill[j] = 0;
                             }
                         }
-                        runs[d] = r;
+                        runs[d] = seg_run(b1, b2, split);
                     }
                     ex += h;
                 }
@@ -1286,22 +1311,46 @@ __global__ void __launch_bounds__(THREADS, kSegCtasPerSm) seg_pass1_kernel(SegAr
         __syncthreads();
         // Write each digit run: consecutive threads write consecutive 16-byte tuples (8-byte words).
         // A destination outside the segment storage (negative included) fails the unsigned bound check.
-        if (cnt == (uint32_t)T) {
+        if (W8 && narrow) {
+            const uint2 *nbuf = reinterpret_cast<const uint2 *>(buf);
+            auto word = [&](const uint2 &x) { return ((unsigned long long)(x.y >> a.b1) << 32) | x.x; };
+            if (cnt == (uint32_t)T) {
+                uint2 t[ITEMS];
+                unsigned long long dst[ITEMS];
+#pragma unroll
+                for (int i = 0; i < ITEMS; i++) t[i] = nbuf[tid + i * THREADS];
+#pragma unroll
+                for (int i = 0; i < ITEMS; i++) dst[i] = seg_dst(&runs[t[i].y & dmask], (uint32_t)(tid + i * THREADS));
+#pragma unroll
+                for (int i = 0; i < ITEMS; i++) {
+                    if (dst[i] < cap)
+                        st_stream8(out8 + dst[i], word(t[i]));
+                    else
+                        set_error(err, kErrBounds);
+                }
+            } else {
+                for (uint32_t j = tid; j < cnt; j += THREADS) {
+                    const uint2 t = nbuf[j];
+                    const unsigned long long dst = seg_dst(&runs[t.y & dmask], j);
+                    if (dst < cap)
+                        st_stream8(out8 + dst, word(t));
+                    else
+                        set_error(err, kErrBounds);
+                }
+            }
+        } else if (cnt == (uint32_t)T) {
 #pragma unroll
             for (int hh = 0; hh < 2; hh++) {
                 tuple_v t[ITEMS / 2];
-                long long dst[ITEMS / 2];
+                unsigned long long dst[ITEMS / 2];
 #pragma unroll
                 for (int i = 0; i < ITEMS / 2; i++) t[i] = buf[tid + (hh * ITEMS / 2 + i) * THREADS];
 #pragma unroll
-                for (int i = 0; i < ITEMS / 2; i++) {
-                    const uint32_t j = (uint32_t)(tid + (hh * ITEMS / 2 + i) * THREADS);
-                    const SegRun r = runs[(uint32_t)t[i].x & dmask];
-                    dst[i] = (j < r.split ? r.base : r.base2) + (long long)j;
-                }
+                for (int i = 0; i < ITEMS / 2; i++)
+                    dst[i] = seg_dst(&runs[(uint32_t)t[i].x & dmask], (uint32_t)(tid + (hh * ITEMS / 2 + i) * THREADS));
 #pragma unroll
                 for (int i = 0; i < ITEMS / 2; i++) {
-                    if ((uint64_t)dst[i] < cap) {
+                    if (dst[i] < cap) {
                         if (W8)
                             st_stream8(out8 + dst[i], w8_word(t[i].x, t[i].y, a.b1));
                         else
@@ -1314,9 +1363,8 @@ __global__ void __launch_bounds__(THREADS, kSegCtasPerSm) seg_pass1_kernel(SegAr
         } else {
             for (uint32_t j = tid; j < cnt; j += THREADS) {
                 const tuple_v t = buf[j];
-                const SegRun r = runs[(uint32_t)t.x & dmask];
-                const long long dst = (j < r.split ? r.base : r.base2) + (long long)j;
-                if ((uint64_t)dst < cap) {
+                const unsigned long long dst = seg_dst(&runs[(uint32_t)t.x & dmask], j);
+                if (dst < cap) {
                     if (W8)
                         st_stream8(out8 + dst, w8_word(t.x, t.y, a.b1));
                     else
@@ -1679,7 +1727,9 @@ __device__ __forceinline__ void mat_write_round(MatRound &r, const unsigned long
 
 // MAT: one pair per match. Without repeated build keys a probe has at most one match, and the block reserves
 // output for a round of eight probes per thread by ballots, so a warp writes consecutive pairs.
-template <bool MULTI, bool MAT = false>
+// LP: the unordered run of a first-match join: one match per probe tuple, whichever comes first; a probe tuple
+// with a second one sets acc->dup_flag, and the join runs again in order. Build key 0 never matches (skip0).
+template <bool MULTI, bool MAT = false, bool LP = false>
 __global__ void __launch_bounds__(kCompactThreads, 2) join_words_kernel(JoinArgs a0, MultiRef mr) {
     __shared__ JoinArgs s_a;
     if (MULTI) {
@@ -1702,6 +1752,7 @@ __global__ void __launch_bounds__(kCompactThreads, 2) join_words_kernel(JoinArgs
     unsigned int *err = &a.counters[kCtrErr];
     const uint32_t nitems = a.counters[kCtrNItems];
     unsigned long long cnt = 0, sum = 0;
+    bool multi = false;
     for (;;) {
         if (tid == 0) {
             s_item = atomicAdd(&a.counters[kCtrItemA], 1u);
@@ -1731,6 +1782,7 @@ __global__ void __launch_bounds__(kCompactThreads, 2) join_words_kernel(JoinArgs
             for (int u = 0; u < UR; u++) {
                 if (r[u] == kNone) continue;
                 const uint32_t hi = (uint32_t)(r[u] >> 32);
+                if (LP && a.skip0 && item.part0 && hi == 0) continue;
                 uint32_t h = __umulhi(oa_hash(hi), nslots);
                 for (uint32_t steps = 0;;) {
                     const unsigned long long cur = atomicCAS(&slots[h], kNone, r[u]);
@@ -1760,6 +1812,7 @@ __global__ void __launch_bounds__(kCompactThreads, 2) join_words_kernel(JoinArgs
             for (uint32_t i = tid; i < nr; i += NT) {
                 const unsigned long long w = R8[i];
                 slots[i] = w;
+                if (LP && a.skip0 && item.part0 && (w >> 32) == 0) continue;
                 nxt[i] = (uint16_t)atomic_exch_u16(&head[oa_hash((uint32_t)(w >> 32)) >> 21], i + 1);
             }
             __syncthreads();
@@ -1785,9 +1838,15 @@ __global__ void __launch_bounds__(kCompactThreads, 2) join_words_kernel(JoinArgs
                 const unsigned long long w = ld_stream8(S8 + j);
                 const uint32_t hi = (uint32_t)(w >> 32);
                 uint32_t steps = 0;
+                bool found = false;
                 for (uint32_t e = head[oa_hash(hi) >> 21]; e; e = nxt[e - 1]) {
                     const unsigned long long b = slots[e - 1];
                     if ((uint32_t)(b >> 32) == hi) {
+                        if (LP && found) {
+                            multi = true;
+                            break;
+                        }
+                        found = true;
                         cnt++;
                         sum += (b & 0xffffffffull) + (w & 0xffffffffull);
                     }
@@ -1852,8 +1911,14 @@ __global__ void __launch_bounds__(kCompactThreads, 2) join_words_kernel(JoinArgs
             for (int u = 0; u < U; u++) {
                 const uint32_t hi = (uint32_t)(s[u] >> 32);
                 // A word past the end (kNone), as a probe key beyond every build key, matches nothing.
+                bool found = false;
                 for (uint32_t steps = 0; e[u] != kNone;) {
                     if ((uint32_t)(e[u] >> 32) == hi) {
+                        if (LP && found) {
+                            multi = true;
+                            break;
+                        }
+                        found = true;
                         cnt++;
                         sum += (e[u] & 0xffffffffull) + (s[u] & 0xffffffffull);
                         if (!dups) break;
@@ -1872,6 +1937,7 @@ __global__ void __launch_bounds__(kCompactThreads, 2) join_words_kernel(JoinArgs
         __syncthreads();
     }
     block_sum2_to(cnt, sum, red, &a.acc->matched, &a.acc->checksum);
+    if (LP) flag_multi(multi, &a.acc->dup_flag);
     join_finish(a, true);
 }
 
@@ -2746,13 +2812,18 @@ struct PhjSizes {
 
 // The two-pass pipelines' geometry: the lowest bits that bring build partitions to kSingleTarget tuples, at
 // most what the caller asked for. Fewer digits make longer runs and fewer, fuller units (2^24 x 2^26 in
-// segment mode: 1.32 ms with 12 bits, 1.40 with 13, 2.00 with 14; 2^24 x 2^28 3.38 / 3.47 / 4.09).
-void radix_geom_by_size(size_t nR, RadixGeom *g) {
+// segment mode: 1.32 ms with 12 bits, 1.40 with 13, 2.00 with 14; 2^24 x 2^28 3.38 / 3.47 / 4.09). Pass 2
+// takes eight of them (pass 1 at least kMinBits1), unless the caller split them: a unit of pass 2 is a (pass-1
+// CTA, digit) chain, and fewer pass-1 digits leave less of its last tile empty (2^26 x 2^28, 14 bits: 4.15 ms
+// with 6 + 8, 4.41 with 7 + 7; 2^25 x 2^26, 13 bits: 1.39 with 5 + 8, 1.51 with 6 + 7; 2^24 x 2^27, 12 bits:
+// 1.77 with 5 + 7, 1.82 with 4 + 8; 16-byte tuples prefer one bit more in pass 1, by 4%).
+constexpr int kMinBits1 = 5;
+void radix_geom_by_size(size_t nR, bool split_given, RadixGeom *g) {
     if (g->passes != 2) return;
+    const int req = g->req_bits;
     int b = 2;
     while (b < g->bits && (nR >> b) > kSingleTarget) b++;
-    const int req = g->req_bits;
-    if (b < g->bits) radix_geom(b, 2, g);
+    if (b < g->bits || !split_given) radix_geom(b, 2, g, b - 8 > kMinBits1 ? b - 8 : kMinBits1);
     g->req_bits = req;
 }
 
@@ -2933,6 +3004,8 @@ int phj_prepare_device() {
                                (int)kCompactSmem));
     HJ_CU(cudaFuncSetAttribute(join_compact_kernel<true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)kCompactSmem));
+    HJ_CU(cudaFuncSetAttribute(join_words_kernel<false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)kOaSmem));
     HJ_CU(cudaFuncSetAttribute(join_words_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOaSmem));
     HJ_CU(cudaFuncSetAttribute(join_first_words_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)kFwSmem));
@@ -3307,12 +3380,16 @@ int phj_enqueue(const RadixGeom &g, bool lp, bool skip0, const ulonglong2 *R, si
         join_small_kernel<false, false><<<num_sms, kJoinThreads, kJoinSmem, st>>>(ja, none);
         nlaunch += 2;
         if (ci_ok) {
-            if (lp)
+            if (lp && !ordered) {
+                join_words_kernel<false, false, true><<<num_sms * 2, kCompactThreads, kOaSmem, st>>>(ja, none);
+            } else if (lp) {
                 join_compact_kernel<false, true, true><<<num_sms * 2, kCompactThreads, kCompactSmem, st>>>(ja);
-            else
-                join_compact_kernel<false, true><<<num_sms * 2, kCompactThreads, kCompactSmem, st>>>(ja);
-            join_small_kernel<false, true><<<num_sms, kJoinThreads, kJoinSmem, st>>>(ja, none);
-            nlaunch += 2;
+                join_small_kernel<false, true><<<num_sms, kJoinThreads, kJoinSmem, st>>>(ja, none);
+                nlaunch++;
+            } else {
+                join_words_kernel<false><<<num_sms * 2, kCompactThreads, kOaSmem, st>>>(ja, none);  // items of every size
+            }
+            nlaunch++;
         }
     }
     HJ_CU(cudaGetLastError());

@@ -28,7 +28,7 @@ namespace hj {
 
 constexpr int kCountThreads = 1024;
 constexpr int kPlaceThreads = 512;  // scatter: one CTA per SM
-constexpr int kWordItems = 16, kTupleItems = kWordItems / 2;  // staged 8-byte / 16-byte elements per thread and tile
+constexpr int kWordItems = 20, kTupleItems = kWordItems / 2;  // staged 8-byte / 16-byte elements per thread and tile
 constexpr int kSingleDigitsPerThread = ((1 << kSingleMaxBits) + kPlaceThreads - 1) / kPlaceThreads;
 
 // The contiguous range of n tuples that block c of G takes (a multiple of 8 tuples, one 128-byte line).
