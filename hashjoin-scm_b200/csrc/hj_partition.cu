@@ -360,6 +360,17 @@ struct ItemAhead {
     uint32_t seg;
 };
 
+// The n-th claim's work item. Pass 2 takes the units by pass-1 digit, every chunk's unit of one digit before
+// the next digit, so that the CTAs of the moment write one digit's stretch of the output (pass 2 of 2^26 x 2^28
+// Zipf keys: 1790 -> 1735 us, of 2^27 x 2^29 uniform keys: 3015 -> 2990 us).
+__device__ __forceinline__ uint32_t item_at(const ScatterArgs &a, uint32_t n, uint32_t nitems) {
+    if (a.pass == 0 || n >= nitems) return n;
+    const uint32_t cR = a.cg.cR, r_items = cR * (uint32_t)a.F1;
+    if (n < r_items) return (n % cR) * (uint32_t)a.F1 + n / cR;
+    const uint32_t m = n - r_items, cS = a.cg.cS;
+    return r_items + (m % cS) * (uint32_t)a.F1 + m / cS;
+}
+
 // Issue the loads that describe `ah.item` (pass 2 units; pass-1 sub-chunks need none).
 __device__ __forceinline__ void item_fetch(const ScatterArgs &a, ItemAhead &ah, uint32_t nitems) {
     ah.stage = 2;
@@ -418,7 +429,7 @@ __device__ __forceinline__ TileSlot next_tile(const ScatterArgs &a, ItemIter &it
     for (;;) {
         while (it.item == ~0u || it.done >= it.len) {
             if (ah.stage == 0) {
-                ah.item = a.item_base + atomicAdd(&a.counters[a.ctr_item], 1u);
+                ah.item = item_at(a, a.item_base + atomicAdd(&a.counters[a.ctr_item], 1u), nitems);
                 ah.stage = 1;
             }
             if (ah.stage == 1) item_fetch(a, ah, nitems);
@@ -441,7 +452,7 @@ __device__ __forceinline__ TileSlot next_tile(const ScatterArgs &a, ItemIter &it
             // one is done. (Pass-1 items are long, and an item held back per CTA lengthens the tail
             // by more than the claim costs.)
             if (a.pass != 0) {
-                ah.item = a.item_base + atomicAdd(&a.counters[a.ctr_item], 1u);
+                ah.item = item_at(a, a.item_base + atomicAdd(&a.counters[a.ctr_item], 1u), nitems);
                 ah.stage = 1;
             }
             item_decode(a, cur.item, cur, it);
@@ -1650,7 +1661,9 @@ __device__ __forceinline__ void join_finish(const JoinArgs &a, bool ci) {
 // counted): two CTAs of 512 threads per SM with 13312 slots each. A probe is one 8-byte shared load when its
 // key sits in its first slot and the build saw no key twice, where a chain costs a head, a word and a link.
 // Slots come from the high product of a multiplicative hash, so the table takes any size: twice the build
-// partition (less for the largest, 10240 tuples). Equal keys sit in a row; a build that walks more than
+// partition (less for the largest, 10240 tuples). A thread walks for four probe words per round (8: 1240 us for
+// 2^27 x 2^29 tuples, 4: 1200, 2: 1378: more overlaps more loads, less lets the warps drift apart).
+// Equal keys sit in a row; a build that walks more than
 // kOaMaxSteps slots (a key repeated often) is done again with chains in the same memory.
 constexpr uint32_t kOaSlots = 13312, kOaMaxSteps = 64, kOaHeads = 2048;
 constexpr size_t kOaSmem = (size_t)kOaSlots * 8;
@@ -1747,7 +1760,7 @@ __global__ void __launch_bounds__(kCompactThreads, 2) join_words_kernel(JoinArgs
     __shared__ unsigned long long s_base;
     if (!(a.ci && ci_applies(a.counters, a.bits))) return;
     const int tid = threadIdx.x;
-    constexpr int NT = kCompactThreads, UR = 4, U = 8;
+        constexpr int NT = kCompactThreads, UR = 4, U = 4;
     constexpr unsigned long long kNone = ~0ull;  // no build word has this high part
     unsigned int *err = &a.counters[kCtrErr];
     const uint32_t nitems = a.counters[kCtrNItems];
@@ -1945,7 +1958,8 @@ __global__ void __launch_bounds__(kCompactThreads, 2) join_words_kernel(JoinArgs
 // high part << 32 | position), equal keys share a slot and lower its position, and the row ids of the winners
 // stand beside the slots. Equal keys never lengthen a walk. A bitmap marks the slots that two build tuples
 // share: a probe that matches one sets acc->dup_flag (see flag_multi). One CTA of 1024 threads per SM, 194 KB;
-// a thread keeps its build tuples in registers from the insert to the row-id store.
+// a thread keeps its build tuples in registers from the insert to the row-id store. Probes in rounds of four
+// (8: 280 us for 2^24 x 2^26 tuples, 4: 244, 2: 264).
 constexpr uint32_t kFwSlots = 16384;
 constexpr size_t kFwSmem = (size_t)kFwSlots * 12 + kFwSlots / 8;
 
@@ -1967,7 +1981,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_words_kernel(JoinA
     __shared__ MatRound mat_round;
     if (!(a.ci && ci_applies(a.counters, a.bits))) return;
     const uint32_t tid = threadIdx.x;
-    constexpr int NT = kJoinThreads, UR = kFirstCap / NT, U = 8;
+        constexpr int NT = kJoinThreads, UR = kFirstCap / NT, U = 4;
     static_assert(UR * NT == kFirstCap, "a thread's build tuples");
     constexpr unsigned long long kNone = ~0ull;  // no build element has this high part
     unsigned int *err = &a.counters[kCtrErr];
@@ -2104,7 +2118,8 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_words_kernel(JoinA
 // First-match join of the one-pass pipeline over {key, position} elements (wide). The match with the lowest
 // position wins, so the partition may hold them in any order. Key, position and row id in
 // separate arrays (20 bytes per build tuple, 16-bit bucket heads and chains: 214 KB, one CTA per SM);
-// a build tuple's row id is gathered from the build relation once.
+// a build tuple's row id is gathered from the build relation once. One probe tuple per round, the next one under
+// way (3e6 x 12e6 sparse keys: 166 us; four unrolled: 175 us).
 constexpr uint32_t kFirstHeads = 8192;
 constexpr size_t kFirstSmem = (size_t)kFirstCap * (8 + 8 + 4 + 2) + kFirstHeads * 2;
 
@@ -2135,7 +2150,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_kernel(JoinArgs a0
     const bool skip0 = a.skip0 != 0;
     unsigned long long cnt = 0, sum = 0;
     bool multi = false;
-    constexpr int U = 4;
+    constexpr int U = 4, UP = MAT ? 4 : 1;  // build and probe tuples per thread and round
     for (;;) {
         if (tid == 0) s_item = atomicAdd(&a.counters[kCtrItemA], 1u);
         __syncthreads();
@@ -2148,7 +2163,11 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_kernel(JoinArgs a0
         uint32_t *head32 = reinterpret_cast<uint32_t *>(head);
         for (uint32_t q = tid; q < (nb + 1) / 2; q += kJoinThreads) head32[q] = 0;
         __syncthreads();
-        const tuple_v *R = a.finR + item.r_begin;
+        const tuple_v *R = a.finR + item.r_begin, *S = a.finS + item.s_begin;
+        const uint32_t ns = item.s_len;
+        tuple_v sv[UP];  // the thread's next probe tuples, under way during the build and the walks before them
+#pragma unroll
+        for (int u = 0; u < UP; u++) sv[u] = tid + u * kJoinThreads < ns ? ld_stream(S + tid + u * kJoinThreads) : make_ulonglong2(0, 0);
         for (uint32_t i0 = tid; i0 < nr; i0 += U * kJoinThreads) {
             tuple_v t[U];
             unsigned long long y[U];
@@ -2175,18 +2194,16 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_kernel(JoinArgs a0
             }
         }
         __syncthreads();
-        const tuple_v *S = a.finS + item.s_begin;
-        const uint32_t ns = item.s_len;
-        for (uint32_t base = 0; base < ns; base += U * kJoinThreads) {
-            tuple_v sv[U];
-            uint32_t best[U], m = 0;
+        for (uint32_t base = 0; base < ns; base += UP * kJoinThreads) {
+            tuple_v nx[UP];
+            uint32_t best[UP], m = 0;
 #pragma unroll
-            for (int u = 0; u < U; u++) {
-                const uint32_t j = base + u * kJoinThreads + tid;
-                sv[u] = j < ns ? ld_stream(S + j) : make_ulonglong2(0, 0);
+            for (int u = 0; u < UP; u++) {
+                const uint32_t j = base + (UP + u) * kJoinThreads + tid;
+                nx[u] = j < ns ? ld_stream(S + j) : make_ulonglong2(0, 0);
             }
 #pragma unroll
-            for (int u = 0; u < U; u++) {
+            for (int u = 0; u < UP; u++) {
                 best[u] = 0;
                 if (base + u * kJoinThreads + tid >= ns) continue;
                 uint32_t e = head[(sv[u].x >> B) & hmask], steps = 0, nm = 0, bp = 0;
@@ -2213,9 +2230,11 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_kernel(JoinArgs a0
             if constexpr (MAT) {
                 unsigned long long o = mat_reserve(m, scan_tmp, &s_base, &a.acc->pairs);
 #pragma unroll
-                for (int u = 0; u < U; u++)
+                for (int u = 0; u < UP; u++)
                     if (best[u]) mat_put(a.mat, o++, rid[best[u] - 1], sv[u].y, err);
             }
+#pragma unroll
+            for (int u = 0; u < UP; u++) sv[u] = nx[u];
         }
         __syncthreads();
     }
@@ -2224,6 +2243,12 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_kernel(JoinArgs a0
     join_finish(a, false);
 }
 
+// Partition join over 16-byte tuples (CI: over the words of compact partitions), every match, or with lp the
+// first by partition order: the build partition in shared memory, chained by 16-bit links from up to 16384
+// heads (two per tuple: a warp waits for its longest chain), one CTA of 1024 threads per SM. Bound by those
+// waits, not by bytes: one probe tuple per thread and round, the next one under way, measured 1530 us for
+// 2^26 x 2^28 sparse keys (one head per tuple and four unrolled walks: 2061 us; one head, one walk: 1744; two
+// heads, three walks: 1781). A table of tagged 4-byte slots in place of the chains took 3060 us, its longest walks being longer.
 template <bool MAT, bool CI = false, bool MULTI = false>
 __global__ void __launch_bounds__(kJoinThreads, 1) join_small_kernel(JoinArgs a0, MultiRef mr) {
     __shared__ JoinArgs s_a;
@@ -2259,6 +2284,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_small_kernel(JoinArgs a0
     const bool skip0 = a.skip0 != 0;
     // Items [0, nA) went to the compact kernel if the build side's keys and row ids fit it.
     const uint32_t first_item = !a.all_items && compact_applies(a) ? a.counters[kCtrNItemsA] : 0u;
+    constexpr int U = MAT ? 4 : 1;  // probe tuples per thread and round
     unsigned long long cnt = 0, sum = 0;
     uint32_t phase = 0;
     bool ok = true, multi = false;
@@ -2269,7 +2295,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_small_kernel(JoinArgs a0
         if (it >= nitems) break;
         const JoinItem item = a.items[it];
         const uint32_t nr = item.r_len;
-        const uint32_t nb = next_pow2_u32(nr);
+        const uint32_t nb = min((uint32_t)kHeadMax, 2 * next_pow2_u32(nr));
         const uint64_t hmask = nb - 1;
         if (!ci && tid == 0) {
             // Order earlier generic-proxy accesses to rt before the async-proxy writes.
@@ -2286,6 +2312,16 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_small_kernel(JoinArgs a0
                         dst + off),
                     "l"(src + off), "r"(sz), "r"(bar)
                     : "memory");
+            }
+        }
+        const tuple_v *S = a.finS + item.s_begin;
+        const uint32_t ns = item.s_len;
+        tuple_v s[U];  // the thread's next probe tuples, under way during the build and the walks before them
+        if (!MAT) {
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const uint32_t j = tid + u * kJoinThreads;
+                s[u] = j < ns ? ld_fin(S, a.finS8 + item.s_begin, j, ci) : make_ulonglong2(0, 0);
             }
         }
         uint32_t *head32 = reinterpret_cast<uint32_t *>(head);
@@ -2313,10 +2349,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_small_kernel(JoinArgs a0
         }
         __syncthreads();
         // Probe.
-        const tuple_v *S = a.finS + item.s_begin;
-        const uint32_t ns = item.s_len;
         if constexpr (MAT) {
-            constexpr int U = 4;  // probe tuples per thread and round
             for (uint32_t base = 0; base < ns; base += U * kJoinThreads) {
                 tuple_v sv[U];
 #pragma unroll
@@ -2363,15 +2396,15 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_small_kernel(JoinArgs a0
                 }
             }
         } else
-        for (uint32_t j0 = tid; j0 < ns; j0 += 4 * kJoinThreads) {
-            tuple_v s[4];
+        for (uint32_t j0 = tid; j0 < ns; j0 += U * kJoinThreads) {
+            tuple_v nx[U];
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
-                const uint32_t j = j0 + u * kJoinThreads;
-                s[u] = j < ns ? ld_fin(S, a.finS8 + item.s_begin, j, ci) : make_ulonglong2(0, 0);
+            for (int u = 0; u < U; u++) {
+                const uint32_t j = j0 + (U + u) * kJoinThreads;
+                nx[u] = j < ns ? ld_fin(S, a.finS8 + item.s_begin, j, ci) : make_ulonglong2(0, 0);
             }
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
+            for (int u = 0; u < U; u++) {
                 const uint32_t j = j0 + u * kJoinThreads;
                 if (j >= ns) continue;
                 const uint64_t k = s[u].x;
@@ -2401,6 +2434,8 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_small_kernel(JoinArgs a0
                     multi |= nm > 1;
                 }
             }
+#pragma unroll
+            for (int u = 0; u < U; u++) s[u] = nx[u];
         }
         __syncthreads();
     }
