@@ -75,7 +75,7 @@ int join_geom(hj_algo_t algo, const hj_params_t &p, size_t nR, size_t nS, bool m
     const int rc = hj::radix_geom(p.num_radix_bits, p.num_passes, g, p.radix_bits_pass1);
     if (rc) return rc;
     if (!(p.flags & kPipelineFlags) && !hj::radix_geom_single(p.num_radix_bits, hj::algo_lp(algo) || mat, nR, nS, g))
-        hj::radix_geom_by_size(nR, p.radix_bits_pass1 > 0, g);
+        hj::radix_geom_by_size(nR, nS, p.radix_bits_pass1 > 0, g);
     return HJ_OK;
 }
 
@@ -108,7 +108,7 @@ int plan_join(hj_algo_t algo, hj_params_t *p, size_t nR, size_t nS, JoinPlan *jp
     } else if (nphj_by_radix(*p, nR, nS)) {
         p->flags &= ~(kPipelineFlags | HJ_F_ORDERED);  // radix joins' flags
         hj::radix_geom(14, 2, &jp->geom);
-        if (!hj::radix_geom_single(14, hj::algo_lp(algo) || mat, nR, nS, &jp->geom)) hj::radix_geom_by_size(nR, false, &jp->geom);
+        if (!hj::radix_geom_single(14, hj::algo_lp(algo) || mat, nR, nS, &jp->geom)) hj::radix_geom_by_size(nR, nS, false, &jp->geom);
     } else {
         return HJ_OK;
     }

@@ -403,7 +403,7 @@ void decide(const hj_ctx *c, size_t nR, size_t nS, int *impl, int *bits, int *pa
 int lane_geom(const hj_batch *b, int j, hj::RadixGeom *g) {
     const bool phj = b->impl[j] == kImplPhj;
     const int rc = hj::radix_geom(phj ? b->bits[j] : 14, phj ? b->passes[j] : 2, g);
-    hj::radix_geom_by_size(b->jobs[j].nR, false, g);
+    hj::radix_geom_by_size(b->jobs[j].nR, b->jobs[j].nS, false, g);
     return rc;
 }
 

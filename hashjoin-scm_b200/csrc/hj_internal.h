@@ -44,7 +44,7 @@ bool radix_geom_single(int bits, bool lp, size_t nR, size_t nS, RadixGeom *g);
 
 // Lower the bits of a two-pass geometry to what a build relation of nR tuples needs, and split them for the
 // passes unless the caller gave the split (a split given for more bits than are needed does not apply).
-void radix_geom_by_size(size_t nR, bool split_given, RadixGeom *g);
+void radix_geom_by_size(size_t nR, size_t nS, bool split_given, RadixGeom *g);
 
 // Joins of at most kSmallMaxBuild build tuples run as one kernel (hj_small.cu).
 constexpr uint32_t kSmallMaxBuild = 8192;
@@ -71,7 +71,9 @@ constexpr int kScatterThreads = 256;
 constexpr int kScatterItems = 8;
 constexpr int kScatterBufs = 2;       // tile buffers per CTA (2: double-buffered TMA loads)
 constexpr int kScatterCtasPerSm = 3;  // resident scatter CTAs per SM (registers and shared memory)
-constexpr int kScatterWordCtasPerSm = 2;  // pass 2 over 8-byte words: 16 words per thread, up to 128 registers
+// Pass 2 over 8-byte words, 16 words per thread: three CTAs per SM (72 KB each) fill one another's barriers;
+// the stable rank's counters (3 KB more) leave room for two. 2^25 x 2^27 tuples: 854 us with two, 735 with three.
+constexpr int scatter_word_ctas(bool stable) { return stable ? 2 : 3; }
 constexpr int kTile = kScatterThreads * kScatterItems;  // tuples per partition tile
 constexpr int kJoinThreads = 1024;
 constexpr int kSmemCap = 10240;        // largest build partition joined in shared memory

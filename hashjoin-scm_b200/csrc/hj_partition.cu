@@ -2851,14 +2851,20 @@ struct PhjSizes {
 // takes eight of them (pass 1 at least kMinBits1), unless the caller split them: a unit of pass 2 is a (pass-1
 // CTA, digit) chain, and fewer pass-1 digits leave less of its last tile empty (2^26 x 2^28, 14 bits: 4.15 ms
 // with 6 + 8, 4.41 with 7 + 7; 2^25 x 2^26, 13 bits: 1.39 with 5 + 8, 1.51 with 6 + 7; 2^24 x 2^27, 12 bits:
-// 1.77 with 5 + 7, 1.82 with 4 + 8; 16-byte tuples prefer one bit more in pass 1, by 4%).
+// 1.77 with 5 + 7, 1.82 with 4 + 8; 16-byte tuples prefer one bit more in pass 1, by 4%). From
+// kWideSplitTuples on pass 2 takes seven: what its CTAs write at a time spreads over more memory with the size
+// (2^26 x 2^28: 4.04 ms with 6 + 8, 4.07 with 7 + 7; 2^27 x 2^28: 4.80 and 4.68; 2^27 x 2^29: 7.73 and 7.49).
 constexpr int kMinBits1 = 5;
-void radix_geom_by_size(size_t nR, bool split_given, RadixGeom *g) {
+constexpr uint64_t kWideSplitTuples = 400000000;
+void radix_geom_by_size(size_t nR, size_t nS, bool split_given, RadixGeom *g) {
     if (g->passes != 2) return;
     const int req = g->req_bits;
     int b = 2;
     while (b < g->bits && (nR >> b) > kSingleTarget) b++;
-    if (b < g->bits || !split_given) radix_geom(b, 2, g, b - 8 > kMinBits1 ? b - 8 : kMinBits1);
+    if (b < g->bits || !split_given) {
+        const int bits2 = (uint64_t)nR + nS >= kWideSplitTuples ? 7 : 8;
+        radix_geom(b, 2, g, b - bits2 > kMinBits1 ? b - bits2 : kMinBits1);
+    }
     g->req_bits = req;
 }
 
@@ -2995,19 +3001,25 @@ static size_t seg_smem_bytes(int bits, bool stable) {
            (stable ? (size_t)(kScatterThreads / 32) * 256 * 2 : 0);
 }
 
+// Dynamic shared memory of scatter_kernel: tile buffers (word tiles: 16 spare bytes each), gbase, running,
+// tdstart, and the digit counts (per warp for the stable rank).
+static constexpr size_t scatter_smem_bytes(bool stable) {
+    return (size_t)kScatterBufs * (kTile * 16 + 16) + 256 * 8 * 2 + 256 * 4 +
+           (stable ? (size_t)(kScatterThreads / 32) * 256 * 2 : (size_t)256 * 4);
+}
+
 int phj_prepare_device() {
     int cur_dev = 0;
     HJ_CU(cudaGetDevice(&cur_dev));
     if (cur_dev < 0 || cur_dev >= 64) return HJ_E_INVAL;
     if (g_attr_done[cur_dev]) return HJ_OK;
-    const size_t scatter_smem = (size_t)kScatterBufs * (kTile * 16 + 16) + 256 * 8 * 2 + 256 * 4 + (kScatterThreads / 32) * 256 * 2;
     HJ_CU(cudaFuncSetAttribute(hist_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 136 * 1024));
     HJ_CU(cudaFuncSetAttribute(plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)((size_t)2 * (1u << kPlanStageBits) * 4)));
     HJ_CU(cudaFuncSetAttribute(scatter_kernel<kScatterThreads, kScatterItems, true, kScatterBufs, kScatterCtasPerSm>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scatter_smem));
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scatter_smem_bytes(true)));
     HJ_CU(cudaFuncSetAttribute(scatter_kernel<kScatterThreads, kScatterItems, false, kScatterBufs, kScatterCtasPerSm>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scatter_smem));
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scatter_smem_bytes(false)));
 #define HJ_SEG_ATTR(KK, W, ST)                                                                             \
     HJ_CU(cudaFuncSetAttribute(seg_pass1_kernel<kScatterThreads, kScatterItems, KK, W, ST>,                  \
                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)seg_smem_bytes(kSegMaxBits, ST)))
@@ -3023,11 +3035,11 @@ int phj_prepare_device() {
 #undef HJ_SEG_ATTR4
 #undef HJ_SEG_ATTR
     HJ_CU(cudaFuncSetAttribute(
-        scatter_kernel<kScatterThreads, 2 * kScatterItems, false, kScatterBufs, kScatterWordCtasPerSm, true>,
-        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scatter_smem));
+        scatter_kernel<kScatterThreads, 2 * kScatterItems, false, kScatterBufs, scatter_word_ctas(false), true>,
+        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scatter_smem_bytes(false)));
     HJ_CU(cudaFuncSetAttribute(
-        scatter_kernel<kScatterThreads, 2 * kScatterItems, true, kScatterBufs, kScatterWordCtasPerSm, true>,
-        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scatter_smem));
+        scatter_kernel<kScatterThreads, 2 * kScatterItems, true, kScatterBufs, scatter_word_ctas(true), true>,
+        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scatter_smem_bytes(true)));
     HJ_CU(cudaFuncSetAttribute(join_small_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kJoinSmem));
     HJ_CU(cudaFuncSetAttribute(join_small_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)kJoinSmem));
@@ -3147,8 +3159,6 @@ int phj_enqueue(const RadixGeom &g, bool lp, bool skip0, const ulonglong2 *R, si
     const int np = g.nparts();
     const int F1 = g.F1, F2 = g.F2;
     constexpr int T = kTile;
-    // tile buffers (word tiles: 16 spare bytes each), gbase, running, tdstart, per-warp digit counts
-    const size_t scatter_smem = (size_t)kScatterBufs * (T * 16 + 16) + 256 * 8 * 2 + 256 * 4 + (kScatterThreads / 32) * 256 * 2;
     const size_t hist_smem = (size_t)np * 4 + (size_t)16 * F1 * 4;  // 16 warps
     ChunkGeom cg;
     cg.chunk = s.chunk;
@@ -3331,13 +3341,13 @@ int phj_enqueue(const RadixGeom &g, bool lp, bool skip0, const ulonglong2 *R, si
 #define HJ_SCATTER(ST)                                                                                         \
     if (words_in) {                                                                                            \
         sa.w8 = 1;                                                                                             \
-        scatter_kernel<kScatterThreads, 2 * kScatterItems, ST, kScatterBufs, kScatterWordCtasPerSm, true>        \
-            <<<num_sms * kScatterWordCtasPerSm, kScatterThreads, scatter_smem, st>>>(sa);                      \
+        scatter_kernel<kScatterThreads, 2 * kScatterItems, ST, kScatterBufs, scatter_word_ctas(ST), true>       \
+            <<<num_sms * scatter_word_ctas(ST), kScatterThreads, scatter_smem_bytes(ST), st>>>(sa);            \
         nlaunch++;                                                                                             \
         sa.w8 = 2;                                                                                             \
     }                                                                                                          \
     scatter_kernel<kScatterThreads, kScatterItems, ST, kScatterBufs, kScatterCtasPerSm>                          \
-        <<<scatter_grid, kScatterThreads, scatter_smem, st>>>(sa)
+        <<<scatter_grid, kScatterThreads, scatter_smem_bytes(ST), st>>>(sa)
             if (stable) {
                 HJ_SCATTER(true);
             } else {
