@@ -83,25 +83,15 @@ int join_geom(hj_algo_t algo, const hj_params_t &p, size_t nR, size_t nS, bool m
 // join reports does not depend on how it was computed, and beyond L2 partitioning both sides beats one
 // random table access per tuple (unique keys, device time: nphj_sc 2^22 x 2^23 191 us against 230 by the
 // table, 2^24 x 2^24 575 against 968, 2^26 x 2^28 4.6 ms against 10.7; nphj_lp 2^24 x 2^26 with four
-// duplicates a key 1.5 against 1.8 ms). Up to kNphjTableBuild the compact table does sit in L2 and wins from
-// about five probe tuples a build tuple (2^22 x 2^26: 892 against 745 us). Below kNphjRadixMinBuild (wall clock
-// per call, unique dense / unique 63-bit / dense with four tuples a key; radix then table):
-//   nphj_sc 2^19 build tuples on, probe side at most twice that: 540000 x 1080000 83 92 89 / 96 96 189,
-//   1500000 x 1500000 94 106 103 / 137 139 349; a smaller one, 300000 x 1200000 80 88 90 / 86 85 189, and
-//   10000 x 10000, 72 74 70 / 63 60 84, lose some form.
-//   nphj_lp (its table is cleared, filled and probed in order) up to 3e6 tuples in all and sixteen probe
-//   tuples a build tuple: 10000 x 10000 74 71 72 / 78 80 93, 200000 x 2700000 99 114 99 / 117 117 142;
-//   beyond either, 1000000 x 4000000 122 167 124 / 154 155 265 and 30000 x 2900000 100 117 100 / 107 107 133.
-// Materialising joins keep the table there (nphj_sc 540000 x 1080000 139 154 385 / 125 128 715, nphj_lp
-// 10000 x 10000 109 105 105 / 88 87 111). A load factor asks for the table itself; build partitions above
-// 6144 tuples on average, and scratch that cannot be had, take it too.
+// duplicates a key 1.5 against 1.8 ms). Below kNphjRadixMinBuild the 16-byte table sits in L2 and is as fast
+// (2^18 x 2^20: both 53 us; 20000 x 20000: 43 against 35), and up to kNphjTableBuild the compact one does,
+// which wins from about five probe tuples a build tuple (2^22 x 2^26: 892 against 745 us). A load factor
+// asks for the table itself; build partitions above 6144 tuples on average, and scratch that cannot be had,
+// take it too.
 constexpr size_t kNphjRadixMinBuild = 1u << 21, kNphjTableBuild = 5000000, kNphjRadixMaxBuild = (size_t)6144 << 14;
-constexpr size_t kNphjScRadixBuild = 1u << 19, kNphjLpRadixTuples = 3000000;
-bool nphj_by_radix(const hj_params_t &p, bool lp, size_t nR, size_t nS, bool mat) {
-    const size_t below = mat ? kNphjRadixMinBuild : (size_t)hj::kSmallMaxBuild + 1;
-    if (p.table_load > 0.0 || nR < below || nR > kNphjRadixMaxBuild || nS >= (1ull << 32)) return false;
-    if (nR >= kNphjRadixMinBuild) return nR > kNphjTableBuild || nS <= 5 * nR;
-    return lp ? nS <= 16 * nR && nR + nS <= kNphjLpRadixTuples : nR >= kNphjScRadixBuild && nS <= 2 * nR;
+bool nphj_by_radix(const hj_params_t &p, size_t nR, size_t nS) {
+    if (p.table_load > 0.0 || nR < kNphjRadixMinBuild || nR > kNphjRadixMaxBuild || nS >= (1ull << 32)) return false;
+    return nR > kNphjTableBuild || nS <= 5 * nR;
 }
 
 // How a join runs: by a radix pipeline (radix, geom, seg) or on the non-partitioned table.
@@ -115,7 +105,7 @@ int plan_join(hj_algo_t algo, hj_params_t *p, size_t nR, size_t nS, JoinPlan *jp
     if (is_phj(algo)) {
         const int rc = join_geom(algo, *p, nR, nS, mat, &jp->geom);
         if (rc) return rc;
-    } else if (nphj_by_radix(*p, hj::algo_lp(algo), nR, nS, mat)) {
+    } else if (nphj_by_radix(*p, nR, nS)) {
         p->flags &= ~(kPipelineFlags | HJ_F_ORDERED);  // radix joins' flags
         hj::radix_geom(14, 2, &jp->geom);
         if (!hj::radix_geom_single(14, hj::algo_lp(algo) || mat, nR, nS, &jp->geom)) hj::radix_geom_by_size(nR, nS, false, &jp->geom);

@@ -50,31 +50,3 @@ def test_two_pass_size(hj, cuda):
         r = hj.join(algo, R, S, on_device=True)
         assert (r.matched_cnt, r.checksum) == hj.pkfk_closed_form(nR, nS), algo
         assert (r.flags, r.physical_passes, r.large_partitions) == (0, 0, 0)
-
-
-@pytest.mark.parametrize("wide", [False, True])
-@pytest.mark.parametrize("algo,nR,nS", [
-    ("nphj_sc", (1 << 19) - 1, 1000), ("nphj_sc", 1 << 19, 1 << 20), ("nphj_sc", 1 << 19, (1 << 20) + 1),
-    ("nphj_lp", 8192, 8192), ("nphj_lp", 8193, 1), ("nphj_lp", 8193, 16 * 8193), ("nphj_lp", 8193, 16 * 8193 + 1),
-    ("nphj_lp", 1_500_000, 1_500_000), ("nphj_lp", 1_500_000, 1_500_001)])
-def test_smaller_sizes(hj, oracle, cuda, algo, nR, nS, wide):
-    """Both sides of each limit below 2^21 build tuples: repeated keys, one of them 300 times, keys 0 and 2^64-1, keys of either width."""
-    rng = np.random.default_rng(nR + nS)
-    R = np.empty((nR, 2), dtype=np.uint64)
-    R[:, 0] = rng.permutation(nR).astype(np.uint64) * (np.uint64(0x9E3779B97F4A7C15) if wide else np.uint64(1))
-    R[nR // 2: nR // 2 + 1000, 0] = R[:1000, 0]
-    R[:: max(1, nR // 300), 0] = R[3, 0]
-    R[5::100_003, 0] = 0
-    R[7::200_003, 0] = np.uint64(2**64 - 1) if wide else np.uint64(1 << 33)
-    S = np.empty((nS, 2), dtype=np.uint64)
-    S[:, 0] = R[rng.integers(0, nR, nS), 0]
-    S[::9, 0] += np.uint64(nR)
-    S[::10_007, 0] = 0
-    R[:, 1] = rng.integers(0, 1 << 32, nR, dtype=np.uint64)
-    S[:, 1] = rng.integers(0, 1 << 32, nS, dtype=np.uint64)
-    dR, dS = dev(cuda, R), dev(cuda, S)
-    want = oracle.join(algo, R, S)
-    for load in (0.0, 0.5):
-        r = hj.join(algo, dR, dS, on_device=True, load=load)
-        assert (r.matched_cnt, r.checksum) == want, load
-        assert (r.flags, r.physical_passes, r.large_partitions) == (0, 0, 0)
