@@ -14,7 +14,7 @@ def dev(cuda, a):
 
 @pytest.mark.parametrize("wide", [False, True])
 @pytest.mark.parametrize("nR,nS", [((1 << 21) - 1, 300_000), (1 << 21, 300_000), ((1 << 21) + 3, 10 * (1 << 21)),
-                                   (5_000_001, 1_000_003)])
+                                   (5_000_001, 1_000_003), (1 << 21, (1 << 22) + 1), (12_000_001, 25_000_000)])
 def test_radix_equals_table_and_oracle(hj, oracle, cuda, nR, nS, wide):
     rng = np.random.default_rng(nR)
     R = np.empty((nR, 2), dtype=np.uint64)
