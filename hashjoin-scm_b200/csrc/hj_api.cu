@@ -79,18 +79,18 @@ int join_geom(hj_algo_t algo, const hj_params_t &p, size_t nR, size_t nS, bool m
     return HJ_OK;
 }
 
-// Non-partitioned joins of these sizes run a radix pipeline (14 bits, or the one-pass geometry): what a
-// join reports does not depend on how it was computed, and beyond L2 partitioning both sides beats one
-// random table access per tuple (wall clock, radix then table; nphj_sc 2^22 x 2^23 dense 196 / 245 us, 63-bit
-// keys 290 / 460; nphj_lp 2^24 x 2^26 with four tuples a key 1.46 / 1.84 ms). The line lies where every form
-// of the keys gains, which a skewed probe side decides: it finds the table's hot lines in L2. With at most two
-// probe tuples a build tuple, Zipf 1.5, dense / 63-bit: nphj_sc 2^21 x 2^22 144 176 / 139 212, 2^23 x 2^24 396
-// 539 / 427 804, nphj_lp 463 767 / 557 821. With up to four, nphj_sc takes the table below 2^25 build tuples (12e6 x
-// 48e6 787 / 737, 2^24 x 2^26 1527 / 1279), nphj_lp below 12e6 (2^23 x 2^25 with 63-bit keys 1004 / 927; 12e6
-// x 48e6 Zipf 1.0 1657 / 1690, dense 868 / 920; 2^25 x 2^27 2900 3969 / 3040 3980). With more, both take it
-// (2^24 x 2^28: 3086 3864 / 2755 3383, nphj_lp 5309 / 3005). Below 2^21 the table sits in L2 (300000 x 300000 Zipf 1.5 96 /
-// 73). A load factor asks for the table itself; build partitions above 6144 tuples on average, and scratch
-// that cannot be had, take it too.
+// Non-partitioned joins of these sizes run a radix pipeline (14 bits, or the one-pass geometry): what a join
+// reports does not depend on how it was computed, and beyond L2 partitioning both sides beats one random
+// table access per tuple (wall clock, radix then table; nphj_sc 2^22 x 2^23 dense 196 / 245 us, 63-bit keys
+// 290 / 460; nphj_lp 2^24 x 2^26 with four tuples a key 1.46 / 1.84 ms). The line lies where every form of
+// the keys gains, which a skewed probe side decides: it finds the table's hot lines in L2. With at most two
+// probe tuples a build tuple, Zipf 1.5, dense / 63-bit: nphj_sc 2^21 x 2^22 144 176 / 139 212, 2^23 x 2^24
+// 396 539 / 427 804, nphj_lp 463 767 / 557 821. With up to four, nphj_sc takes the table below 2^25 build
+// tuples (12e6 x 48e6 787 / 737, 2^24 x 2^26 1527 / 1279), nphj_lp below 12e6 (2^23 x 2^25 with 63-bit keys
+// 1004 / 927; 12e6 x 48e6 Zipf 1.0 1657 / 1690, dense 868 / 920; 2^25 x 2^27 2900 3969 / 3040 3980). With
+// more, both take it (2^24 x 2^28: 3086 3864 / 2755 3383, nphj_lp 5309 / 3005). Below 2^21 the table sits in
+// L2 (300000 x 300000 Zipf 1.5 96 / 73). A load factor asks for the table itself; build partitions above 6144
+// tuples on average, and scratch that cannot be had, take it too.
 constexpr size_t kNphjRadixMinBuild = 1u << 21, kNphjScWide = 1u << 25, kNphjLpWide = 12000000;
 constexpr size_t kNphjRadixMaxBuild = (size_t)6144 << 14;
 bool nphj_by_radix(const hj_params_t &p, bool lp, size_t nR, size_t nS) {

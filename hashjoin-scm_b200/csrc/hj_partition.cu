@@ -29,16 +29,21 @@
 //                      order), staged in shared memory sorted by digit and written back as coalesced
 //                      16-byte streaming stores per digit run (the shared-memory analogue of the
 //                      reference's SWWCB + non-temporal flush). No inter-CTA waiting.
-//   join_compact       when keys (after the radix shift) and row ids fit 32 bits: persistent CTAs take
-//                      (partition, S chunk) items; 12-byte table entries with u16 bucket heads and chains
-//                      built by shared-memory atomics; S streamed with evict-first vector loads
+//   join_words         compact final partitions (8-byte words): persistent CTAs take (partition, S chunk)
+//                      items; an open-addressing table of the words in shared memory
+//   join_compact       tuples whose keys (after the radix shift) and row ids fit 32 bits, and ordered
+//                      first-match joins over words: words with u16 bucket heads and chains
 //   join_small         the general case: R_p arrives in shared memory by one TMA bulk copy, 16-byte
 //                      entries, u16 head/next chains
+//   join_first*        first-match joins of the one-pass pipeline, by input position
 //   join_large_*       partitions whose R side exceeds shared memory: chains in global memory
 // The join kernels have a materialising variant (MAT) for the ptr_* joins: one (r.row_id, s.row_id)
 // pair per match instead of the sums.
 //
-// Segment mode (joins that count every match, two passes, <= 14 bits, from 2^26 tuples): no histogram
+// Build relations that few partitions cover go through one pass instead (hj_single.cu), those of at most
+// kSmallMaxBuild tuples through one kernel (hj_small.cu); the join kernels here serve both pipelines.
+//
+// Segment mode (two passes, <= 14 bits, from 2^26 tuples): no histogram
 // pass. seg_pass1_kernel writes pass 1 into per-(CTA, relation, digit) chains of tile-sized segments
 // and counts each CTA's joint histogram itself; colscan/plan/units then treat the pass-1 CTAs as the
 // chunks, and pass 2 (scatter_kernel) walks the chains as its units.
@@ -3043,8 +3048,6 @@ int phj_prepare_device() {
     HJ_CU(cudaFuncSetAttribute(join_small_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kJoinSmem));
     HJ_CU(cudaFuncSetAttribute(join_small_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)kJoinSmem));
-    HJ_CU(cudaFuncSetAttribute(join_compact_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)kCompactSmem));
     HJ_CU(cudaFuncSetAttribute(join_compact_kernel<false, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)kCompactSmem));
     HJ_CU(cudaFuncSetAttribute(join_compact_kernel<false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(1024, 1) single_plan(SingleArgs a0, PlanArgs p
 }
 
 // ------------------------------------------------------------------------------------------------
-// 3. Scatter. Tiles of 8192 8-byte or 4096 16-byte elements: a thread takes 16 (8) elements, all their loads
+// 3. Scatter. Tiles of 10240 8-byte or 5120 16-byte elements: a thread takes 20 (10) elements, all their loads
 //    in flight together and issued under the previous tile's write-out; their ranks within their digit come
 //    from shared-memory atomics; a block scan over the digits gives each digit's start in the tile; the tile
 //    is staged in digit order and written out, consecutive threads to consecutive places of a digit's run. A

@@ -89,7 +89,8 @@ typedef struct {
     uint32_t flags;       /* HJ_F_* bits */
     double table_load;    /* NPHJ global table load factor; 0 selects 0.4 for build relations of up to
                              5 M tuples (about L2-sized tables, where shorter probe chains pay) and 0.5
-                             above */
+                             above, and lets the join run a radix pipeline at sizes where that is faster
+                             (same result); a value > 0 asks for the table */
     int radix_bits_pass1; /* two passes: bits of pass 1 (NUM_RADIX_BITS_PASS1 of phj_asymm_radix,
                              src/algo/phj_asymm_radix.h:10-19); 0 selects bits / 2. Clamped to the
                              split where each pass has 1..8 bits. */
@@ -101,7 +102,11 @@ typedef struct {
 #define HJ_F_NO_TIMING   0x1u /* skip the per-phase CUDA events (buildpart/probejoin stay 0) */
 #define HJ_F_PINNED_HOST 0x2u /* host inputs are already page-locked */
 #define HJ_F_PHASE_TIMES 0x4u /* also time each kernel group (fills hj_result_t.phase) */
-/* Radix joins (two passes, <= 14 bits) from 2^27 tuples run in segment mode: pass 1 writes chains of
+/* A radix join takes the shortest pipeline that its sizes allow, whatever num_radix_bits and num_passes ask
+ * for: at most 8192 build tuples one kernel, then one partition pass over the fewest bits that bring build
+ * partitions to shared-memory size (up to 11 bits), then two passes with the bits asked for or fewer. The
+ * flags HJ_F_SEGMENTS, HJ_F_EXACT, HJ_F_WIDE and HJ_F_WORDS name a two-pass pipeline and run it as asked.
+ * Radix joins in two passes of <= 14 bits from 2^26 tuples run in segment mode: pass 1 writes chains of
  * fixed-size segments and counts the histograms itself, so no histogram pass reads the relations first
  * (if the larger scratch does not fit, the exact-offset pipeline runs). First-match joins (lp) keep each
  * build partition in input order there too: every pass-1 CTA takes a contiguous range of the build
@@ -121,7 +126,8 @@ typedef struct {
 /* phj_radix_lp keeps the first match in input order among equal build keys. It first runs with the
  * partition passes of phj_radix_bc (no order kept), and the joins note whether any probe tuple matched
  * two build tuples; only then is the first match order-dependent, and the join runs again with ordered
- * passes (each build partition in input order, stable ranks). The context remembers the last build
+ * passes (each build partition in input order, stable ranks). (In one pass or one kernel the first match
+ * is found by input position, and nothing runs twice.) The context remembers the last build
  * relation (pointer and size) that needed this; its next joins there run ordered at once. Both runs
  * together are one join: one result, and its times include both. Such joins are not replayed from a
  * CUDA graph. HJ_F_ORDERED runs the ordered passes at once. */
@@ -129,8 +135,8 @@ typedef struct {
 
 /* hj_result_t.phase[] slots (seconds), filled with HJ_F_PHASE_TIMES. PHJ: histogram, plan, partition
  * pass 1, partition pass 2, shared-memory partition joins, global-memory (large) partition joins
- * (segment mode: no histogram pass, so that slot is 0 and pass 1 includes the counting).
- * NPHJ: build, -, -, -, probe, -. */
+ * (segment mode: no histogram pass, so that slot is 0 and pass 1 includes the counting; one kernel: all in
+ * the join slot). NPHJ: build, -, -, -, probe, -. */
 enum { HJ_PH_HIST = 0, HJ_PH_PLAN = 1, HJ_PH_PASS1 = 2, HJ_PH_PASS2 = 3, HJ_PH_JOIN = 4, HJ_PH_LARGE = 5,
        HJ_PH_COUNT = 6 };
 
@@ -146,7 +152,7 @@ typedef struct {
     double total;
     double h2d;       /* seconds spent copying host inputs to the device (0 for device inputs) */
     int status;
-    int physical_passes; /* partition passes the device ran (PHJ only) */
+    int physical_passes; /* partition passes the device ran, 0 to 2 (PHJ only) */
     uint64_t large_partitions; /* partitions joined through the global-memory path (PHJ only) */
     double phase[HJ_PH_COUNT]; /* per-kernel-group seconds (HJ_F_PHASE_TIMES) */
     uint32_t kernel_launches;  /* kernels this join launched */
@@ -310,7 +316,7 @@ typedef struct {
 typedef struct {
     double seconds;              /* device time of the whole batch (CUDA events) */
     uint32_t kernel_launches;    /* kernels the batch launches */
-    int waves;                   /* waves of non-partitioned joins */
+    int waves;                   /* waves of joins */
     int nphj_jobs, phj_jobs;
 } hj_batch_stats_t;
 
