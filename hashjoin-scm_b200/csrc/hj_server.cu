@@ -206,11 +206,11 @@ void wave_layout(const std::vector<Request> &reqs, int num_sms, WaveLayout *L) {
 }
 
 // Waves of fewer mid-size requests than this keep the table form: a lone one is done sooner by two launches over
-// an L2-sized table than by the one-pass pipeline's nine (20000 x 20000: 35 against 43 us); a burst is done
+// an L2-sized table than by the one-pass pipeline's nine (20000 x 20000: 35 against 43 us); a full burst is done
 // sooner in one pass (64 joins of 2^10..2^18 build tuples queued together: 729 us by tables, 363 in one pass).
-// Bursts as they arrive, 64 requests of 2^10..2^16 build tuples: 417 us with 4 here, 405 with 8, 378 with 16, 386
-// by tables; of 2^10..2^18: 568, 602, 593, 614.
-constexpr size_t kOnePassWaveMin = 16;
+// Waves that form while requests arrive stand between: 64 requests of 2^10..2^16 build tuples took 605 us with 4
+// or 16 here, 584 with 32, 587 by tables; of 2^10..2^18 555 with any.
+constexpr size_t kOnePassWaveMin = 32;
 
 std::vector<hj::WaveJoin> wave_joins(const std::vector<Request> &reqs) {
     std::vector<hj::WaveJoin> v;

@@ -61,3 +61,16 @@ def test_server_bursts(hj, oracle, cuda, budget):
                 c = got[ids[i]]
                 assert (c.status, c.matched_cnt, c.checksum) == (0, *oracle.join(a, R, S)), (a, R.shape, S.shape)
         assert srv.stats().in_use_bytes == 0
+
+
+def test_server_full_bursts(hj, oracle, cuda):
+    """Enough requests at once that waves hold more mid-size ones than the one-pass form asks for (32)."""
+    host = [j for j in joins(np.random.default_rng(63)) if len(j[1]) > 8192]
+    dev = [(cuda.from_numpy(R.view(np.int64)).cuda(), cuda.from_numpy(S.view(np.int64)).cuda()) for _, R, S in host]
+    want = [oracle.join(*j) for j in host]
+    with hj.Server(0, slots=4, hbm_budget_bytes=2e9) as srv:
+        ids = [srv.submit(host[i][0], *dev[i], on_device=True) for _ in range(12) for i in range(len(host))]
+        got = srv.wait_all(ids)
+        for n, rid in enumerate(ids):
+            c = got[rid]
+            assert (c.status, c.matched_cnt, c.checksum) == (0, *want[n % len(host)]), host[n % len(host)][0]
