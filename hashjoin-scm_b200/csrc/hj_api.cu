@@ -469,6 +469,8 @@ int hj_join_ctx(hj_ctx_t *c, hj_algo_t algo, const hj_params_t *pin, const hj_tu
         key.bits_pass1 = p.radix_bits_pass1;
         key.table_load = p.table_load;
         key.seg = seg;
+        key.radix = radix;
+        key.one_pass = one_pass;  // differs between calls with and without a watchdog
         key.arena = c->arena;
         key.arena_bytes = c->arena_bytes;
     }

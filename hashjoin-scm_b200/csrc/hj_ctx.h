@@ -21,13 +21,15 @@ struct hj_graph_key {
     uint32_t flags = 0;
     int bits = 0, passes = 0, bits_pass1 = 0;
     double table_load = 0;
-    bool seg = false;
+    bool seg = false, radix = false;
+    bool one_pass = false;  // the enqueued work leaves the result in acc_host, without its large partitions
     const char *arena = nullptr;
     size_t arena_bytes = 0;
     bool operator==(const hj_graph_key &o) const {
         return algo == o.algo && R == o.R && S == o.S && nR == o.nR && nS == o.nS && flags == o.flags &&
                bits == o.bits && passes == o.passes && bits_pass1 == o.bits_pass1 && table_load == o.table_load &&
-               seg == o.seg && arena == o.arena && arena_bytes == o.arena_bytes;
+               seg == o.seg && radix == o.radix && one_pass == o.one_pass && arena == o.arena &&
+               arena_bytes == o.arena_bytes;
     }
 };
 

@@ -54,3 +54,22 @@ def test_many_keys_eviction_and_arena_growth(hj, oracle, cuda):
             big_R, big_S = rel(rng, 400_000, 800_000), rel(rng, 900_000, 800_000)
             r = hj.join("nphj_sc", dev(cuda, big_R), dev(cuda, big_S), on_device=True, ctx=ctx)
             assert (r.matched_cnt, r.checksum) == oracle.join("nphj_sc", big_R, big_S)
+
+
+@pytest.mark.parametrize("algo", ["phj_radix_bc", "phj_radix_lp"])
+@pytest.mark.parametrize("first", [0, 60_000])
+def test_watchdog_and_plain_calls_keep_their_own_graphs(hj, oracle, cuda, algo, first):
+    """A hot build key makes a partition beyond shared memory, which a one-pass join without a watchdog runs in
+    a second step and one with a watchdog in the same enqueue: calls on the same buffers that differ only in
+    the watchdog must not replay each other's graph."""
+    rng = np.random.default_rng(33)
+    R, S = rel(rng, 60_000, 80_000), rel(rng, 150_000, 90_000)
+    R[10_000:30_000, 0] = R[3, 0]
+    S[:500, 0] = R[3, 0]
+    dR, dS = dev(cuda, R), dev(cuda, S)
+    want = oracle.join(algo, R, S)
+    with hj.Context(0) as ctx:
+        for ms in [first] * 3 + [60_000 - first] * 3 + [first] * 2:
+            r = hj.join(algo, dR, dS, on_device=True, ctx=ctx, watchdog_ms=ms)
+            assert (r.matched_cnt, r.checksum) == want, ms
+            assert r.large_partitions >= 1
