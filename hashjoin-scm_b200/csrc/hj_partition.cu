@@ -2449,7 +2449,13 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_small_kernel(JoinArgs a0
     join_finish(a, ci);
 }
 
-// Large partitions: chained tables in global memory, one flattened index space for all of them.
+// Large partitions: chained tables in global memory, one flattened index space for all of them. Buckets are the
+// top bits of a multiplicative hash of the key above the radix bits: the keys of a large partition often share
+// more than those (ids in the high half of the key), and low bits of them would then make one chain of all.
+__device__ __forceinline__ uint64_t large_bucket(uint64_t high, uint32_t nb_log) {
+    return nb_log ? (high * 0x9e3779b97f4a7c15ull) >> (64 - nb_log) : 0ull;
+}
+
 __device__ __forceinline__ int find_large(const LargePart *L, int nl, uint64_t g, bool by_r) {
     int lo = 0, hi = nl;  // largest l with flat[l] <= g
     while (hi - lo > 1) {
@@ -2559,7 +2565,7 @@ __device__ __forceinline__ void large_build(const JoinArgs &a, uint32_t blk, uin
             if ((int)lane != __ffs(peers) - 1) continue;
             const LargePart &L = a.large[l];
             const LargeAgg t = large_agg(a.large_table, L);
-            const uint64_t h = (r.x >> bshift) & ((1ull << L.nb_log) - 1);
+            const uint64_t h = large_bucket(r.x >> bshift, L.nb_log);
             const uint32_t node = large_agg_find_or_insert(t, a, ci, L.r_begin, L.r_len, h, r.x, (uint32_t)i,
                                                            &a.counters[kCtrErr]);
             if (!node) continue;
@@ -2579,7 +2585,7 @@ __device__ __forceinline__ void large_build(const JoinArgs &a, uint32_t blk, uin
         if (a.skip0 && k == 0 && (!ci || L.part0)) continue;
         uint32_t *head = a.large_table + L.table_off;
         uint32_t *nxt = head + (1ull << L.nb_log);
-        const uint64_t h = (k >> bshift) & ((1ull << L.nb_log) - 1);
+        const uint64_t h = large_bucket(k >> bshift, L.nb_log);
         nxt[i] = atomicExch(&head[h], (uint32_t)(i + 1));
     }
 }
@@ -2609,7 +2615,7 @@ __device__ __forceinline__ void large_probe(const JoinArgs &a, uint32_t blk, uin
                 const uint32_t *head = a.large_table + Lp->table_off;
                 const uint32_t *nxt = head + (1ull << Lp->nb_log);
                 unsigned long long best_y = 0;
-                e0 = head[(s.x >> bshift) & ((1ull << Lp->nb_log) - 1)];
+                e0 = head[large_bucket(s.x >> bshift, Lp->nb_log)];
                 uint64_t steps = 0;
                 for (uint32_t e = e0; e;) {
                     const tuple_v r = fin_r(a, ci, Lp->r_begin + e - 1);
@@ -2652,7 +2658,7 @@ __device__ __forceinline__ void large_probe(const JoinArgs &a, uint32_t blk, uin
             const LargePart &L = a.large[l];
             const tuple_v s = ld_fin(a.finS, a.finS8, L.s_begin + (g - L.s_flat), ci);
             const LargeAgg t = large_agg(a.large_table, L);
-            uint32_t e = t.head[(s.x >> bshift) & ((1ull << L.nb_log) - 1)];
+            uint32_t e = t.head[large_bucket(s.x >> bshift, L.nb_log)];
             uint64_t steps = 0;
             while (e && fin_r(a, ci, L.r_begin + e - 1).x != s.x) {
                 e = t.next[e - 1];
@@ -2685,7 +2691,7 @@ __device__ __forceinline__ void large_probe(const JoinArgs &a, uint32_t blk, uin
         const tuple_v s = ld_fin(a.finS, a.finS8, L.s_begin + (g - L.s_flat), ci);
         const uint32_t *head = a.large_table + L.table_off;
         const uint32_t *nxt = head + (1ull << L.nb_log);
-        uint32_t e = head[(s.x >> bshift) & ((1ull << L.nb_log) - 1)];
+        uint32_t e = head[large_bucket(s.x >> bshift, L.nb_log)];
         uint32_t best = 0, nm = 0;
         unsigned long long best_y = 0;  // the match's row id, or its input position (lp_pos)
         uint64_t steps = 0;

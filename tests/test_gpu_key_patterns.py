@@ -1,0 +1,62 @@
+"""Build keys with structure (strides, ids in the high half, packed fields) through every route that partitions by
+key bits, against the oracle. The tables of partitions beyond shared memory, the chains in shared memory and the
+partitions themselves must not degenerate on them: a join here takes well under a millisecond, and one that
+walks a chain of all its build tuples per tuple takes seconds, so the time is bounded far from both."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+ALGOS = ["phj_radix_bc", "phj_radix_lp", "nphj_sc", "nphj_lp"]
+PATTERNS = {
+    "x4": lambda k: k * np.uint64(4),
+    "x2^11": lambda k: k << np.uint64(11),
+    "x2^14": lambda k: k << np.uint64(14),
+    "x2^32": lambda k: k << np.uint64(32),
+    "packed": lambda k: ((k >> np.uint64(8)) << np.uint64(40)) | ((k & np.uint64(255)) << np.uint64(20)),
+}
+
+
+def relations(rng, nR, nS, pattern, dup=1, rid_bits=32):
+    """Every build key `dup` times; a quarter of the probe tuples without a match."""
+    f = PATTERNS[pattern]
+    n = max(1, nR // dup)
+    R, S = np.empty((nR, 2), dtype=np.uint64), np.empty((nS, 2), dtype=np.uint64)
+    R[:, 0] = f(rng.permutation(nR).astype(np.uint64) % np.uint64(n))  # key 0 included
+    S[:, 0] = f(rng.integers(0, n + n // 3 + 1, nS, dtype=np.uint64))
+    R[:, 1] = rng.integers(0, 1 << rid_bits, nR, dtype=np.uint64)
+    S[:, 1] = rng.integers(0, 1 << rid_bits, nS, dtype=np.uint64)
+    return R, S
+
+
+def dev(cuda, a):
+    return cuda.from_numpy(np.ascontiguousarray(a).view(np.int64)).cuda()
+
+
+@pytest.mark.parametrize("algo", ALGOS)
+@pytest.mark.parametrize("pattern", list(PATTERNS))
+@pytest.mark.parametrize("nR", [20_000, 300_000])
+def test_single_joins(hj, oracle, cuda, nR, pattern, algo):
+    """Partitions beyond shared memory whose keys share bits above the radix bits too."""
+    rng = np.random.default_rng(nR)
+    for dup in (1, 3):
+        R, S = relations(rng, nR, 2 * nR + 7, pattern, dup)
+        want = oracle.join(algo, R, S)
+        for flags in (0, hj.HJ_F_EXACT) if algo.startswith("phj") else (0,):
+            r = hj.join(algo, dev(cuda, R), dev(cuda, S), on_device=True, flags=flags)
+            assert (r.matched_cnt, r.checksum) == want, (dup, flags)
+            assert r.total < 0.1, (dup, flags)
+
+
+@pytest.mark.parametrize("algo", ["phj_radix_bc", "phj_radix_lp"])
+@pytest.mark.parametrize("pattern", ["x2^14", "x2^32"])
+def test_materialised_large_partitions(hj, oracle, cuda, pattern, algo):
+    rng = np.random.default_rng(5)
+    R, S = relations(rng, 60_000, 90_000, pattern)
+    R[:, 1] = np.arange(1, R.shape[0] + 1, dtype=np.uint64)
+    S[:, 1] = np.arange(1, S.shape[0] + 1, dtype=np.uint64)
+    want = oracle.join_pairs(algo, R, S)
+    out = cuda.zeros((want.shape[0], 2), dtype=cuda.int64, device="cuda")
+    r = hj.join_mat(algo, dev(cuda, R), dev(cuda, S), pairs=out, on_device=True)
+    got = out.cpu().numpy().view(np.uint64)
+    assert r.matched_cnt == want.shape[0]
+    assert np.array_equal(got[np.lexsort((got[:, 1], got[:, 0]))], want)
