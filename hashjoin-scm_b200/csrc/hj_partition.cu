@@ -1460,6 +1460,18 @@ __device__ __forceinline__ tuple_v fin_r(const JoinArgs &a, bool ci, uint64_t i)
     return a.finR[i];
 }
 
+// Chain head of a key among 2^nb_log (1..14) in shared memory: hashed, since a partition's keys may share the low
+// bits above the radix bits too (as for the large partitions' tables). Two 32-bit products: the radix bits, equal
+// in a partition, only shift the result, so they need not be shifted out (a 64-bit product of the shifted key
+// cost hr joins of 3e6 x 12e6 sparse keys 1.7%).
+__device__ __forceinline__ uint32_t head_of(unsigned long long key, uint32_t nb_log) {
+    return ((uint32_t)key * 0x9e3779b1u + (uint32_t)(key >> 32) * 0x85ebca6bu) >> (32 - nb_log);
+}
+// log2 of the number of heads for nr build tuples: the next power of two, times two if `twice`, at least 2.
+__device__ __forceinline__ uint32_t heads_log(uint32_t nr, bool twice, uint32_t max_log) {
+    return min(max_log, max(1u, (nr <= 1 ? 0u : 32u - __clz(nr - 1)) + (twice ? 1u : 0u)));
+}
+
 constexpr int kHeadMax = 16384;  // next_pow_2(kSmemCap)
 constexpr size_t kJoinSmem = (size_t)kSmemCap * 16 + kHeadMax * 2 + (size_t)kSmemCap * 2;
 
@@ -1516,10 +1528,9 @@ __global__ void __launch_bounds__(kCompactThreads, 2) join_compact_kernel(JoinAr
         if (it >= nA) break;
         const JoinItem item = a.items[it];
         const uint32_t nr = item.r_len;
-        const uint32_t nb = next_pow2_u32(nr);
-        const uint64_t hmask = nb - 1;
+        const uint32_t nb_log = heads_log(nr, false, 13);
         uint32_t *head32 = reinterpret_cast<uint32_t *>(head);
-        for (uint32_t q = tid; q < (nb + 1) / 2; q += kCompactThreads) head32[q] = 0;
+        for (uint32_t q = tid; q < (1u << nb_log) / 2; q += kCompactThreads) head32[q] = 0;
         __syncthreads();
         // Load and chain the build side; lp_join skips key 0, which reads as an empty slot there (in
         // compact final partitions such a key's words have a high part that no probe word has).
@@ -1538,7 +1549,7 @@ __global__ void __launch_bounds__(kCompactThreads, 2) join_compact_kernel(JoinAr
                 if (i >= nr) continue;
                 rw[i] = ((t[u].x >> B) << 32) | (t[u].y & 0xffffffffull);
                 if (skip0 && t[u].x == 0 && (!ci || item.part0)) continue;
-                nxt[i] = (uint16_t)atomic_exch_u16(&head[(t[u].x >> B) & hmask], i + 1);
+                nxt[i] = (uint16_t)atomic_exch_u16(&head[head_of(t[u].x >> B, nb_log)], i + 1);
             }
         }
         __syncthreads();
@@ -1560,7 +1571,7 @@ __global__ void __launch_bounds__(kCompactThreads, 2) join_compact_kernel(JoinAr
                     mm[u] = best[u] = 0;
                     if (base + u * kCompactThreads + tid >= ns) continue;
                     const uint64_t khi = sv[u].x >> B;
-                    uint32_t e = head[khi & hmask], steps = 0;
+                    uint32_t e = head[head_of(khi, nb_log)], steps = 0;
                     while (e) {
                         if ((rw[e - 1] >> 32) == khi) {
                             if (!lp) mm[u]++;
@@ -1585,7 +1596,7 @@ __global__ void __launch_bounds__(kCompactThreads, 2) join_compact_kernel(JoinAr
                         continue;
                     }
                     const uint64_t khi = sv[u].x >> B;
-                    uint32_t e = head[khi & hmask], steps = 0;
+                    uint32_t e = head[head_of(khi, nb_log)], steps = 0;
                     while (e && steps++ <= nr) {
                         const unsigned long long w = rw[e - 1];
                         if ((w >> 32) == khi) mat_put(a.mat, o++, w & 0xffffffffull, sv[u].y, err);
@@ -1608,7 +1619,7 @@ __global__ void __launch_bounds__(kCompactThreads, 2) join_compact_kernel(JoinAr
                 const uint32_t j = j0 + u * kCompactThreads;
                 if (j >= ns) continue;
                 const uint64_t khi = sv[u].x >> B;
-                uint32_t e = head[khi & hmask];
+                uint32_t e = head[head_of(khi, nb_log)];
                 uint32_t best = 0, steps = 0, nm = 0;
                 while (e) {
                     const unsigned long long w = rw[e - 1];
@@ -2125,7 +2136,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_words_kernel(JoinA
 // separate arrays (20 bytes per build tuple, 16-bit bucket heads and chains: 214 KB, one CTA per SM);
 // a build tuple's row id is gathered from the build relation once. One probe tuple per round, the next one under
 // way (3e6 x 12e6 sparse keys: 166 us; four unrolled: 175 us).
-constexpr uint32_t kFirstHeads = 8192;
+constexpr uint32_t kFirstHeadsLog = 13, kFirstHeads = 1u << kFirstHeadsLog;
 constexpr size_t kFirstSmem = (size_t)kFirstCap * (8 + 8 + 4 + 2) + kFirstHeads * 2;
 
 template <bool MAT, bool MULTI = false>
@@ -2151,7 +2162,6 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_kernel(JoinArgs a0
     unsigned int *err = &a.counters[kCtrErr];
     const uint32_t nitems = a.counters[kCtrNItems];
     if (a.ci && ci_applies(a.counters, a.bits)) return;  // join_first_words_kernel
-    const int B = a.bits;
     const bool skip0 = a.skip0 != 0;
     unsigned long long cnt = 0, sum = 0;
     bool multi = false;
@@ -2163,10 +2173,9 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_kernel(JoinArgs a0
         if (it >= nitems) break;
         const JoinItem item = a.items[it];
         const uint32_t nr = item.r_len;
-        const uint32_t nb = min(next_pow2_u32(nr), kFirstHeads);
-        const uint64_t hmask = nb - 1;
+        const uint32_t nb_log = heads_log(nr, false, kFirstHeadsLog);
         uint32_t *head32 = reinterpret_cast<uint32_t *>(head);
-        for (uint32_t q = tid; q < (nb + 1) / 2; q += kJoinThreads) head32[q] = 0;
+        for (uint32_t q = tid; q < (1u << nb_log) / 2; q += kJoinThreads) head32[q] = 0;
         __syncthreads();
         const tuple_v *R = a.finR + item.r_begin, *S = a.finS + item.s_begin;
         const uint32_t ns = item.s_len;
@@ -2195,7 +2204,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_kernel(JoinArgs a0
                 rid[i] = y[u];
                 pos[i] = (uint32_t)t[u].y;
                 if (skip0 && k == 0) continue;
-                nxt[i] = (uint16_t)atomic_exch_u16(&head[(k >> B) & hmask], i + 1);
+                nxt[i] = (uint16_t)atomic_exch_u16(&head[head_of(k, nb_log)], i + 1);
             }
         }
         __syncthreads();
@@ -2211,7 +2220,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_kernel(JoinArgs a0
             for (int u = 0; u < UP; u++) {
                 best[u] = 0;
                 if (base + u * kJoinThreads + tid >= ns) continue;
-                uint32_t e = head[(sv[u].x >> B) & hmask], steps = 0, nm = 0, bp = 0;
+                uint32_t e = head[head_of(sv[u].x, nb_log)], steps = 0, nm = 0, bp = 0;
                 while (e) {
                     if (kx[e - 1] == sv[u].x) {
                         const uint32_t p = pos[e - 1];
@@ -2284,7 +2293,6 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_small_kernel(JoinArgs a0
     // Compiled once per partition layout; only the launch matching the device's choice runs.
     if (CI != (a.ci && ci_applies(a.counters, a.bits))) return;
     constexpr bool ci = CI;
-    const int B = ci ? 0 : a.bits;  // shift from a stored x to the key's bits above the radix bits
     const bool lp = a.lp != 0;
     const bool skip0 = a.skip0 != 0;
     // Items [0, nA) went to the compact kernel if the build side's keys and row ids fit it.
@@ -2300,8 +2308,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_small_kernel(JoinArgs a0
         if (it >= nitems) break;
         const JoinItem item = a.items[it];
         const uint32_t nr = item.r_len;
-        const uint32_t nb = min((uint32_t)kHeadMax, 2 * next_pow2_u32(nr));
-        const uint64_t hmask = nb - 1;
+        const uint32_t nb_log = heads_log(nr, true, 14);  // up to kHeadMax
         if (!ci && tid == 0) {
             // Order earlier generic-proxy accesses to rt before the async-proxy writes.
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -2330,7 +2337,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_small_kernel(JoinArgs a0
             }
         }
         uint32_t *head32 = reinterpret_cast<uint32_t *>(head);
-        for (uint32_t q = tid; q < (nb + 1) / 2; q += kJoinThreads) head32[q] = 0;
+        for (uint32_t q = tid; q < (1u << nb_log) / 2; q += kJoinThreads) head32[q] = 0;
         if (ci) {
             // Compact final partitions: expand the build side's words into {key >> bits, row id}.
             for (uint32_t i = tid; i < nr; i += kJoinThreads)
@@ -2349,7 +2356,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_small_kernel(JoinArgs a0
         for (uint32_t i = tid; i < nr; i += kJoinThreads) {
             const uint64_t k = rt[i].x;
             if (skip0 && k == 0 && (!ci || item.part0)) continue;
-            const uint32_t h = (uint32_t)((k >> B) & hmask);
+            const uint32_t h = head_of(k, nb_log);
             nxt[i] = (uint16_t)atomic_exch_u16(&head[h], i + 1);
         }
         __syncthreads();
@@ -2368,7 +2375,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_small_kernel(JoinArgs a0
                     mm[u] = best[u] = 0;
                     if (base + u * kJoinThreads + tid >= ns) continue;
                     const uint64_t k = sv[u].x;
-                    uint32_t e = head[(k >> B) & hmask], steps = 0;
+                    uint32_t e = head[head_of(k, nb_log)], steps = 0;
                     while (e) {
                         if (rt[e - 1].x == k) {
                             if (!lp) mm[u]++;
@@ -2393,7 +2400,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_small_kernel(JoinArgs a0
                         continue;
                     }
                     const uint64_t k = sv[u].x;
-                    uint32_t e = head[(k >> B) & hmask], steps = 0;
+                    uint32_t e = head[head_of(k, nb_log)], steps = 0;
                     while (e && steps++ <= nr) {
                         if (rt[e - 1].x == k) mat_put(a.mat, o++, rt[e - 1].y, sv[u].y, err);
                         e = nxt[e - 1];
@@ -2413,7 +2420,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_small_kernel(JoinArgs a0
                 const uint32_t j = j0 + u * kJoinThreads;
                 if (j >= ns) continue;
                 const uint64_t k = s[u].x;
-                uint32_t e = head[(k >> B) & hmask];
+                uint32_t e = head[head_of(k, nb_log)];
                 uint32_t best = 0, nm = 0;
                 uint32_t steps = 0;
                 while (e) {

@@ -190,10 +190,6 @@ __host__ __device__ __forceinline__ uint32_t ceil_div_u64(uint64_t a, uint64_t b
     return (uint32_t)((a + b - 1) / b);
 }
 
-__device__ __forceinline__ uint32_t next_pow2_u32(uint32_t x) {
-    return x <= 1 ? 1u : 1u << (32 - __clz(x - 1));
-}
-
 struct PlanArgs {
     int bits, passes, b1, F1, F2;
     uint64_t nR, nS;

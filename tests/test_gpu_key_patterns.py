@@ -34,7 +34,7 @@ def dev(cuda, a):
 
 @pytest.mark.parametrize("algo", ALGOS)
 @pytest.mark.parametrize("pattern", list(PATTERNS))
-@pytest.mark.parametrize("nR", [20_000, 300_000])
+@pytest.mark.parametrize("nR", [9_000, 20_000, 300_000])
 def test_single_joins(hj, oracle, cuda, nR, pattern, algo):
     """Partitions beyond shared memory whose keys share bits above the radix bits too."""
     rng = np.random.default_rng(nR)
@@ -60,3 +60,27 @@ def test_materialised_large_partitions(hj, oracle, cuda, pattern, algo):
     got = out.cpu().numpy().view(np.uint64)
     assert r.matched_cnt == want.shape[0]
     assert np.array_equal(got[np.lexsort((got[:, 1], got[:, 0]))], want)
+
+
+@pytest.mark.parametrize("algo", ALGOS)
+def test_partitions_of_keys_that_share_low_bits(hj, cuda, algo):
+    """Partitions that fit shared memory, whose keys are equal in 24 bits above the radix bits: no slower than five
+    times the same join of mixed keys (one chain per partition: over twenty times)."""
+    nR, nS = 1 << 20, 1 << 21
+    g = cuda.Generator(device="cuda")
+    g.manual_seed(1)
+    R = cuda.empty((nR, 2), dtype=cuda.int64, device="cuda")
+    S = cuda.empty((nS, 2), dtype=cuda.int64, device="cuda")
+    r, s = cuda.randperm(nR, generator=g, device="cuda"), cuda.randint(0, nR, (nS,), generator=g, device="cuda")
+    R[:, 1], S[:, 1] = cuda.arange(nR, device="cuda") << 20, cuda.arange(nS, device="cuda")
+    rid = cuda.empty(nR, dtype=cuda.int64, device="cuda")
+    rid[r] = R[:, 1]
+    want = (nS, int((rid[s] + S[:, 1]).sum()))
+    times = []
+    for f in (lambda k: k * 0x1E3779B97F4A7C15 & 0x7FFFFFFFFFFFFFFF, lambda k: (k << 32) | (k & 255)):
+        R[:, 0], S[:, 0] = f(r + 1), f(s + 1)  # key 0 never matches in phj_radix_lp
+        with hj.Context(0) as ctx:
+            res = [hj.join(algo, R, S, on_device=True, ctx=ctx) for _ in range(5)]
+        assert all((q.matched_cnt, q.checksum) == want for q in res)
+        times.append(min(q.total for q in res))
+    assert times[1] < 5 * times[0], times
