@@ -2746,25 +2746,29 @@ __global__ void join_large_probe(JoinArgs a) {
     large_probe<MAT>(a, blockIdx.x, gridDim.x);
 }
 
-// End of a wave, one block per join: its partitions beyond shared memory (rare: the block takes all three
-// steps by itself) and its error word.
-__global__ void __launch_bounds__(kJoinThreads, 1) multi_finish(const MultiJob *jobs) {
+// The large-partition steps of a wave of joins, over a map of (job, block) as its other steps: a block of a job
+// without large partitions returns at once. (With one block per job a batch of four
+// 2^21 x 2^23 joins whose partitions were all large took 98.7 ms, one with a hot build key in each 10.3.) Step 2
+// hands over the error word.
+template <int STEP>
+__global__ void __launch_bounds__(kMultiLargeThreads) multi_large(MultiRef mr) {
+    const uint2 e = mr.map[blockIdx.x];
+    const MultiJob &job = mr.jobs[e.x];
+    const bool any = job.ja.counters[kCtrNLarge] != 0;
+    if (!any && (STEP != 2 || e.y != 0)) return;
     __shared__ JoinArgs a;
-    multi_copy(&a, &jobs[blockIdx.x].ja);
+    const uint32_t nblk = job.large_blocks;
+    multi_copy(&a, &job.ja);
     __syncthreads();
-    if (a.counters[kCtrNLarge]) {
-        large_clear(a, 0, 1);
-        __threadfence();
-        __syncthreads();
-        large_build(a, 0, 1);
-        __threadfence();
-        __syncthreads();
-        large_probe<false>(a, 0, 1);
+    if (any) {
+        if (STEP == 0) large_clear(a, e.y, nblk);
+        if (STEP == 1) large_build(a, e.y, nblk);
+        if (STEP == 2) large_probe<false>(a, e.y, nblk);
         __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        const uint32_t e = *reinterpret_cast<const volatile uint32_t *>(&a.counters[kCtrErr]);
-        if (e) atomicOr(&a.acc->error, e);
+    if (STEP == 2 && threadIdx.x == 0) {
+        const uint32_t err = *reinterpret_cast<const volatile uint32_t *>(&a.counters[kCtrErr]);
+        if (err) atomicOr(&a.acc->error, err);
     }
 }
 
@@ -3135,10 +3139,11 @@ static int large_launch(const JoinArgs &ja, bool mat, const PhjScratch &s, JoinA
     return HJ_OK;
 }
 
-int multi_join_launch(const MultiJob *jobs, int njobs, const uint2 *every_map, unsigned every_blocks,
-                      const uint2 *first_map, unsigned first_blocks, cudaStream_t st, uint32_t *launches) {
+int multi_join_launch(const MultiJob *jobs, const uint2 *every_map, unsigned every_blocks, const uint2 *first_map,
+                      unsigned first_blocks, const uint2 *large_map, unsigned large_blocks, cudaStream_t st,
+                      uint32_t *launches) {
     const JoinArgs none = {};
-    const MultiRef every = {jobs, every_map}, first = {jobs, first_map};
+    const MultiRef every = {jobs, every_map}, first = {jobs, first_map}, large = {jobs, large_map};
     if (every_blocks) {
         join_words_kernel<true><<<every_blocks, kCompactThreads, kOaSmem, st>>>(none, every);
         join_small_kernel<false, false, true><<<every_blocks, kJoinThreads, kJoinSmem, st>>>(none, every);
@@ -3149,8 +3154,10 @@ int multi_join_launch(const MultiJob *jobs, int njobs, const uint2 *every_map, u
         join_first_kernel<false, true><<<first_blocks, kJoinThreads, kFirstSmem, st>>>(none, first);
         *launches += 2;
     }
-    multi_finish<<<njobs, kJoinThreads, 0, st>>>(jobs);
-    *launches += 1;
+    multi_large<0><<<large_blocks, kMultiLargeThreads, 0, st>>>(large);
+    multi_large<1><<<large_blocks, kMultiLargeThreads, 0, st>>>(large);
+    multi_large<2><<<large_blocks, kMultiLargeThreads, 0, st>>>(large);
+    *launches += 3;
     HJ_CU(cudaGetLastError());
     return HJ_OK;
 }

@@ -397,7 +397,10 @@ struct MultiJob {
     JoinArgs ja;
     uint32_t grid;         // blocks of the count and the scatter
     uint32_t plan_blocks;  // blocks of the plan
+    uint32_t large_blocks; // blocks of the large-partition steps
+    uint32_t pad;
 };
+constexpr int kMultiLargeThreads = 256;
 static_assert(sizeof(MultiJob) % 8 == 0 && sizeof(SingleArgs) % 8 == 0 && sizeof(PlanArgs) % 8 == 0 &&
               sizeof(JoinArgs) % 8 == 0, "copied by 8-byte words");
 
@@ -427,10 +430,11 @@ void single_args(const RadixGeom &g, bool lp, bool skip0, bool ci_ok, const ulon
                  const ulonglong2 *S, size_t nS, const PhjScratch &s, JoinAccum *acc, bool clear_acc, bool agg_ok,
                  SingleArgs *a, PlanArgs *pa);
 // The steps of a wave of one-pass joins (hj_wave.cu): partition phase, partition joins (maps of the joins
-// that count every match and of the first-match ones), large partitions and error words.
+// that count every match and of the first-match ones), large partitions and error words (a map of all).
 int multi_partition_launch(const MultiJob *jobs, const uint2 *part_map, unsigned part_blocks, const uint2 *plan_map,
                            unsigned plan_blocks, int max_bits, cudaStream_t st, uint32_t *launches);
-int multi_join_launch(const MultiJob *jobs, int njobs, const uint2 *every_map, unsigned every_blocks,
-                      const uint2 *first_map, unsigned first_blocks, cudaStream_t st, uint32_t *launches);
+int multi_join_launch(const MultiJob *jobs, const uint2 *every_map, unsigned every_blocks, const uint2 *first_map,
+                      unsigned first_blocks, const uint2 *large_map, unsigned large_blocks, cudaStream_t st,
+                      uint32_t *launches);
 
 }  // namespace hj

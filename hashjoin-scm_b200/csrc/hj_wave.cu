@@ -63,6 +63,11 @@ uint32_t join_blocks(const WaveJoin &j, const Pieces &pc, int num_sms) {
     return blocks((uint64_t)j.nR + j.nS, pc.join, 2 * (uint32_t)num_sms);
 }
 
+// Blocks of a join's large-partition steps, which return at once for most joins: few, up to what fills the GPU.
+uint32_t large_blocks(const WaveJoin &j, int num_sms) {
+    return blocks((uint64_t)j.nR + j.nS, kWavePartTuples, 4 * (uint32_t)num_sms);
+}
+
 // Probe tuples per block of a small join: no fewer than twice its build side, which every block reads.
 uint64_t small_range(const WaveJoin &j, const Pieces &pc) { return std::max<uint64_t>(pc.small, 2 * j.nR); }
 
@@ -89,6 +94,7 @@ void wave_plan(const WaveJoin *joins, size_t n, int num_sms, WavePlan *wp) {
         wp->n_part += part_grid(j, pc, num_sms);
         wp->n_plan += (2u * (unsigned)g.F1 + 31) / 32;
         (j.lp ? wp->n_first : wp->n_every) += join_blocks(j, pc, num_sms);
+        wp->n_large += large_blocks(j, num_sms);
         wp->max_bits = std::max(wp->max_bits, g.bits);
         wp->scratch_bytes += a256(phj_scratch_bytes(g, j.nR, j.nS, (int)part_grid(j, pc, num_sms)));
     }
@@ -105,6 +111,7 @@ void wave_plan(const WaveJoin *joins, size_t n, int num_sms, WavePlan *wp) {
     wp->plan_off = put(8 * (size_t)wp->n_plan);
     wp->every_off = put(8 * (size_t)wp->n_every);
     wp->first_off = put(8 * (size_t)wp->n_first);
+    wp->large_off = put(8 * (size_t)wp->n_large);
     wp->image_bytes = o;
 }
 
@@ -114,9 +121,9 @@ int wave_image(const WaveJoin *joins, size_t n, int num_sms, const WavePlan &wp,
     MChunk *ch = reinterpret_cast<MChunk *>(image + wp.chunk_off);
     uint2 *part = reinterpret_cast<uint2 *>(image + wp.part_off), *plan = reinterpret_cast<uint2 *>(image + wp.plan_off);
     uint2 *every = reinterpret_cast<uint2 *>(image + wp.every_off);
-    uint2 *first = reinterpret_cast<uint2 *>(image + wp.first_off);
+    uint2 *first = reinterpret_cast<uint2 *>(image + wp.first_off), *large = reinterpret_cast<uint2 *>(image + wp.large_off);
     const Pieces pc = pieces_of(joins, n, num_sms);
-    unsigned nj = 0, ns = 0, nc = 0, npt = 0, npl = 0, ne = 0, nf = 0;
+    unsigned nj = 0, ns = 0, nc = 0, npt = 0, npl = 0, ne = 0, nf = 0, nl = 0;
     for (size_t q = 0; q < n; q++) {
         const WaveJoin &j = joins[q];
         if (!j.nR || !j.nS) continue;
@@ -146,6 +153,8 @@ int wave_image(const WaveJoin *joins, size_t n, int num_sms, const WavePlan &wp,
         m.plan_blocks = (2u * (unsigned)g.F1 + 31) / 32;
         for (uint32_t b = 0; b < G; b++) part[npt++] = make_uint2(nj, b);
         for (uint32_t b = 0; b < m.plan_blocks; b++) plan[npl++] = make_uint2(nj, b);
+        m.large_blocks = large_blocks(j, num_sms);
+        for (uint32_t b = 0; b < m.large_blocks; b++) large[nl++] = make_uint2(nj, b);
         const uint32_t jb = join_blocks(j, pc, num_sms);
         for (uint32_t b = 0; b < jb; b++) {
             if (j.lp)
@@ -156,7 +165,7 @@ int wave_image(const WaveJoin *joins, size_t n, int num_sms, const WavePlan &wp,
         mj[nj++] = m;
     }
     const bool same = nj == wp.n_jobs && ns == wp.n_small && nc == wp.n_chunks && npt == wp.n_part && npl == wp.n_plan &&
-                      ne == wp.n_every && nf == wp.n_first;
+                      ne == wp.n_every && nf == wp.n_first && nl == wp.n_large;
     return same ? HJ_OK : HJ_E_INVAL;
 }
 
@@ -173,7 +182,8 @@ int wave_enqueue(const WavePlan &wp, const char *image_dev, cudaStream_t st, uin
         auto map = [&](size_t off) { return reinterpret_cast<const uint2 *>(image_dev + off); };
         rc = multi_partition_launch(jobs, map(wp.part_off), wp.n_part, map(wp.plan_off), wp.n_plan, wp.max_bits, st, &l);
         if (!rc)
-            rc = multi_join_launch(jobs, (int)wp.n_jobs, map(wp.every_off), wp.n_every, map(wp.first_off), wp.n_first, st, &l);
+            rc = multi_join_launch(jobs, map(wp.every_off), wp.n_every, map(wp.first_off), wp.n_first, map(wp.large_off),
+                                   wp.n_large, st, &l);
     }
     if (launches) *launches += l;
     return rc;

@@ -107,8 +107,8 @@ bool wave_takes(size_t nR, size_t nS);
 // caller's (image: host copy of what goes to the device).
 struct WavePlan {
     size_t scratch_bytes = 0, image_bytes = 0;
-    size_t jobs_off, small_off, chunk_off, part_off, plan_off, every_off, first_off;
-    unsigned n_jobs = 0, n_small = 0, n_chunks = 0, n_part = 0, n_plan = 0, n_every = 0, n_first = 0;
+    size_t jobs_off, small_off, chunk_off, part_off, plan_off, every_off, first_off, large_off;
+    unsigned n_jobs = 0, n_small = 0, n_chunks = 0, n_part = 0, n_plan = 0, n_every = 0, n_first = 0, n_large = 0;
     int max_bits = 0;
     size_t max_build = 0;
 };

@@ -84,3 +84,42 @@ def test_partitions_of_keys_that_share_low_bits(hj, cuda, algo):
         assert all((q.matched_cnt, q.checksum) == want for q in res)
         times.append(min(q.total for q in res))
     assert times[1] < 5 * times[0], times
+
+
+@pytest.mark.parametrize("kind", ["x16", "hot"])
+def test_batch_jobs_with_large_partitions(hj, cuda, kind):
+    """Batch jobs of millions of tuples whose partitions exceed shared memory, or whose hot build key's does: the
+    answer, and a time of the order of a single join's (one block per job for these partitions: 20 times it)."""
+    nR, nS = 1 << 21, 1 << 23
+    g = cuda.Generator(device="cuda")
+    g.manual_seed(2)
+    jobs, want, alone = [], [], []
+    for i, algo in enumerate(("nphj_sc", "phj_radix_lp", "nphj_lp", "phj_radix_bc")):
+        k = cuda.randperm(nR, generator=g, device="cuda") + 1
+        s = cuda.randint(1, nR + nR // 4, (nS,), generator=g, device="cuda")
+        if kind == "hot":
+            k[nR // 4: 3 * nR // 4] = k[0]
+            s[: nS // 2] = k[0]
+        R, S = (cuda.empty((n, 2), dtype=cuda.int64, device="cuda") for n in (nR, nS))
+        R[:, 1], S[:, 1] = cuda.randperm(nR, generator=g, device="cuda"), cuda.arange(nS, device="cuda")
+        cnt = cuda.bincount(k, minlength=2 * nR)
+        if algo.endswith("lp"):
+            first = cuda.full((2 * nR,), nR, device="cuda").scatter_reduce_(0, k, cuda.arange(nR, device="cuda"), "amin")
+            m = (cnt[s] > 0).to(cuda.int64)
+            total = ((R[:, 1][first[s].clamp(max=nR - 1)] + S[:, 1]) * m).sum()
+        else:
+            m = cnt[s]
+            total = (cuda.zeros(2 * nR, dtype=cuda.int64, device="cuda").index_add_(0, k, R[:, 1])[s] + m * S[:, 1]).sum()
+        want.append((int(m.sum()), int(total) % 2**64))
+        R[:, 0], S[:, 0] = (k, s) if kind == "hot" else (k * 16, s * 16)
+        jobs.append((algo, R, S))
+        with hj.Context(0) as ctx:
+            alone.append(min(hj.join("phj_radix_" + ("lp" if algo.endswith("lp") else "bc"), R, S, on_device=True,
+                                     ctx=ctx).total for _ in range(3)))
+    with hj.Context(0) as ctx, hj.Batch(ctx, jobs) as b:
+        stats = []
+        for _ in range(3):
+            res, st = b.run()
+            assert [(r.status, r.matched_cnt, r.checksum) for r in res] == [(0, *w) for w in want]
+            stats.append(st.seconds)
+    assert min(stats) < 3 * sum(alone), (stats, alone)
