@@ -7,11 +7,13 @@
 // results and writes them to the caller's pinned host record, so there is nothing to clear before and
 // nothing to copy after the kernel (whole calls: phj_radix_bc 1000 x 4000 158 -> 29 us).
 //
-// The table: 32-bit bucket heads, tuples and 16-bit chain links by build position (22 bytes per tuple plus
-// the heads, at most 208 KB, one CTA of 1024 threads per SM). Keys may share low bits, so buckets are
-// taken from the top of a multiplicative hash. First-match joins take the lowest position on the chain,
-// which is the first in input order. Bound by the read of the probe relation (four 16-byte loads per
-// thread in flight) when that is large, else by the latency of its four dependent steps.
+// The table, where every match counts: tuples, 32-bit bucket heads and 16-bit chain links by build position (at
+// most 176 KB, one CTA of 1024 threads per SM). Keys may share low bits, so buckets are taken from the top of a
+// multiplicative hash. First-match joins need one place per key, not a walk over its duplicates (8192 build
+// tuples on eight keys, 2^22 probes: 3050 us with chains, 42 with one place): an open-addressing table of
+// build positions, at most half full, in which equal keys lower the position they share, and a bit per slot that
+// tells which two tuples share (at most 194 KB). Bound by the read of the probe relation (four 16-byte
+// loads per thread in flight) when that is large, else by the latency of its four dependent steps.
 #include <cstdio>
 
 #include "hj_common.cuh"
@@ -35,14 +37,20 @@ struct SmallArgs {
     JoinAccum *out;   // pinned host memory
 };
 
-struct SmallTable {  // in dynamic shared memory
+// In dynamic shared memory: 2^nb_log heads with chains, or (lp) twice as many slots and their duplicate bits.
+struct SmallTable {
     tuple_v *rt;        // [nR]
-    uint32_t *head;     // [2^nb_log]
+    uint32_t *head;     // [2^nb_log], or slots [2^(nb_log + 1)]
     uint16_t *nxt;      // [nR]
+    uint32_t *dup;      // [slots / 32]
+    uint32_t entries;   // heads or slots
     int shift;
-    __device__ __forceinline__ SmallTable(unsigned char *smem, uint32_t nR, int nb_log)
+    __device__ __forceinline__ SmallTable(unsigned char *smem, uint32_t nR, int nb_log, bool lp)
         : rt(reinterpret_cast<tuple_v *>(smem)), head(reinterpret_cast<uint32_t *>(rt + nR)),
-          nxt(reinterpret_cast<uint16_t *>(head + (1u << nb_log))), shift(64 - nb_log) {}
+          entries(1u << (nb_log + (lp ? 1 : 0))), shift(64 - nb_log - (lp ? 1 : 0)) {
+        nxt = reinterpret_cast<uint16_t *>(head + entries);
+        dup = head + entries;
+    }
     __device__ __forceinline__ uint32_t bucket(unsigned long long key) const {
         return (uint32_t)((key * 0x9e3779b97f4a7c15ull) >> shift);
     }
@@ -54,8 +62,8 @@ struct SmallSums {
 };
 
 // Build the whole table and probe it with S[j0], S[j0 + stride], ... below end. All threads of the block.
-__device__ __forceinline__ void small_block(const SmallTable &tb, const tuple_v *R, uint32_t nR, int nb_log, bool lp,
-                                            bool skip0, const tuple_v *S, uint64_t j0, uint64_t stride, uint64_t end,
+__device__ __forceinline__ void small_block(const SmallTable &tb, const tuple_v *R, uint32_t nR, bool lp, bool skip0,
+                                            const tuple_v *S, uint64_t j0, uint64_t stride, uint64_t end,
                                             SmallSums &o) {
     const int tid = threadIdx.x;
     constexpr int UR = kSmallMaxBuild / kSmallThreads, U = 4;
@@ -72,8 +80,9 @@ __device__ __forceinline__ void small_block(const SmallTable &tb, const tuple_v 
         const uint32_t i = tid + u * kSmallThreads;
         if (i < nR) t[u] = __ldg(R + i);
     }
-    for (uint32_t q = tid; q < (1u << nb_log); q += kSmallThreads) tb.head[q] = 0;
-    __syncthreads();
+    for (uint32_t q = tid; q < tb.entries; q += kSmallThreads) tb.head[q] = 0;
+    if (lp)
+        for (uint32_t q = tid; q < (tb.entries + 31) / 32; q += kSmallThreads) tb.dup[q] = 0;
 #pragma unroll
     for (int u = 0; u < UR; u++) {
         const uint32_t i = tid + u * kSmallThreads;
@@ -81,8 +90,32 @@ __device__ __forceinline__ void small_block(const SmallTable &tb, const tuple_v 
         tb.rt[i] = t[u];
         o.kor |= t[u].x;
         o.ror |= t[u].y;
-        if (skip0 && t[u].x == 0) continue;
-        tb.nxt[i] = (uint16_t)atomicExch(&tb.head[tb.bucket(t[u].x)], i + 1);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < UR; u++) {
+        const uint32_t i = tid + u * kSmallThreads;
+        if (i >= nR) break;
+        const unsigned long long k = tb.rt[i].x;
+        if (skip0 && k == 0) continue;
+        uint32_t h = tb.bucket(k);
+        if (!lp) {
+            tb.nxt[i] = (uint16_t)atomicExch(&tb.head[h], i + 1);
+            continue;
+        }
+        for (uint32_t steps = 0;; h = (h + 1) & (tb.entries - 1)) {
+            const uint32_t cur = atomicCAS(&tb.head[h], 0u, i + 1);
+            if (!cur) break;
+            if (tb.rt[cur - 1].x == k) {
+                atomicMin(&tb.head[h], i + 1);
+                atomicOr(&tb.dup[h >> 5], 1u << (h & 31));
+                break;
+            }
+            if (++steps >= tb.entries) {
+                o.over = true;
+                break;
+            }
+        }
     }
     __syncthreads();
     for (; j0 < end; j0 += U * stride) {
@@ -96,28 +129,24 @@ __device__ __forceinline__ void small_block(const SmallTable &tb, const tuple_v 
         for (int u = 0; u < U; u++) {
             if (j0 + u * stride >= end) continue;
             o.sor |= s[u].y;
-            uint32_t e = tb.head[tb.bucket(s[u].x)];
-            uint32_t best = 0, nm = 0, steps = 0;
+            uint32_t h = tb.bucket(s[u].x), steps = 0;
+            uint32_t e = tb.head[h];
             while (e) {
                 const tuple_v r = tb.rt[e - 1];
                 if (r.x == s[u].x) {
+                    o.cnt++;
+                    o.sum += r.y + s[u].y;
                     if (lp) {
-                        if (nm++ == 0 || e < best) best = e;
-                    } else {
-                        o.cnt++;
-                        o.sum += r.y + s[u].y;
+                        o.multi |= (tb.dup[h >> 5] >> (h & 31)) & 1u;
+                        break;
                     }
                 }
-                e = tb.nxt[e - 1];
-                if (++steps > nR) {
+                h = (h + 1) & (tb.entries - 1);
+                e = lp ? tb.head[h] : tb.nxt[e - 1];
+                if (++steps > tb.entries) {
                     o.over = true;
                     break;
                 }
-            }
-            if (nm) {  // first match
-                o.cnt++;
-                o.sum += tb.rt[best - 1].y + s[u].y;
-                o.multi |= nm > 1;
             }
         }
 #pragma unroll
@@ -132,9 +161,9 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_multi(const SmallJob *
     __shared__ unsigned long long red[64];
     const MChunk ch = chunks[blockIdx.x];
     const SmallJob J = jobs[ch.job];
-    const SmallTable tb(smem, J.nR, J.nb_log);
+    const SmallTable tb(smem, J.nR, J.nb_log, J.lp != 0);
     SmallSums o;
-    small_block(tb, J.R, J.nR, J.nb_log, J.lp != 0, J.skip0 != 0, J.S, ch.begin + threadIdx.x, kSmallThreads,
+    small_block(tb, J.R, J.nR, J.lp != 0, J.skip0 != 0, J.S, ch.begin + threadIdx.x, kSmallThreads,
                 ch.begin + ch.len, o);
     block_sum2_to(o.cnt, o.sum, red, &J.acc->matched, &J.acc->checksum);
     if (__syncthreads_or(o.over) && threadIdx.x == 0) set_error(&J.acc->error, kErrProbeLimit);
@@ -145,9 +174,9 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_join(SmallArgs a) {
     __shared__ unsigned long long s_red[5][kSmallThreads / 32];
     __shared__ bool s_last;
     const int tid = threadIdx.x;
-    const SmallTable tb(smem, a.nR, a.nb_log);
+    const SmallTable tb(smem, a.nR, a.nb_log, a.lp != 0);
     SmallSums o;
-    small_block(tb, a.R, a.nR, a.nb_log, a.lp != 0, a.skip0 != 0, a.S, (uint64_t)blockIdx.x * kSmallThreads + tid,
+    small_block(tb, a.R, a.nR, a.lp != 0, a.skip0 != 0, a.S, (uint64_t)blockIdx.x * kSmallThreads + tid,
                 (uint64_t)gridDim.x * kSmallThreads, a.nS, o);
     unsigned long long cnt = o.cnt, sum = o.sum, kor = o.kor, ror = o.ror, sor = o.sor;
     const bool multi = o.multi, over = o.over;
@@ -235,21 +264,25 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_join(SmallArgs a) {
         }                                                                             \
     } while (0)
 
-int small_prepare_device() {
-    HJ_CU(cudaFuncSetAttribute(small_multi, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               kSmallMaxBuild * (16 + 4 + 2)));
-    HJ_CU(cudaFuncSetAttribute(small_join, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               kSmallMaxBuild * (16 + 4 + 2)));
-    return HJ_OK;
-}
-
 static int small_buckets_log(size_t nR) {
     int b = 1;
     while ((1u << b) < nR) b++;
     return b;
 }
 
-static size_t small_smem(size_t nR) { return nR * 16 + ((size_t)4 << small_buckets_log(nR)) + nR * 2; }
+// Shared memory of a join: tuples, then heads and links, or (lp) slots and their duplicate bits. A wave takes the
+// larger form for its largest build side.
+static size_t small_smem(size_t nR, bool lp) {
+    const size_t heads = (size_t)1 << small_buckets_log(nR);
+    return nR * 16 + (lp ? 2 * heads * 4 + (2 * heads + 31) / 32 * 4 : heads * 4 + nR * 2);
+}
+
+int small_prepare_device() {
+    const int most = (int)small_smem(kSmallMaxBuild, true);
+    HJ_CU(cudaFuncSetAttribute(small_multi, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    HJ_CU(cudaFuncSetAttribute(small_join, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    return HJ_OK;
+}
 
 void small_job(bool lp, bool skip0, const ulonglong2 *R, size_t nR, const ulonglong2 *S, JoinAccum *acc, SmallJob *j) {
     j->R = R;
@@ -262,7 +295,7 @@ void small_job(bool lp, bool skip0, const ulonglong2 *R, size_t nR, const ulongl
 }
 
 int small_multi_launch(const SmallJob *jobs, const MChunk *chunks, unsigned nchunks, size_t max_build, cudaStream_t st) {
-    small_multi<<<nchunks, kSmallThreads, small_smem(max_build), st>>>(jobs, chunks);
+    small_multi<<<nchunks, kSmallThreads, small_smem(max_build, true), st>>>(jobs, chunks);
     HJ_CU(cudaGetLastError());
     return HJ_OK;
 }
@@ -285,7 +318,7 @@ int small_enqueue(bool lp, bool skip0, int flag_bits, const ulonglong2 *R, size_
     const uint64_t want = ((uint64_t)nS + kSmallThreads - 1) / kSmallThreads;
     const uint64_t sms = (uint64_t)(num_sms < kSmallMaxGrid ? num_sms : kSmallMaxGrid);
     const unsigned grid = (unsigned)(want < 1 ? 1 : want < sms ? want : sms);
-    small_join<<<grid, kSmallThreads, small_smem(nR), st>>>(a);
+    small_join<<<grid, kSmallThreads, small_smem(nR, lp), st>>>(a);
     HJ_CU(cudaGetLastError());
     return HJ_OK;
 }

@@ -52,3 +52,30 @@ def test_small_builds(hj, oracle, cuda, nR, nS, kind):
                 two = hj.join(algo, dR, dS, on_device=True, ctx=ctx, flags=hj.HJ_F_EXACT)
                 assert (two.matched_cnt, two.checksum) == want, algo
                 assert two.flags == got[0].flags, algo
+
+
+@pytest.mark.parametrize("nR", [2, 33, 1024, 8192])
+@pytest.mark.parametrize("keys", [1, 8])
+def test_first_match_of_few_keys(hj, oracle, cuda, nR, keys):
+    """First-match joins with one place per key: a build relation on one or eight keys, in a join and in a batch,
+    takes no longer for many probes than one of distinct keys (a walk over the duplicates: a hundred times)."""
+    rng = np.random.default_rng(nR)
+    nS = 1 << 19
+    R, S = relations(rng, nR, nS, "plain")
+    few = R.copy()
+    few[:, 0] = rng.integers(1, keys + 1, nR, dtype=np.uint64) * np.uint64(1 << 33)
+    fewS = S.copy()
+    fewS[:, 0] = rng.integers(0, keys + 2, nS, dtype=np.uint64) * np.uint64(1 << 33)
+    for algo in ("nphj_lp", "phj_radix_lp"):
+        times = []
+        for r, s in ((R, S), (few, fewS)):
+            dr, ds, want = dev(cuda, r), dev(cuda, s), oracle.join(algo, r, s)
+            with hj.Context(0) as ctx:
+                got = [hj.join(algo, dr, ds, on_device=True, ctx=ctx) for _ in range(4)]
+                assert all((g.matched_cnt, g.checksum) == want for g in got), algo
+                ordered = [g.flags & hj.HJ_RES_ORDERED_PASSES != 0 for g in got]
+                assert not any(ordered) if r is R or algo == "nphj_lp" else ordered[-1] == (keys < nR), algo
+                times.append(min(g.total for g in got))
+                with hj.Batch(ctx, [(algo, dr, ds)] * 2) as b:
+                    assert [(g.matched_cnt, g.checksum) for g in b.run()[0]] == [want] * 2
+        assert times[1] < 5 * times[0] + 20e-6, times
