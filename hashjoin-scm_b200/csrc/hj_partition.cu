@@ -2133,11 +2133,18 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_words_kernel(JoinA
 
 // First-match join of the one-pass pipeline over {key, position} elements (wide). The match with the lowest
 // position wins, so the partition may hold them in any order. Key, position and row id in
-// separate arrays (20 bytes per build tuple, 16-bit bucket heads and chains: 214 KB, one CTA per SM);
-// a build tuple's row id is gathered from the build relation once. One probe tuple per round, the next one under
-// way (3e6 x 12e6 sparse keys: 166 us; four unrolled: 175 us).
+// separate arrays (20 bytes per build tuple, 16-bit bucket heads and chains: 215 KB, one CTA per SM);
+// a build tuple's row id is gathered from the build relation once. A build tuple that finds its own key at the
+// head lowers that node's position instead of becoming a node; a partition where that happened has its chains
+// gone over once, a thread per head, which leaves one node per key with its first position and row id, and a bit
+// that there were more. (2^22 x 2^24 tuples of mixed 63-bit keys with 1 / 4 / 1000 a key: 510 / 615 / 18300 us with
+// every duplicate a node, 529 / 542 / 602 now; 2^21 x 2^22 with one key 1000 times and half of the probes on it:
+// 7680 and 203 us, the global table 2040. Looking through the whole chain before each insert: 560 us with 1 a
+// key.) One probe tuple per round, the next one under way (3e6 x 12e6 sparse keys: 166 us; four unrolled: 175).
 constexpr uint32_t kFirstHeadsLog = 13, kFirstHeads = 1u << kFirstHeadsLog;
-constexpr size_t kFirstSmem = (size_t)kFirstCap * (8 + 8 + 4 + 2) + kFirstHeads * 2;
+constexpr size_t kFirstSmem = (size_t)kFirstCap * (8 + 8 + 4 + 2) + kFirstHeads * 2 + kFirstCap / 8;
+constexpr uint32_t kFirstMerged = 0x8000;  // nxt of a tuple merged into a node: this bit, and the node's index + 1
+static_assert(kFirstCap < kFirstMerged && kFirstCap % 32 == 0, "an index and the bit fit a link");
 
 template <bool MAT, bool MULTI = false>
 __global__ void __launch_bounds__(kJoinThreads, 1) join_first_kernel(JoinArgs a0, MultiRef mr) {
@@ -2154,8 +2161,9 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_kernel(JoinArgs a0
     uint32_t *pos = reinterpret_cast<uint32_t *>(rid + kFirstCap);         // [kFirstCap]
     uint16_t *head = reinterpret_cast<uint16_t *>(pos + kFirstCap);        // [kFirstHeads]
     uint16_t *nxt = head + kFirstHeads;                                    // [kFirstCap]
+    uint32_t *dup = reinterpret_cast<uint32_t *>(nxt + kFirstCap);         // [kFirstCap / 32]
     __shared__ unsigned long long red[64];
-    __shared__ uint32_t s_item;
+    __shared__ uint32_t s_item, s_dups;
     __shared__ uint32_t scan_tmp[32];
     __shared__ unsigned long long s_base;
     const int tid = threadIdx.x;
@@ -2167,7 +2175,10 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_kernel(JoinArgs a0
     bool multi = false;
     constexpr int U = 4, UP = MAT ? 4 : 1;  // build and probe tuples per thread and round
     for (;;) {
-        if (tid == 0) s_item = atomicAdd(&a.counters[kCtrItemA], 1u);
+        if (tid == 0) {
+            s_item = atomicAdd(&a.counters[kCtrItemA], 1u);
+            s_dups = 0;
+        }
         __syncthreads();
         const uint32_t it = s_item;
         if (it >= nitems) break;
@@ -2176,6 +2187,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_kernel(JoinArgs a0
         const uint32_t nb_log = heads_log(nr, false, kFirstHeadsLog);
         uint32_t *head32 = reinterpret_cast<uint32_t *>(head);
         for (uint32_t q = tid; q < (1u << nb_log) / 2; q += kJoinThreads) head32[q] = 0;
+        for (uint32_t q = tid; q < (nr + 31) / 32; q += kJoinThreads) dup[q] = 0;
         __syncthreads();
         const tuple_v *R = a.finR + item.r_begin, *S = a.finS + item.s_begin;
         const uint32_t ns = item.s_len;
@@ -2199,15 +2211,78 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_kernel(JoinArgs a0
             for (int u = 0; u < U; u++) {
                 const uint32_t i = i0 + u * kJoinThreads;
                 if (i >= nr) continue;
-                const unsigned long long k = t[u].x;
-                kx[i] = k;
+                kx[i] = t[u].x;
                 rid[i] = y[u];
                 pos[i] = (uint32_t)t[u].y;
-                if (skip0 && k == 0) continue;
-                nxt[i] = (uint16_t)atomic_exch_u16(&head[head_of(k, nb_log)], i + 1);
             }
         }
         __syncthreads();
+        bool twice = false;
+        for (uint32_t i = tid; i < nr; i += kJoinThreads) {
+            const unsigned long long k = kx[i];
+            if (skip0 && k == 0) continue;
+            const uint32_t h = head_of(k, nb_log), shift = (h & 1) * 16;
+            uint32_t *word = head32 + (h >> 1);
+            uint32_t old = *reinterpret_cast<volatile uint32_t *>(word);
+            for (;;) {  // lock-free: a failed CAS means another thread's succeeded
+                const uint32_t e = (old >> shift) & 0xffffu;
+                if (e && kx[e - 1] == k) {
+                    atomicMin(&pos[e - 1], pos[i]);
+                    nxt[i] = (uint16_t)(kFirstMerged | e);
+                    twice = true;
+                    break;
+                }
+                nxt[i] = (uint16_t)e;
+                const uint32_t seen = atomicCAS(word, old, (old & ~(0xffffu << shift)) | ((i + 1) << shift));
+                if (seen == old) break;
+                old = seen;
+            }
+        }
+        if (twice) s_dups = 1u;
+        __syncthreads();
+        const bool dups = s_dups != 0;
+        if (dups) {
+            // Row ids of the tuples whose position won, and duplicate bits; then what is left of one key in a
+            // chain (nodes that were not next to each other).
+            for (uint32_t i = tid; i < nr; i += kJoinThreads) {
+                const uint32_t e = nxt[i];
+                if (!(e & kFirstMerged) || (skip0 && kx[i] == 0)) continue;
+                const uint32_t r = (e & (kFirstMerged - 1)) - 1;
+                if (pos[r] == pos[i]) rid[r] = rid[i];
+                atomicOr(&dup[r >> 5], 1u << (r & 31));
+            }
+            __syncthreads();
+            for (uint32_t q = tid; q < 1u << nb_log; q += kJoinThreads) {
+                for (uint32_t r = head[q]; r; r = nxt[r - 1]) {
+                    // Take the nodes behind r with its key out of the chain.
+                    const unsigned long long k = kx[r - 1];
+                    uint32_t prev = r, first = r, fp = pos[r - 1];
+                    bool gap = false, any = false;  // any: bits of the nodes taken out pass to r
+                    for (uint32_t e = nxt[r - 1], next; e; e = next) {
+                        const uint32_t p = pos[e - 1];
+                        next = nxt[e - 1];
+                        if (kx[e - 1] == k) {
+                            gap = any = true;
+                            if (p < fp) {
+                                fp = p;
+                                first = e;
+                            }
+                        } else {
+                            if (gap) nxt[prev - 1] = (uint16_t)e;
+                            gap = false;
+                            prev = e;
+                        }
+                    }
+                    if (gap) nxt[prev - 1] = 0;
+                    if (any) {
+                        pos[r - 1] = fp;
+                        rid[r - 1] = rid[first - 1];
+                        atomicOr(&dup[(r - 1) >> 5], 1u << ((r - 1) & 31));
+                    }
+                }
+            }
+            __syncthreads();
+        }
         for (uint32_t base = 0; base < ns; base += UP * kJoinThreads) {
             tuple_v nx[UP];
             uint32_t best[UP], m = 0;
@@ -2238,7 +2313,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_kernel(JoinArgs a0
                 if (!best[u]) continue;
                 m++;
                 if (!MAT) sum += rid[best[u] - 1] + sv[u].y;
-                multi |= nm > 1;
+                multi |= nm > 1 || (dups && (dup[(best[u] - 1) >> 5] >> ((best[u] - 1) & 31)) & 1u);
             }
             cnt += m;
             if constexpr (MAT) {

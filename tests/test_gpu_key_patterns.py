@@ -123,3 +123,28 @@ def test_batch_jobs_with_large_partitions(hj, cuda, kind):
             assert [(r.status, r.matched_cnt, r.checksum) for r in res] == [(0, *w) for w in want]
             stats.append(st.seconds)
     assert min(stats) < 3 * sum(alone), (stats, alone)
+
+
+@pytest.mark.parametrize("algo,nR", [("phj_radix_lp", 1 << 20), ("nphj_lp", (1 << 21) + 5)])
+@pytest.mark.parametrize("copies", [2, 1000])
+def test_first_match_of_repeated_wide_keys(hj, oracle, cuda, algo, nR, copies):
+    """First matches over 16-byte tuples: one node per key, so that repeated keys cost a probe no walk; the joins'
+    sums, the pairs' retrieved row ids, and a time of the order of distinct keys' (a walk over 1000: ten times)."""
+    rng = np.random.default_rng(copies)
+    nS, times = 1 << 21, []
+    for c in (1, copies):
+        n = nR // c
+        R, S = np.empty((nR, 2), dtype=np.uint64), np.empty((nS, 2), dtype=np.uint64)
+        R[:, 0] = (rng.permutation(nR).astype(np.uint64) % np.uint64(n) + np.uint64(1)) * np.uint64(0x1E3779B97F4A7C15)
+        S[:, 0] = rng.integers(1, n + n // 4 + 2, nS, dtype=np.uint64) * np.uint64(0x1E3779B97F4A7C15)
+        R[:, 1], S[:, 1] = np.arange(1, nR + 1, dtype=np.uint64), np.arange(1, nS + 1, dtype=np.uint64)
+        want, dR, dS = oracle.join(algo, R, S), dev(cuda, R), dev(cuda, S)
+        with hj.Context(0) as ctx:
+            got = [hj.join(algo, dR, dS, on_device=True, ctx=ctx) for _ in range(4)]
+            assert all((r.matched_cnt, r.checksum) == want for r in got)
+            times.append(min(r.total for r in got))
+            r = hj.join_mat(algo, dR, dS, on_device=True, ctx=ctx)
+            assert (r.matched_cnt, r.checksum) == want
+            if algo.startswith("phj"):
+                assert bool(got[0].flags & hj.HJ_RES_ORDERED_PASSES) == (c > 1)
+    assert times[1] < 3 * times[0], times
