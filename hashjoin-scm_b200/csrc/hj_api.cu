@@ -69,28 +69,41 @@ bool want_seg(hj_algo_t algo, const hj_params_t &p, const hj::RadixGeom &g, size
 // Flags that name a pipeline or its element layout: the two-pass pipelines run as asked.
 constexpr uint32_t kPipelineFlags = HJ_F_SEGMENTS | HJ_F_EXACT | HJ_F_WIDE | HJ_F_WORDS | HJ_F_TEST_STALL;
 
+// One-pass radix joins of at most kRawDigitsMaxBuild build tuples partition by the key's own low bits, as asked, larger
+// ones by mix_key (which a materialising join, whose large partitions walk every duplicate, always does). Keys
+// that share low bits overfill a few of the raw partitions; a join that finds most of its build tuples in partitions
+// beyond shared memory is run again by mix_key (2^21 x 2^23 multiples of 4: 809 us with the global tables of such
+// partitions, 332 run again, 480 in two passes of 14 bits; dense keys 155). At kRerunMinBuild build tuples and
+// below the tables are as fast (multiples of 2^14, 2^16 x 2^18: 103 us and 106 run again, 2^18 x 2^20: 161 and 127).
+// Mixing costs dense keys 1% in one pass, 2.5% in two.
+constexpr size_t kRawDigitsMaxBuild = 1u << 21, kRerunMinBuild = 1u << 16;
+
 // The geometry of a radix join: the one-pass pipeline where the build relation needs few partitions,
 // unless the flags name another, else as asked.
 int join_geom(hj_algo_t algo, const hj_params_t &p, size_t nR, size_t nS, bool mat, hj::RadixGeom *g) {
     const int rc = hj::radix_geom(p.num_radix_bits, p.num_passes, g, p.radix_bits_pass1);
     if (rc) return rc;
-    if (!(p.flags & kPipelineFlags) && !hj::radix_geom_single(p.num_radix_bits, hj::algo_lp(algo) || mat, nR, nS, g))
+    if (p.flags & kPipelineFlags) return HJ_OK;
+    if (hj::radix_geom_single(p.num_radix_bits, hj::algo_lp(algo) || mat, nR, nS, g))
+        g->mix = mat || nR > kRawDigitsMaxBuild;
+    else
         hj::radix_geom_by_size(nR, nS, p.radix_bits_pass1 > 0, g);
     return HJ_OK;
 }
 
-// Non-partitioned joins of these sizes run a radix pipeline (14 bits, or the one-pass geometry): what a join
-// reports does not depend on how it was computed, and beyond L2 partitioning both sides beats one random
-// table access per tuple (wall clock, radix then table; nphj_sc 2^22 x 2^23 dense 196 / 245 us, 63-bit keys
-// 290 / 460; nphj_lp 2^24 x 2^26 with four tuples a key 1.46 / 1.84 ms). The line lies where every form of
-// the keys gains, which a skewed probe side decides: it finds the table's hot lines in L2. With at most two
+// Non-partitioned joins of these sizes run a radix pipeline (14 bits, or the one-pass geometry; partitions of
+// mix_key, so that the keys' low bits matter as little as to the table's hash): what a join reports does not
+// depend on how it was computed, and beyond L2 partitioning both sides beats one random table access per tuple
+// (wall clock, radix then table; nphj_sc 2^22 x 2^23 dense 193 / 247 us, multiples of 4 209 / 247, 63-bit keys 290 /
+// 460; nphj_lp 2^24 x 2^26 with four tuples a key 1.45 / 1.82 ms). The line lies where every measured form of the
+// keys gains, which a skewed probe side decides: it finds the table's hot lines in L2. With at most two
 // probe tuples a build tuple, Zipf 1.5, dense / 63-bit: nphj_sc 2^21 x 2^22 144 176 / 139 212, 2^23 x 2^24
 // 396 539 / 427 804, nphj_lp 463 767 / 557 821. With up to four, nphj_sc takes the table below 2^25 build
 // tuples (12e6 x 48e6 787 / 737, 2^24 x 2^26 1527 / 1279), nphj_lp below 12e6 (2^23 x 2^25 with 63-bit keys
-// 1004 / 927; 12e6 x 48e6 Zipf 1.0 1657 / 1690, dense 868 / 920; 2^25 x 2^27 2900 3969 / 3040 3980). With
+// 1004 / 927; 12e6 x 48e6 Zipf 1.0 1657 / 1690, dense 868 / 920). With
 // more, both take it (2^24 x 2^28: 3086 3864 / 2755 3383, nphj_lp 5309 / 3005). Below 2^21 the table sits in
-// L2 (300000 x 300000 Zipf 1.5 96 / 73). A load factor asks for the table itself; build partitions above 6144
-// tuples on average, and scratch that cannot be had, take it too.
+// L2 (300000 x 300000 Zipf 1.5 96 / 73). First matches take the table beyond one pass (plan_join). A load factor asks
+// for the table itself; build partitions above 6144 tuples on average, and scratch that cannot be had, take it too.
 constexpr size_t kNphjRadixMinBuild = 1u << 21, kNphjScWide = 1u << 25, kNphjLpWide = 12000000;
 constexpr size_t kNphjRadixMaxBuild = (size_t)6144 << 14;
 bool nphj_by_radix(const hj_params_t &p, bool lp, size_t nR, size_t nS) {
@@ -110,9 +123,14 @@ int plan_join(hj_algo_t algo, hj_params_t *p, size_t nR, size_t nS, JoinPlan *jp
         const int rc = join_geom(algo, *p, nR, nS, mat, &jp->geom);
         if (rc) return rc;
     } else if (nphj_by_radix(*p, hj::algo_lp(algo), nR, nS)) {
-        p->flags &= ~(kPipelineFlags | HJ_F_ORDERED);  // radix joins' flags
         hj::radix_geom(14, 2, &jp->geom);
-        if (!hj::radix_geom_single(14, hj::algo_lp(algo) || mat, nR, nS, &jp->geom)) hj::radix_geom_by_size(nR, nS, false, &jp->geom);
+        if (!hj::radix_geom_single(14, hj::algo_lp(algo) || mat, nR, nS, &jp->geom)) {
+            // Two passes join first matches in partition order, where a probe walks all duplicates of its key.
+            if (hj::algo_lp(algo)) return HJ_OK;
+            hj::radix_geom_by_size(nR, nS, false, &jp->geom);
+        }
+        p->flags &= ~(kPipelineFlags | HJ_F_ORDERED);  // radix joins' flags
+        jp->geom.mix = true;  // as the table's hash, whatever bits the keys share
     } else {
         return HJ_OK;
     }
@@ -389,9 +407,7 @@ int hj_join_ctx(hj_ctx_t *c, hj_algo_t algo, const hj_params_t *pin, const hj_tu
     // are not captured into a graph; a build relation that needed it runs ordered at once next time.
     // The one-pass pipeline needs neither: its build elements carry their input position. It reports
     // HJ_RES_ORDERED_PASSES for the joins that the two-pass pipelines would have run ordered.
-    // A non-partitioned join in two passes runs ordered at once: it must not pay for two runs where the table
-    // would have been one.
-    const bool lp_first = radix && hj::algo_lp(algo) && (is_phj(algo) || geom.single) && !(p.flags & (HJ_F_ORDERED | HJ_F_TEST_STALL)) &&
+    const bool lp_first = radix && hj::algo_lp(algo) && !(p.flags & (HJ_F_ORDERED | HJ_F_TEST_STALL)) &&
                           p.watchdog_ms <= 0 && !(c->lp_ordered_R == (const void *)R && c->lp_ordered_nR == nR);
     const bool lp_try = lp_first && !geom.single && !small;
     const bool lp_ordered = radix && hj::algo_lp(algo) && !lp_first;
@@ -546,12 +562,31 @@ int hj_join_ctx(hj_ctx_t *c, hj_algo_t algo, const hj_params_t *pin, const hj_tu
         CU_OR(cudaStreamSynchronize(st), out->status = HJ_E_DEVICE);
     }
     JoinAccum res = *c->acc_host;
+    unsigned long long raw_large = 0;  // large partitions of the digits asked for, when the join ran again by mix_key
+    hj::RadixGeom run_geom = geom;
+    if (one_pass && !geom.mix && nR > kRerunMinBuild && res.large_build > nR / 2) {
+        raw_large = res.large_parts;
+        run_geom.mix = true;
+        hj::PhjScratch s;
+        hj::phj_carve(run_geom, nR, nS, c->num_sms, cur, &s, false);
+        uint32_t again = 0;
+        rc = hj::phj_enqueue(run_geom, hj::algo_lp(algo), hj::algo_skip0(algo), dR, nR, dS, nS, s, acc, st,
+                             timing ? c->ev_mid : nullptr, c->num_sms, ph, &again, nullptr, 0, true, c->acc_host);
+        launches += again;
+        if (rc) {
+            cudaStreamSynchronize(st);
+            return out->status = rc;
+        }
+        if (timing) CU_OR(cudaEventRecord(c->ev_end, st), out->status = HJ_E_DEVICE);
+        CU_OR(cudaStreamSynchronize(st), out->status = HJ_E_DEVICE);
+        res = *c->acc_host;
+    }
     if (one_pass && res.large_parts) {
         // Partitions beyond shared memory (rare: a hot build key, or keys that share their low bits) are
         // joined by a second batch of kernels, launched only now that there are some.
         hj::PhjScratch s;
-        hj::phj_carve(geom, nR, nS, c->num_sms, cur, &s, false);
-        rc = hj::phj_large_enqueue(geom, hj::algo_lp(algo), hj::algo_skip0(algo), dR, nR, nS, s, acc, st, c->num_sms,
+        hj::phj_carve(run_geom, nR, nS, c->num_sms, cur, &s, false);
+        rc = hj::phj_large_enqueue(run_geom, hj::algo_lp(algo), hj::algo_skip0(algo), dR, nR, nS, s, acc, st, c->num_sms,
                                    &launches);
         if (rc) return out->status = rc;
         if (phases) CU_OR(cudaEventRecord(c->ev_ph[HJ_PH_COUNT], st), out->status = HJ_E_DEVICE);
@@ -566,7 +601,7 @@ int hj_join_ctx(hj_ctx_t *c, hj_algo_t algo, const hj_params_t *pin, const hj_tu
     }
     out->matched_cnt = res.matched;
     out->checksum = res.checksum;
-    out->large_partitions = is_phj(algo) ? res.large_parts : 0;
+    out->large_partitions = !is_phj(algo) ? 0 : raw_large ? raw_large : res.large_parts;
     out->flags = is_phj(algo) ? (uint32_t)res.flags : 0u;
     if (lp_first && !lp_try) lp_rerun = res.dup_flag != 0;
     if (is_phj(algo) && (lp_ordered || lp_rerun)) out->flags |= HJ_RES_ORDERED_PASSES;

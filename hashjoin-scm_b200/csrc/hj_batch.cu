@@ -404,6 +404,7 @@ int lane_geom(const hj_batch *b, int j, hj::RadixGeom *g) {
     const bool phj = b->impl[j] == kImplPhj;
     const int rc = hj::radix_geom(phj ? b->bits[j] : 14, phj ? b->passes[j] : 2, g);
     hj::radix_geom_by_size(b->jobs[j].nR, b->jobs[j].nS, false, g);
+    g->mix = g->mix || !phj;  // the hashed table it would have used does not depend on the keys' low bits
     return rc;
 }
 

@@ -33,7 +33,7 @@ struct JoinAccum {
     unsigned long long pairs;   // materialising joins: output slots reserved so far
     unsigned long long flags;   // HJ_RES_* bits of hj_result_t.flags
     unsigned long long wide_rids;  // materialising joins: OR of the row ids' high halves (mat_columns)
-    unsigned long long pad;
+    unsigned long long large_build;  // one-pass joins: build tuples in large partitions
 };
 
 __device__ __forceinline__ void set_error(unsigned int *err, uint32_t bit) { atomicOr(err, bit); }

@@ -21,6 +21,7 @@ struct RadixGeom {
     int F1, F2;     // fanouts (F2 = 1 for one pass)
     bool single = false;  // the one-pass pipeline (hj_single.cu): bits <= kSingleMaxBits, passes 1
     int req_bits = 0;     // the radix bits asked for (bits is smaller in the one-pass pipeline)
+    bool mix = false;     // partitions by the low bits of mix_key (hj_partition.cuh) instead of the key's own
     int nparts() const { return 1 << bits; }
 };
 

@@ -59,14 +59,20 @@ namespace hj {
 // histogram and into the warp's histogram of the pass-1 digit, ORing together all row ids and (BUILD)
 // all keys: their widths decide whether the compact join table and the compact final partitions apply
 // (a value fits k bits iff the OR of all values does).
-template <bool BUILD>
+template <bool BUILD, bool MIX>
 __device__ __forceinline__ void hist_range_warp(const tuple_v *__restrict__ in, uint64_t lo, uint64_t hi,
                                                 uint32_t *sh_hist, uint32_t *wsub, uint64_t mask, uint32_t m1,
-                                                unsigned long long &kor, unsigned long long &ror) {
+                                                int bits, unsigned long long &kor, unsigned long long &ror) {
     uint64_t i = lo + (threadIdx.x & 31u);
     for (; i + 96 < hi; i += 128) {
-        const tuple_v t0 = ld_stream(in + i), t1 = ld_stream(in + i + 32);
-        const tuple_v t2 = ld_stream(in + i + 64), t3 = ld_stream(in + i + 96);
+        tuple_v t0 = ld_stream(in + i), t1 = ld_stream(in + i + 32);
+        tuple_v t2 = ld_stream(in + i + 64), t3 = ld_stream(in + i + 96);
+        if (MIX) {
+            t0.x = mix_key(t0.x, bits, kMixMul);
+            t1.x = mix_key(t1.x, bits, kMixMul);
+            t2.x = mix_key(t2.x, bits, kMixMul);
+            t3.x = mix_key(t3.x, bits, kMixMul);
+        }
         atomicAdd(&sh_hist[t0.x & mask], 1u);
         atomicAdd(&sh_hist[t1.x & mask], 1u);
         atomicAdd(&sh_hist[t2.x & mask], 1u);
@@ -79,7 +85,8 @@ __device__ __forceinline__ void hist_range_warp(const tuple_v *__restrict__ in, 
         ror |= t0.y | t1.y | t2.y | t3.y;
     }
     for (; i < hi; i += 32) {
-        const tuple_v t = ld_stream(in + i);
+        tuple_v t = ld_stream(in + i);
+        if (MIX) t.x = mix_key(t.x, bits, kMixMul);
         atomicAdd(&sh_hist[t.x & mask], 1u);
         atomicAdd(&wsub[(uint32_t)t.x & m1], 1u);
         if (BUILD) kor |= t.x;
@@ -93,6 +100,7 @@ __device__ __forceinline__ void hist_range_warp(const tuple_v *__restrict__ in, 
 //    sub-chunk's digit histogram is complete after a warp barrier and no CTA barrier interrupts the
 //    stream of loads. Every bin is written.
 // ------------------------------------------------------------------------------------------------
+template <bool MIX>
 __global__ void __launch_bounds__(512) hist_chunk_kernel(const tuple_v *__restrict__ R, size_t nR,
                                                          const tuple_v *__restrict__ S, size_t nS, int bits,
                                                          int F1, ChunkGeom cg, uint32_t *__restrict__ chunk_hist,
@@ -118,9 +126,9 @@ __global__ void __launch_bounds__(512) hist_chunk_kernel(const tuple_v *__restri
         const uint64_t lo = clo + (uint64_t)j * cg.sub < chi ? clo + (uint64_t)j * cg.sub : chi;
         const uint64_t hi = lo + cg.sub < chi ? lo + cg.sub : chi;
         if (rel == 0)
-            hist_range_warp<true>(in, lo, hi, sh_hist, wsub, mask, m1, kor, ror);
+            hist_range_warp<true, MIX>(in, lo, hi, sh_hist, wsub, mask, m1, bits, kor, ror);
         else
-            hist_range_warp<false>(in, lo, hi, sh_hist, wsub, mask, m1, kor, ror);
+            hist_range_warp<false, MIX>(in, lo, hi, sh_hist, wsub, mask, m1, bits, kor, ror);
         __syncwarp();
         uint32_t *so = subhist + ((size_t)c * cg.spc + j) * F1;
         for (int v = lane; v < F1; v += 32) {
@@ -564,6 +572,10 @@ __device__ __forceinline__ unsigned digit_peers_n(uint32_t d, int nbits) {
     return peers;
 }
 
+// The pass that reads the relations takes mix_key for the key; words only occur later.
+__device__ __forceinline__ void elem_mix(tuple_v &v, int bits) { v.x = mix_key(v.x, bits, kMixMul); }
+__device__ __forceinline__ void elem_mix(unsigned long long &, int) {}
+
 // Digit of an element in this pass: (key >> shift) & mask; a word holds key >> b1, which is pass 2's shift.
 __device__ __forceinline__ uint32_t elem_digit(const tuple_v &v, int shift, uint64_t dmask) {
     return (uint32_t)((v.x >> shift) & dmask);
@@ -572,7 +584,8 @@ __device__ __forceinline__ uint32_t elem_digit(unsigned long long v, int, uint64
     return (uint32_t)((v >> 32) & dmask);
 }
 
-template <int THREADS, int ITEMS, bool STABLE, int NBUF, int MINB, bool WIN = false>
+// MIX (pass 0 only): partition by mix_key, and store it in place of the key; pass 1 then finds it in its input.
+template <int THREADS, int ITEMS, bool STABLE, int NBUF, int MINB, bool WIN = false, bool MIX = false>
 __global__ void __launch_bounds__(THREADS, MINB) scatter_kernel(ScatterArgs a) {
     using E = typename ScatterElem<WIN>::type;
     constexpr int T = THREADS * ITEMS;
@@ -708,6 +721,7 @@ __global__ void __launch_bounds__(THREADS, MINB) scatter_kernel(ScatterArgs a) {
 #pragma unroll
             for (int i = 0; i < ITEMS; i++) {
                 v[i] = buf[w * 32 * ITEMS + i * 32 + lane];
+                if (MIX) elem_mix(v[i], a.bits);
                 d[i] = elem_digit(v[i], a.shift, dmask);
             }
         } else {
@@ -716,6 +730,7 @@ __global__ void __launch_bounds__(THREADS, MINB) scatter_kernel(ScatterArgs a) {
                 const uint32_t idx = (uint32_t)(w * 32 * ITEMS + i * 32 + lane);
                 if (idx < cnt) {
                     v[i] = buf[idx];
+                    if (MIX) elem_mix(v[i], a.bits);
                     d[i] = elem_digit(v[i], a.shift, dmask);
                 } else {
                     v[i] = E{};
@@ -980,7 +995,8 @@ __device__ __forceinline__ void seg_flush(uint32_t *jh, uint32_t *row, int nbins
 // order. Probe tiles keep the atomic rank: their order inside a partition changes no result.
 // Build key 0 of first-match joins needs nothing here: its word (high part 0) reaches key 0's final
 // partition, whose joins skip it (JoinItem::part0); a select per word cost pass 1 3%.
-template <int THREADS, int ITEMS, int K, bool W8 = false, bool STABLE_R = false>
+// MIX: partition by mix_key, and store it in place of the key.
+template <int THREADS, int ITEMS, int K, bool W8 = false, bool STABLE_R = false, bool MIX = false>
 __global__ void __launch_bounds__(THREADS, kSegCtasPerSm) seg_pass1_kernel(SegArgs a) {
     constexpr int T = THREADS * ITEMS;
     static_assert(T == kTile, "a tile fills one segment of tuples");
@@ -1125,6 +1141,7 @@ __global__ void __launch_bounds__(THREADS, kSegCtasPerSm) seg_pass1_kernel(SegAr
 #pragma unroll
             for (int i = 0; i < ITEMS; i++) {
                 v[i] = buf[w * 32 * ITEMS + i * 32 + lane];
+                if (MIX) v[i].x = mix_key(v[i].x, a.bits, kMixMul);
                 const uint32_t d = (uint32_t)v[i].x & dmask;
                 if (!st) rk[i] = atomicAdd(&thist[d], 1u);
                 const uint32_t bin = (uint32_t)(v[i].x & bmask);
@@ -1139,6 +1156,7 @@ __global__ void __launch_bounds__(THREADS, kSegCtasPerSm) seg_pass1_kernel(SegAr
                 const uint32_t idx = (uint32_t)(w * 32 * ITEMS + i * 32 + lane);
                 if (idx < cnt) {
                     v[i] = buf[idx];
+                    if (MIX) v[i].x = mix_key(v[i].x, a.bits, kMixMul);
                     const uint32_t d = (uint32_t)v[i].x & dmask;
                     if (!st) rk[i] = atomicAdd(&thist[d], 1u);
                     const uint32_t bin = (uint32_t)(v[i].x & bmask);
@@ -1666,6 +1684,7 @@ __device__ __forceinline__ void join_finish(const JoinArgs &a, bool ci) {
     r.error = acc->error | *reinterpret_cast<const volatile uint32_t *>(&a.counters[kCtrErr]);
     r.dup_flag = acc->dup_flag;
     r.large_parts = a.counters[kCtrNLarge];
+    r.large_build = ld_u64_pair(&a.counters[kCtrLargeR]);
     if (a.ci && ci_applies(a.counters, a.flag_bits)) r.flags = HJ_RES_COMPACT_PARTITIONS;
     *a.host_out = r;
     // Large partitions add to the result after this: start them from zero.
@@ -2531,11 +2550,14 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_small_kernel(JoinArgs a0
     join_finish(a, ci);
 }
 
-// Large partitions: chained tables in global memory, one flattened index space for all of them. Buckets are the
-// top bits of a multiplicative hash of the key above the radix bits: the keys of a large partition often share
-// more than those (ids in the high half of the key), and low bits of them would then make one chain of all.
+// Large partitions: chained tables in global memory, one flattened index space for all of them. A bucket is the low
+// bits of the key above the radix bits, changed by a hash of the bits above those (as mix_key): the keys of a
+// large partition often share more low bits than the radix bits (ids in the high half of the key) and would make
+// one chain of all, while runs of them keep neighbouring buckets (2^26 x 2^28 multiples of 4, 24.2 ms; 26.2 with a
+// full hash).
 __device__ __forceinline__ uint64_t large_bucket(uint64_t high, uint32_t nb_log) {
-    return nb_log ? (high * 0x9e3779b97f4a7c15ull) >> (64 - nb_log) : 0ull;
+    if (!nb_log) return 0;
+    return (high ^ (((high >> nb_log) * 0x9e3779b97f4a7c15ull) >> (64 - nb_log))) & ((1ull << nb_log) - 1);
 }
 
 __device__ __forceinline__ int find_large(const LargePart *L, int nl, uint64_t g, bool by_r) {
@@ -2865,6 +2887,7 @@ int radix_geom(int bits, int passes, RadixGeom *g, int b1_req) {
     g->bits = bits;
     g->req_bits = bits;
     g->single = false;
+    g->mix = false;
     g->passes = P;
     int b1 = bits / 2;
     if (b1_req > 0) {
@@ -2942,6 +2965,8 @@ struct PhjSizes {
     ChunkGeom cg;
 };
 
+// With fewer bits than asked for, keys that share low bits would overfill the partitions they fall into (2^24 x 2^26
+// multiples of 4: 1.5 ms with 14 bits, 5.8 with 12), so the partitions are then those of mix_key.
 // The two-pass pipelines' geometry: the lowest bits that bring build partitions to kSingleTarget tuples, at
 // most what the caller asked for. Fewer digits make longer runs and fewer, fuller units (2^24 x 2^26 in
 // segment mode: 1.32 ms with 12 bits, 1.40 with 13, 2.00 with 14; 2^24 x 2^28 3.38 / 3.47 / 4.09). Pass 2
@@ -2962,6 +2987,7 @@ void radix_geom_by_size(size_t nR, size_t nS, bool split_given, RadixGeom *g) {
         const int bits2 = (uint64_t)nR + nS >= kWideSplitTuples ? 7 : 8;
         radix_geom(b, 2, g, b - bits2 > kMinBits1 ? b - bits2 : kMinBits1);
     }
+    g->mix = b < req;
     g->req_bits = req;
 }
 
@@ -3110,21 +3136,31 @@ int phj_prepare_device() {
     HJ_CU(cudaGetDevice(&cur_dev));
     if (cur_dev < 0 || cur_dev >= 64) return HJ_E_INVAL;
     if (g_attr_done[cur_dev]) return HJ_OK;
-    HJ_CU(cudaFuncSetAttribute(hist_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 136 * 1024));
+    HJ_CU(cudaFuncSetAttribute(hist_chunk_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 136 * 1024));
+    HJ_CU(cudaFuncSetAttribute(hist_chunk_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 136 * 1024));
     HJ_CU(cudaFuncSetAttribute(plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)((size_t)2 * (1u << kPlanStageBits) * 4)));
     HJ_CU(cudaFuncSetAttribute(scatter_kernel<kScatterThreads, kScatterItems, true, kScatterBufs, kScatterCtasPerSm>,
                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scatter_smem_bytes(true)));
     HJ_CU(cudaFuncSetAttribute(scatter_kernel<kScatterThreads, kScatterItems, false, kScatterBufs, kScatterCtasPerSm>,
                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scatter_smem_bytes(false)));
-#define HJ_SEG_ATTR(KK, W, ST)                                                                             \
-    HJ_CU(cudaFuncSetAttribute(seg_pass1_kernel<kScatterThreads, kScatterItems, KK, W, ST>,                  \
+    HJ_CU(cudaFuncSetAttribute(
+        scatter_kernel<kScatterThreads, kScatterItems, true, kScatterBufs, kScatterCtasPerSm, false, true>,
+        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scatter_smem_bytes(true)));
+    HJ_CU(cudaFuncSetAttribute(
+        scatter_kernel<kScatterThreads, kScatterItems, false, kScatterBufs, kScatterCtasPerSm, false, true>,
+        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scatter_smem_bytes(false)));
+#define HJ_SEG_ATTR(KK, W, ST, MX)                                                                         \
+    HJ_CU(cudaFuncSetAttribute(seg_pass1_kernel<kScatterThreads, kScatterItems, KK, W, ST, MX>,              \
                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)seg_smem_bytes(kSegMaxBits, ST)))
-#define HJ_SEG_ATTR4(W, ST) \
-    HJ_SEG_ATTR(1, W, ST);  \
-    HJ_SEG_ATTR(2, W, ST);  \
-    HJ_SEG_ATTR(4, W, ST);  \
-    HJ_SEG_ATTR(8, W, ST)
+#define HJ_SEG_ATTR4(W, ST)        \
+    HJ_SEG_ATTR(1, W, ST, false);  \
+    HJ_SEG_ATTR(2, W, ST, false);  \
+    HJ_SEG_ATTR(4, W, ST, false);  \
+    HJ_SEG_ATTR(8, W, ST, false);  \
+    HJ_SEG_ATTR(1, W, ST, true);   \
+    HJ_SEG_ATTR(2, W, ST, true);   \
+    HJ_SEG_ATTR(4, W, ST, true)
     HJ_SEG_ATTR4(false, false);
     HJ_SEG_ATTR4(true, false);
     HJ_SEG_ATTR4(false, true);
@@ -3280,7 +3316,7 @@ int phj_enqueue(const RadixGeom &g, bool lp, bool skip0, const ulonglong2 *R, si
     // 9.01 against 10.68 ms).
     const bool exact_words =
         !segm && ci_ok && g.passes == 2 && ((test_flags & 4) || cg.chunk / (uint64_t)F1 >= 2ull * kTile);
-    if (segm && (g.passes != 2 || g.bits > kSegMaxBits)) return HJ_E_INVAL;
+    if (segm && (g.passes != 2 || g.bits > kSegMaxBits || (g.mix && F1 > 128))) return HJ_E_INVAL;
     {
         const int rc = phj_prepare_device();
         if (rc) return rc;
@@ -3318,25 +3354,33 @@ int phj_enqueue(const RadixGeom &g, bool lp, bool skip0, const ulonglong2 *R, si
         // Ordered first-match joins keep every build partition in input order (the stable build-relation form).
         const size_t sm = seg_smem_bytes(g.bits, stable);
         auto launch_pass1 = [&](bool words) {
-#define HJ_SEG_LAUNCH_W(KK, W)                                                                                   \
-    if (stable)                                                                                                  \
-        seg_pass1_kernel<kScatterThreads, kScatterItems, KK, W, true><<<s.seg_grid, kScatterThreads, sm, st>>>(ga); \
-    else                                                                                                         \
-        seg_pass1_kernel<kScatterThreads, kScatterItems, KK, W, false><<<s.seg_grid, kScatterThreads, sm, st>>>(ga)
-#define HJ_SEG_LAUNCH(KK)         \
-    if (words) {                  \
-        HJ_SEG_LAUNCH_W(KK, true);  \
-    } else {                      \
-        HJ_SEG_LAUNCH_W(KK, false); \
+#define HJ_SEG_LAUNCH_W(KK, W, MX)                                                                                   \
+    if (stable)                                                                                                      \
+        seg_pass1_kernel<kScatterThreads, kScatterItems, KK, W, true, MX><<<s.seg_grid, kScatterThreads, sm, st>>>(ga); \
+    else                                                                                                             \
+        seg_pass1_kernel<kScatterThreads, kScatterItems, KK, W, false, MX><<<s.seg_grid, kScatterThreads, sm, st>>>(ga)
+#define HJ_SEG_LAUNCH(KK, MX)           \
+    if (words) {                        \
+        HJ_SEG_LAUNCH_W(KK, true, MX);  \
+    } else {                            \
+        HJ_SEG_LAUNCH_W(KK, false, MX); \
     }
-            if (F1 <= 32) {
-                HJ_SEG_LAUNCH(1);
+            if (g.mix) {  // at most 7 bits in pass 1
+                if (F1 <= 32) {
+                    HJ_SEG_LAUNCH(1, true);
+                } else if (F1 <= 64) {
+                    HJ_SEG_LAUNCH(2, true);
+                } else {
+                    HJ_SEG_LAUNCH(4, true);
+                }
+            } else if (F1 <= 32) {
+                HJ_SEG_LAUNCH(1, false);
             } else if (F1 <= 64) {
-                HJ_SEG_LAUNCH(2);
+                HJ_SEG_LAUNCH(2, false);
             } else if (F1 <= 128) {
-                HJ_SEG_LAUNCH(4);
+                HJ_SEG_LAUNCH(4, false);
             } else {
-                HJ_SEG_LAUNCH(8);
+                HJ_SEG_LAUNCH(8, false);
             }
 #undef HJ_SEG_LAUNCH
 #undef HJ_SEG_LAUNCH_W
@@ -3355,8 +3399,12 @@ int phj_enqueue(const RadixGeom &g, bool lp, bool skip0, const ulonglong2 *R, si
         nlaunch++;
     } else {
         // 1. per-chunk histograms
-        hist_chunk_kernel<<<nchunks, 512, hist_smem, st>>>(R, nR, S, nS, g.bits, F1, cg, s.chunk_hist, s.subhist,
-                                                           s.counters + kCtrMaxKey);
+        if (g.mix)
+            hist_chunk_kernel<true><<<nchunks, 512, hist_smem, st>>>(R, nR, S, nS, g.bits, F1, cg, s.chunk_hist, s.subhist,
+                                                                     s.counters + kCtrMaxKey);
+        else
+            hist_chunk_kernel<false><<<nchunks, 512, hist_smem, st>>>(R, nR, S, nS, g.bits, F1, cg, s.chunk_hist, s.subhist,
+                                                                      s.counters + kCtrMaxKey);
         HJ_CU(cudaGetLastError());
     }
     if (!g.single) {
@@ -3444,8 +3492,12 @@ int phj_enqueue(const RadixGeom &g, bool lp, bool skip0, const ulonglong2 *R, si
         nlaunch++;                                                                                             \
         sa.w8 = 2;                                                                                             \
     }                                                                                                          \
-    scatter_kernel<kScatterThreads, kScatterItems, ST, kScatterBufs, kScatterCtasPerSm>                          \
-        <<<scatter_grid, kScatterThreads, scatter_smem_bytes(ST), st>>>(sa)
+    if (g.mix && pass == 0)                                                                                     \
+        scatter_kernel<kScatterThreads, kScatterItems, ST, kScatterBufs, kScatterCtasPerSm, false, true>         \
+            <<<scatter_grid, kScatterThreads, scatter_smem_bytes(ST), st>>>(sa);                               \
+    else                                                                                                       \
+        scatter_kernel<kScatterThreads, kScatterItems, ST, kScatterBufs, kScatterCtasPerSm>                      \
+            <<<scatter_grid, kScatterThreads, scatter_smem_bytes(ST), st>>>(sa)
             if (stable) {
                 HJ_SCATTER(true);
             } else {

@@ -13,7 +13,8 @@
 //                   partitions
 //   single_scatter  CTA c reads its ranges again, last tuple first (what the count read last is still in
 //                   L2), takes each element's place from a shared-memory cursor per digit and stores it
-// The partitions are those of `bits` low key bits, so the join kernels are the two-pass pipelines'.
+// The partitions are those of `bits` low bits of the key or of mix_key, so the join kernels are the two-pass
+// pipelines'.
 //
 // Elements: compact words ci_word (8 bytes) when the widths allow them, else tuples. First-match joins
 // need the lowest input position among equal build keys; their build elements are 16 bytes, {ci_word,
@@ -90,14 +91,14 @@ __global__ void __launch_bounds__(kCountThreads, 1) single_count(SingleArgs a0, 
             for (int u = 0; u < U; u++) t[u] = ld_twice(in + i + u * kCountThreads);
 #pragma unroll
             for (int u = 0; u < U; u++) {
-                atomicAdd(&mine[(uint32_t)t[u].x & mask], 1u);
+                atomicAdd(&mine[(uint32_t)mix_key(t[u].x, a.bits, a.mul) & mask], 1u);
                 kor |= t[u].x;
                 ror |= t[u].y;
             }
         }
         for (; i < hi; i += kCountThreads) {
             const tuple_v t = ld_twice(in + i);
-            atomicAdd(&mine[(uint32_t)t.x & mask], 1u);
+            atomicAdd(&mine[(uint32_t)mix_key(t.x, a.bits, a.mul) & mask], 1u);
             kor |= t.x;
             ror |= t.y;
         }
@@ -332,6 +333,7 @@ __device__ __noinline__ void single_scatter_rel(const SingleArgs &a, int rel, ui
         uint32_t rk[ITEMS / 2];  // ranks, two 16-bit ones per word
 #pragma unroll
         for (int q = 0; q < ITEMS; q++) {
+            t[q].x = mix_key(t[q].x, bits, a.mul);
             v[q] = Elem::stage(t[q], lo + base + q * NT + tid, bits, mask, z0);
             uint32_t r = 0;
             if (q * NT + tid < m) r = atomicAdd(&cnt[Elem::digit(v[q], mask)], 1u);
@@ -459,6 +461,7 @@ void single_args(const RadixGeom &g, bool lp, bool skip0, bool ci_ok, const ulon
     a.S = S;
     a.nR = nR;
     a.nS = nS;
+    a.mul = g.mix ? kMixMul : 0;
     a.bits = g.bits;
     a.copies = single_copies(g.bits);
     a.hist = s.chunk_hist;

@@ -34,6 +34,7 @@ RadixGeom geom_of(const WaveJoin &j) {
     g.F1 = 1 << b;
     g.F2 = 1;
     g.single = true;
+    g.mix = true;
     return g;
 }
 

@@ -153,7 +153,7 @@ typedef struct {
     double h2d;       /* seconds spent copying host inputs to the device (0 for device inputs) */
     int status;
     int physical_passes; /* partition passes the device ran, 0 to 2 (PHJ only) */
-    uint64_t large_partitions; /* partitions joined through the global-memory path (PHJ only) */
+    uint64_t large_partitions; /* partitions whose build side exceeded shared memory (PHJ only) */
     double phase[HJ_PH_COUNT]; /* per-kernel-group seconds (HJ_F_PHASE_TIMES) */
     uint32_t kernel_launches;  /* kernels this join launched */
     uint32_t flags;            /* HJ_RES_* bits */

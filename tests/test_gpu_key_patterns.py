@@ -148,3 +148,63 @@ def test_first_match_of_repeated_wide_keys(hj, oracle, cuda, algo, nR, copies):
             if algo.startswith("phj"):
                 assert bool(got[0].flags & hj.HJ_RES_ORDERED_PASSES) == (c > 1)
     assert times[1] < 3 * times[0], times
+
+
+STRIDES = {"x1": lambda k: k, "x4": lambda k: k * 4, "x2^14": lambda k: k << 14, "x2^32": lambda k: k << 32}
+
+
+@pytest.mark.parametrize("algo,nR,nS", [
+    ("phj_radix_bc", 1 << 17, 1 << 18), ("phj_radix_lp", 1 << 21, 1 << 21),   # raw digits, run again by mix_key
+    ("phj_radix_bc", (1 << 21) + 1, 1 << 22), ("phj_radix_lp", (1 << 21) + 1, 1 << 22),  # one pass by mix_key
+    ("nphj_sc", 1 << 21, 1 << 22), ("nphj_lp", (1 << 21) + 7, 1 << 22),
+    ("phj_radix_bc", (1 << 24) + 1, 1 << 24), ("phj_radix_lp", (1 << 24) + 1, 1 << 24),  # two passes, exact offsets
+    ("phj_radix_bc", (1 << 24) + 1, 3 << 24), ("phj_radix_lp", (1 << 24) + 1, 3 << 24),  # two passes, segments
+    ("nphj_sc", (1 << 24) + 1, 1 << 25), ("nphj_lp", (1 << 24) + 1, 1 << 25)])            # segments; the table
+def test_strided_keys(hj, cuda, algo, nR, nS):
+    """Distinct keys with a stride: the answer, no partition beyond shared memory where mix_key picks them, and no
+    more than four times a dense join's time (raw digits of such keys: six to ten times)."""
+    g = cuda.Generator(device="cuda")
+    g.manual_seed(nR)
+    R, S = (cuda.empty((n, 2), dtype=cuda.int64, device="cuda") for n in (nR, nS))
+    r = cuda.randperm(nR, generator=g, device="cuda")
+    s = cuda.randint(0, nR + nR // 4, (nS,), generator=g, device="cuda")
+    R[:, 1], S[:, 1] = cuda.randperm(nR, generator=g, device="cuda"), cuda.arange(nS, device="cuda")
+    rid = cuda.empty(nR, dtype=cuda.int64, device="cuda")
+    rid[r] = R[:, 1]
+    hit = s < nR
+    want = (int(hit.sum()), int((rid[s[hit]] + S[:, 1][hit]).sum()))
+    times = {}
+    for name, f in STRIDES.items():
+        R[:, 0], S[:, 0] = f(r + 1), f(s + 1)
+        with hj.Context(0) as ctx:
+            res = [hj.join(algo, R, S, on_device=True, ctx=ctx) for _ in range(4)]
+        assert all((q.matched_cnt, q.checksum) == want for q in res), name
+        raw = algo.startswith("phj") and nR <= 1 << 21
+        assert raw or all(q.large_partitions == 0 for q in res), name
+        times[name] = min(q.total for q in res)
+    assert max(times.values()) < 4 * times["x1"], times
+
+
+@pytest.mark.parametrize("algo", ["phj_radix_bc", "phj_radix_lp"])
+@pytest.mark.parametrize("kind", ["strided", "hot"])
+def test_run_again_by_mixed_keys(hj, oracle, cuda, algo, kind):
+    """A join whose raw digits overfill most of the build side's partitions runs again: duplicates, key 0, wide row
+    ids, the same partitions reported, with phase times, from a graph and from host memory; and a hot key, whose
+    partition is too large by either digits."""
+    rng = np.random.default_rng(77)
+    nR, nS = 100_000, 230_000
+    if kind == "strided":
+        R, S = relations(rng, nR, nS, "x2^14", dup=3, rid_bits=40)
+    else:
+        R, S = relations(rng, nR, nS, "x4", rid_bits=32)
+        R[20_000:90_000, 0] = R[1, 0]
+        S[:3000, 0] = R[1, 0]
+    want = oracle.join(algo, R, S)
+    dR, dS = dev(cuda, R), dev(cuda, S)
+    with hj.Context(0) as ctx:
+        got = [hj.join(algo, dR, dS, on_device=True, ctx=ctx, flags=hj.HJ_F_PHASE_TIMES) for _ in range(4)]
+        got += [hj.join(algo, R, S, ctx=ctx), hj.join(algo, dR, dS, on_device=True, ctx=ctx, watchdog_ms=60_000)]
+    for r in got:
+        assert (r.matched_cnt, r.checksum) == want
+        assert r.large_partitions == got[0].large_partitions >= 1
+        assert r.total > 0
