@@ -184,17 +184,33 @@ int ensure_arena(hj_ctx *c, size_t bytes) {
     return HJ_OK;
 }
 
-// Scratch for the plan; one that cannot be had falls back to a plan that needs less (segment mode to the
-// exact-offset pipeline, a non-partitioned join's radix pipeline to the table).
-int ensure_plan(hj_ctx *c, hj_algo_t algo, const hj_params_t &p, size_t nR, size_t nS, bool host_inputs, JoinPlan *jp) {
-    int rc = ensure_arena(c, scratch_need(*jp, p, nR, nS, host_inputs, c->num_sms));
+// Whether the arena can be as large as this: it is, or the device has the memory for it. A plan that has a smaller one
+// to fall back to asks first, so that an arena which serves that one is not given up for an allocation that
+// fails, with the join graphs, at every call.
+bool arena_may_grow(hj_ctx *c, size_t bytes) {
+    if (c->arena_bytes >= bytes) return true;
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return bytes <= free_b + c->arena_bytes;
+}
+
+// Scratch for the plan (need: its bytes); one that cannot be had falls back to a plan that needs less (segment mode to
+// the exact-offset pipeline, a non-partitioned join's radix pipeline to the table).
+template <class Need>
+int ensure_plan(hj_ctx *c, hj_algo_t algo, JoinPlan *jp, const Need &need) {
+    const bool table = jp->radix && !is_phj(algo);  // a plan to fall back to
+    auto attempt = [&](bool last) { return last || arena_may_grow(c, need()) ? ensure_arena(c, need()) : (int)HJ_E_OOM; };
+    int rc = attempt(!jp->seg && !table);
     if (rc == HJ_E_OOM && jp->seg) {
         jp->seg = false;
-        rc = ensure_arena(c, scratch_need(*jp, p, nR, nS, host_inputs, c->num_sms));
+        rc = attempt(!table);
     }
-    if (rc == HJ_E_OOM && jp->radix && !is_phj(algo)) {
+    if (rc == HJ_E_OOM && table) {
         *jp = JoinPlan();
-        rc = ensure_arena(c, scratch_need(*jp, p, nR, nS, host_inputs, c->num_sms));
+        rc = ensure_arena(c, need());
     }
     return rc;
 }
@@ -339,7 +355,7 @@ int hj_ctx_reserve(hj_ctx_t *c, hj_algo_t algo, const hj_params_t *pin, size_t n
     if (rc) return rc;
     DeviceGuard g(c->device);
     std::lock_guard<std::mutex> lk(c->mu);
-    return ensure_plan(c, algo, p, nR, nS, !p.inputs_on_device, &jp);
+    return ensure_plan(c, algo, &jp, [&] { return scratch_need(jp, p, nR, nS, !p.inputs_on_device, c->num_sms); });
 }
 
 int hj_join_ctx(hj_ctx_t *c, hj_algo_t algo, const hj_params_t *pin, const hj_tuple_t *R, size_t nR,
@@ -365,7 +381,7 @@ int hj_join_ctx(hj_ctx_t *c, hj_algo_t algo, const hj_params_t *pin, const hj_tu
         out->physical_passes = 0;
         if (host_in) rc = ensure_arena(c, kAccBytes + align256(nR * 16) + align256(nS * 16));
     } else {
-        rc = ensure_plan(c, algo, p, nR, nS, host_in, &jp);
+        rc = ensure_plan(c, algo, &jp, [&] { return scratch_need(jp, p, nR, nS, host_in, c->num_sms); });
     }
     if (rc) return out->status = rc;
     const bool radix = jp.radix, seg = jp.seg && !small;
@@ -665,15 +681,7 @@ static int join_mat(hj_ctx *c, hj_algo_t algo, hj_params_t p, const hj_tuple_t *
         if (pairs_in_arena) need += align256(cap * 16);
         return need;
     };
-    rc = ensure_arena(c, need_of());
-    if (rc == HJ_E_OOM && jp.seg) {
-        jp.seg = false;
-        rc = ensure_arena(c, need_of());
-    }
-    if (rc == HJ_E_OOM && jp.radix && !is_phj(algo)) {
-        jp = JoinPlan();
-        rc = ensure_arena(c, need_of());
-    }
+    rc = ensure_plan(c, algo, &jp, need_of);
     if (rc) return out->status = rc;
     const bool seg = jp.seg;
     const hj::RadixGeom &geom = jp.geom;
