@@ -517,22 +517,38 @@ static int plan_one(hj_ctx_t *c, const hj_batch_job_t *jobs, int njobs, const hj
 // Empirical tuning of a batch (HJ_F_TUNE): plan it under a few table budgets around the current one,
 // time each plan's graph, keep the fastest and leave its budget in the context's tuner. Timings of
 // single joins in isolation do not predict a batch well (waves share tables' L2 room, partitioned
-// joins overlap the waves on their own branch), the batch itself does.
+// joins overlap the waves on their own branch), the batch itself does. Budgets that lead to the same plan are timed
+// once, and a batch whose plan does not depend on the budget leaves the tuner as it is.
 int hj_batch_plan(hj_ctx_t *c, const hj_batch_job_t *jobs, int njobs, const hj_params_t *p, hj_batch_t **out) {
     if (!c || !out) return HJ_E_INVAL;
     if (!(p && (p->flags & HJ_F_TUNE))) return plan_one(c, jobs, njobs, p, out);
     *out = nullptr;
+    if (njobs < 0 || (njobs && !jobs)) return HJ_E_INVAL;
     const hj_tuner_t saved = c->tuner;
     const double base = saved.nphj_max_table_bytes > 0 ? saved.nphj_max_table_bytes : 64e6;
     const double scales[] = {1.0 / 32, 1.0 / 16, 0.125, 0.25, 0.5, 1.0, 2.0, 4.0};
     hj_batch_t *best = nullptr;
     double best_s = 1e300, best_budget = base;
-    std::vector<int> last_impl;
+    // What the tuner's decisions change of a plan: nothing for the joins of one-pass waves, the geometry of the
+    // others; with table waves (memory is short) every decision.
+    std::vector<int> last, seen;
+    bool tables = false, differ = false;
+    auto decisions = [&] {
+        std::vector<int> v;
+        for (int j = 0; j < njobs; j++) {
+            int impl = 0, bits = 0, passes = 0;
+            if (tables || !hj::wave_takes(jobs[j].nR, jobs[j].nS)) decide(c, jobs[j].nR, jobs[j].nS, &impl, &bits, &passes);
+            v.insert(v.end(), {impl, bits, passes});
+        }
+        return v;
+    };
     for (double sc : scales) {
         hj_tuner_t t = saved;
         t.nphj_max_table_bytes = base * sc;
         t.calibrated = 0;  // the table-budget rule
         c->tuner = t;
+        seen = decisions();
+        if (best && seen == last) continue;
         hj_batch_t *b = nullptr;
         int rc = plan_one(c, jobs, njobs, p, &b);
         if (rc) {
@@ -540,11 +556,12 @@ int hj_batch_plan(hj_ctx_t *c, const hj_batch_job_t *jobs, int njobs, const hj_p
             if (best) hj_batch_destroy(best);
             return rc;
         }
-        if (best && b->impl == last_impl) {  // same decisions as the previous budget: nothing to time
-            hj_batch_destroy(b);
-            continue;
+        if (!tables && !b->waves.empty()) {
+            tables = true;
+            seen = decisions();
         }
-        last_impl = b->impl;
+        differ = differ || best;
+        last = seen;
         double s = 1e300;
         for (int rep = 0; rep < 3 && !rc; rep++) {
             hj_batch_stats_t st;
@@ -567,8 +584,10 @@ int hj_batch_plan(hj_ctx_t *c, const hj_batch_job_t *jobs, int njobs, const hj_p
         }
     }
     c->tuner = saved;
-    c->tuner.nphj_max_table_bytes = best_budget;
-    c->tuner.calibrated = 0;
+    if (differ) {
+        c->tuner.nphj_max_table_bytes = best_budget;
+        c->tuner.calibrated = 0;
+    }
     *out = best;
     return HJ_OK;
 }
@@ -910,8 +929,8 @@ int hj_join_batch(hj_ctx_t *c, const hj_batch_job_t *jobs, int njobs, const hj_p
     return rc;
 }
 
-// Calibration: time both implementations on PK-FK joins of growing build size (|S| = 8 |R|) and set
-// the table budget to the largest build whose non-partitioned join was faster.
+// Calibration: time both implementations, as the decisions choose between them (the global table; the exact-offset
+// pipeline with the decision's bits), on PK-FK joins of growing build size (|S| = 8 |R|) and fit the cost model.
 int hj_tuner_calibrate(hj_ctx_t *c, double *report, int report_len) {
     if (!c) return HJ_E_INVAL;
     int dev_prev = -1;
@@ -950,6 +969,7 @@ int hj_tuner_calibrate(hj_ctx_t *c, double *report, int report_len) {
                 c->tuner = saved;
                 p.num_radix_bits = b;
                 p.num_passes = ps;
+                p.flags = HJ_F_EXACT;  // the pipeline that the server runs for this decision
                 algo = HJ_ALGO_PHJ_RADIX_BC;
             }
             for (int rep = 0; rep < 4; rep++) {

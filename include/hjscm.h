@@ -276,7 +276,8 @@ void hj_pkfk_closed_form(size_t nR, size_t nS, uint64_t *matched, uint64_t *chec
  * -------------------------------------------------------------------------------------------- */
 #define HJ_F_NO_GRAPH 0x8u /* batches: launch the kernels one by one instead of one captured graph */
 #define HJ_F_TUNE 0x10u    /* batches: plan under a few table budgets around the tuner's, time each plan
-                              on the device (the joins run), keep the fastest and its budget */
+                              on the device (the joins run), keep the fastest and its budget; budgets
+                              that lead to the same plan are timed once, and if all do the tuner stays */
 
 #define HJ_TUNER_LEVELS 8
 
@@ -308,8 +309,10 @@ typedef struct {
     uint64_t matched_cnt;
     uint64_t checksum;
     int status;                  /* HJ_OK or an HJ_E_* code for this join */
-    int impl;                    /* what ran: 0 = non-partitioned table, 1 = radix-partitioned */
-    int num_radix_bits;          /* radix-partitioned joins: bits and passes chosen */
+    int impl;                    /* the tuner's decision: 0 = non-partitioned table, 1 = radix-partitioned.
+                                    Joins of up to 12.58 M build tuples run in one-pass waves whatever it is,
+                                    unless memory is short */
+    int num_radix_bits;          /* decision 1: its bits and passes */
     int num_passes;
 } hj_batch_result_t;
 
@@ -317,7 +320,7 @@ typedef struct {
     double seconds;              /* device time of the whole batch (CUDA events) */
     uint32_t kernel_launches;    /* kernels the batch launches */
     int waves;                   /* waves of joins */
-    int nphj_jobs, phj_jobs;
+    int nphj_jobs, phj_jobs;     /* joins by the tuner's decision (hj_batch_result_t.impl) */
 } hj_batch_stats_t;
 
 typedef struct hj_batch hj_batch_t;
