@@ -439,7 +439,7 @@ int hj_join_ctx(hj_ctx_t *c, hj_algo_t algo, const hj_params_t *pin, const hj_tu
             if (timing && hj::record_event(c->ev_start, st) != cudaSuccess) return HJ_E_DEVICE;
             for (int i = 0; ph && i < HJ_PH_LARGE; i++)
                 if (hj::record_event(ph[i], st) != cudaSuccess) return HJ_E_DEVICE;
-            int erc = hj::phj_prepare_device();
+            int erc = hj::phj_prepare_device(false, false);
             if (!erc)
                 erc = hj::small_enqueue(hj::algo_lp(algo), hj::algo_skip0(algo), is_phj(algo) ? geom.req_bits : -1, dR,
                                         nR, dS, nS, reinterpret_cast<hj::SmallPart *>(c->small_buf + 256),

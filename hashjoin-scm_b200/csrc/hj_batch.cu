@@ -835,7 +835,7 @@ static int plan_tables(hj_ctx_t *c, const hj_batch_job_t *jobs, int njobs, const
         b->waves.push_back(w);
     }
     b->phj_scratch = cur;
-    if (hj::phj_prepare_device()) return fail(HJ_E_DEVICE);
+    if (hj::phj_prepare_device(false, true)) return fail(HJ_E_DEVICE);
     if (b->use_graph) {
         if (cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) return fail(HJ_E_DEVICE);
         int rc = enqueue_batch(b);

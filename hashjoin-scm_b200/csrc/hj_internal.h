@@ -121,9 +121,10 @@ struct PhjScratch {
 // relation and pass-1 digit).
 bool phj_seg_applies(const RadixGeom &g, bool lp, size_t nR, size_t nS);
 
-// Kernel attributes (dynamic shared memory limits) for the current device; phj_enqueue calls it too,
-// but callers that capture a stream into a graph call it before the capture.
-int phj_prepare_device();
+// Kernel attributes (dynamic shared memory limits) for the current device: of the kernels that every join may
+// use, and of segment mode's or of the exact-offset pipeline's pass by mix_key. phj_enqueue calls it too, but
+// callers that capture a stream into a graph call it before the capture.
+int phj_prepare_device(bool seg, bool mix);
 
 // seg: lay the scratch out for segment mode (callers pass phj_seg_applies(...) or false).
 size_t phj_scratch_bytes(const RadixGeom &g, size_t nR, size_t nS, int num_sms, bool seg = false);

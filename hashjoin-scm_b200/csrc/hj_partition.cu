@@ -47,6 +47,7 @@
 // pass. seg_pass1_kernel writes pass 1 into per-(CTA, relation, digit) chains of tile-sized segments
 // and counts each CTA's joint histogram itself; colscan/plan/units then treat the pass-1 CTAs as the
 // chunks, and pass 2 (scatter_kernel) walks the chains as its units.
+#include <atomic>
 #include <cstdio>
 
 #include "hj_common.cuh"
@@ -3114,8 +3115,6 @@ void phj_carve(const RadixGeom &g, size_t nR, size_t nS, int num_sms, char *base
         }                                                                             \
     } while (0)
 
-static bool g_attr_done[64] = {};
-
 // Dynamic shared memory of seg_pass1_kernel: two tile buffers, per-digit state, 2^bits 16-bit counters,
 // and for the stable build-relation rank one 16-bit counter per (warp, digit).
 static size_t seg_smem_bytes(int bits, bool stable) {
@@ -3131,42 +3130,48 @@ static constexpr size_t scatter_smem_bytes(bool stable) {
            (stable ? (size_t)(kScatterThreads / 32) * 256 * 2 : (size_t)256 * 4);
 }
 
-int phj_prepare_device() {
-    int cur_dev = 0;
-    HJ_CU(cudaGetDevice(&cur_dev));
-    if (cur_dev < 0 || cur_dev >= 64) return HJ_E_INVAL;
-    if (g_attr_done[cur_dev]) return HJ_OK;
-    HJ_CU(cudaFuncSetAttribute(hist_chunk_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 136 * 1024));
+// Segment mode's pass 1, by the key's digits or by mix_key.
+template <bool MIX>
+static int prepare_segments() {
+#define HJ_SEG_ATTR(KK, W, ST)                                                                             \
+    HJ_CU(cudaFuncSetAttribute(seg_pass1_kernel<kScatterThreads, kScatterItems, KK, W, ST, MIX>,             \
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)seg_smem_bytes(kSegMaxBits, ST)))
+#define HJ_SEG_ATTR4(KK)         \
+    HJ_SEG_ATTR(KK, false, false); \
+    HJ_SEG_ATTR(KK, true, false);  \
+    HJ_SEG_ATTR(KK, false, true);  \
+    HJ_SEG_ATTR(KK, true, true)
+    HJ_SEG_ATTR4(1);
+    HJ_SEG_ATTR4(2);
+    HJ_SEG_ATTR4(4);
+    if constexpr (!MIX) {
+        HJ_SEG_ATTR4(8);
+    }
+#undef HJ_SEG_ATTR4
+#undef HJ_SEG_ATTR
+    return HJ_OK;
+}
+
+// The exact-offset pipeline's kernels that partition by mix_key.
+static int prepare_mixed() {
     HJ_CU(cudaFuncSetAttribute(hist_chunk_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 136 * 1024));
-    HJ_CU(cudaFuncSetAttribute(plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)((size_t)2 * (1u << kPlanStageBits) * 4)));
-    HJ_CU(cudaFuncSetAttribute(scatter_kernel<kScatterThreads, kScatterItems, true, kScatterBufs, kScatterCtasPerSm>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scatter_smem_bytes(true)));
-    HJ_CU(cudaFuncSetAttribute(scatter_kernel<kScatterThreads, kScatterItems, false, kScatterBufs, kScatterCtasPerSm>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scatter_smem_bytes(false)));
     HJ_CU(cudaFuncSetAttribute(
         scatter_kernel<kScatterThreads, kScatterItems, true, kScatterBufs, kScatterCtasPerSm, false, true>,
         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scatter_smem_bytes(true)));
     HJ_CU(cudaFuncSetAttribute(
         scatter_kernel<kScatterThreads, kScatterItems, false, kScatterBufs, kScatterCtasPerSm, false, true>,
         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scatter_smem_bytes(false)));
-#define HJ_SEG_ATTR(KK, W, ST, MX)                                                                         \
-    HJ_CU(cudaFuncSetAttribute(seg_pass1_kernel<kScatterThreads, kScatterItems, KK, W, ST, MX>,              \
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)seg_smem_bytes(kSegMaxBits, ST)))
-#define HJ_SEG_ATTR4(W, ST)        \
-    HJ_SEG_ATTR(1, W, ST, false);  \
-    HJ_SEG_ATTR(2, W, ST, false);  \
-    HJ_SEG_ATTR(4, W, ST, false);  \
-    HJ_SEG_ATTR(8, W, ST, false);  \
-    HJ_SEG_ATTR(1, W, ST, true);   \
-    HJ_SEG_ATTR(2, W, ST, true);   \
-    HJ_SEG_ATTR(4, W, ST, true)
-    HJ_SEG_ATTR4(false, false);
-    HJ_SEG_ATTR4(true, false);
-    HJ_SEG_ATTR4(false, true);
-    HJ_SEG_ATTR4(true, true);
-#undef HJ_SEG_ATTR4
-#undef HJ_SEG_ATTR
+    return HJ_OK;
+}
+
+static int prepare_all() {
+    HJ_CU(cudaFuncSetAttribute(hist_chunk_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 136 * 1024));
+    HJ_CU(cudaFuncSetAttribute(plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)((size_t)2 * (1u << kPlanStageBits) * 4)));
+    HJ_CU(cudaFuncSetAttribute(scatter_kernel<kScatterThreads, kScatterItems, true, kScatterBufs, kScatterCtasPerSm>,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scatter_smem_bytes(true)));
+    HJ_CU(cudaFuncSetAttribute(scatter_kernel<kScatterThreads, kScatterItems, false, kScatterBufs, kScatterCtasPerSm>,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scatter_smem_bytes(false)));
     HJ_CU(cudaFuncSetAttribute(
         scatter_kernel<kScatterThreads, 2 * kScatterItems, false, kScatterBufs, scatter_word_ctas(false), true>,
         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scatter_smem_bytes(false)));
@@ -3206,8 +3211,24 @@ int phj_prepare_device() {
         if (!rc) rc = small_prepare_device();
         if (rc) return rc;
     }
-    g_attr_done[cur_dev] = true;
     return nphj_prepare_device();
+}
+
+// In parts, as setting an attribute loads the kernel (a process's first server took 24 ms to create with all of them,
+// 16 without the pass-1 forms that it does not use).
+int phj_prepare_device(bool seg, bool mix) {
+    static std::atomic<unsigned> done[64];
+    int cur_dev = 0;
+    HJ_CU(cudaGetDevice(&cur_dev));
+    if (cur_dev < 0 || cur_dev >= 64) return HJ_E_INVAL;
+    const unsigned want = 1u | (!seg && mix ? 2u : 0u) | (seg ? (mix ? 8u : 4u) : 0u), have = done[cur_dev].load();
+    int rc = HJ_OK;
+    if (want & ~have & 1u) rc = prepare_all();
+    if (!rc && (want & ~have & 2u)) rc = prepare_mixed();
+    if (!rc && (want & ~have & 4u)) rc = prepare_segments<false>();
+    if (!rc && (want & ~have & 8u)) rc = prepare_segments<true>();
+    if (!rc) done[cur_dev].fetch_or(want);
+    return rc;
 }
 
 JoinArgs join_args(const RadixGeom &g, bool lp, bool skip0, const ulonglong2 *R, size_t nR, const PhjScratch &s,
@@ -3318,7 +3339,7 @@ int phj_enqueue(const RadixGeom &g, bool lp, bool skip0, const ulonglong2 *R, si
         !segm && ci_ok && g.passes == 2 && ((test_flags & 4) || cg.chunk / (uint64_t)F1 >= 2ull * kTile);
     if (segm && (g.passes != 2 || g.bits > kSegMaxBits || (g.mix && F1 > 128))) return HJ_E_INVAL;
     {
-        const int rc = phj_prepare_device();
+        const int rc = phj_prepare_device(segm, g.mix);
         if (rc) return rc;
     }
     if (!g.single) HJ_CU(cudaMemsetAsync(s.counters, 0, kNumCounters * 4, st));  // the one-pass count clears them

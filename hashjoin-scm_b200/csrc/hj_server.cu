@@ -755,7 +755,7 @@ int hj_server_create(const hj_server_config_t *cfg, hj_server_t **out) {
     }
     s->pool_bytes = want;
     s->pool.init(want);
-    hj::phj_prepare_device();
+    hj::phj_prepare_device(false, false);
     int prio_lo = 0, prio_hi = 0;
     cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi);
     s->slots.resize(cfg->slots);
