@@ -601,11 +601,19 @@ __global__ void __launch_bounds__(256) nphj_probe_mat(NphjArgs a) {
     }
 }
 
+// Whether n pairs are worth the columns: reading both relations for them costs as much as the gathers save at about a
+// quarter of a pair per tuple (retrieve phase, columns and not: 2^24 x 2^26 tuples, 67 M pairs 1980 / 2440 us, 27 M
+// 1012 / 1028, 17 M 746 / 666, 0.7 M 316 / 45; 2^23 x 2^24, 6.7 M 196 / 225, 4.2 M 163 / 154).
+__device__ __forceinline__ bool mat_columns_pay(unsigned long long n, unsigned long long nR, unsigned long long nS) {
+    return 4 * n >= nR + nS;
+}
+
 // Row-id columns for the retrieve phase: the low 32 bits of every row id, and in acc->wide_rids the OR of the
 // high ones.
-__global__ void mat_columns(const tuple_v *__restrict__ R, unsigned long long nR, const tuple_v *__restrict__ S,
+__global__ void mat_columns(const unsigned long long *n_dev, unsigned long long cap, const tuple_v *__restrict__ R, unsigned long long nR, const tuple_v *__restrict__ S,
                             unsigned long long nS, uint32_t *__restrict__ colR, uint32_t *__restrict__ colS,
                             JoinAccum *acc) {
+    if (!mat_columns_pay(min(*n_dev, cap), nR, nS)) return;
     unsigned long long wide = 0;
     constexpr int U = 4;
     const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
@@ -637,7 +645,7 @@ __global__ void mat_retrieve(const ulonglong2 *__restrict__ pairs, const unsigne
                              const uint32_t *__restrict__ colS, JoinAccum *acc) {
     unsigned long long n = *n_dev;
     if (n > cap) n = cap;
-    const bool col = colR && *reinterpret_cast<volatile unsigned long long *>(&acc->wide_rids) == 0;
+    const bool col = colR && mat_columns_pay(n, nR, nS) && *reinterpret_cast<volatile unsigned long long *>(&acc->wide_rids) == 0;
     unsigned long long sum = 0;
     bool bad = false;
     // Eight pairs per thread and step: their 16 gathers are all in flight before any is summed.
@@ -842,7 +850,7 @@ int mat_retrieve_enqueue(const ulonglong2 *pairs, const unsigned long long *n_de
     if ((nR + nS) * 16 > kMatColumnsFrom && (nR + nS) * 4 <= scratch_bytes) {
         colR = reinterpret_cast<uint32_t *>(scratch);
         colS = colR + nR;
-        mat_columns<<<num_sms * 4, 512, 0, st>>>(R, nR, S, nS, colR, colS, acc);
+        mat_columns<<<num_sms * 4, 512, 0, st>>>(n_dev, cap, R, nR, S, nS, colR, colS, acc);
         *launches += 1;
     }
     mat_retrieve<<<num_sms * 8, 256, 0, st>>>(pairs, n_dev, cap, R, nR, S, nS, colR, colS, acc);

@@ -98,3 +98,27 @@ def test_empty_relations(hj, cuda):
         assert (r.matched_cnt, r.checksum) == (0, 0)
         r = hj.join_mat(algo, one, one)
         assert (r.matched_cnt, r.checksum) == (1, 2)
+
+
+@pytest.mark.parametrize("algo", ["phj_radix_bc", "nphj_lp"])
+@pytest.mark.parametrize("pairs", [0, 1, (1 << 20) + (1 << 19) - 1, (1 << 20) + (1 << 19), (1 << 20) + (1 << 19) + 1])
+def test_retrieve_of_few_pairs(hj, cuda, algo, pairs):
+    """The retrieve phase gathers from row-id columns where there is a pair for every fourth tuple at least, else from
+    the relations (2^21 x 2^22 tuples, on both sides of that line), and a few pairs cost it next to nothing."""
+    nR, nS = 1 << 21, 1 << 22
+    g = cuda.Generator(device="cuda")
+    g.manual_seed(6)
+    R, S = (cuda.empty((n, 2), dtype=cuda.int64, device="cuda") for n in (nR, nS))
+    R[:, 0] = cuda.randperm(nR, generator=g, device="cuda") + 1
+    S[:, 0] = nR + 5
+    at = cuda.randperm(nS, generator=g, device="cuda")[:pairs]
+    S[at, 0] = cuda.randint(1, nR + 1, (pairs,), generator=g, device="cuda")
+    R[:, 1], S[:, 1] = cuda.randperm(nR, generator=g, device="cuda") + 1, cuda.randperm(nS, generator=g, device="cuda") + 1
+    rid = cuda.zeros(nR + 6, dtype=cuda.int64, device="cuda")
+    rid[R[:, 0]] = R[:, 1]
+    want = int((R[:, 1][rid[S[at, 0]] - 1] + S[:, 1][S[at, 1] - 1]).sum())
+    with hj.Context(0) as ctx:
+        res = [hj.join_mat(algo, R, S, on_device=True, ctx=ctx) for _ in range(4)]
+    assert all((r.matched_cnt, r.checksum) == (pairs, want) for r in res)
+    if pairs <= 1:
+        assert min(r.retrieve for r in res) < 25e-6
