@@ -169,6 +169,29 @@ __device__ __forceinline__ void tma_load_1d(void *dst_smem, const void *src, uin
     }
 }
 
+// Segment mode (hj_segments.cu).
+constexpr uint32_t kSegSlab = 32;          // segment ids a CTA takes from the global counter at once
+constexpr int kSegCtasPerSm = 2;           // shared memory: two tile buffers + 32 KB of counters
+constexpr int kSegMaxBits = 14;
+int seg_prepare_device(bool mix);
+// Pass 1 into segment chains, with the per-CTA histograms. words_too: in 8-byte words where the widths allow them;
+// stable: every build partition keeps input order (ordered first-match joins); stall: the test hook.
+int seg_pass1_enqueue(const RadixGeom &g, const ulonglong2 *R, size_t nR, const ulonglong2 *S, size_t nS,
+                      const PhjScratch &s, bool words_too, bool stable, bool stall, cudaStream_t st, uint32_t *launches);
+
+// Lanes of the warp whose digit equals this lane's: one ballot per digit bit (NB bits).
+template <int NB>
+__device__ __forceinline__ unsigned digit_peers(uint32_t d) {
+    unsigned peers = 0xffffffffu;
+#pragma unroll
+    for (int b = 0; b < NB; b++) {
+        const unsigned bit = (d >> b) & 1u;
+        const unsigned bal = __ballot_sync(0xffffffffu, bit);
+        peers &= bal ^ (bit - 1u);  // bit ? bal : ~bal
+    }
+    return peers;
+}
+
 // Chunking of the two relations (identical for the histogram and both scatter passes).
 struct ChunkGeom {
     uint64_t chunk;  // tuples per chunk (a multiple of the tile)
