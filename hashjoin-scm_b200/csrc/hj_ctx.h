@@ -52,7 +52,8 @@ struct hj_ctx {
     size_t arena_bytes = 0;
     hj::JoinAccum *acc_host = nullptr;  // pinned
     char *copy_buf = nullptr;           // page-locked pieces of copies from pageable memory (hj_hostcopy.cu)
-    std::vector<cudaEvent_t> copy_ev;   // one per piece: its last copy has been read
+    static constexpr int kCopyEvents = 8;
+    cudaEvent_t copy_ev[kCopyEvents] = {};  // one per piece: its last copy has been read
     char *small_buf = nullptr;          // device: the ticket and partial results of one-kernel joins
     bool gave_up = false;               // a watchdog gave up on a join: the next one waits for ev_done
     hj_tuner_t tuner = {};              // autotuner state used by batches

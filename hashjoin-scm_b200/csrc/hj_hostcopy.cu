@@ -3,13 +3,13 @@
 // A copy from pageable memory goes through the driver's own staging on one thread, at about 10 GB/s of the
 // ~55 GB/s the link carries: 8.1 ms of an 8.2 ms join of 2^20 x 2^22 host tuples. Here up to kCopyThreads
 // threads of the call copy 2 MB pieces into page-locked buffers, two per thread, and issue the pieces'
-// copies on the join's stream: 2.4 ms for the same join (3 threads 2.9, 6 threads 2.5, 12 threads of 1 MB
-// pieces 3.9: the threads then wait for each other in the driver). The buffers (16 MB) belong to the context, are allocated by its first large pageable
-// copy and freed with it; the threads end before the call goes on. Page-locked sources, and copies too small
-// to repay the threads, take the plain copy, and so does a call that cannot get buffers or threads.
+// copies on the join's stream: 2.4 to 2.8 ms for the same join, whole calls on different machines (on the one where
+// it took 2.4: 3 threads 2.9, 6 threads 2.5, 12 threads of 1 MB pieces 3.9, which then wait for each other in the
+// driver). The buffers (16 MB) belong to the context, are allocated by its first large pageable copy and freed
+// with it; the threads end before the call goes on. Page-locked sources, and copies too small to repay the
+// threads, take the plain copy, and so does a call that cannot get buffers; fewer threads copy more pieces each.
 #include <atomic>
 #include <cstring>
-#include <system_error>
 #include <thread>
 
 #include "hj_ctx.h"
@@ -20,6 +20,7 @@ namespace hj {
 namespace {
 
 constexpr int kCopyThreads = 4, kCopyBuffers = 2 * kCopyThreads;
+static_assert(kCopyBuffers == hj_ctx::kCopyEvents, "an event per buffer");
 constexpr size_t kCopyPiece = 2u << 20, kCopyMin = 4u << 20;
 constexpr int kMaxCopies = 2;
 
@@ -39,14 +40,13 @@ bool get_buffers(hj_ctx *c) {
         c->copy_buf = nullptr;
         return false;
     }
-    for (int i = 0; i < kCopyBuffers; i++) {
-        cudaEvent_t ev;
+    for (cudaEvent_t &ev : c->copy_ev) {
         if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) {
             cudaGetLastError();
+            ev = nullptr;
             free_copy_buffers(c);
             return false;
         }
-        c->copy_ev.push_back(ev);
     }
     return true;
 }
@@ -54,8 +54,10 @@ bool get_buffers(hj_ctx *c) {
 }  // namespace
 
 void free_copy_buffers(hj_ctx *c) {
-    for (cudaEvent_t ev : c->copy_ev) cudaEventDestroy(ev);
-    c->copy_ev.clear();
+    for (cudaEvent_t &ev : c->copy_ev) {
+        if (ev) cudaEventDestroy(ev);
+        ev = nullptr;
+    }
     if (c->copy_buf) cudaFreeHost(c->copy_buf);
     c->copy_buf = nullptr;
 }
@@ -114,7 +116,7 @@ int copy_in(hj_ctx *c, const HostCopy *copies, int ncopies, bool pinned, cudaStr
     int started = 1;
     try {
         for (; started < want; started++) threads[started] = std::thread(work, started);
-    } catch (const std::system_error &) {  // fewer threads: those that started, and this one, do all pieces
+    } catch (...) {  // no more threads (or memory for them): those that started, and this one, do all pieces
     }
     work(0);
     for (int w = 1; w < started; w++) threads[w].join();

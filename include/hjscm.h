@@ -189,7 +189,8 @@ const char *hj_algo_name(hj_algo_t algo);
  * serialised, joins on different contexts may run concurrently. */
 int hj_ctx_create(int device, hj_ctx_t **out);
 int hj_ctx_destroy(hj_ctx_t *ctx);
-/* Pre-size the scratch arena for a join of the given shape, so that later joins allocate nothing. */
+/* Pre-size the scratch arena for a join of the given shape, so that later joins allocate no device memory (the
+ * first large copy from pageable host memory also allocates 16 MB of page-locked buffers). */
 int hj_ctx_reserve(hj_ctx_t *ctx, hj_algo_t algo, const hj_params_t *p, size_t nR, size_t nS);
 /* Bytes of device scratch the context currently holds. */
 size_t hj_ctx_scratch_bytes(const hj_ctx_t *ctx);
