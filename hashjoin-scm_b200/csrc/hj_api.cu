@@ -168,6 +168,11 @@ hj_graph_entry *find_graph(hj_ctx *c, const hj_graph_key &k) {
     return nullptr;
 }
 
+void refuse_arena(hj_ctx *c, size_t bytes) {
+    c->refused_bytes = bytes;
+    c->refused_at = std::chrono::steady_clock::now();
+}
+
 int ensure_arena(hj_ctx *c, size_t bytes) {
     if (c->arena_bytes >= bytes) return HJ_OK;
     CU_OR(cudaStreamSynchronize(c->stream), HJ_E_DEVICE);
@@ -178,6 +183,7 @@ int ensure_arena(hj_ctx *c, size_t bytes) {
     if (cudaMalloc(&c->arena, bytes) != cudaSuccess) {
         cudaGetLastError();
         c->arena = nullptr;
+        refuse_arena(c, bytes);
         return HJ_E_OOM;
     }
     c->arena_bytes = bytes;
@@ -186,15 +192,21 @@ int ensure_arena(hj_ctx *c, size_t bytes) {
 
 // Whether the arena can be as large as this: it is, or the device has the memory for it. A plan that has a smaller one
 // to fall back to asks first, so that an arena which serves that one is not given up for an allocation that
-// fails, with the join graphs, at every call.
+// fails, with the join graphs, at every call. Asking the driver takes 0.07 to 1 ms, so a refusal stands for a second.
 bool arena_may_grow(hj_ctx *c, size_t bytes) {
     if (c->arena_bytes >= bytes) return true;
+    if (c->refused_bytes && bytes >= c->refused_bytes &&
+        std::chrono::steady_clock::now() - c->refused_at < std::chrono::seconds(1))
+        return false;
+    c->refused_bytes = 0;
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
         cudaGetLastError();
         return true;
     }
-    return bytes <= free_b + c->arena_bytes;
+    if (bytes <= free_b + c->arena_bytes) return true;
+    refuse_arena(c, bytes);
+    return false;
 }
 
 // Scratch for the plan (need: its bytes); one that cannot be had falls back to a plan that needs less (segment mode to

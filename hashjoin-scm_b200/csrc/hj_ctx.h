@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <chrono>
 #include <cstdint>
 #include <mutex>
 #include <vector>
@@ -50,6 +51,8 @@ struct hj_ctx {
     cudaEvent_t ev_ph[HJ_PH_COUNT + 1] = {};
     char *arena = nullptr;
     size_t arena_bytes = 0;
+    size_t refused_bytes = 0;  // an arena of this size was refused, at refused_at (0: none; see arena_may_grow)
+    std::chrono::steady_clock::time_point refused_at;
     hj::JoinAccum *acc_host = nullptr;  // pinned
     char *copy_buf = nullptr;           // page-locked pieces of copies from pageable memory (hj_hostcopy.cu)
     static constexpr int kCopyEvents = 8;
