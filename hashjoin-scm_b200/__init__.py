@@ -218,7 +218,8 @@ def join(algo: str, R, S, *, bits: int = 14, passes: int = 2, device: int = 0, o
     """Run one join (synchronous). Raises JoinError on a non-zero status when check is set.
     bits_pass1: pass-1 radix bits of a two-pass join (None: 11 for phj_asymm_radix_* names, as the
     reference's NUM_RADIX_BITS_PASS1 default, else an even split). load: the non-partitioned joins'
-    table load factor (0: 0.4 for build relations up to 5 M tuples, 0.5 above)."""
+    table load factor (0: 0.4 for build relations up to 5 M tuples, 0.5 above, or a radix pipeline instead of
+    the table at sizes where that is faster; the result is the same)."""
     L = lib()
     a = ALGOS[algo]
     if bits_pass1 is None:

@@ -69,10 +69,10 @@ __device__ __forceinline__ void hist_range_warp(const tuple_v *__restrict__ in, 
         tuple_v t0 = ld_stream(in + i), t1 = ld_stream(in + i + 32);
         tuple_v t2 = ld_stream(in + i + 64), t3 = ld_stream(in + i + 96);
         if (MIX) {
-            t0.x = mix_key(t0.x, bits, kMixMul);
-            t1.x = mix_key(t1.x, bits, kMixMul);
-            t2.x = mix_key(t2.x, bits, kMixMul);
-            t3.x = mix_key(t3.x, bits, kMixMul);
+            t0.x = mix_key(t0.x, bits);
+            t1.x = mix_key(t1.x, bits);
+            t2.x = mix_key(t2.x, bits);
+            t3.x = mix_key(t3.x, bits);
         }
         atomicAdd(&sh_hist[t0.x & mask], 1u);
         atomicAdd(&sh_hist[t1.x & mask], 1u);
@@ -87,7 +87,7 @@ __device__ __forceinline__ void hist_range_warp(const tuple_v *__restrict__ in, 
     }
     for (; i < hi; i += 32) {
         tuple_v t = ld_stream(in + i);
-        if (MIX) t.x = mix_key(t.x, bits, kMixMul);
+        if (MIX) t.x = mix_key(t.x, bits);
         atomicAdd(&sh_hist[t.x & mask], 1u);
         atomicAdd(&wsub[(uint32_t)t.x & m1], 1u);
         if (BUILD) kor |= t.x;
@@ -561,7 +561,7 @@ __device__ __forceinline__ unsigned digit_peers_n(uint32_t d, int nbits) {
 }
 
 // The pass that reads the relations takes mix_key for the key; words only occur later.
-__device__ __forceinline__ void elem_mix(tuple_v &v, int bits) { v.x = mix_key(v.x, bits, kMixMul); }
+__device__ __forceinline__ void elem_mix(tuple_v &v, int bits) { v.x = mix_key(v.x, bits); }
 __device__ __forceinline__ void elem_mix(unsigned long long &, int) {}
 
 // Digit of an element in this pass: (key >> shift) & mask; a word holds key >> b1, which is pass 2's shift.

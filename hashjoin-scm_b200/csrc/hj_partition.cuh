@@ -202,15 +202,16 @@ struct ChunkGeom {
 };
 
 // The key that a pass partitions by and stores where the geometry says so (RadixGeom::mix): the low `bits` bits
-// changed by a multiplicative hash of those above, which stay, so equal keys stay equal, distinct ones distinct, 0
+// changed by a hash of those above, which stay, so equal keys stay equal, distinct ones distinct, 0
 // stays 0, and a run of 2^bits consecutive keys still takes every digit once. Keys with a stride, or with their
 // ids in the high half, then spread over the partitions evenly (strides of 1..64 and of powers of 2 and 10 up to
-// 2^43, 2^20 to 2^24 keys: the largest partition at most 1.25 times the average), where their own low bits put them into a few that no longer fit
-// shared memory. mul: kMixMul, or 0 for the key itself. The multiplier is unrelated to those of the joins'
-// tables, which hash the same bits.
-constexpr unsigned long long kMixMul = 0xd6e8feb86659fd93ull;
-__host__ __device__ __forceinline__ unsigned long long mix_key(unsigned long long key, int bits, unsigned long long mul) {
-    return key ^ (((key >> bits) * mul) >> (64 - bits));
+// 2^43, 2^20 to 6e6 keys: the largest partition at most 1.11 times the average), where their own low bits put them
+// into a few that no longer fit shared memory. Two 32-bit products (a 64-bit one costs the one-pass scatter 6%,
+// these 4%), with odd multipliers taken for that evenness out of a dozen pairs, and because the runs that such keys
+// make in the joins' tables, which hash the same bits, stay below 13 slots (others: up to 135).
+constexpr uint32_t kMixLow = 0x7feb352du, kMixHigh = 0x846ca68bu;
+__device__ __forceinline__ unsigned long long mix_key(unsigned long long key, int bits) {
+    return key ^ ((((uint32_t)key >> bits) * kMixLow + (uint32_t)(key >> 32) * kMixHigh) >> (32 - bits));
 }
 
 __device__ __forceinline__ uint64_t ld_u64_pair(const uint32_t *p) {
@@ -383,7 +384,6 @@ __device__ __forceinline__ void plan_body(const PlanArgs &a, const uint32_t *tot
 struct SingleArgs {
     const tuple_v *R, *S;
     uint64_t nR, nS;
-    unsigned long long mul;  // mix_key's multiplier
     int bits;                // P = 2^bits partitions
     int copies;              // count: histograms per CTA (its warps spread over them)
     uint32_t *hist;          // [2][G][P]: rows of R, rows of S; exclusive prefixes after single_plan

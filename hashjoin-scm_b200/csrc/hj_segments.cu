@@ -278,7 +278,7 @@ __global__ void __launch_bounds__(THREADS, kSegCtasPerSm) seg_pass1_kernel(SegAr
 #pragma unroll
             for (int i = 0; i < ITEMS; i++) {
                 v[i] = buf[w * 32 * ITEMS + i * 32 + lane];
-                if (MIX) v[i].x = mix_key(v[i].x, a.bits, kMixMul);
+                if (MIX) v[i].x = mix_key(v[i].x, a.bits);
                 const uint32_t d = (uint32_t)v[i].x & dmask;
                 if (!st) rk[i] = atomicAdd(&thist[d], 1u);
                 const uint32_t bin = (uint32_t)(v[i].x & bmask);
@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(THREADS, kSegCtasPerSm) seg_pass1_kernel(SegAr
                 const uint32_t idx = (uint32_t)(w * 32 * ITEMS + i * 32 + lane);
                 if (idx < cnt) {
                     v[i] = buf[idx];
-                    if (MIX) v[i].x = mix_key(v[i].x, a.bits, kMixMul);
+                    if (MIX) v[i].x = mix_key(v[i].x, a.bits);
                     const uint32_t d = (uint32_t)v[i].x & dmask;
                     if (!st) rk[i] = atomicAdd(&thist[d], 1u);
                     const uint32_t bin = (uint32_t)(v[i].x & bmask);

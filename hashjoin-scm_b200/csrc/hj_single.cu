@@ -1,4 +1,4 @@
-// hj_single.cu - the one-pass partition phase of radix joins whose build relation needs at most 2^12
+// hj_single.cu - the one-pass partition phase of radix joins whose build relation needs at most 2^11
 // partitions.
 //
 // The number of radix bits a caller asks for (NUM_RADIX_BITS, 14 by default) fits build relations of
@@ -55,7 +55,8 @@ __device__ __forceinline__ tuple_v ld_twice(const tuple_v *p) {
 //    the shared-memory increments return nothing. With few partitions the warps spread over `copies`
 //    histograms, since 32 lanes on a handful of counters serialise.
 // ------------------------------------------------------------------------------------------------
-template <bool MULTI>
+// MIX (always in a wave): digits of mix_key.
+template <bool MULTI, bool MIX>
 __global__ void __launch_bounds__(kCountThreads, 1) single_count(SingleArgs a0, MultiRef mr) {
     extern __shared__ uint32_t sh[];  // [copies][P]
     __shared__ SingleArgs s_a;
@@ -91,14 +92,14 @@ __global__ void __launch_bounds__(kCountThreads, 1) single_count(SingleArgs a0, 
             for (int u = 0; u < U; u++) t[u] = ld_twice(in + i + u * kCountThreads);
 #pragma unroll
             for (int u = 0; u < U; u++) {
-                atomicAdd(&mine[(uint32_t)mix_key(t[u].x, a.bits, a.mul) & mask], 1u);
+                atomicAdd(&mine[(uint32_t)(MIX ? mix_key(t[u].x, a.bits) : t[u].x) & mask], 1u);
                 kor |= t[u].x;
                 ror |= t[u].y;
             }
         }
         for (; i < hi; i += kCountThreads) {
             const tuple_v t = ld_twice(in + i);
-            atomicAdd(&mine[(uint32_t)mix_key(t.x, a.bits, a.mul) & mask], 1u);
+            atomicAdd(&mine[(uint32_t)(MIX ? mix_key(t.x, a.bits) : t.x) & mask], 1u);
             kor |= t.x;
             ror |= t.y;
         }
@@ -283,8 +284,9 @@ __device__ __forceinline__ uint32_t place_scan(uint32_t v, uint32_t *tmp) {
     return __reduce_add_sync(0xffffffffu, lane < w ? tmp[lane] : 0u) + x - v;
 }
 
-// Place one relation's range. A function of its own per mode: inlined side by side the modes spilled.
-template <int MODE>
+// Place one relation's range. A function of its own per mode: inlined side by side the modes spilled. MIX: the key
+// becomes mix_key when it is staged.
+template <int MODE, bool MIX>
 __device__ __noinline__ void single_scatter_rel(const SingleArgs &a, int rel, uint32_t blk, uint32_t G) {
     using Elem = SingleElem<MODE>;
     using E = typename Elem::Staged;
@@ -333,7 +335,7 @@ __device__ __noinline__ void single_scatter_rel(const SingleArgs &a, int rel, ui
         uint32_t rk[ITEMS / 2];  // ranks, two 16-bit ones per word
 #pragma unroll
         for (int q = 0; q < ITEMS; q++) {
-            t[q].x = mix_key(t[q].x, bits, a.mul);
+            if (MIX) t[q].x = mix_key(t[q].x, bits);
             v[q] = Elem::stage(t[q], lo + base + q * NT + tid, bits, mask, z0);
             uint32_t r = 0;
             if (q * NT + tid < m) r = atomicAdd(&cnt[Elem::digit(v[q], mask)], 1u);
@@ -387,7 +389,7 @@ __device__ __noinline__ void single_scatter_rel(const SingleArgs &a, int rel, ui
     __syncthreads();
 }
 
-template <bool MULTI>
+template <bool MULTI, bool MIX>
 __global__ void __launch_bounds__(kPlaceThreads, 1) single_scatter(SingleArgs a0, MultiRef mr) {
     __shared__ SingleArgs s_a;
     uint32_t blk = blockIdx.x, G = gridDim.x;
@@ -405,15 +407,15 @@ __global__ void __launch_bounds__(kPlaceThreads, 1) single_scatter(SingleArgs a0
     for (int rel = 1; rel >= 0; rel--) {
         if (rel == 0 && a.lp) {
             if (ci)
-                single_scatter_rel<kModePosWord>(a, rel, blk, G);
+                single_scatter_rel<kModePosWord, MIX>(a, rel, blk, G);
             else
-                single_scatter_rel<kModePos>(a, rel, blk, G);
+                single_scatter_rel<kModePos, MIX>(a, rel, blk, G);
         } else if (narrow) {
-            single_scatter_rel<kModeWord>(a, rel, blk, G);
+            single_scatter_rel<kModeWord, MIX>(a, rel, blk, G);
         } else if (ci) {
-            single_scatter_rel<kModeTupleWord>(a, rel, blk, G);
+            single_scatter_rel<kModeTupleWord, MIX>(a, rel, blk, G);
         } else {
-            single_scatter_rel<kModeTuple>(a, rel, blk, G);
+            single_scatter_rel<kModeTuple, MIX>(a, rel, blk, G);
         }
     }
 }
@@ -444,10 +446,10 @@ uint32_t single_grid(size_t nR, size_t nS, int num_sms) {
     } while (0)
 
 int single_prepare_device() {
-    HJ_CU(cudaFuncSetAttribute(single_scatter<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)single_scatter_smem(kSingleMaxBits)));
-    HJ_CU(cudaFuncSetAttribute(single_scatter<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)single_scatter_smem(kSingleMaxBits)));
+    const int most = (int)single_scatter_smem(kSingleMaxBits);
+    HJ_CU(cudaFuncSetAttribute(single_scatter<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    HJ_CU(cudaFuncSetAttribute(single_scatter<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    HJ_CU(cudaFuncSetAttribute(single_scatter<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     return HJ_OK;
 }
 
@@ -461,7 +463,6 @@ void single_args(const RadixGeom &g, bool lp, bool skip0, bool ci_ok, const ulon
     a.S = S;
     a.nR = nR;
     a.nS = nS;
-    a.mul = g.mix ? kMixMul : 0;
     a.bits = g.bits;
     a.copies = single_copies(g.bits);
     a.hist = s.chunk_hist;
@@ -506,11 +507,17 @@ int single_partition_enqueue(const RadixGeom &g, bool lp, bool skip0, bool ci_ok
     PlanArgs pa;
     single_args(g, lp, skip0, ci_ok, R, nR, S, nS, s, acc, clear_acc, agg_ok, &a, &pa);
     const MultiRef none = {};
-    single_count<false><<<G, kCountThreads, (size_t)a.copies * P * 4, st>>>(a, none);
+    if (g.mix)
+        single_count<false, true><<<G, kCountThreads, (size_t)a.copies * P * 4, st>>>(a, none);
+    else
+        single_count<false, false><<<G, kCountThreads, (size_t)a.copies * P * 4, st>>>(a, none);
     if (ph) HJ_CU(record_event(ph[1], st));
     single_plan<false><<<(2 * P + 31) / 32, 1024, (size_t)2 * P * 4, st>>>(a, pa, G, none);
     if (ph) HJ_CU(record_event(ph[2], st));
-    single_scatter<false><<<G, kPlaceThreads, single_scatter_smem(g.bits), st>>>(a, none);
+    if (g.mix)
+        single_scatter<false, true><<<G, kPlaceThreads, single_scatter_smem(g.bits), st>>>(a, none);
+    else
+        single_scatter<false, false><<<G, kPlaceThreads, single_scatter_smem(g.bits), st>>>(a, none);
     HJ_CU(cudaGetLastError());
     if (ph) {
         HJ_CU(record_event(ph[3], st));
@@ -525,9 +532,9 @@ int multi_partition_launch(const MultiJob *jobs, const uint2 *part_map, unsigned
     const SingleArgs none_a = {};
     const PlanArgs none_p = {};
     const MultiRef part = {jobs, part_map}, plan = {jobs, plan_map};
-    single_count<true><<<part_blocks, kCountThreads, kCountSmem, st>>>(none_a, part);
+    single_count<true, true><<<part_blocks, kCountThreads, kCountSmem, st>>>(none_a, part);
     single_plan<true><<<plan_blocks, 1024, (size_t)8 << max_bits, st>>>(none_a, none_p, 0, plan);
-    single_scatter<true><<<part_blocks, kPlaceThreads, single_scatter_smem(max_bits), st>>>(none_a, part);
+    single_scatter<true, true><<<part_blocks, kPlaceThreads, single_scatter_smem(max_bits), st>>>(none_a, part);
     HJ_CU(cudaGetLastError());
     *launches += 3;
     return HJ_OK;

@@ -1,10 +1,11 @@
-// hj_wave.cuh - waves of non-partitioned joins.
+// hj_wave.cuh - waves: many independent joins with one launch per step over flat lists of (join, range) items, so
+// that the launch count does not grow with the number of joins.
 //
-// A wave runs many independent joins, each with its own global hash table, with one multi-join build
-// kernel and one multi-join probe kernel over flat lists of (join, range) chunks, so the launch count
-// does not grow with the number of joins. Batches (hj_batch.cu) pack their small joins into waves at
-// plan time; the join server (hj_server.cu) forms a wave from the small requests queued at each
-// dispatch (continuous batching).
+// Two forms. In the first (MJob, WaveDev) each join has its own global hash table: one multi-join build kernel
+// and one multi-join probe kernel. In the second (WaveJoin, WavePlan, below) joins have no global table: shared-memory
+// tables for small build sides, the one-pass radix pipeline for the others. Batches (hj_batch.cu) pack their joins
+// into waves at plan time, of the first form only when the second's scratch cannot be had; the join server
+// (hj_server.cu) forms a wave from the requests queued at each dispatch (continuous batching).
 #pragma once
 
 #include <cuda_runtime.h>

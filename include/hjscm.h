@@ -90,7 +90,8 @@ typedef struct {
     double table_load;    /* NPHJ global table load factor; 0 selects 0.4 for build relations of up to
                              5 M tuples (about L2-sized tables, where shorter probe chains pay) and 0.5
                              above, and lets the join run a radix pipeline at sizes where that is faster
-                             (same result); a value > 0 asks for the table */
+                             (same result); a value > 0 asks for the table (build relations of at most
+                             8192 tuples run as one kernel all the same) */
     int radix_bits_pass1; /* two passes: bits of pass 1 (NUM_RADIX_BITS_PASS1 of phj_asymm_radix,
                              src/algo/phj_asymm_radix.h:10-19); 0 selects bits / 2. Clamped to the
                              split where each pass has 1..8 bits. */
@@ -104,7 +105,10 @@ typedef struct {
 #define HJ_F_PHASE_TIMES 0x4u /* also time each kernel group (fills hj_result_t.phase) */
 /* A radix join takes the shortest pipeline that its sizes allow, whatever num_radix_bits and num_passes ask
  * for: at most 8192 build tuples one kernel, then one partition pass over the fewest bits that bring build
- * partitions to shared-memory size (up to 11 bits), then two passes with the bits asked for or fewer. The
+ * partitions to shared-memory size (up to 11 bits), then two passes with the bits asked for or fewer. With fewer bits
+ * than asked for and more than 2^21 build tuples the partitions are those of a mixed key, so that keys which share
+ * low bits still spread; up to 2^21 they are the key's low bits, and the join runs again by the mixed key when most
+ * of the build side falls into partitions beyond shared memory (both runs are one join, its times include both). The
  * flags HJ_F_SEGMENTS, HJ_F_EXACT, HJ_F_WIDE and HJ_F_WORDS name a two-pass pipeline and run it as asked.
  * Radix joins in two passes of <= 14 bits from 2^26 tuples run in segment mode: pass 1 writes chains of
  * fixed-size segments and counts the histograms itself, so no histogram pass reads the relations first
@@ -160,9 +164,10 @@ typedef struct {
     double retrieve;           /* materialising joins: seconds of the retrieve phase (included in total) */
 } hj_result_t;
 
-/* hj_result_t.flags: the last partition pass stored the final partitions as 8-byte words
- * (key >> radix bits) << 32 | row id, which the joins read (radix joins without per-match output and
- * without the key-0 rule, when every build key >> radix bits is below 2^31 and every row id below 2^32). */
+/* hj_result_t.flags: the widths allow final partitions of 8-byte words (key >> radix bits) << 32 | row id: every
+ * build key >> num_radix_bits below 2^31 and every row id below 2^32 (radix joins without per-match output). Two
+ * passes with the bits asked for store and read them then; with fewer bits, or in one kernel, the keys may have to
+ * be narrower by the difference for that, and the flag still tells about num_radix_bits. */
 #define HJ_RES_COMPACT_PARTITIONS 0x1u
 /* hj_result_t.flags: segment mode stored the pass-1 chains as 8-byte words (key >> pass-1 bits) << 32 |
  * row id as well (every build key >> pass-1 bits below 2^31, every row id below 2^32), so pass 1 wrote

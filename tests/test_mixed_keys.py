@@ -1,5 +1,5 @@
 """mix_key, the key that joins partition by where its own low bits are not taken as they are: restated from the kernels'
-header, with the multiplier read from it. Bijective for every number of radix bits, 0 stays 0, the high bits stay,
+header, with the multipliers read from it. Bijective for every number of radix bits, 0 stays 0, the high bits stay,
 and keys with structure spread evenly over the partitions."""
 import pathlib
 import re
@@ -8,12 +8,15 @@ import numpy as np
 import pytest
 
 HEADER = pathlib.Path(__file__).resolve().parents[1] / "hashjoin-scm_b200" / "csrc" / "hj_partition.cuh"
-MUL = np.uint64(int(re.search(r"kMixMul = (0x[0-9a-f]+)ull", HEADER.read_text()).group(1), 16))
+LOW, HIGH = (np.uint64(int(x, 16)) for x in
+             re.search(r"kMixLow = (0x[0-9a-f]+)u, kMixHigh = (0x[0-9a-f]+)u", HEADER.read_text()).groups())
+U32 = np.uint64(0xFFFFFFFF)
 
 
 def mix(key, bits):
+    low, high = (key & U32) >> np.uint64(bits), key >> np.uint64(32)
     with np.errstate(over="ignore"):
-        return key ^ (((key >> np.uint64(bits)) * MUL) >> np.uint64(64 - bits))
+        return key ^ (((low * LOW + high * HIGH) & U32) >> np.uint64(32 - bits))
 
 
 @pytest.mark.parametrize("bits", range(1, 16))
@@ -29,7 +32,7 @@ def test_bijective(bits):
     assert np.array_equal(np.sort(run), np.arange(1 << bits, dtype=np.uint64))  # a run takes every digit once
 
 
-@pytest.mark.parametrize("bits,n", [(4, 90_000), (8, 1 << 20), (10, 1 << 22), (11, 6_000_000)])
+@pytest.mark.parametrize("bits,n", [(4, 90_000), (8, 1 << 20), (10, 1 << 22), (11, 6_000_000), (12, 1 << 24)])
 @pytest.mark.parametrize("stride", [1, 2, 3, 4, 10, 16, 60, 100, 1000, 1 << 11, 1 << 14, 10**6, 10**7, 1 << 20, 1 << 32, 3 << 32, 1 << 40])
 def test_even_partitions(bits, n, stride):
     """The largest partition stays within shared memory's 10240 tuples where the average is 6144 at most."""
