@@ -1111,6 +1111,10 @@ __device__ __forceinline__ void join_finish(const JoinArgs &a, bool ci) {
     a.acc->dup_flag = a.acc->error = 0;
 }
 
+// Large-partition steps 0 (clear) and 1 (build) of a wave's job, by the blocks of its partition joins, which come as
+// two launches (one per element layout): the first clears, the second builds, multi_large probes.
+__device__ __noinline__ void multi_large_step(const JoinArgs &a, int step, uint32_t blk, uint32_t nblk);
+
 // Partition join over compact words in an open-addressing table of the words themselves (every match
 // counted): two CTAs of 512 threads per SM with 13312 slots each. A probe is one 8-byte shared load when its
 // key sits in its first slot and the build saw no key twice, where a chain costs a head, a word and a link.
@@ -1203,6 +1207,7 @@ __global__ void __launch_bounds__(kCompactThreads, 2) join_words_kernel(JoinArgs
         const uint2 e = mr.map[blockIdx.x];
         multi_copy(&s_a, &mr.jobs[e.x].ja);
         __syncthreads();
+        multi_large_step(s_a, 0, e.y, mr.jobs[e.x].join_blocks);
     }
     const JoinArgs &a = MULTI ? s_a : a0;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -1424,6 +1429,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_words_kernel(JoinA
         const uint2 e = mr.map[blockIdx.x];
         multi_copy(&s_a, &mr.jobs[e.x].ja);
         __syncthreads();
+        multi_large_step(s_a, 0, e.y, mr.jobs[e.x].join_blocks);
     }
     const JoinArgs &a = MULTI ? s_a : a0;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -1591,6 +1597,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_kernel(JoinArgs a0
         const uint2 e = mr.map[blockIdx.x];
         multi_copy(&s_a, &mr.jobs[e.x].ja);
         __syncthreads();
+        multi_large_step(s_a, 1, e.y, mr.jobs[e.x].join_blocks);
     }
     const JoinArgs &a = MULTI ? s_a : a0;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -1783,6 +1790,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_small_kernel(JoinArgs a0
         const uint2 e = mr.map[blockIdx.x];
         multi_copy(&s_a, &mr.jobs[e.x].ja);
         __syncthreads();
+        multi_large_step(s_a, 1, e.y, mr.jobs[e.x].join_blocks);
     }
     const JoinArgs &a = MULTI ? s_a : a0;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -2262,27 +2270,32 @@ __global__ void join_large_probe(JoinArgs a) {
     large_probe<MAT>(a, blockIdx.x, gridDim.x);
 }
 
-// The large-partition steps of a wave of joins, over a map of (job, block) as its other steps: a block of a job
-// without large partitions returns at once. (With one block per job a batch of four
-// 2^21 x 2^23 joins whose partitions were all large took 98.7 ms, one with a hot build key in each 10.3.) Step 2
+__device__ __noinline__ void multi_large_step(const JoinArgs &a, int step, uint32_t blk, uint32_t nblk) {
+    if (!a.counters[kCtrNLarge]) return;
+    if (step == 0)
+        large_clear(a, blk, nblk);
+    else
+        large_build(a, blk, nblk);
+    __syncthreads();
+}
+
+// The last large-partition step of a wave of joins, the probe, over a map of (job, block) as its other steps: a block
+// of a job without large partitions returns at once. (With one block per job for all three steps a batch of four
+// 2^21 x 2^23 joins whose partitions were all large took 98.7 ms, one with a hot build key in each 10.3.) It also
 // hands over the error word.
-template <int STEP>
 __global__ void __launch_bounds__(kMultiLargeThreads) multi_large(MultiRef mr) {
     const uint2 e = mr.map[blockIdx.x];
     const MultiJob &job = mr.jobs[e.x];
     const bool any = job.ja.counters[kCtrNLarge] != 0;
-    if (!any && (STEP != 2 || e.y != 0)) return;
+    if (!any && e.y != 0) return;
     __shared__ JoinArgs a;
-    const uint32_t nblk = job.large_blocks;
     multi_copy(&a, &job.ja);
     __syncthreads();
     if (any) {
-        if (STEP == 0) large_clear(a, e.y, nblk);
-        if (STEP == 1) large_build(a, e.y, nblk);
-        if (STEP == 2) large_probe<false>(a, e.y, nblk);
+        large_probe<false>(a, e.y, job.large_blocks);
         __syncthreads();
     }
-    if (STEP == 2 && threadIdx.x == 0) {
+    if (threadIdx.x == 0) {
         const uint32_t err = *reinterpret_cast<const volatile uint32_t *>(&a.counters[kCtrErr]);
         if (err) atomicOr(&a.acc->error, err);
     }
@@ -2674,10 +2687,8 @@ int multi_join_launch(const MultiJob *jobs, const uint2 *every_map, unsigned eve
         join_first_kernel<false, true><<<first_blocks, kJoinThreads, kFirstSmem, st>>>(none, first);
         *launches += 2;
     }
-    multi_large<0><<<large_blocks, kMultiLargeThreads, 0, st>>>(large);
-    multi_large<1><<<large_blocks, kMultiLargeThreads, 0, st>>>(large);
-    multi_large<2><<<large_blocks, kMultiLargeThreads, 0, st>>>(large);
-    *launches += 3;
+    multi_large<<<large_blocks, kMultiLargeThreads, 0, st>>>(large);
+    *launches += 1;
     HJ_CU(cudaGetLastError());
     return HJ_OK;
 }

@@ -433,8 +433,8 @@ struct MultiJob {
     JoinArgs ja;
     uint32_t grid;         // blocks of the count and the scatter
     uint32_t plan_blocks;  // blocks of the plan
-    uint32_t large_blocks; // blocks of the large-partition steps
-    uint32_t pad;
+    uint32_t join_blocks;  // blocks of the partition joins
+    uint32_t large_blocks; // blocks of the large-partition probe
 };
 constexpr int kMultiLargeThreads = 256;
 static_assert(sizeof(MultiJob) % 8 == 0 && sizeof(SingleArgs) % 8 == 0 && sizeof(PlanArgs) % 8 == 0 &&

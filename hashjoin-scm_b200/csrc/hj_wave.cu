@@ -64,7 +64,7 @@ uint32_t join_blocks(const WaveJoin &j, const Pieces &pc, int num_sms) {
     return blocks((uint64_t)j.nR + j.nS, pc.join, 2 * (uint32_t)num_sms);
 }
 
-// Blocks of a join's large-partition steps, which return at once for most joins: few, up to what fills the GPU.
+// Blocks of a join's large-partition probe, which return at once for most joins: few, up to what fills the GPU.
 uint32_t large_blocks(const WaveJoin &j, int num_sms) {
     return blocks((uint64_t)j.nR + j.nS, kWavePartTuples, 4 * (uint32_t)num_sms);
 }
@@ -154,9 +154,10 @@ int wave_image(const WaveJoin *joins, size_t n, int num_sms, const WavePlan &wp,
         m.plan_blocks = (2u * (unsigned)g.F1 + 31) / 32;
         for (uint32_t b = 0; b < G; b++) part[npt++] = make_uint2(nj, b);
         for (uint32_t b = 0; b < m.plan_blocks; b++) plan[npl++] = make_uint2(nj, b);
+        m.join_blocks = join_blocks(j, pc, num_sms);
         m.large_blocks = large_blocks(j, num_sms);
         for (uint32_t b = 0; b < m.large_blocks; b++) large[nl++] = make_uint2(nj, b);
-        const uint32_t jb = join_blocks(j, pc, num_sms);
+        const uint32_t jb = m.join_blocks;
         for (uint32_t b = 0; b < jb; b++) {
             if (j.lp)
                 first[nf++] = make_uint2(nj, b);
