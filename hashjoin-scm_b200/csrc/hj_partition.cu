@@ -897,12 +897,13 @@ __device__ __forceinline__ tuple_v fin_r(const JoinArgs &a, bool ci, uint64_t i)
     return a.finR[i];
 }
 
-// Chain head of a key among 2^nb_log (1..14) in shared memory: hashed, since a partition's keys may share the low
-// bits above the radix bits too (as for the large partitions' tables). Two 32-bit products: the radix bits, equal
-// in a partition, only shift the result, so they need not be shifted out (a 64-bit product of the shifted key
-// cost hr joins of 3e6 x 12e6 sparse keys 1.7%).
-__device__ __forceinline__ uint32_t head_of(unsigned long long key, uint32_t nb_log) {
-    return ((uint32_t)key * 0x9e3779b1u + (uint32_t)(key >> 32) * 0x85ebca6bu) >> (32 - nb_log);
+// Chain head among 2^nb_log (1..14) in shared memory of a key's bits above the radix bits: the low ones, changed by
+// a hash of those above (as mix_key), since a partition's keys may share those low bits too. Runs of keys keep a head
+// each, as without the hash (a hash of all bits cost dense keys in 16-byte tuples 3.5%).
+__device__ __forceinline__ uint32_t head_of(unsigned long long high, uint32_t nb_log) {
+    const uint32_t lo = (uint32_t)high;
+    return (lo ^ (((lo >> nb_log) * 0x9e3779b1u + (uint32_t)(high >> 32) * 0x85ebca6bu) >> (32 - nb_log))) &
+           ((1u << nb_log) - 1u);
 }
 // log2 of the number of heads for nr build tuples: the next power of two, times two if `twice`, at least 2.
 __device__ __forceinline__ uint32_t heads_log(uint32_t nr, bool twice, uint32_t max_log) {
@@ -1615,6 +1616,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_kernel(JoinArgs a0
     unsigned int *err = &a.counters[kCtrErr];
     const uint32_t nitems = a.counters[kCtrNItems];
     if (a.ci && ci_applies(a.counters, a.bits)) return;  // join_first_words_kernel
+    const int B = a.bits;
     const bool skip0 = a.skip0 != 0;
     unsigned long long cnt = 0, sum = 0;
     bool multi = false;
@@ -1666,7 +1668,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_kernel(JoinArgs a0
         for (uint32_t i = tid; i < nr; i += kJoinThreads) {
             const unsigned long long k = kx[i];
             if (skip0 && k == 0) continue;
-            const uint32_t h = head_of(k, nb_log), shift = (h & 1) * 16;
+            const uint32_t h = head_of(k >> B, nb_log), shift = (h & 1) * 16;
             uint32_t *word = head32 + (h >> 1);
             uint32_t old = *reinterpret_cast<volatile uint32_t *>(word);
             for (;;) {  // lock-free: a failed CAS means another thread's succeeded
@@ -1740,7 +1742,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_kernel(JoinArgs a0
             for (int u = 0; u < UP; u++) {
                 best[u] = 0;
                 if (base + u * kJoinThreads + tid >= ns) continue;
-                uint32_t e = head[head_of(sv[u].x, nb_log)], steps = 0, nm = 0, bp = 0;
+                uint32_t e = head[head_of(sv[u].x >> B, nb_log)], steps = 0, nm = 0, bp = 0;
                 while (e) {
                     if (kx[e - 1] == sv[u].x) {
                         const uint32_t p = pos[e - 1];
@@ -1814,6 +1816,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_small_kernel(JoinArgs a0
     // Compiled once per partition layout; only the launch matching the device's choice runs.
     if (CI != (a.ci && ci_applies(a.counters, a.bits))) return;
     constexpr bool ci = CI;
+    const int B = ci ? 0 : a.bits;  // shift from a stored x to the key's bits above the radix bits
     const bool lp = a.lp != 0;
     const bool skip0 = a.skip0 != 0;
     // Items [0, nA) went to the compact kernel if the build side's keys and row ids fit it.
@@ -1877,7 +1880,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_small_kernel(JoinArgs a0
         for (uint32_t i = tid; i < nr; i += kJoinThreads) {
             const uint64_t k = rt[i].x;
             if (skip0 && k == 0 && (!ci || item.part0)) continue;
-            const uint32_t h = head_of(k, nb_log);
+            const uint32_t h = head_of(k >> B, nb_log);
             nxt[i] = (uint16_t)atomic_exch_u16(&head[h], i + 1);
         }
         __syncthreads();
@@ -1896,7 +1899,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_small_kernel(JoinArgs a0
                     mm[u] = best[u] = 0;
                     if (base + u * kJoinThreads + tid >= ns) continue;
                     const uint64_t k = sv[u].x;
-                    uint32_t e = head[head_of(k, nb_log)], steps = 0;
+                    uint32_t e = head[head_of(k >> B, nb_log)], steps = 0;
                     while (e) {
                         if (rt[e - 1].x == k) {
                             if (!lp) mm[u]++;
@@ -1921,7 +1924,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_small_kernel(JoinArgs a0
                         continue;
                     }
                     const uint64_t k = sv[u].x;
-                    uint32_t e = head[head_of(k, nb_log)], steps = 0;
+                    uint32_t e = head[head_of(k >> B, nb_log)], steps = 0;
                     while (e && steps++ <= nr) {
                         if (rt[e - 1].x == k) mat_put(a.mat, o++, rt[e - 1].y, sv[u].y, err);
                         e = nxt[e - 1];
@@ -1941,7 +1944,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_small_kernel(JoinArgs a0
                 const uint32_t j = j0 + u * kJoinThreads;
                 if (j >= ns) continue;
                 const uint64_t k = s[u].x;
-                uint32_t e = head[head_of(k, nb_log)];
+                uint32_t e = head[head_of(k >> B, nb_log)];
                 uint32_t best = 0, nm = 0;
                 uint32_t steps = 0;
                 while (e) {
