@@ -681,7 +681,11 @@ __global__ void mat_retrieve(const ulonglong2 *__restrict__ pairs, const unsigne
     if ((threadIdx.x & 31) == 0 && sum) atomicAdd(&acc->checksum, sum);
 }
 
-constexpr size_t kMatColumnsFrom = 64u << 20;  // bytes of both relations
+// Columns pay from relations that no longer fit L2 on, while the build side's column is not far beyond it (retrieve
+// phase, columns and not: 2^24 x 2^27 4.08 / 5.33 ms, 2^25 x 2^27 5.34 / 6.08, 2^26 x 2^28 12.5 / 12.9, 2^27 x 2^28
+// 14.0 / 13.4, 2^27 x 2^29 27.8 / 26.9).
+constexpr size_t kMatColumnsFrom = 64u << 20;       // bytes of both relations
+constexpr size_t kMatColumnsMaxBuild = 1u << 26;
 
 // Default load factor of the global table: 0.4 for build relations up to 5 M tuples, 0.5 above. Below
 // that size the table is about the size of L2 and shorter probe chains pay for the larger table
@@ -845,9 +849,8 @@ int nphj_enqueue(bool lp, bool skip0, const ulonglong2 *R, size_t nR, const ulon
 int mat_retrieve_enqueue(const ulonglong2 *pairs, const unsigned long long *n_dev, unsigned long long cap,
                          const ulonglong2 *R, size_t nR, const ulonglong2 *S, size_t nS, void *scratch,
                          size_t scratch_bytes, JoinAccum *acc, cudaStream_t st, int num_sms, uint32_t *launches) {
-    // Columns pay once the relations no longer fit L2, if the scratch holds them.
     uint32_t *colR = nullptr, *colS = nullptr;
-    if ((nR + nS) * 16 > kMatColumnsFrom && (nR + nS) * 4 <= scratch_bytes) {
+    if ((nR + nS) * 16 > kMatColumnsFrom && nR <= kMatColumnsMaxBuild && (nR + nS) * 4 <= scratch_bytes) {
         colR = reinterpret_cast<uint32_t *>(scratch);
         colS = colR + nR;
         mat_columns<<<num_sms * 4, 512, 0, st>>>(n_dev, cap, R, nR, S, nS, colR, colS, acc);

@@ -122,3 +122,20 @@ def test_retrieve_of_few_pairs(hj, cuda, algo, pairs):
     assert all((r.matched_cnt, r.checksum) == (pairs, want) for r in res)
     if pairs <= 1:
         assert min(r.retrieve for r in res) < 25e-6
+
+
+@pytest.mark.parametrize("nR", [1 << 26, (1 << 26) + 1])
+def test_retrieve_around_the_largest_columns(hj, cuda, nR):
+    nS = 1 << 26
+    R, S = (cuda.empty((n, 2), dtype=cuda.int64, device="cuda") for n in (nR, nS))
+    g = cuda.Generator(device="cuda")
+    g.manual_seed(3)
+    R[:, 0] = cuda.randperm(nR, generator=g, device="cuda")
+    S[:, 0] = cuda.randint(0, nR, (nS,), generator=g, device="cuda")
+    R[:, 1], S[:, 1] = cuda.arange(1, nR + 1, device="cuda"), cuda.arange(1, nS + 1, device="cuda")
+    rid = cuda.empty(nR, dtype=cuda.int64, device="cuda")
+    rid[R[:, 0]] = R[:, 1]
+    want = int(rid[S[:, 0]].sum()) + nS * (nS + 1) // 2
+    del rid
+    r = hj.join_mat("phj_radix_bc", R, S, on_device=True)
+    assert (r.matched_cnt, r.checksum) == (nS, want)
