@@ -897,13 +897,14 @@ __device__ __forceinline__ tuple_v fin_r(const JoinArgs &a, bool ci, uint64_t i)
     return a.finR[i];
 }
 
-// Chain head among 2^nb_log (1..14) in shared memory of a key's bits above the radix bits: the low ones, changed by
-// a hash of those above (as mix_key), since a partition's keys may share those low bits too. Runs of keys keep a head
-// each, as without the hash (a hash of all bits cost dense keys in 16-byte tuples 3.5%).
-__device__ __forceinline__ uint32_t head_of(unsigned long long high, uint32_t nb_log) {
-    const uint32_t lo = (uint32_t)high;
-    return (lo ^ (((lo >> nb_log) * 0x9e3779b1u + (uint32_t)(high >> 32) * 0x85ebca6bu) >> (32 - nb_log))) &
-           ((1u << nb_log) - 1u);
+// Chain head among 2^nb_log (1..14) in shared memory of a key's bits above the B lowest (the radix bits): the next
+// nb_log bits, changed by a hash of those above (as mix_key), since a partition's keys may share those bits too. Runs
+// of keys keep a head each, as without the hash (a hash of all bits cost dense keys in 16-byte tuples 3.5%). Four
+// dependent instructions: a probe waits for them.
+__device__ __forceinline__ uint32_t head_of(unsigned long long key, int B, uint32_t nb_log) {
+    const uint32_t lo = (uint32_t)key, hi = (uint32_t)(key >> 32);
+    const uint32_t f = ((lo >> (B + nb_log)) * 0x9e3779b1u + hi * 0x85ebca6bu) >> (32 - nb_log);
+    return (__funnelshift_r(lo, hi, B) ^ f) & ((1u << nb_log) - 1u);
 }
 // log2 of the number of heads for nr build tuples: the next power of two, times two if `twice`, at least 2.
 __device__ __forceinline__ uint32_t heads_log(uint32_t nr, bool twice, uint32_t max_log) {
@@ -987,7 +988,7 @@ __global__ void __launch_bounds__(kCompactThreads, 2) join_compact_kernel(JoinAr
                 if (i >= nr) continue;
                 rw[i] = ((t[u].x >> B) << 32) | (t[u].y & 0xffffffffull);
                 if (skip0 && t[u].x == 0 && (!ci || item.part0)) continue;
-                nxt[i] = (uint16_t)atomic_exch_u16(&head[head_of(t[u].x >> B, nb_log)], i + 1);
+                nxt[i] = (uint16_t)atomic_exch_u16(&head[head_of(t[u].x >> B, 0, nb_log)], i + 1);
             }
         }
         __syncthreads();
@@ -1009,7 +1010,7 @@ __global__ void __launch_bounds__(kCompactThreads, 2) join_compact_kernel(JoinAr
                     mm[u] = best[u] = 0;
                     if (base + u * kCompactThreads + tid >= ns) continue;
                     const uint64_t khi = sv[u].x >> B;
-                    uint32_t e = head[head_of(khi, nb_log)], steps = 0;
+                    uint32_t e = head[head_of(khi, 0, nb_log)], steps = 0;
                     while (e) {
                         if ((rw[e - 1] >> 32) == khi) {
                             if (!lp) mm[u]++;
@@ -1034,7 +1035,7 @@ __global__ void __launch_bounds__(kCompactThreads, 2) join_compact_kernel(JoinAr
                         continue;
                     }
                     const uint64_t khi = sv[u].x >> B;
-                    uint32_t e = head[head_of(khi, nb_log)], steps = 0;
+                    uint32_t e = head[head_of(khi, 0, nb_log)], steps = 0;
                     while (e && steps++ <= nr) {
                         const unsigned long long w = rw[e - 1];
                         if ((w >> 32) == khi) mat_put(a.mat, o++, w & 0xffffffffull, sv[u].y, err);
@@ -1057,7 +1058,7 @@ __global__ void __launch_bounds__(kCompactThreads, 2) join_compact_kernel(JoinAr
                 const uint32_t j = j0 + u * kCompactThreads;
                 if (j >= ns) continue;
                 const uint64_t khi = sv[u].x >> B;
-                uint32_t e = head[head_of(khi, nb_log)];
+                uint32_t e = head[head_of(khi, 0, nb_log)];
                 uint32_t best = 0, steps = 0, nm = 0;
                 while (e) {
                     const unsigned long long w = rw[e - 1];
@@ -1579,17 +1580,76 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_words_kernel(JoinA
 // First-match join of the one-pass pipeline over {key, position} elements (wide). The match with the lowest
 // position wins, so the partition may hold them in any order. Key, position and row id in
 // separate arrays (20 bytes per build tuple, 16-bit bucket heads and chains: 215 KB, one CTA per SM);
-// a build tuple's row id is gathered from the build relation once. A build tuple that finds its own key at the
-// head lowers that node's position instead of becoming a node; a partition where that happened has its chains
-// gone over once, a thread per head, which leaves one node per key with its first position and row id, and a bit
-// that there were more. (2^22 x 2^24 tuples of mixed 63-bit keys with 1 / 4 / 1000 a key: 510 / 615 / 18300 us with
-// every duplicate a node, 529 / 542 / 602 now; 2^21 x 2^22 with one key 1000 times and half of the probes on it:
-// 7680 and 203 us, the global table 2040. Looking through the whole chain before each insert: 560 us with 1 a
-// key.) One probe tuple per round, the next one under way (3e6 x 12e6 sparse keys: 166 us; four unrolled: 175).
+// a build tuple's row id is gathered from the build relation once. A build tuple that loses a head to its own key
+// lowers that node's position instead of becoming a node, and flags the partition, which happens where a key is
+// repeated a few dozen times; first_merge then leaves one node per key, with its first position and row id, and a
+// bit that there were more. Fewer duplicates are walked. (2^22 x 2^24 tuples of mixed 63-bit keys, 4 / 1000 a key:
+// 615 / 18300 us with every duplicate walked, 601 / 632 now; 2^21 x 2^22 with one key 1000 times and half of the
+// probes on it: 7680 and 200 us, the global table 2040. Distinct keys, 3e6 x 9e6: 147 and 151 us for this join; a
+// look at the head's key before each insert 163, at the whole chain 170, walks measured in the probe 165.) One
+// probe tuple per round, the next one under way (3e6 x 12e6 sparse keys: 166 us; four unrolled: 175).
 constexpr uint32_t kFirstHeadsLog = 13, kFirstHeads = 1u << kFirstHeadsLog;
 constexpr size_t kFirstSmem = (size_t)kFirstCap * (8 + 8 + 4 + 2) + kFirstHeads * 2 + kFirstCap / 8;
 constexpr uint32_t kFirstMerged = 0x8000;  // nxt of a tuple merged into a node: this bit, and the node's index + 1
 static_assert(kFirstCap < kFirstMerged && kFirstCap % 32 == 0, "an index and the bit fit a link");
+
+struct FirstTable {  // the table of join_first_kernel
+    unsigned long long *kx, *rid;
+    uint32_t *pos, *dup;
+    uint16_t *head, *nxt;
+    uint32_t nr, nb_log;
+    bool skip0;
+};
+
+// One node per key: the others of a chain leave it, and the node takes the first position among them and its row id. A
+// thread per head; all threads of the block, before a probe walks.
+__device__ __noinline__ void first_merge(const FirstTable &t) {
+    unsigned long long *kx = t.kx, *rid = t.rid;
+    uint32_t *pos = t.pos, *dup = t.dup;
+    uint16_t *head = t.head, *nxt = t.nxt;
+    const uint32_t nr = t.nr, nb_log = t.nb_log, tid = threadIdx.x;
+    const bool skip0 = t.skip0;
+    // Row ids of the tuples whose position won, and duplicate bits; then what is left of one key in a
+    // chain (nodes that were not next to each other).
+    for (uint32_t i = tid; i < nr; i += kJoinThreads) {
+        const uint32_t e = nxt[i];
+        if (!(e & kFirstMerged) || (skip0 && kx[i] == 0)) continue;
+        const uint32_t r = (e & (kFirstMerged - 1)) - 1;
+        if (pos[r] == pos[i]) rid[r] = rid[i];
+        atomicOr(&dup[r >> 5], 1u << (r & 31));
+    }
+    __syncthreads();
+    for (uint32_t q = tid; q < 1u << nb_log; q += kJoinThreads) {
+        for (uint32_t r = head[q]; r; r = nxt[r - 1]) {
+            // Take the nodes behind r with its key out of the chain.
+            const unsigned long long k = kx[r - 1];
+            uint32_t prev = r, first = r, fp = pos[r - 1];
+            bool gap = false, any = false;  // any: bits of the nodes taken out pass to r
+            for (uint32_t e = nxt[r - 1], next; e; e = next) {
+                const uint32_t p = pos[e - 1];
+                next = nxt[e - 1];
+                if (kx[e - 1] == k) {
+                    gap = any = true;
+                    if (p < fp) {
+                        fp = p;
+                        first = e;
+                    }
+                } else {
+                    if (gap) nxt[prev - 1] = (uint16_t)e;
+                    gap = false;
+                    prev = e;
+                }
+            }
+            if (gap) nxt[prev - 1] = 0;
+            if (any) {
+                pos[r - 1] = fp;
+                rid[r - 1] = rid[first - 1];
+                atomicOr(&dup[(r - 1) >> 5], 1u << ((r - 1) & 31));
+            }
+        }
+    }
+    __syncthreads();
+}
 
 template <bool MAT, bool MULTI = false>
 __global__ void __launch_bounds__(kJoinThreads, 1) join_first_kernel(JoinArgs a0, MultiRef mr) {
@@ -1641,6 +1701,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_kernel(JoinArgs a0
         tuple_v sv[UP];  // the thread's next probe tuples, under way during the build and the walks before them
 #pragma unroll
         for (int u = 0; u < UP; u++) sv[u] = tid + u * kJoinThreads < ns ? ld_stream(S + tid + u * kJoinThreads) : make_ulonglong2(0, 0);
+        bool twice = false;
         for (uint32_t i0 = tid; i0 < nr; i0 += U * kJoinThreads) {
             tuple_v t[U];
             unsigned long long y[U];
@@ -1662,73 +1723,38 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_kernel(JoinArgs a0
                 rid[i] = y[u];
                 pos[i] = (uint32_t)t[u].y;
             }
-        }
-        __syncthreads();
-        bool twice = false;
-        for (uint32_t i = tid; i < nr; i += kJoinThreads) {
-            const unsigned long long k = kx[i];
-            if (skip0 && k == 0) continue;
-            const uint32_t h = head_of(k >> B, nb_log), shift = (h & 1) * 16;
-            uint32_t *word = head32 + (h >> 1);
-            uint32_t old = *reinterpret_cast<volatile uint32_t *>(word);
-            for (;;) {  // lock-free: a failed CAS means another thread's succeeded
-                const uint32_t e = (old >> shift) & 0xffffu;
-                if (e && kx[e - 1] == k) {
-                    atomicMin(&pos[e - 1], pos[i]);
-                    nxt[i] = (uint16_t)(kFirstMerged | e);
-                    twice = true;
-                    break;
+            __threadfence_block();  // before these become heads: a thread that loses a head reads its key
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const uint32_t i = i0 + u * kJoinThreads;
+                const unsigned long long k = t[u].x;
+                if (i >= nr || (skip0 && k == 0)) continue;
+                const uint32_t h = head_of(k, B, nb_log), shift = (h & 1) * 16;
+                uint32_t *word = head32 + (h >> 1);
+                uint32_t old = *reinterpret_cast<volatile uint32_t *>(word), e;
+                for (;;) {  // lock-free: a failed CAS means another thread's succeeded
+                    e = (old >> shift) & 0xffffu;
+                    const uint32_t seen = atomicCAS(word, old, (old & ~(0xffffu << shift)) | ((i + 1) << shift));
+                    if (seen == old) break;
+                    __threadfence_block();
+                    old = seen;
+                    e = (seen >> shift) & 0xffffu;
+                    if (e && *reinterpret_cast<volatile unsigned long long *>(&kx[e - 1]) == k) {
+                        atomicMin(&pos[e - 1], (uint32_t)t[u].y);
+                        e |= kFirstMerged;
+                        twice = true;
+                        break;
+                    }
                 }
                 nxt[i] = (uint16_t)e;
-                const uint32_t seen = atomicCAS(word, old, (old & ~(0xffffu << shift)) | ((i + 1) << shift));
-                if (seen == old) break;
-                old = seen;
             }
         }
         if (twice) s_dups = 1u;
         __syncthreads();
-        const bool dups = s_dups != 0;
-        if (dups) {
-            // Row ids of the tuples whose position won, and duplicate bits; then what is left of one key in a
-            // chain (nodes that were not next to each other).
-            for (uint32_t i = tid; i < nr; i += kJoinThreads) {
-                const uint32_t e = nxt[i];
-                if (!(e & kFirstMerged) || (skip0 && kx[i] == 0)) continue;
-                const uint32_t r = (e & (kFirstMerged - 1)) - 1;
-                if (pos[r] == pos[i]) rid[r] = rid[i];
-                atomicOr(&dup[r >> 5], 1u << (r & 31));
-            }
-            __syncthreads();
-            for (uint32_t q = tid; q < 1u << nb_log; q += kJoinThreads) {
-                for (uint32_t r = head[q]; r; r = nxt[r - 1]) {
-                    // Take the nodes behind r with its key out of the chain.
-                    const unsigned long long k = kx[r - 1];
-                    uint32_t prev = r, first = r, fp = pos[r - 1];
-                    bool gap = false, any = false;  // any: bits of the nodes taken out pass to r
-                    for (uint32_t e = nxt[r - 1], next; e; e = next) {
-                        const uint32_t p = pos[e - 1];
-                        next = nxt[e - 1];
-                        if (kx[e - 1] == k) {
-                            gap = any = true;
-                            if (p < fp) {
-                                fp = p;
-                                first = e;
-                            }
-                        } else {
-                            if (gap) nxt[prev - 1] = (uint16_t)e;
-                            gap = false;
-                            prev = e;
-                        }
-                    }
-                    if (gap) nxt[prev - 1] = 0;
-                    if (any) {
-                        pos[r - 1] = fp;
-                        rid[r - 1] = rid[first - 1];
-                        atomicOr(&dup[(r - 1) >> 5], 1u << ((r - 1) & 31));
-                    }
-                }
-            }
-            __syncthreads();
+        const bool merged = s_dups != 0;
+        if (merged) {
+            const FirstTable table = {kx, rid, pos, dup, head, nxt, nr, nb_log, skip0};
+            first_merge(table);
         }
         for (uint32_t base = 0; base < ns; base += UP * kJoinThreads) {
             tuple_v nx[UP];
@@ -1742,7 +1768,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_kernel(JoinArgs a0
             for (int u = 0; u < UP; u++) {
                 best[u] = 0;
                 if (base + u * kJoinThreads + tid >= ns) continue;
-                uint32_t e = head[head_of(sv[u].x >> B, nb_log)], steps = 0, nm = 0, bp = 0;
+                uint32_t e = head[head_of(sv[u].x, B, nb_log)], steps = 0, nm = 0, bp = 0;
                 while (e) {
                     if (kx[e - 1] == sv[u].x) {
                         const uint32_t p = pos[e - 1];
@@ -1760,7 +1786,8 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_first_kernel(JoinArgs a0
                 if (!best[u]) continue;
                 m++;
                 if (!MAT) sum += rid[best[u] - 1] + sv[u].y;
-                multi |= nm > 1 || (dups && (dup[(best[u] - 1) >> 5] >> ((best[u] - 1) & 31)) & 1u);
+                multi |= nm > 1;
+                if (merged) multi |= (dup[(best[u] - 1) >> 5] >> ((best[u] - 1) & 31)) & 1u;
             }
             cnt += m;
             if constexpr (MAT) {
@@ -1880,7 +1907,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_small_kernel(JoinArgs a0
         for (uint32_t i = tid; i < nr; i += kJoinThreads) {
             const uint64_t k = rt[i].x;
             if (skip0 && k == 0 && (!ci || item.part0)) continue;
-            const uint32_t h = head_of(k >> B, nb_log);
+            const uint32_t h = head_of(k, B, nb_log);
             nxt[i] = (uint16_t)atomic_exch_u16(&head[h], i + 1);
         }
         __syncthreads();
@@ -1899,7 +1926,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_small_kernel(JoinArgs a0
                     mm[u] = best[u] = 0;
                     if (base + u * kJoinThreads + tid >= ns) continue;
                     const uint64_t k = sv[u].x;
-                    uint32_t e = head[head_of(k >> B, nb_log)], steps = 0;
+                    uint32_t e = head[head_of(k, B, nb_log)], steps = 0;
                     while (e) {
                         if (rt[e - 1].x == k) {
                             if (!lp) mm[u]++;
@@ -1924,7 +1951,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_small_kernel(JoinArgs a0
                         continue;
                     }
                     const uint64_t k = sv[u].x;
-                    uint32_t e = head[head_of(k >> B, nb_log)], steps = 0;
+                    uint32_t e = head[head_of(k, B, nb_log)], steps = 0;
                     while (e && steps++ <= nr) {
                         if (rt[e - 1].x == k) mat_put(a.mat, o++, rt[e - 1].y, sv[u].y, err);
                         e = nxt[e - 1];
@@ -1944,7 +1971,7 @@ __global__ void __launch_bounds__(kJoinThreads, 1) join_small_kernel(JoinArgs a0
                 const uint32_t j = j0 + u * kJoinThreads;
                 if (j >= ns) continue;
                 const uint64_t k = s[u].x;
-                uint32_t e = head[head_of(k >> B, nb_log)];
+                uint32_t e = head[head_of(k, B, nb_log)];
                 uint32_t best = 0, nm = 0;
                 uint32_t steps = 0;
                 while (e) {
